@@ -36,7 +36,7 @@ UNITS = [
     ("ensc_batch.cu", []),
     ("ensc_capi.cu", []),
 ]
-HEADERS = ["ensc_device.cuh", "ensc_kernels.h", "ensc_instance.h"]
+HEADERS = ["ensc_cycle.cuh", "ensc_device.cuh", "ensc_kernels.h", "ensc_instance.h", "ensc_run.cuh", "ensc_stage.cuh"]
 
 
 def nvcc() -> str:

@@ -48,7 +48,9 @@ struct ensc_handle {
     Ctl* ctl_host = nullptr;       // pinned mirror
     int grid_e = 1, grid_n = 1;
     int chunk = 32;
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graph = nullptr;   // cycles of the per-phase kernels
+    ensc::RunPlan run{};               // resident runs (grid 0: the graph)
+    ensc::RunSync* sync = nullptr;
     bool kinetic0_done = false;
     double* amp = nullptr;         // device gravity amplitude table
     // output snapshots (ensc_snapshot_begin / ensc_snapshot_wait): a device
@@ -144,6 +146,51 @@ int build_graph(ensc_handle* h) {
     return ENSC_OK;
 }
 
+// Most cycles of one resident-run launch (tens of ms on the meshes that run
+// resident): the host looks at the control block between launches.
+constexpr int64_t kRunCycles = 4096;
+
+// The launches that rebuild what a handle steps with after its material or
+// loads changed: the graph carries them by value, a resident run takes them
+// with every launch.
+int loads_changed(ensc_handle* h) { return h->graph ? build_graph(h) : ENSC_OK; }
+
+// Enqueues up to `cycles` cycles of a step call: its first (arm, which sets
+// the call's limits: max_cycles in all) or a later part.
+int enqueue_cycles(ensc_handle* h, int64_t cycles, bool arm, int64_t max_cycles, double step_end, double pause) {
+    if (h->run.grid) {
+        int64_t left = cycles;
+        while (left > 0) {
+            const int64_t n = std::min(left, kRunCycles);
+            ensc::RunArgs a{step_end, pause, max_cycles, arm ? 1 : 0, static_cast<int32_t>(n), h->run.tiles_per_warp};
+            const cudaError_t e =
+                mixed(h) ? ensc::launch_run_mixed(h->run, h->E, h->N, h->M, h->ctl, h->P, h->sync, a, h->stream)
+                         : ensc::launch_run_fp64(h->run, h->E, h->N, h->M, h->ctl, h->P, h->sync, a, h->stream);
+            if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources) {
+                // fewer SMs are open to this process than the device has:
+                // the per-phase kernels need no resident grid
+                cudaGetLastError();
+                h->run = ensc::RunPlan{};
+                break;
+            }
+            if (e != cudaSuccess) return cuda_err(h, "resident run", e);
+            arm = false;
+            left -= n;
+        }
+        h->fe_valid = true;
+        if (left == 0) return ENSC_OK;
+        cycles = left;
+    }
+    if (!h->graph)
+        if (int rc = build_graph(h)) return rc;
+    if (arm) ensc::launch_arm(h->ctl, step_end, max_cycles, h->stream, pause);
+    const int64_t launches = (cycles + h->chunk - 1) / h->chunk;
+    for (int64_t i = 0; i < launches; ++i) CK(h, cudaGraphLaunch(h->graph, h->stream));
+    CK(h, cudaGetLastError());
+    h->fe_valid = true;
+    return ENSC_OK;
+}
+
 int read_ctl(ensc_handle* h) {
     CK(h, cudaMemcpyAsync(h->ctl_host, h->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -232,9 +279,17 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
     h->grid_e = static_cast<int>(std::min<int64_t>(ge, static_cast<int64_t>(occ_e) * prop.multiProcessorCount));
     h->grid_n = static_cast<int>(std::min<int64_t>(gn, static_cast<int64_t>(occ_n) * prop.multiProcessorCount));
 
+    // resident runs where the mesh fits on chip (slot assembly)
+    if (!ih.patch && prop.cooperativeLaunch)
+        h->run = mx ? ensc::plan_run_mixed(h->ne, h->plastic, prop.multiProcessorCount)
+                    : ensc::plan_run_fp64(h->ne, h->plastic, prop.multiProcessorCount);
+
     // ---- device memory: the instance block plus partial sums and control ----
-    const size_t pbytes = (3 * static_cast<size_t>(h->grid_e) + 2 * static_cast<size_t>(h->grid_n)) * sizeof(double);
-    const size_t small = (pbytes + 255) / 256 * 256 + (sizeof(Ctl) + 255) / 256 * 256;
+    // (one partial slot per block of the larger of the two launch forms)
+    const int pe = std::max(h->grid_e, h->run.grid), pn = std::max(h->grid_n, h->run.grid);
+    const size_t pbytes = (3 * static_cast<size_t>(pe) + 2 * static_cast<size_t>(pn)) * sizeof(double);
+    const size_t poff = (pbytes + 255) / 256 * 256, coff = (sizeof(Ctl) + 255) / 256 * 256;
+    const size_t small = poff + coff + (sizeof(ensc::RunSync) + 255) / 256 * 256;
     cudaError_t ce = cudaMalloc(&h->arena, ih.bytes + small);
     if (ce != cudaSuccess) {
         cuda_err(h, "cudaMalloc(instance)", ce);
@@ -269,11 +324,16 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
     h->n_partials = ih.n_pnodes;
     char* tail = static_cast<char*>(h->arena) + ih.bytes;
     h->P.elem = reinterpret_cast<double*>(tail);
-    h->P.node = h->P.elem + 3 * h->grid_e;
-    h->P.n_elem_blocks = h->grid_e;
-    h->P.n_node_blocks = h->grid_n;
-    h->ctl = reinterpret_cast<Ctl*>(tail + (pbytes + 255) / 256 * 256);
+    h->P.node = h->P.elem + 3 * pe;
+    h->P.n_elem_blocks = pe;
+    h->P.n_node_blocks = pn;
+    h->ctl = reinterpret_cast<Ctl*>(tail + poff);
+    h->sync = reinterpret_cast<ensc::RunSync*>(tail + poff + coff);
     ce = cudaMemsetAsync(tail, 0, small, h->stream);
+    ensc::RunSync sync0{};
+    sync0.pre_len = ensc::kInfBits;
+    for (ensc::RunMins& m : sync0.mins) m = ensc::RunMins{ensc::kInfBits, ensc::kInfBits};
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(h->sync, &sync0, sizeof(sync0), cudaMemcpyHostToDevice, h->stream);
     if (ce != cudaSuccess) {
         cuda_err(h, "cudaMemset(partials)", ce);
         return fail(ENSC_ERR_CUDA);
@@ -308,8 +368,10 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
         cuda_err(h, "init pass", ce);
         return fail(ENSC_ERR_CUDA);
     }
-    rc = build_graph(h);
-    if (rc) return fail(rc);
+    if (!h->run.grid) {
+        rc = build_graph(h);
+        if (rc) return fail(rc);
+    }
     *out = h;
     return ENSC_OK;
 }
@@ -349,7 +411,7 @@ int ensc_set_gravity(ensc_handle* h, int32_t on, double value, const double dir[
     h->M.gravity_on = on;
     h->M.gravity_value = value;
     for (int i = 0; i < 3; ++i) h->M.gravity_dir[i] = dir ? dir[i] : 0.0;
-    return build_graph(h);
+    return loads_changed(h);
 }
 
 int ensc_set_gravity_amplitude(ensc_handle* h, int32_t n_points, const double* time_value) {
@@ -360,7 +422,7 @@ int ensc_set_gravity_amplitude(ensc_handle* h, int32_t n_points, const double* t
     if (n_points == 0) {
         h->M.amp = nullptr;
         h->M.amp_n = 0;
-        return build_graph(h);
+        return loads_changed(h);
     }
     if (!h->amp) {
         cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&h->amp), 2 * sizeof(double) * ENSC_MAX_AMPLITUDE_POINTS);
@@ -374,19 +436,14 @@ int ensc_set_gravity_amplitude(ensc_handle* h, int32_t n_points, const double* t
     CK(h, cudaStreamSynchronize(h->stream));
     h->M.amp = h->amp;
     h->M.amp_n = n_points;
-    return build_graph(h);
+    return loads_changed(h);
 }
 
 int ensc_step_async(ensc_handle* h, int64_t max_cycles, double step_end_time) {
     if (!h || max_cycles < 0) return ENSC_ERR_ARG;
     if (max_cycles == 0) return ENSC_OK;
     DevGuard dg(h->device);
-    ensc::launch_arm(h->ctl, step_end_time, max_cycles, h->stream);
-    const int64_t launches = (max_cycles + h->chunk - 1) / h->chunk;
-    for (int64_t i = 0; i < launches; ++i) CK(h, cudaGraphLaunch(h->graph, h->stream));
-    CK(h, cudaGetLastError());
-    h->fe_valid = true;
-    return ENSC_OK;
+    return enqueue_cycles(h, max_cycles, true, max_cycles, step_end_time, HUGE_VAL);
 }
 
 int ensc_step_until_async(ensc_handle* h, int64_t max_cycles, double step_end_time, double pause_time) {
@@ -395,20 +452,13 @@ int ensc_step_until_async(ensc_handle* h, int64_t max_cycles, double step_end_ti
         return set_err(h, ENSC_ERR_ARG, "ensc_step_until_async: at most 2^24 cycles per call");
     if (max_cycles == 0) return ENSC_OK;
     DevGuard dg(h->device);
-    ensc::launch_arm(h->ctl, step_end_time, max_cycles, h->stream, pause_time);
-    const int64_t launches = (max_cycles + h->chunk - 1) / h->chunk;
-    for (int64_t i = 0; i < launches; ++i) CK(h, cudaGraphLaunch(h->graph, h->stream));
-    CK(h, cudaGetLastError());
-    h->fe_valid = true;
-    return ENSC_OK;
+    return enqueue_cycles(h, max_cycles, true, max_cycles, step_end_time, pause_time);
 }
 
 int ensc_sync(ensc_handle* h, ensc_step_report* report) {
     if (!h) return ENSC_ERR_ARG;
     DevGuard dg(h->device);
     const int64_t before = h->ctl_host->cycles_done;
-    ensc::launch_between(h->ctl, h->P, 1, h->stream);
-    CK(h, cudaGetLastError());
     int rc = read_ctl(h);
     if (rc) return rc;
     fill_report(h, before, report);
@@ -424,27 +474,21 @@ int ensc_step_until(ensc_handle* h, int64_t max_cycles, double step_end_time, do
     if (!h || max_cycles < 0) return ENSC_ERR_ARG;
     DevGuard dg(h->device);
     const int64_t before = h->ctl_host->cycles_done;
-    if (max_cycles > 0) {
-        ensc::launch_arm(h->ctl, step_end_time, max_cycles, h->stream, pause_time);
-        // launch graphs in batches; between batches read the control block
-        // to stop once time reached step_end
-        const int64_t batch = std::max<int64_t>(1, 4096 / h->chunk);
-        int64_t launched = 0;
-        const int64_t needed = (max_cycles + h->chunk - 1) / h->chunk;
-        while (launched < needed) {
-            const int64_t n = std::min(batch, needed - launched);
-            for (int64_t i = 0; i < n; ++i) CK(h, cudaGraphLaunch(h->graph, h->stream));
-            launched += n;
-            h->fe_valid = true;
-            int rc = read_ctl(h);
-            if (rc) return rc;
-            if (h->ctl_host->done || h->ctl_host->status) break;
-        }
+    if (max_cycles == 0) {
+        int rc = read_ctl(h);
+        if (rc) return rc;
     }
-    ensc::launch_between(h->ctl, h->P, 1, h->stream);
-    CK(h, cudaGetLastError());
-    int rc = read_ctl(h);
-    if (rc) return rc;
+    // launch in batches; after each, the control block tells whether the call
+    // is over (step end or pause reached, cycles spent, or a status)
+    const int64_t batch = (kRunCycles + h->chunk - 1) / h->chunk * h->chunk;
+    for (int64_t launched = 0; launched < max_cycles;) {
+        const int64_t n = std::min(batch, max_cycles - launched);
+        int rc = enqueue_cycles(h, n, launched == 0, max_cycles, step_end_time, pause_time);
+        if (!rc) rc = read_ctl(h);
+        if (rc) return rc;
+        launched += n;
+        if (h->ctl_host->done || h->ctl_host->status) break;
+    }
     fill_report(h, before, report);
     return status_code(h, h->ctl_host->status);
 }
@@ -671,6 +715,12 @@ int ensc_profile(ensc_handle* h, int64_t max_cycles, double step_end_time, doubl
     }
     cudaEvent_t ev[6];
     for (int i = 0; i < 6; ++i) CK(h, cudaEventCreate(&ev[i]));
+    if (h->run.grid) {
+        // the node pass fills fewer partial slots than a resident run: what
+        // the runs left is folded, and no kinetic energy stays in the others
+        ensc::launch_between(h->ctl, h->P, 1, h->stream);
+        CK(h, cudaMemsetAsync(h->P.node, 0, h->P.n_node_blocks * sizeof(double), h->stream));
+    }
     ensc::launch_arm(h->ctl, step_end_time, max_cycles, h->stream);
     int rc = ENSC_OK;
     for (int64_t c = 0; c < max_cycles && rc == ENSC_OK; ++c) {
@@ -707,7 +757,7 @@ int64_t ensc_device_bytes(const ensc_handle* h) {
     return static_cast<int64_t>(h->arena_bytes + (h->staging_owned ? h->staging_bytes : 0));
 }
 
-int32_t ensc_kernels_per_cycle(const ensc_handle* h) { return h ? 4 : 0; }
+int32_t ensc_kernels_per_cycle(const ensc_handle* h) { return h && !h->run.grid ? 4 : 0; }
 
 int ensc_assembly(const ensc_handle* h, int32_t* assembly, int64_t* patches, int64_t* partials) {
     if (!h) return ENSC_ERR_ARG;

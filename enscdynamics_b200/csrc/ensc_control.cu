@@ -2,6 +2,7 @@
 // stable-time-step arithmetic reproduces the reference's
 // update_minVertex_perMaterial_and_dt (Explicit3D/source/exDyna3D.cpp:663-686)
 // and run()'s last-step clamp (:90-97) operation by operation.
+#include "ensc_cycle.cuh"
 #include "ensc_device.cuh"
 #include "ensc_kernels.h"
 
@@ -44,40 +45,6 @@ __device__ double fixed_sum_strided(const double* a, int n, int stride) {
     return r;
 }
 
-// First half of update_minVertex_perMaterial_and_dt for the next cycle
-// (exDyna3D.cpp:663-686) and computeSate's clock advance (:775-780): rotate
-// dt_i_1 <- dt_i and advance time, unless the total-time clamp (:682-685)
-// could fire, which needs the cycle's minimum element edge first
-// (edge_prepass + begin_exact).  Caller has checked done / step end.
-__device__ __forceinline__ void cycle_begin(Ctl* ctl) {
-    ctl->dts_cur = bits_ord(ctl->dts_next);
-    ctl->dts_next = kInfBits;
-    ctl->len_min = kInfBits;
-    const double dt_prev = ctl->dt_i;
-    ctl->dt_prev = dt_prev;
-    const double time = ctl->time;
-    const double time_prev = time + dt_prev;
-    // the new dt is factor * min(edge / c, dts_cur) <= factor * dts_cur
-    const double bound = ctl->dts_cur * ctl->factor;
-    const double rem = ctl->total_time - time_prev;
-    const int exact = (rem > 0.0 && rem < bound) ? 1 : 0;
-    ctl->need_exact = exact;
-    ctl->dt_final = 0;
-    if (!exact) {
-        double dt_i_1 = dt_prev;
-        if (time + dt_i_1 > ctl->step_end) {
-            const double r = ctl->step_end - time;
-            dt_i_1 = r;
-            ctl->dt_i = r;
-            ctl->dt_final = 1;
-        }
-        ctl->dt_i_1 = dt_i_1;
-        double t = time + dt_i_1;
-        if (t > ctl->total_time) t = ctl->total_time;
-        ctl->time = t;
-    }
-}
-
 // mode 0: the first half of update_minVertex_perMaterial_and_dt for the
 // next cycle: rotate dt_i_1 <- dt_i, advance time (computeSate :775-780) and
 // fix dt_i_1 unless the total-time clamp (:682-685) could fire, which needs
@@ -115,33 +82,6 @@ __global__ void __launch_bounds__(kCtlThreads) k_between(Ctl* ctl, Partials P, i
         return;
     }
     cycle_begin(ctl);
-}
-
-// Rest of update_minVertex_perMaterial_and_dt and run()'s clamp for a cycle
-// that needed the exact edge minimum (len_min_bits: that minimum, as
-// ordered bits).
-__device__ __forceinline__ void begin_exact(Ctl* ctl, unsigned long long len_min_bits) {
-    const double time = ctl->time;
-    double dt_i_1 = ctl->dt_prev;
-    const double time_prev = time + dt_i_1;
-    double d = bits_ord(len_min_bits) / ctl->wos;
-    d = d < ctl->dts_cur ? d : ctl->dts_cur;
-    double dt_i = d * ctl->factor;
-    if ((ctl->total_time - time_prev) < dt_i && (ctl->total_time - time_prev) > 0.0) {
-        dt_i = ctl->total_time - time_prev;
-        dt_i_1 = dt_i;
-    }
-    if (time + dt_i_1 > ctl->step_end) {
-        const double r = ctl->step_end - time;
-        dt_i = r;
-        dt_i_1 = r;
-    }
-    ctl->dt_i = dt_i;
-    ctl->dt_i_1 = dt_i_1;
-    ctl->dt_final = 1;
-    double t = time + dt_i_1;
-    if (t > ctl->total_time) t = ctl->total_time;
-    ctl->time = t;
 }
 
 // Minimum element edge over the current coordinates (min_ele_edge,

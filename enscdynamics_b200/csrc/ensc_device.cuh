@@ -428,8 +428,10 @@ __host__ __device__ inline int16_t* v_lo_rows(void* v, int64_t nn_pad) {
 template <int W, typename T>
 __device__ __forceinline__ void ld_row(const T* p, T (&o)[W]) {
     constexpr int kBytes = W * static_cast<int>(sizeof(T));
-    static_assert(kBytes % 16 == 0 || kBytes == 8 || kBytes == 4, "16-byte chunks or one 8- or 4-byte chunk");
-    if constexpr (kBytes == 4) {
+    static_assert(kBytes % 16 == 0 || kBytes == 8 || kBytes == 4 || W == 1, "16-byte chunks or one smaller chunk");
+    if constexpr (W == 1) {
+        o[0] = *p;
+    } else if constexpr (kBytes == 4) {
         const uint32_t q = *reinterpret_cast<const uint32_t*>(p);
         memcpy(o, &q, 4);
     } else if constexpr (kBytes == 8) {
@@ -446,8 +448,10 @@ __device__ __forceinline__ void ld_row(const T* p, T (&o)[W]) {
 template <int W, typename T>
 __device__ __forceinline__ void st_row(T* p, const T (&v)[W]) {
     constexpr int kBytes = W * static_cast<int>(sizeof(T));
-    static_assert(kBytes % 16 == 0 || kBytes == 8 || kBytes == 4, "16-byte chunks or one 8- or 4-byte chunk");
-    if constexpr (kBytes == 4) {
+    static_assert(kBytes % 16 == 0 || kBytes == 8 || kBytes == 4 || W == 1, "16-byte chunks or one smaller chunk");
+    if constexpr (W == 1) {
+        *p = v[0];
+    } else if constexpr (kBytes == 4) {
         uint32_t q;
         memcpy(&q, v, 4);
         *reinterpret_cast<uint32_t*>(p) = q;
@@ -464,10 +468,11 @@ __device__ __forceinline__ void st_row(T* p, const T (&v)[W]) {
         }
     }
 }
-// W (2 or 4) consecutive bytes as one word, byte j of node j in bits 8j..8j+7.
+// W (1, 2 or 4) consecutive bytes as one word, byte j of node j in bits 8j..8j+7.
 template <int W>
 __device__ __forceinline__ uint32_t ld_bytes(const uint8_t* p) {
-    static_assert(W == 2 || W == 4, "2 or 4 bytes");
+    static_assert(W == 1 || W == 2 || W == 4, "1, 2 or 4 bytes");
+    if (W == 1) return *p;
     if (W == 4) return *reinterpret_cast<const uint32_t*>(p);
     return *reinterpret_cast<const uint16_t*>(p);
 }

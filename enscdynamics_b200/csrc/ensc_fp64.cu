@@ -9,6 +9,7 @@
 // launched inside a CUDA graph; see ensc_capi.cu for the orchestration.
 #include "ensc_device.cuh"
 #include "ensc_kernels.h"
+#include "ensc_run.cuh"
 #include "ensc_stage.cuh"
 
 #include <algorithm>
@@ -150,27 +151,40 @@ __device__ __forceinline__ Fp64Src fp64_src_global(const ElemArrays& E, int64_t 
                    static_cast<const double*>(E.bt), E.ne_pad, e};
 }
 
+// Where one element's evolving rows are written: rows of `stride` entries
+// with the element at `i` (the instance's global arrays, or the shared-memory
+// tile that a resident run keeps them in).
+struct Fp64Out {
+    double* sig;            // [6] rows
+    double* qia;            // [12] rows
+    double* eps;
+    int64_t stride, i;
+};
+
+__device__ __forceinline__ Fp64Out fp64_out_global(const ElemArrays& E, int64_t e) {
+    return Fp64Out{static_cast<double*>(E.sigma), static_cast<double*>(E.qia), static_cast<double*>(E.eps_p), E.ne_pad,
+                   e};
+}
+
 // One element of the FP64 element pass (the kernel comment below has the
-// reference mapping), shared by the single-instance, staged and batched
-// kernels; inputs come from S, outputs go to the instance's arrays at
-// element e.  SMEM / BT_SMEM: S's rows / B0^T rows
+// reference mapping), shared by the single-instance, staged, batched and
+// resident-run kernels; inputs come from S, the evolving rows go to O and the
+// forces to the instance's force array at element e.  Node rows are read with
+// plain loads: a resident run rewrites them between its cycles.  SMEM / BT_SMEM: S's rows / B0^T rows
 // are in shared memory.  PF: node rows the body reads later are prefetched
 // into L1 once the connectivity is known (bit 0 the velocities, bit 1 the
 // displacements).
 template <bool PLASTIC, bool INIT, bool SMEM = false, bool BT_SMEM = false, int PF = 0>
 __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArrays& N, const Material& M,
-                                             const Fp64Src& S, const double dt1, const int64_t e, double& dts,
-                                             double& len, double& e_int, double& e_hg, double& e_vis,
+                                             const Fp64Src& S, const Fp64Out& O, const double dt1, const int64_t e,
+                                             double& dts, double& len, double& e_int, double& e_hg, double& e_vis,
                                              int32_t& bad) {
-    const int64_t ss = S.stride, si = S.i, bs = S.bt_stride;
+    const int64_t ss = S.stride, si = S.i, bs = S.bt_stride, os = O.stride, oi = O.i;
     const int64_t ep = E.ne_pad, np = N.nn_pad;
-    double* sig = static_cast<double*>(E.sigma);
-    double* qia = static_cast<double*>(E.qia);
-    double* epsp = static_cast<double*>(E.eps_p);
-    double* __restrict__ fe = static_cast<double*>(E.fe);
-    const double* __restrict__ X = N.x;
-    const double* __restrict__ U = N.u;
-    const double* __restrict__ V = static_cast<const double*>(N.v);
+    double* fe = static_cast<double*>(E.fe);
+    const double* X = N.x;
+    const double* U = N.u;
+    const double* V = static_cast<const double*>(N.v);
     const double G = M.G, lam = M.lambda;
 
     const double* bte = S.bt + S.bt_i;
@@ -315,12 +329,12 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
             s[3] = s[3] * r;
             s[4] = s[4] * r;
             s[5] = s[5] * r;
-            if (!INIT) epsp[e] = ep_old + dl;
+            if (!INIT) O.eps[oi] = ep_old + dl;
         }
     }
     if (!INIT) {
 #pragma unroll
-        for (int i = 0; i < 6; ++i) sig[i * ep + e] = s[i];
+        for (int i = 0; i < 6; ++i) O.sig[i * os + oi] = s[i];
     }
     const double V0 = S.vol0[si];
     const double Vc = J * V0;
@@ -344,7 +358,7 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             const double q = __fma_rn(DR, HIA[i][kk], S.qia[(4 * i + kk) * ss + si]);
-            if (!INIT) qia[(4 * i + kk) * ep + e] = q;
+            if (!INIT) O.qia[(4 * i + kk) * os + oi] = q;
             Gq[i][kk] = __fma_rn(CR, HIA[i][kk], q);
         }
     // bulk viscosity pressure (:1073-1109)
@@ -439,7 +453,7 @@ __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_FP64) k_element(E
         const bool live = e0 < ne;
         const int64_t e = live ? e0 : 0;
         double dts = DBL_MAX, len = DBL_MAX;
-        if (live) element_body<PLASTIC, INIT>(E, N, M, fp64_src_global(E, e), dt1, e, dts, len, e_int, e_hg, e_vis, bad);
+        if (live) element_body<PLASTIC, INIT>(E, N, M, fp64_src_global(E, e), fp64_out_global(E, e), dt1, e, dts, len, e_int, e_hg, e_vis, bad);
         dts_min = dts < dts_min ? dts : dts_min;
         len_min = len < len_min ? len : len_min;
     }
@@ -457,8 +471,8 @@ __device__ __forceinline__ void node_body(const ElemArrays& E, const NodeArrays&
                                           const double dt_i, const double dt_i_1, const double amp, const int64_t n, double& kin,
                                           double& wext, int32_t& bad) {
     const int64_t np = N.nn_pad, ep = E.ne_pad;
-    const double* __restrict__ fe = static_cast<const double*>(E.fe);
-    double* __restrict__ V = static_cast<double*>(N.v);
+    const double* fe = static_cast<const double*>(E.fe);
+    double* V = static_cast<double*>(N.v);
     const double half = (dt_i + dt_i_1);
     const double dt_avg = (dt_i + dt_i_1) / 2.0;
 
@@ -663,7 +677,7 @@ __global__ void __launch_bounds__(kStageTileF64, BT ? kStageMinbF64 : kStageMinb
                             BT ? d + kF64StageRows * T : static_cast<const double*>(E.bt),
                             BT ? static_cast<int64_t>(T) : E.ne_pad, BT ? static_cast<int64_t>(tid) : e};
             double dts, len;
-            element_body<PLASTIC, false, true, BT>(E, N, M, S, dt1, e, dts, len, e_int, e_hg, e_vis, bad);
+            element_body<PLASTIC, false, true, BT>(E, N, M, S, fp64_out_global(E, e), dt1, e, dts, len, e_int, e_hg, e_vis, bad);
             dts_min = dts < dts_min ? dts : dts_min;
             len_min = len < len_min ? len : len_min;
         }
@@ -845,8 +859,8 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
                             kF64WarpBt ? static_cast<int64_t>(T) : E.ne_pad,
                             kF64WarpBt ? static_cast<int64_t>(lane) : e};
             double dts, len;
-            element_body<PLASTIC, false, true, kF64WarpBt, ENSC_F64_PREFETCH>(E, N, M, S, dt1, e, dts, len, e_int,
-                                                                              e_hg, e_vis, bad);
+            element_body<PLASTIC, false, true, kF64WarpBt, ENSC_F64_PREFETCH>(E, N, M, S, fp64_out_global(E, e), dt1, e,
+                                                                              dts, len, e_int, e_hg, e_vis, bad);
             dts_min = dts < dts_min ? dts : dts_min;
             len_min = len < len_min ? len : len_min;
         }
@@ -881,8 +895,8 @@ template <int W>
 __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i, const double dt_i_1, const double amp,
                                            const int64_t n0, double& kin, double& wext, int32_t& bad) {
     const int64_t np = N.np, nn = N.nn;
-    const double* __restrict__ fe = static_cast<const double*>(N.fe);
-    double* __restrict__ V = static_cast<double*>(N.v);
+    const double* fe = static_cast<const double*>(N.fe);
+    double* V = static_cast<double*>(N.v);
     const double half = (dt_i + dt_i_1);
     const double dt_avg = (dt_i + dt_i_1) / 2.0;
     double f[3][W];
@@ -997,6 +1011,61 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_FP64) k_node(Elem
     block_sum<kNodeThreads, 2, 2u>(v2, P.node, P.n_node_blocks, blockIdx.x);
 }
 
+// ---- resident runs (ensc_run.cuh) -----------------------------------------
+// 8 warps per SM as in the warp-pipelined pass; a tile of 32 elements takes
+// 12.8 KB, so that 17 tiles fit an SM and 148 SMs hold 75,776 elements at two
+// tiles per warp.
+constexpr int kRunWarpsF64 = 8;
+template <bool PLASTIC>
+struct RunFp64 {
+    static constexpr uint32_t kTileBytes = 8u * 32u * 4u + (kF64StageRows + 24) * 32u * 8u;
+    __device__ static const uint32_t* conn(const unsigned char* tile) {
+        return reinterpret_cast<const uint32_t*>(tile);
+    }
+    __device__ static void load_tile(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t base, int lane) {
+        static_assert(kF64WarpBt && kF64WarpStageBytes == kTileBytes, "the warp-pipelined pass's stage");
+        f64_warp_stage_issue<PLASTIC>(E, dst, bar, base, lane);
+    }
+    __device__ static void store_tile(const ElemArrays& E, const unsigned char* tile, int64_t base, int lane) {
+        const double* d = reinterpret_cast<const double*>(tile + 8 * 32 * 4);
+        const int64_t e = base + lane;
+        if (e >= E.ne) return;
+        for (int r = 0; r < 18; ++r) const_cast<double*>(f64_stage_row(E, r))[e] = d[r * 32 + lane];
+        if (PLASTIC) const_cast<double*>(f64_stage_row(E, 21))[e] = d[21 * 32 + lane];
+    }
+    __device__ static void element(const ElemArrays& E, const NodeArrays& N, const Material& M, unsigned char* tile,
+                                   double dt1, int64_t e, int lane, double& dts, double& len, double& e_int,
+                                   double& e_hg, double& e_vis, int32_t& bad) {
+        double* d = reinterpret_cast<double*>(tile + 8 * 32 * 4);
+        const Fp64Src S{conn(tile), d, d + 6 * 32, d + 18 * 32, d + 19 * 32, d + 20 * 32, d + 21 * 32, 32, lane,
+                        d + kF64StageRows * 32, 32, lane};
+        const Fp64Out O{d, d + 6 * 32, d + 21 * 32, 32, lane};
+        element_body<PLASTIC, false, true, true, ENSC_F64_PREFETCH>(E, N, M, S, O, dt1, e, dts, len, e_int, e_hg,
+                                                                     e_vis, bad);
+    }
+    // one node per thread while the grid has a thread for every node
+    __device__ static void nodes(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i,
+                                 double dt_i_1, double amp, int64_t t0, int64_t stride, double& kin, double& wext,
+                                 int32_t& bad) {
+        if (E.slot_major) {
+            const NodeView nv = node_view(E, N, M, nullptr);
+            if (N.nn <= stride) {
+                if (t0 < N.nn) node_group<1>(nv, dt_i, dt_i_1, amp, t0, kin, wext, bad);
+            } else {
+                for (int64_t g = t0; g * 2 < N.nn; g += stride)
+                    node_group<2>(nv, dt_i, dt_i_1, amp, g * 2, kin, wext, bad);
+            }
+        } else {
+            for (int64_t n = t0; n < N.nn; n += stride) node_body(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
+        }
+    }
+};
+
+template <bool PLASTIC, bool CLUSTER>
+__global__ void __launch_bounds__(32 * kRunWarpsF64, 1)
+    k_run_fp64(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P, RunSync* sync, RunArgs a) {
+    run_cycles<RunFp64<PLASTIC>, CLUSTER>(E, N, M, ctl, P, sync, a);
+}
 
 // ---- batched instances --------------------------------------------------------
 // Element tiles of kStageTileF64 elements and node tiles of
@@ -1173,7 +1242,8 @@ __global__ void __launch_bounds__(kF64BatchTile, 256 / kF64BatchTile) k_element_
             const Fp64Src S{reinterpret_cast<const uint32_t*>(st), dr, dr + 6 * TT, dr + 18 * TT, dr + 19 * TT,
                             dr + 20 * TT, dr + 21 * TT, TT, tid, dr + kF64StageRows * TT, TT, tid};
             double d1, l1;
-            element_body<true, false, true, true, ENSC_F64_PREFETCH>(E, N, d.M, S, dt1, e, d1, l1, ei, eh, ev, bad);
+            element_body<true, false, true, true, ENSC_F64_PREFETCH>(E, N, d.M, S, fp64_out_global(E, e), dt1, e, d1, l1,
+                                                                     ei, eh, ev, bad);
             dts = d1 < dts ? d1 : dts;
             len = l1 < len ? l1 : len;
         }
@@ -1349,6 +1419,21 @@ int occupancy_element_batch_fp64() {
                          static_cast<int>(kF64BatchStageSmem));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_batch_fp64, kF64BatchTile, kF64BatchStageSmem);
     return nb;
+}
+
+RunPlan plan_run_fp64(int64_t ne, bool plastic, int sms) {
+    return plastic ? plan_run(k_run_fp64<true, true>, k_run_fp64<true, false>, ne, sms, kRunWarpsF64,
+                              RunFp64<true>::kTileBytes)
+                   : plan_run(k_run_fp64<false, true>, k_run_fp64<false, false>, ne, sms, kRunWarpsF64,
+                              RunFp64<false>::kTileBytes);
+}
+cudaError_t launch_run_fp64(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
+                            const Partials& P, RunSync* sync, const RunArgs& a, cudaStream_t st) {
+    if (M.plastic)
+        return p.cluster ? launch_run(k_run_fp64<true, true>, p, st, E, N, M, ctl, P, sync, a)
+                         : launch_run(k_run_fp64<true, false>, p, st, E, N, M, ctl, P, sync, a);
+    return p.cluster ? launch_run(k_run_fp64<false, true>, p, st, E, N, M, ctl, P, sync, a)
+                     : launch_run(k_run_fp64<false, false>, p, st, E, N, M, ctl, P, sync, a);
 }
 
 int batch_element_tile_fp64() { return kF64BatchTile; }

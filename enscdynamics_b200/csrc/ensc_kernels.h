@@ -130,6 +130,41 @@ constexpr int kNodeUnrollMixed = ENSC_NODE_UNROLL_MIXED;
 constexpr int kNodeThreads = 256;
 constexpr int kCtlThreads = 256;
 
+// ---- resident runs (ensc_run.cuh) ----
+// Minima of one cycle's element phase, as ordered bits.
+struct RunMins {
+    unsigned long long dts, len;
+};
+// Grid-wide state of a resident run, zero and +inf between launches: the
+// arrival counter (low half; upper half: blocks that saw an error, 16 bits per
+// phase), the raised status bits, the blocks that have left.
+struct alignas(128) RunSync {
+    unsigned long long arrive;
+    int32_t status, left;
+    unsigned long long pre_len;
+    unsigned long long pad;
+    RunMins mins[3];
+};
+struct RunArgs {
+    double step_end, pause;
+    long long max_cycles;      // with arm: the limits of the step call (k_arm)
+    int32_t arm;
+    int32_t launch_cycles;     // most cycles of this launch
+    int32_t tiles_per_warp;
+};
+// Launch geometry of an instance's resident runs; grid 0: the mesh does not
+// fit, use the per-phase kernels.
+struct RunPlan {
+    int grid = 0, threads = 0, cluster = 0, tiles_per_warp = 0;
+    size_t smem = 0;
+};
+RunPlan plan_run_fp64(int64_t ne, bool plastic, int sms);
+RunPlan plan_run_mixed(int64_t ne, bool plastic, int sms);
+cudaError_t launch_run_fp64(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
+                            const Partials& P, RunSync* sync, const RunArgs& a, cudaStream_t st);
+cudaError_t launch_run_mixed(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
+                             const Partials& P, RunSync* sync, const RunArgs& a, cudaStream_t st);
+
 // FP64 (ensc_fp64.cu, built with -fmad=false)
 void launch_element_fp64(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl, const Partials& P,
                          int grid, bool init, cudaStream_t st);

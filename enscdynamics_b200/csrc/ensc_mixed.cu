@@ -16,6 +16,7 @@
 // (double, ENSC_MIXED_UREF); v float with 16-bit residual rows.
 #include "ensc_device.cuh"
 #include "ensc_kernels.h"
+#include "ensc_run.cuh"
 #include "ensc_stage.cuh"
 
 #include <cfloat>
@@ -174,26 +175,38 @@ __device__ __forceinline__ void corner_values(T (&c)[8], T (&a)[8]) {
     for (int j = 0; j < 8; ++j) a[j] = c[kBits[j]];
 }
 
+// Where one element's evolving rows are written: the instance's own arrays,
+// or the shared-memory tile that a resident run keeps them in.
+struct MixedOut {
+    float* sig;             // [6] rows
+    float* qia;             // [12] rows
+    float* eps;
+    int64_t stride, i;
+};
+
+__device__ __forceinline__ MixedOut mixed_out_global(const ElemArrays& E, int64_t e) {
+    return MixedOut{static_cast<float*>(E.sigma), static_cast<float*>(E.qia), static_cast<float*>(E.eps_p), E.ne_pad, e};
+}
+
 // One element of the mixed element pass (see the kernel comment below);
-// shared by the single-instance, staged and batched kernels.  Inputs come
-// from S, outputs go to the instance's arrays at element e.
+// shared by the single-instance, staged, batched and resident-run kernels.
+// Inputs come from S, the evolving rows go to O and the forces to the
+// instance's force array at element e.  Node rows are read with plain loads:
+// a resident run rewrites them between its cycles.
 // PF: node rows prefetched into L1 at the start (bit 0 velocities, bit 1
 // coordinate components 1 and 2).
 // FOUT: the 24 nodal forces go to fout[3 * 8] (component-major) instead of
 // the instance's force array, for the patch assembly.
 template <bool PLASTIC, bool INIT, bool SMEM = false, int PF = 0, bool FOUT = false>
 __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const NodeArrays& N, const Material& M,
-                                                   const MixedSrc& S, const float dt1, const double dt1d,
-                                                   const int64_t e, double& dts, double& len, double& e_int,
-                                                   double& e_hg, double& e_vis, int32_t& bad,
+                                                   const MixedSrc& S, const MixedOut& O, const float dt1,
+                                                   const double dt1d, const int64_t e, double& dts, double& len,
+                                                   double& e_int, double& e_hg, double& e_vis, int32_t& bad,
                                                    float* fout = nullptr) {
-    const int64_t ep = E.ne_pad, np = N.nn_pad, ss = S.stride, si = S.i;
-    float* sig = static_cast<float*>(E.sigma);
-    float* qia = static_cast<float*>(E.qia);
-    float* epsp = static_cast<float*>(E.eps_p);
-    float* __restrict__ fe = static_cast<float*>(E.fe);
-    const double* __restrict__ X = N.x;
-    const float* __restrict__ V = static_cast<const float*>(N.v);
+    const int64_t ep = E.ne_pad, np = N.nn_pad, ss = S.stride, si = S.i, os = O.stride, oi = O.i;
+    float* fe = static_cast<float*>(E.fe);
+    const double* X = N.x;
+    const float* V = static_cast<const float*>(N.v);
     const float G = M.mc.G;
     const float lam_hi = M.mc.lam_hi, lam_lo = M.mc.lam_lo;
     const float g2_hi = M.mc.g2_hi, g2_lo = M.mc.g2_lo;
@@ -383,12 +396,12 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
             s[3] *= r;
             s[4] *= r;
             s[5] *= r;
-            if (!INIT) epsp[e] = ep_old + dl;
+            if (!INIT) O.eps[oi] = ep_old + dl;
         }
     }
     if (!INIT) {
 #pragma unroll
-        for (int i = 0; i < 6; ++i) sig[i * ep + e] = s[i];
+        for (int i = 0; i < 6; ++i) O.sig[i * os + oi] = s[i];
     }
     const float Vc = static_cast<float>(static_cast<double>(J) * S.vol0[si]);
     {
@@ -406,7 +419,7 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             const float q = fmaf(DR, HIA[i][kk], S.qia[(4 * i + kk) * ss + si]);
-            if (!INIT) qia[(4 * i + kk) * ep + e] = q;
+            if (!INIT) O.qia[(4 * i + kk) * os + oi] = q;
             Gq[i][kk] = fmaf(CR, HIA[i][kk], q);
         }
     const bool visc = !(fabsf(vr) < 1.0e-10f);
@@ -509,8 +522,8 @@ __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_MIXED)
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < ne; e += stride) {
         double dts, len;
-        element_body_mixed<PLASTIC, INIT>(E, N, M, mixed_src_global(E, e), dt1, dt1d, e, dts, len, e_int, e_hg, e_vis,
-                                          bad);
+        element_body_mixed<PLASTIC, INIT>(E, N, M, mixed_src_global(E, e), mixed_out_global(E, e), dt1, dt1d, e, dts, len,
+                                          e_int, e_hg, e_vis, bad);
         dts_min = fmin(dts_min, dts);
         len_min = fmin(len_min, len);
     }
@@ -628,8 +641,8 @@ __global__ void __launch_bounds__(kStageTile, ENSC_STAGE_MINB_MIXED)
                              kStageTile,
                              tid};
             double dts, len;
-            element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(E, N, M, S, dt1, dt1d, e, dts, len, e_int,
-                                                                          e_hg, e_vis, bad);
+            element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(E, N, M, S, mixed_out_global(E, e), dt1, dt1d, e,
+                                                                          dts, len, e_int, e_hg, e_vis, bad);
             dts_min = fmin(dts_min, dts);
             len_min = fmin(len_min, len);
         }
@@ -736,8 +749,8 @@ __global__ void __launch_bounds__(kStageTile, ENSC_STAGE_MINB_MIXED)
                              kStageTile,
                              tid};
             double dts, len;
-            element_body_mixed<PLASTIC, INIT, true, ENSC_MIXED_PREFETCH, true>(E, N, M, S, dt1, dt1d, e, dts, len,
-                                                                               e_int, e_hg, e_vis, bad, fo);
+            element_body_mixed<PLASTIC, INIT, true, ENSC_MIXED_PREFETCH, true>(E, N, M, S, mixed_out_global(E, e), dt1, dt1d,
+                                                                               e, dts, len, e_int, e_hg, e_vis, bad, fo);
             dts_min = fmin(dts_min, dts);
             len_min = fmin(len_min, len);
         }
@@ -815,8 +828,8 @@ __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeA
                                                 const double dt_i, const double dt_i_1, const double amp, const int64_t n,
                                                 double& kin, double& wext, int32_t& bad) {
     const int64_t np = N.nn_pad, ep = E.ne_pad;
-    const float* __restrict__ fe = static_cast<const float*>(E.fe);
-    float* __restrict__ V = static_cast<float*>(N.v);
+    const float* fe = static_cast<const float*>(E.fe);
+    float* V = static_cast<float*>(N.v);
     [[maybe_unused]] const float hdt = static_cast<float>(0.5 * (dt_i + dt_i_1));
     [[maybe_unused]] const float hdt_lo = static_cast<float>(0.5 * (dt_i + dt_i_1) - static_cast<double>(hdt));
     const double dt_avg = 0.5 * (dt_i + dt_i_1);
@@ -906,8 +919,8 @@ __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double
                                                  const double amp, const int64_t n0, double& kin, double& wext,
                                                  int32_t& bad) {
     const int64_t np = N.np, nn = N.nn;
-    const float* __restrict__ fe = static_cast<const float*>(N.fe);
-    float* __restrict__ V = static_cast<float*>(N.v);
+    const float* fe = static_cast<const float*>(N.fe);
+    float* V = static_cast<float*>(N.v);
     [[maybe_unused]] const float hdt = static_cast<float>(0.5 * (dt_i + dt_i_1));
     [[maybe_unused]] const float hdt_lo = static_cast<float>(0.5 * (dt_i + dt_i_1) - static_cast<double>(hdt));
     const double dt_avg = 0.5 * (dt_i + dt_i_1);
@@ -1089,6 +1102,66 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_MIXED) k_node_mix
     block_sum_d<kNodeThreads, 2, 2u>(v2, P.node, P.n_node_blocks, blockIdx.x);
 }
 
+// ---- resident runs (ensc_run.cuh) -----------------------------------------
+// 16 warps per SM as in the staged pass; a tile of 32 elements takes 6.1 KB,
+// so that 148 SMs hold 151,552 elements at two tiles per warp.
+constexpr int kRunWarpsMixed = 16;
+template <bool PLASTIC>
+struct RunMixed {
+    static constexpr uint32_t kV0Off = kStageWordRows * 32u * 4u;
+    static constexpr uint32_t kTileBytes = kV0Off + 32u * 8u;
+    __device__ static const uint32_t* conn(const unsigned char* tile) {
+        return reinterpret_cast<const uint32_t*>(tile);
+    }
+    __device__ static void load_tile(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t base, int lane) {
+        constexpr int rows = PLASTIC ? kStageWordRows : kStageWordRows - 1;
+        if (lane == 0) mbar_arrive_expect_tx(bar, rows * 32u * 4u + 32u * 8u);
+        __syncwarp();
+        for (int r = lane; r <= rows; r += 32) {
+            if (r < rows) bulk_g2s(dst + r * (32u * 4u), stage_row(E, r) + base, 32u * 4u, bar);
+            else bulk_g2s(dst + kV0Off, E.vol0 + base, 32u * 8u, bar);
+        }
+    }
+    __device__ static void store_tile(const ElemArrays& E, const unsigned char* tile, int64_t base, int lane) {
+        const float* d = reinterpret_cast<const float*>(tile);
+        const int64_t e = base + lane;
+        if (e >= E.ne) return;
+        for (int r = 26; r < 44; ++r) const_cast<float*>(stage_row(E, r))[e] = d[r * 32 + lane];
+        if (PLASTIC) const_cast<float*>(stage_row(E, 45))[e] = d[45 * 32 + lane];
+    }
+    __device__ static void element(const ElemArrays& E, const NodeArrays& N, const Material& M, unsigned char* tile,
+                                   double dt1, int64_t e, int lane, double& dts, double& len, double& e_int,
+                                   double& e_hg, double& e_vis, int32_t& bad) {
+        float* st = reinterpret_cast<float*>(tile);
+        const MixedSrc S{conn(tile), st + 8 * 32, reinterpret_cast<const double*>(tile + kV0Off), st + 44 * 32,
+                         st + 26 * 32, st + 32 * 32, st + 45 * 32, 32, lane};
+        const MixedOut O{st + 26 * 32, st + 32 * 32, st + 45 * 32, 32, lane};
+        element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(E, N, M, S, O, static_cast<float>(dt1), dt1, e,
+                                                                      dts, len, e_int, e_hg, e_vis, bad);
+    }
+    // one node per thread while the grid has a thread for every node
+    __device__ static void nodes(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i,
+                                 double dt_i_1, double amp, int64_t t0, int64_t stride, double& kin, double& wext,
+                                 int32_t& bad) {
+        if (E.slot_major) {
+            const NodeView nv = node_view(E, N, M, nullptr);
+            if (N.nn <= stride) {
+                if (t0 < N.nn) node_group_mixed<1, false>(nv, dt_i, dt_i_1, amp, t0, kin, wext, bad);
+            } else {
+                for (int64_t g = t0; g * 2 < N.nn; g += stride)
+                    node_group_mixed<2, false>(nv, dt_i, dt_i_1, amp, g * 2, kin, wext, bad);
+            }
+        } else {
+            for (int64_t n = t0; n < N.nn; n += stride) node_body_mixed(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
+        }
+    }
+};
+
+template <bool PLASTIC, bool CLUSTER>
+__global__ void __launch_bounds__(32 * kRunWarpsMixed, 1)
+    k_run_mixed(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P, RunSync* sync, RunArgs a) {
+    run_cycles<RunMixed<PLASTIC>, CLUSTER>(E, N, M, ctl, P, sync, a);
+}
 
 // The last cycle's acceleration in mixed precision (see k_acceleration in
 // the FP64 stepper): the FP32 force sum, gravity and the FP32 acceleration
@@ -1343,8 +1416,8 @@ __global__ void __launch_bounds__(kStageTile / EPT, ENSC_BATCH_MINB_MIXED) k_ele
                                  kStageTile,
                                  li};
                 double d1, l1;
-                element_body_mixed<true, false, true, ENSC_BATCH_MIXED_PREFETCH, true>(E, N, M, S, dt1, dt1d, e, d1, l1,
-                                                                                      ei, eh, ev, bad, fo);
+                element_body_mixed<true, false, true, ENSC_BATCH_MIXED_PREFETCH, true>(E, N, M, S, mixed_out_global(E, e), dt1,
+                                                                                      dt1d, e, d1, l1, ei, eh, ev, bad, fo);
                 dts = fmin(dts, d1);
                 len = fmin(len, l1);
                 if (!patch) {
@@ -1575,6 +1648,21 @@ int occupancy_element_batch_mixed(int ept) {
     else
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_batch_mixed<1, false>, kStageTile, kBatchStageSmem);
     return nb;
+}
+
+RunPlan plan_run_mixed(int64_t ne, bool plastic, int sms) {
+    return plastic ? plan_run(k_run_mixed<true, true>, k_run_mixed<true, false>, ne, sms, kRunWarpsMixed,
+                              RunMixed<true>::kTileBytes)
+                   : plan_run(k_run_mixed<false, true>, k_run_mixed<false, false>, ne, sms, kRunWarpsMixed,
+                              RunMixed<false>::kTileBytes);
+}
+cudaError_t launch_run_mixed(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
+                             const Partials& P, RunSync* sync, const RunArgs& a, cudaStream_t st) {
+    if (M.plastic)
+        return p.cluster ? launch_run(k_run_mixed<true, true>, p, st, E, N, M, ctl, P, sync, a)
+                         : launch_run(k_run_mixed<true, false>, p, st, E, N, M, ctl, P, sync, a);
+    return p.cluster ? launch_run(k_run_mixed<false, true>, p, st, E, N, M, ctl, P, sync, a)
+                     : launch_run(k_run_mixed<false, false>, p, st, E, N, M, ctl, P, sync, a);
 }
 
 int batch_element_tile(bool mixed_precision) { return mixed_precision ? kStageTile : batch_element_tile_fp64(); }

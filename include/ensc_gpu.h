@@ -254,7 +254,9 @@ int ensc_profile(ensc_handle* h, int64_t max_cycles, double step_end_time, doubl
 /* Device bytes held by the handle. */
 int64_t ensc_device_bytes(const ensc_handle* h);
 
-/* Number of kernel launches one cycle issues (for launch accounting). */
+/* Number of kernel launches one cycle issues (for launch accounting); 0 where
+ * the instance is small enough to stay on chip, so that one launch runs all
+ * cycles of a step call (up to 4096 of them). */
 int32_t ensc_kernels_per_cycle(const ensc_handle* h);
 
 /* The force assembly the instance uses (ENSC_ASSEMBLY_SLOT or _PATCH), and
