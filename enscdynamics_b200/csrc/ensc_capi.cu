@@ -281,8 +281,8 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
 
     // resident runs where the mesh fits on chip (slot assembly)
     if (!ih.patch && prop.cooperativeLaunch)
-        h->run = mx ? ensc::plan_run_mixed(h->ne, h->plastic, prop.multiProcessorCount)
-                    : ensc::plan_run_fp64(h->ne, h->plastic, prop.multiProcessorCount);
+        h->run = mx ? ensc::plan_run_mixed(h->ne, h->nn, h->plastic, prop.multiProcessorCount)
+                    : ensc::plan_run_fp64(h->ne, h->nn, h->plastic, prop.multiProcessorCount);
 
     // ---- device memory: the instance block plus partial sums and control ----
     // (one partial slot per block of the larger of the two launch forms)
@@ -331,7 +331,7 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
     h->sync = reinterpret_cast<ensc::RunSync*>(tail + poff + coff);
     ce = cudaMemsetAsync(tail, 0, small, h->stream);
     ensc::RunSync sync0{};
-    sync0.pre_len = ensc::kInfBits;
+    sync0.pre = ensc::kInfBits;
     for (ensc::RunMins& m : sync0.mins) m = ensc::RunMins{ensc::kInfBits, ensc::kInfBits};
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(h->sync, &sync0, sizeof(sync0), cudaMemcpyHostToDevice, h->stream);
     if (ce != cudaSuccess) {

@@ -7,6 +7,21 @@
 
 namespace ensc {
 
+// x / c for a divisor used many times, rc = 1 / c rounded to nearest: a
+// quotient estimate corrected twice by its exact remainder, which rounds as the
+// division does (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990: an estimate within one unit in the last
+// place and one correction with a correctly rounded reciprocal suffice; the
+// first correction brings the estimate there).  For normal x, c and quotient;
+// zero stays zero and a non-finite x gives a non-finite quotient.  Five
+// dependent operations without the branch and the call of a general
+// division.
+__device__ __forceinline__ double div_by(double x, double c, double rc) {
+    double q = x * rc;
+    q = __fma_rn(__fma_rn(-q, c, x), rc, q);
+    return __fma_rn(__fma_rn(-q, c, x), rc, q);
+}
+
 // True when the instance must not begin another cycle (a status was raised,
 // the step end, the cycle budget or the pause time is reached).
 __device__ __forceinline__ bool cycle_stops(const Ctl* ctl, int32_t status) {
@@ -76,10 +91,11 @@ __device__ __forceinline__ void begin_exact(Ctl* ctl, unsigned long long len_min
 }
 
 // The cycle's stable dt once the element pass has left its edge minimum
-// (update_minVertex_perMaterial_and_dt, exDyna3D.cpp:673-679).
-__device__ __forceinline__ double cycle_dt(const Ctl* ctl, unsigned long long len_min_bits) {
+// (update_minVertex_perMaterial_and_dt, exDyna3D.cpp:673-679); inv_wos =
+// 1 / ctl->wos.
+__device__ __forceinline__ double cycle_dt(const Ctl* ctl, unsigned long long len_min_bits, double inv_wos) {
     if (ctl->dt_final) return ctl->dt_i;
-    double d = bits_ord(len_min_bits) / ctl->wos;
+    double d = div_by(bits_ord(len_min_bits), ctl->wos, inv_wos);
     const double tmp = ctl->dts_cur;
     d = d < tmp ? d : tmp;
     return d * ctl->factor;

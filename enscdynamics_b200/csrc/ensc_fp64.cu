@@ -314,7 +314,7 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
     if (PLASTIC) {
         // J2 radial return, linear isotropic hardening (no reference
         // counterpart; the elastic instantiation omits it).
-        const double pm = ((s[0] + s[1]) + s[2]) / 3.0;
+        const double pm = div_by((s[0] + s[1]) + s[2], 3.0, 1.0 / 3.0);
         const double d0 = s[0] - pm, d1 = s[1] - pm, d2 = s[2] - pm;
         const double j2 = 0.5 * ((d0 * d0 + d1 * d1) + d2 * d2) + ((s[3] * s[3] + s[4] * s[4]) + s[5] * s[5]);
         const double seq = sqrt(3.0 * j2);
@@ -419,10 +419,10 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
     }
     // compute_dtStable (:828-834)
     {
-        const double cd = M.wos;
+        const double cd = M.wos, rcd = M.mc.inv_wos;
         const double m0 = vr < 0.0 ? vr : 0.0;
-        const double xi = M.cvisl - M.cvisq * M.cvisq * len / cd * m0;
-        dts = (sqrt(1.0 + xi * xi) - xi) * len / cd;
+        const double xi = M.cvisl - div_by(M.cvisq * M.cvisq * len, cd, rcd) * m0;
+        dts = div_by((sqrt(1.0 + xi * xi) - xi) * len, cd, rcd);
     }
     if (!isfinite(dts)) bad |= ST_NONFINITE;
 }
@@ -466,7 +466,9 @@ __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_FP64) k_element(E
 }
 
 // One node of the node pass (see the kernel comment below); shared by the
-// single-instance and batched kernels.
+// single-instance, batched and resident-run kernels (KIN: sum the kinetic
+// energy).
+template <bool KIN = true>
 __device__ __forceinline__ void node_body(const ElemArrays& E, const NodeArrays& N, const Material& M,
                                           const double dt_i, const double dt_i_1, const double amp, const int64_t n, double& kin,
                                           double& wext, int32_t& bad) {
@@ -559,7 +561,7 @@ __device__ __forceinline__ void node_body(const ElemArrays& E, const NodeArrays&
         N.x[c * np + n] = N.x[c * np + n] + dt_i * vn;
         const double vb = 0.5 * (vo + vn);
         wext = wext + (g + r) * dt_avg * vb;
-        kin = kin + 0.5 * (vn * vn) / im;
+        if (KIN) kin = kin + 0.5 * (vn * vn) / im;
         if (!isfinite(vn)) bad |= ST_NONFINITE;
     }
 }
@@ -891,15 +893,31 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
 // added as the zeros they hold, as the reference adds all 8 slot vectors:
 // the slot-major rows start zeroed and only the slot's element writes them.
 // Nodes at or past nn (row padding) are loaded and stored back unchanged.
+//
+// pre (resident runs): the nodes' own rows, loaded while the grid still works
+// on the forces; such a run sums its kinetic energy once, at its end.
 template <int W>
-__device__ __forceinline__ void node_group(const NodeView& N, const double dt_i, const double dt_i_1, const double amp,
-                                           const int64_t n0, double& kin, double& wext, int32_t& bad) {
-    const int64_t np = N.np, nn = N.nn;
+struct NodeRowsF64 {
+    double im[W], v[3][W], u[3][W], x[3][W];
+    uint32_t code;
+};
+template <int W>
+__device__ __forceinline__ void node_rows_load(const NodeView& N, const int64_t n0, NodeRowsF64<W>& r) {
+    ld_row<W>(N.inv_mass + n0, r.im);
+    r.code = ld_bytes<W>(N.bc + n0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        ld_row<W>(static_cast<const double*>(N.v) + c * N.np + n0, r.v[c]);
+        ld_row<W>(N.u + c * N.np + n0, r.u[c]);
+        ld_row<W>(N.x + c * N.np + n0, r.x[c]);
+    }
+}
+
+// The forces of W consecutive nodes, added up in slot order.
+template <int W>
+__device__ __forceinline__ void node_forces(const NodeView& N, const int64_t n0, double (&f)[3][W]) {
+    const int64_t np = N.np;
     const double* fe = static_cast<const double*>(N.fe);
-    double* V = static_cast<double*>(N.v);
-    const double half = (dt_i + dt_i_1);
-    const double dt_avg = (dt_i + dt_i_1) / 2.0;
-    double f[3][W];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -921,15 +939,52 @@ __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i,
             }
         }
     }
+}
+
+// PRE: rows and forces come in pre and fpre.
+template <int W, bool PRE = false>
+__device__ __forceinline__ void node_group(const NodeView& N, const double dt_i, const double dt_i_1, const double amp,
+                                           const int64_t n0, double& kin, double& wext, int32_t& bad,
+                                           const NodeRowsF64<W>* pre = nullptr,
+                                           const double (*fpre)[W] = nullptr) {
+    const int64_t np = N.np, nn = N.nn;
+    double* V = static_cast<double*>(N.v);
+    const double half = (dt_i + dt_i_1);
+    const double dt_avg = (dt_i + dt_i_1) / 2.0;
+    double f[3][W];
+    if constexpr (PRE) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int j = 0; j < W; ++j) f[c][j] = fpre[c][j];
+    } else {
+        node_forces<W>(N, n0, f);
+    }
     double im[W];
-    ld_row<W>(N.inv_mass + n0, im);
-    const uint32_t code = ld_bytes<W>(N.bc + n0);
+    uint32_t code;
+    if constexpr (PRE) {
+#pragma unroll
+        for (int j = 0; j < W; ++j) im[j] = pre->im[j];
+        code = pre->code;
+    } else {
+        ld_row<W>(N.inv_mass + n0, im);
+        code = ld_bytes<W>(N.bc + n0);
+    }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         double vo[W], uo[W], xo[W], vn[W], un[W], xn[W];
-        ld_row<W>(V + c * np + n0, vo);
-        ld_row<W>(N.u + c * np + n0, uo);
-        ld_row<W>(N.x + c * np + n0, xo);
+        if constexpr (PRE) {
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                vo[j] = pre->v[c][j];
+                uo[j] = pre->u[c][j];
+                xo[j] = pre->x[c][j];
+            }
+        } else {
+            ld_row<W>(V + c * np + n0, vo);
+            ld_row<W>(N.u + c * np + n0, uo);
+            ld_row<W>(N.x + c * np + n0, xo);
+        }
 #pragma unroll
         for (int j = 0; j < W; ++j) {
             vn[j] = vo[j];
@@ -960,7 +1015,7 @@ __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i,
             xn[j] = xo[j] + dt_i * vn[j];
             const double vb = 0.5 * (vo[j] + vn[j]);
             wext = wext + (g + r) * dt_avg * vb;
-            kin = kin + 0.5 * (vn[j] * vn[j]) / im[j];
+            if (!PRE) kin = kin + 0.5 * (vn[j] * vn[j]) / im[j];
             if (!isfinite(vn[j])) bad |= ST_NONFINITE;
         }
         st_row<W>(V + c * np + n0, vn);
@@ -1043,28 +1098,52 @@ struct RunFp64 {
         element_body<PLASTIC, false, true, true, ENSC_F64_PREFETCH>(E, N, M, S, O, dt1, e, dts, len, e_int, e_hg,
                                                                      e_vis, bad);
     }
-    // one node per thread while the grid has a thread for every node
-    __device__ static void nodes(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i,
-                                 double dt_i_1, double amp, int64_t t0, int64_t stride, double& kin, double& wext,
-                                 int32_t& bad) {
-        if (E.slot_major) {
-            const NodeView nv = node_view(E, N, M, nullptr);
-            if (N.nn <= stride) {
-                if (t0 < N.nn) node_group<1>(nv, dt_i, dt_i_1, amp, t0, kin, wext, bad);
-            } else {
-                for (int64_t g = t0; g * 2 < N.nn; g += stride)
-                    node_group<2>(nv, dt_i, dt_i_1, amp, g * 2, kin, wext, bad);
-            }
-        } else {
-            for (int64_t n = t0; n < N.nn; n += stride) node_body(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
+    // W nodes per thread, their rows loaded ahead of the forces; a thread's
+    // further nodes (meshes with more than 2 per thread) load both together.
+    // Meshes whose nodes repeat slots read their lists node by node.
+    template <int W>
+    struct Nodes {
+        NodeRowsF64<W> rows;
+        double f[3][W];
+        __device__ void load(const ElemArrays& E, const NodeArrays& N, const Material& M, int64_t t0) {
+            if (E.slot_major && t0 * W < N.nn) node_rows_load<W>(node_view(E, N, M, nullptr), t0 * W, rows);
         }
+        __device__ void gather(const ElemArrays& E, const NodeArrays& N, const Material& M, int64_t t0) {
+            if (E.slot_major && t0 * W < N.nn) node_forces<W>(node_view(E, N, M, nullptr), t0 * W, f);
+        }
+        __device__ void update(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i, double dt_i_1,
+                               double amp, int64_t t0, int64_t stride, double& wext, int32_t& bad) {
+            double kin = 0.0;
+            if (E.slot_major) {
+                const NodeView nv = node_view(E, N, M, nullptr);
+                if (t0 * W < N.nn) node_group<W, true>(nv, dt_i, dt_i_1, amp, t0 * W, kin, wext, bad, &rows, f);
+                if (W > 1)
+                    for (int64_t g = t0 + stride; g * W < N.nn; g += stride) {
+                        node_rows_load<W>(nv, g * W, rows);
+                        node_forces<W>(nv, g * W, f);
+                        node_group<W, true>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad, &rows, f);
+                    }
+            } else {
+                for (int64_t n = t0; n < N.nn; n += stride)
+                    node_body<false>(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
+            }
+        }
+    };
+    __device__ static double kinetic(const NodeArrays& N, int64_t n) {
+        const double* V = static_cast<const double*>(N.v);
+        double kin = 0.0;
+        for (int c = 0; c < 3; ++c) {
+            const double v = V[c * N.nn_pad + n];
+            kin = kin + 0.5 * (v * v) / N.inv_mass[n];
+        }
+        return kin;
     }
 };
 
-template <bool PLASTIC, bool CLUSTER>
+template <bool PLASTIC, bool CLUSTER, int W>
 __global__ void __launch_bounds__(32 * kRunWarpsF64, 1)
     k_run_fp64(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P, RunSync* sync, RunArgs a) {
-    run_cycles<RunFp64<PLASTIC>, CLUSTER>(E, N, M, ctl, P, sync, a);
+    run_cycles<RunFp64<PLASTIC>, CLUSTER, W>(E, N, M, ctl, P, sync, a);
 }
 
 // ---- batched instances --------------------------------------------------------
@@ -1421,19 +1500,20 @@ int occupancy_element_batch_fp64() {
     return nb;
 }
 
-RunPlan plan_run_fp64(int64_t ne, bool plastic, int sms) {
-    return plastic ? plan_run(k_run_fp64<true, true>, k_run_fp64<true, false>, ne, sms, kRunWarpsF64,
-                              RunFp64<true>::kTileBytes)
-                   : plan_run(k_run_fp64<false, true>, k_run_fp64<false, false>, ne, sms, kRunWarpsF64,
-                              RunFp64<false>::kTileBytes);
+RunPlan plan_run_fp64(int64_t ne, int64_t nn, bool plastic, int sms) {
+    return plastic ? plan_run(k_run_fp64<true, true, 1>, k_run_fp64<true, true, 2>, k_run_fp64<true, false, 1>,
+                              k_run_fp64<true, false, 2>, ne, nn, sms, kRunWarpsF64, RunFp64<true>::kTileBytes)
+                   : plan_run(k_run_fp64<false, true, 1>, k_run_fp64<false, true, 2>, k_run_fp64<false, false, 1>,
+                              k_run_fp64<false, false, 2>, ne, nn, sms, kRunWarpsF64, RunFp64<false>::kTileBytes);
 }
 cudaError_t launch_run_fp64(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
                             const Partials& P, RunSync* sync, const RunArgs& a, cudaStream_t st) {
-    if (M.plastic)
-        return p.cluster ? launch_run(k_run_fp64<true, true>, p, st, E, N, M, ctl, P, sync, a)
-                         : launch_run(k_run_fp64<true, false>, p, st, E, N, M, ctl, P, sync, a);
-    return p.cluster ? launch_run(k_run_fp64<false, true>, p, st, E, N, M, ctl, P, sync, a)
-                     : launch_run(k_run_fp64<false, false>, p, st, E, N, M, ctl, P, sync, a);
+    using K = void (*)(ElemArrays, NodeArrays, Material, Ctl*, Partials, RunSync*, RunArgs);
+    static const K kernels[8] = {k_run_fp64<false, false, 1>, k_run_fp64<false, false, 2>, k_run_fp64<false, true, 1>,
+                                 k_run_fp64<false, true, 2>,  k_run_fp64<true, false, 1>,  k_run_fp64<true, false, 2>,
+                                 k_run_fp64<true, true, 1>,   k_run_fp64<true, true, 2>};
+    return launch_run(kernels[(M.plastic ? 4 : 0) + (p.cluster ? 2 : 0) + p.node_width - 1], p, st, E, N, M, ctl, P,
+                      sync, a);
 }
 
 int batch_element_tile_fp64() { return kF64BatchTile; }

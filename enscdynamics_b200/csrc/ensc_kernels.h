@@ -77,13 +77,6 @@ constexpr int kNodeUnrollMixed = ENSC_NODE_UNROLL_MIXED;
 #ifndef ENSC_NODE_ALL_SLOTS
 #define ENSC_NODE_ALL_SLOTS 1
 #endif
-// 1: the mixed node passes load the nodes' own rows (v, its residual, x,
-// the inverse mass, the BC code) before the force slots, so that all the
-// group's loads are in flight together (measured on B200: node pass 4%
-// faster, bit-identical)
-#ifndef ENSC_NODE_LOAD_FIRST
-#define ENSC_NODE_LOAD_FIRST 1
-#endif
 #ifndef ENSC_NODE_BATCH_MINB_MIXED
 #define ENSC_NODE_BATCH_MINB_MIXED 2
 #endif
@@ -135,15 +128,15 @@ constexpr int kCtlThreads = 256;
 struct RunMins {
     unsigned long long dts, len;
 };
-// Grid-wide state of a resident run, zero and +inf between launches: the
-// arrival counter (low half; upper half: blocks that saw an error, 16 bits per
-// phase), the raised status bits, the blocks that have left.
+// Grid-wide state of a resident run; between launches the minima are +inf and
+// the rest zero.
 struct alignas(128) RunSync {
-    unsigned long long arrive;
-    int32_t status, left;
-    unsigned long long pre_len;
-    unsigned long long pad;
-    RunMins mins[3];
+    unsigned long long arrive;  // arrivals; 8 bits each from bit 48 and 56: blocks that saw an error in
+                                // an element phase and in a node phase
+    int32_t status, left;       // raised status bits, blocks that have left
+    unsigned long long pad[14];
+    RunMins mins[3];            // element phases of three cycles in turn
+    unsigned long long pre;     // edge minimum of a cycle the total-time clamp may shorten
 };
 struct RunArgs {
     double step_end, pause;
@@ -156,10 +149,11 @@ struct RunArgs {
 // fit, use the per-phase kernels.
 struct RunPlan {
     int grid = 0, threads = 0, cluster = 0, tiles_per_warp = 0;
+    int node_width = 1;        // nodes per thread of the node phase
     size_t smem = 0;
 };
-RunPlan plan_run_fp64(int64_t ne, bool plastic, int sms);
-RunPlan plan_run_mixed(int64_t ne, bool plastic, int sms);
+RunPlan plan_run_fp64(int64_t ne, int64_t nn, bool plastic, int sms);
+RunPlan plan_run_mixed(int64_t ne, int64_t nn, bool plastic, int sms);
 cudaError_t launch_run_fp64(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
                             const Partials& P, RunSync* sync, const RunArgs& a, cudaStream_t st);
 cudaError_t launch_run_mixed(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,

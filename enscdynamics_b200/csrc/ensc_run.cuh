@@ -7,8 +7,8 @@
 // keeps its element tiles (connectivity, geometry, sigma, QIA, eps_p) in
 // shared memory from the first cycle to the last, and the element and node
 // phases of each cycle are separated by barriers of the grid: a hardware
-// cluster barrier where one cluster holds the mesh, else an arrival counter
-// in global memory.  Node rows and element forces go through L2 as in the
+// cluster barrier where one cluster holds the mesh, else an arrival counter in
+// global memory.  Node rows and element forces go through L2 as in the
 // per-phase kernels.
 //
 // The scalar control (ensc_cycle.cuh) is evaluated by thread 0 of every block
@@ -37,6 +37,7 @@ struct RunShared {
     int32_t go, exact;
     double dt1, dt_i, dt_i_1, amp;
     int32_t cycles;                // cycles begun in this launch
+    int32_t last;
     unsigned int bar;              // arrivals that complete the next barrier
     unsigned long long w_dts[kRunMaxWarps], w_len[kRunMaxWarps];
     // cluster barrier: what each block of the cluster published
@@ -63,31 +64,36 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, unsigned long long v) 
 __device__ __forceinline__ void st_cluster32(uint32_t addr, int32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void cluster_barrier() {
+__device__ __forceinline__ void cluster_arrive() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// Adds one arrival (and `extra` in the upper half) and waits until `target`
-// arrivals have been counted; returns the counter as seen then, or all ones
-// when the bounded wait expired.  One thread per block, between block
-// barriers: the release of the arrival covers what the block wrote before,
-// the acquire what it reads after.
-__device__ __forceinline__ unsigned long long grid_arrive_wait(unsigned long long* word, unsigned long long extra,
-                                                               unsigned int target) {
+// ---- barrier of the grid ----
+// One thread per block, between block barriers: adds its arrival (the
+// release covers what the block wrote before) and polls until `target`
+// arrivals have been counted (the acquire covers what it reads after).
+// Returns the counter as seen then, or all ones when the bounded wait
+// expired.  With 148 blocks on B200 the bare barrier takes 2,460 clocks, two
+// trips to L2 and back, and 3,460 behind 9 stores per thread.  Forms with a
+// second hop (one collector that publishes, a tree of counters) took 3,100 to
+// 4,350 bare; every block reading a table of all blocks, twice that.
+__device__ __forceinline__ unsigned long long grid_barrier(unsigned long long* word, unsigned long long extra,
+                                                           unsigned int target) {
     unsigned long long v;
-    __threadfence();
-    asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;" : "=l"(v) : "l"(word), "l"(extra + 1ull) : "memory");
-    v += extra + 1ull;
-    if (static_cast<unsigned int>(v) < target) {
-        const long long t0 = clock64();
-        do {
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
-            if (static_cast<unsigned int>(v) >= target) break;
-            if (clock64() - t0 > kStageWaitCycles) return ~0ull;
-        } while (true);
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(extra + 1ull) : "memory");
+    const long long t0 = clock64();
+    while (true) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+        if (static_cast<unsigned int>(v) >= target) return v;
+        if (clock64() - t0 > kStageWaitCycles) return ~0ull;
     }
-    __threadfence();
+}
+constexpr unsigned long long kRunErrElem = 1ull << 48, kRunErrNode = 1ull << 56;
+
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -112,9 +118,11 @@ __device__ __forceinline__ void run_begin(RunShared& sh, int32_t status, int lau
 //   Pol::load_tile(E, dst, bar, base, lane)   bulk copies of a tile
 //   Pol::store_tile(E, tile, base, lane)      its evolving rows back to global memory
 //   Pol::element(E, N, M, tile, dt1, e, lane, ...)
-//   Pol::nodes(E, N, M, dt_i, dt_i_1, amp, t0, stride, kin, wext, bad)
+//   Pol::Nodes<W>                             a thread's W nodes: load (their rows), gather (their
+//                                             forces), update
+//   Pol::kinetic(N, n)                        kinetic energy of node n
 // Blocks of 32 * nw threads; warp w of the grid owns the tiles w, w + W, ...
-template <class Pol, bool CLUSTER>
+template <class Pol, bool CLUSTER, int W>
 __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
                                            const Partials& P, RunSync* sync, const RunArgs& a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -142,9 +150,14 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
         if (!sh.c.done) run_begin(sh, sh.c.status, a.launch_cycles);
     }
     __syncthreads();
-    const bool any = sh.go != 0;
+    if (!sh.go) {
+        // nothing to run: only the limits and `done` change, to the same
+        // values whichever of the old and new ones another block reads
+        if (tid == 0 && block == 0) *ctl = sh.c;
+        return;
+    }
     bool loaded = true;
-    if (any && mine > 0) {
+    if (mine > 0) {
         const uint32_t bar = smem_addr(&sh.mbar[wid]);
         if (lane == 0) {
             mbar_init(bar, mine);
@@ -156,13 +169,13 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
         loaded = mbar_wait_bounded(bar, 0);
         loaded = __all_sync(0xffffffffu, loaded);
     }
-    double e_int = 0.0, e_hg = 0.0, e_vis = 0.0, kin = 0.0, wext = 0.0;
+    double e_int = 0.0, e_hg = 0.0, e_vis = 0.0, wext = 0.0;
     const int64_t t0 = static_cast<int64_t>(block) * blockDim.x + tid;
     const int64_t stride = static_cast<int64_t>(nblocks) * blockDim.x;
     bool failed = false;
-    int32_t err_a = 0;
+    int32_t err = 0;  // warp 0: an error was published
     while (sh.go) {
-        const int slot = sh.cycles % 3;
+        const int set = sh.cycles % 3;
         if (sh.exact) {
             // a cycle the total-time clamp may shorten: the edge minimum first
             double m = DBL_MAX;
@@ -180,19 +193,35 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
                 m = t < m ? t : m;
             }
             const unsigned long long b = run_warp_min(ord_bits(m));
-            if (lane == 0) atomicMin(&sync->pre_len, b);
+            if (lane == 0) sh.w_len[wid] = b;
             __syncthreads();
-            if (CLUSTER) {
-                __threadfence();
-                cluster_barrier();
-            }
-            if (tid == 0) {
-                if (!CLUSTER) {
+            unsigned long long l = kInfBits;
+            if (wid == 0) {
+                l = run_warp_min(lane < nw ? sh.w_len[lane] : kInfBits);
+                if (CLUSTER) {
+                    if (lane < nblocks) st_cluster(map_to_rank(smem_addr(&sh.c_len[block]), lane), l);
+                } else if (lane == 0) {
+                    atomicMin(&sync->pre, l);
                     sh.bar += nblocks;
-                    if (grid_arrive_wait(&sync->arrive, 0, sh.bar) == ~0ull) failed = true;
+                    if (grid_barrier(&sync->arrive, 0, sh.bar) == ~0ull) failed = true;
+                    l = ld_relaxed(&sync->pre);
                 }
-                begin_exact(&sh.c, atomicOr(&sync->pre_len, 0ull));
-                sh.dt1 = sh.c.dt_i_1;
+            }
+            if (CLUSTER) {
+                cluster_arrive();
+                cluster_wait();
+            }
+            if (wid == 0) {
+                if (CLUSTER) l = run_warp_min(lane < nblocks ? sh.c_len[lane] : kInfBits);
+                if (lane == 0) {
+                    begin_exact(&sh.c, l);
+                    sh.dt1 = sh.c.dt_i_1;
+                }
+            }
+            if (CLUSTER) {
+                // c_len is written again at the end of the element phase
+                cluster_arrive();
+                cluster_wait();
             }
             failed = __syncthreads_or(failed);
             if (failed) break;
@@ -220,8 +249,8 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
         }
         int any_bad = __syncthreads_or(bad);
         if (wid == 0) {
-            unsigned long long d = run_warp_min(lane < nw ? sh.w_dts[lane] : kInfBits);
-            unsigned long long l = run_warp_min(lane < nw ? sh.w_len[lane] : kInfBits);
+            const unsigned long long d = run_warp_min(lane < nw ? sh.w_dts[lane] : kInfBits);
+            const unsigned long long l = run_warp_min(lane < nw ? sh.w_len[lane] : kInfBits);
             if (CLUSTER) {
                 if (lane < nblocks) {
                     st_cluster(map_to_rank(smem_addr(&sh.c_dts[block]), lane), d);
@@ -229,70 +258,82 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
                     st_cluster32(map_to_rank(smem_addr(&sh.c_bad[0][block]), lane), any_bad);
                 }
             } else if (lane == 0) {
-                atomicMin(&sync->mins[slot].dts, d);
-                atomicMin(&sync->mins[slot].len, l);
+                atomicMin(&sync->mins[set].dts, d);
+                atomicMin(&sync->mins[set].len, l);
             }
         }
-        if (CLUSTER) cluster_barrier();
+        // the thread's own node rows are on their way while the grid finishes
+        typename Pol::template Nodes<W> nodes;
+        if (CLUSTER) cluster_arrive();
+        nodes.load(E, N, M, t0);
+        if (CLUSTER) {
+            cluster_wait();
+        } else {
+            if (tid == 0) {
+                sh.bar += nblocks;
+                const unsigned long long v = grid_barrier(&sync->arrive, any_bad ? kRunErrElem : 0, sh.bar);
+                if (v == ~0ull) failed = true;
+                err |= static_cast<int32_t>((v >> 48) & 0xffu);
+            }
+            if (__syncthreads_or(failed)) {
+                failed = true;
+                break;
+            }
+        }
+        // the forces are added up while thread 0 turns the minima into dt
+        unsigned long long d = 0, l = 0;
+        if (!CLUSTER && tid == 0) {
+            d = ld_relaxed(&sync->mins[set].dts);
+            l = ld_relaxed(&sync->mins[set].len);
+        }
+        nodes.gather(E, N, M, t0);
         if (wid == 0) {
-            unsigned long long d, l;
             if (CLUSTER) {
                 d = run_warp_min(lane < nblocks ? sh.c_dts[lane] : kInfBits);
                 l = run_warp_min(lane < nblocks ? sh.c_len[lane] : kInfBits);
-                err_a |= __any_sync(0xffffffffu, lane < nblocks && sh.c_bad[0][lane] != 0);
-            } else if (lane == 0) {
-                sh.bar += nblocks;
-                const unsigned long long v = grid_arrive_wait(&sync->arrive, any_bad ? 1ull << 32 : 0ull, sh.bar);
-                if (v == ~0ull) failed = true;
-                err_a |= static_cast<int32_t>((v >> 32) & 0xffffu);
-                d = *reinterpret_cast<volatile unsigned long long*>(&sync->mins[slot].dts);
-                l = *reinterpret_cast<volatile unsigned long long*>(&sync->mins[slot].len);
+                err |= __any_sync(0xffffffffu, lane < nblocks && sh.c_bad[0][lane] != 0);
             }
             if (lane == 0) {
                 Ctl* c = &sh.c;
                 c->dts_next = d;
                 c->len_min = l;
-                const double dt_i = cycle_dt(c, l);
+                const double dt_i = cycle_dt(c, l, M.mc.inv_wos);
                 if (!c->dt_final) c->dt_i = dt_i;
                 c->cycles_done += 1;
                 sh.dt_i = dt_i;
                 sh.dt_i_1 = c->dt_i_1;
                 sh.amp = (M.gravity_on && M.amp_n > 0) ? gravity_amplitude(M.amp, M.amp_n, c->time, dt_i) : 1.0;
                 if (!(dt_i > 0.0) || !isfinite(dt_i)) {
-                    err_a |= 1;
+                    err |= 1;
                     atomicOr(&sync->status, ST_BAD_DT);
                 }
-                if (block == 0) {
-                    // the slot two cycles on restarts from +inf (its last
+                if (!CLUSTER && block == 0) {
+                    // the set of the next cycle restarts from +inf (its last
                     // readers passed the previous cycle's barriers)
-                    sync->mins[(slot + 1) % 3] = RunMins{kInfBits, kInfBits};
-                    if (sh.exact) sync->pre_len = kInfBits;
+                    sync->mins[(set + 1) % 3] = RunMins{kInfBits, kInfBits};
+                    if (sh.exact) sync->pre = kInfBits;
                 }
             }
         }
-        if (__syncthreads_or(failed)) {
-            failed = true;
-            break;
-        }
+        __syncthreads();
         // ---- node phase
         int32_t nbad = 0;
-        kin = 0.0;
-        Pol::nodes(E, N, M, sh.dt_i, sh.dt_i_1, sh.amp, t0, stride, kin, wext, nbad);
+        nodes.update(E, N, M, sh.dt_i, sh.dt_i_1, sh.amp, t0, stride, wext, nbad);
         if (nbad) atomicOr(&sync->status, nbad);
         any_bad = __syncthreads_or(nbad);
         if (CLUSTER) {
             if (tid < nblocks) st_cluster32(map_to_rank(smem_addr(&sh.c_bad[1][block]), tid), any_bad);
-            cluster_barrier();
+            cluster_arrive();
+            cluster_wait();
         }
         if (wid == 0) {
-            int32_t err = err_a;
             if (CLUSTER) {
                 err |= __any_sync(0xffffffffu, lane < nblocks && sh.c_bad[1][lane] != 0);
             } else if (lane == 0) {
                 sh.bar += nblocks;
-                const unsigned long long v = grid_arrive_wait(&sync->arrive, any_bad ? 1ull << 48 : 0ull, sh.bar);
+                const unsigned long long v = grid_barrier(&sync->arrive, any_bad ? kRunErrNode : 0, sh.bar);
                 if (v == ~0ull) failed = true;
-                err |= static_cast<int32_t>(v >> 48);
+                err |= static_cast<int32_t>(v >> 56);
             }
             if (lane == 0) run_begin(sh, err, a.launch_cycles);
         }
@@ -301,17 +342,13 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
             break;
         }
     }
-    if (!any) {
-        // nothing to run: only the limits and `done` change, to the same
-        // values whichever of the old and new ones another block reads
-        if (tid == 0 && block == 0) *ctl = sh.c;
-        return;
-    }
     // ---- end of the launch: the evolving element rows, the energy partials
     // and the control block back to global memory
     for (int s = 0; s < mine && loaded; ++s)
         Pol::store_tile(E, wtiles + s * Pol::kTileBytes, (w0 + s * wstride) * 32, lane);
     if (tid == 0 && failed) atomicOr(&sync->status, ST_TIMEOUT);
+    double kin = 0.0;
+    for (int64_t n = t0; n < N.nn; n += stride) kin = kin + Pol::kinetic(N, n);
     double v5[5] = {e_int, e_hg, e_vis, wext, kin};
     __shared__ double red[5][kRunMaxWarps];
 #pragma unroll
@@ -331,22 +368,20 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
             // the latest kinetic energy: this run's blocks hold all of it
             for (int i = block; i < P.n_node_blocks; i += nblocks) P.node[i] = i == block ? s : 0.0;
     }
+    // the last block out leaves the control block and a fresh sync area
     __threadfence();
     __syncthreads();
-    if (tid == 0) {
-        // the last block out leaves the control block and a fresh sync area
-        if (atomicAdd(&sync->left, 1) == nblocks - 1) {
-            __threadfence();
-            sh.c.status |= atomicExch(&sync->status, 0);
-            sh.c.energy_pending = 1;
-            for (int i = 0; i < 6; ++i) sh.c.energy[i] = ctl->energy[i];
-            *ctl = sh.c;
-            for (int i = 0; i < 3; ++i) sync->mins[i] = RunMins{kInfBits, kInfBits};
-            sync->pre_len = kInfBits;
-            sync->arrive = 0;
-            sync->left = 0;
-        }
-    }
+    if (tid == 0) sh.last = atomicAdd(&sync->left, 1) == nblocks - 1;
+    __syncthreads();
+    if (!sh.last || tid != 0) return;
+    __threadfence();
+    sh.c.status |= atomicExch(&sync->status, 0);
+    sh.c.energy_pending = 1;
+    *ctl = sh.c;
+    for (int i = 0; i < 3; ++i) sync->mins[i] = RunMins{kInfBits, kInfBits};
+    sync->pre = kInfBits;
+    sync->arrive = 0;
+    sync->left = 0;
 }
 
 // ---- host side ----
@@ -358,8 +393,12 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
 constexpr size_t kRunSmemMax = 227 * 1024 - sizeof(RunShared) - 5 * kRunMaxWarps * sizeof(double) - 256;
 
 template <typename K>
-RunPlan plan_run(K cluster_kernel, K grid_kernel, int64_t ne, int sms, int max_warps, uint32_t tile_bytes) {
+RunPlan plan_run(K cluster_kernel_1, K cluster_kernel_2, K grid_kernel_1, K grid_kernel_2, int64_t ne, int64_t nn,
+                 int sms, int max_warps, uint32_t tile_bytes) {
     RunPlan p;
+    // one node per thread while there is a thread for every node
+    auto width = [nn](const RunPlan& q) { return nn <= static_cast<int64_t>(q.grid) * q.threads ? 1 : 2; };
+    sms = sms < 255 ? sms : 255;  // the error counts have 8 bits
     const int64_t tiles = (ne + 31) / 32;
     if (tiles <= 4 * kRunMaxCluster) {
         int c = 1;
@@ -368,6 +407,8 @@ RunPlan plan_run(K cluster_kernel, K grid_kernel, int64_t ne, int sms, int max_w
         p.grid = p.cluster = c;
         p.tiles_per_warp = 1;
         p.smem = static_cast<size_t>(4) * tile_bytes;
+        p.node_width = width(p);
+        K cluster_kernel = p.node_width == 1 ? cluster_kernel_1 : cluster_kernel_2;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(c);
         cfg.blockDim = dim3(p.threads);
@@ -393,6 +434,8 @@ RunPlan plan_run(K cluster_kernel, K grid_kernel, int64_t ne, int sms, int max_w
     p.threads = static_cast<int>(32 * w);
     const int64_t k = (tiles + p.grid * w - 1) / (p.grid * w);
     const size_t need = static_cast<size_t>(w * k) * tile_bytes;
+    p.node_width = width(p);
+    K grid_kernel = p.node_width == 1 ? grid_kernel_1 : grid_kernel_2;
     int nb = 0;
     if (need > kRunSmemMax ||
         cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
