@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
 // on the forces; such a run sums its kinetic energy once, at its end.
 template <int W>
 struct NodeRowsF64 {
-    double im[W], v[3][W], u[3][W], x[3][W];
+    double im[W], rim[W], v[3][W], u[3][W], x[3][W];  // rim: 1 / im, under gravity
     uint32_t code;
 };
 template <int W>
@@ -910,6 +910,10 @@ __device__ __forceinline__ void node_rows_load(const NodeView& N, const int64_t 
         ld_row<W>(static_cast<const double*>(N.v) + c * N.np + n0, r.v[c]);
         ld_row<W>(N.u + c * N.np + n0, r.u[c]);
         ld_row<W>(N.x + c * N.np + n0, r.x[c]);
+    }
+    if (N.gravity_on) {
+#pragma unroll
+        for (int j = 0; j < W; ++j) r.rim[j] = 1.0 / r.im[j];
     }
 }
 
@@ -994,7 +998,9 @@ __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i,
             double a = f[c][j];
             double g = 0.0;
             if (N.gravity_on) {
-                g = amp * N.gravity_value * N.gravity_dir[c] / im[j];
+                const double w = amp * N.gravity_value * N.gravity_dir[c];
+                if constexpr (PRE) g = div_by(w, im[j], pre->rim[j]);
+                else g = w / im[j];
                 a = a + g;
             }
             const uint32_t cc = (code >> (8 * j + 2 * c)) & 3u;
