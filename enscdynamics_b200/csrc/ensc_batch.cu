@@ -4,7 +4,7 @@
 // Instances are sub-allocated from a CUDA memory pool owned by the batch (the
 // arena, bounded by a byte budget); each keeps the single-instance layout of
 // ensc_instance.h in its block.  A device table of instance descriptors and
-// two tile lists (32-element and 32-node tiles, each inside one instance)
+// two tile lists (element tiles and node tiles, each inside one instance)
 // drive one persistent launch per phase for all instances, each with its own
 // clock, dt and material.  The cycle is captured once as a CUDA graph; adding
 // or removing instances rewrites the tables in place, so the graph stays
@@ -32,7 +32,7 @@ struct Slot {
     bool used = false;
     void* block = nullptr;
     size_t bytes = 0;
-    int64_t nn = 0, ne = 0, nn_pad = 0, ne_pad = 0;
+    int64_t nn = 0, ne = 0, nn_pad = 0;
     bool plastic = false;
     ensc::ElemArrays E{};
     ensc::NodeArrays N{};
@@ -50,7 +50,6 @@ struct Slot {
 // and threads per block of the node pass.
 struct Tune {
     int mult_e = 1, mult_n = 1, chunk = 32, node_threads = ensc::kNodeThreads;
-    int ept = 1;  // elements per thread of the element pass
 };
 
 }  // namespace
@@ -105,8 +104,7 @@ struct ensc_batch {
     int64_t tune_etiles = 0;
     int tunings = 0;  // completed tunings
     cudaGraphExec_t graph = nullptr;
-    int graph_chunk = 0, graph_ge = 0, graph_gn = 0, graph_nt = 0, graph_ept = 0;
-    int occ_e2 = 1;  // resident element-pass blocks per SM at 2 elements per thread (mixed)
+    int graph_chunk = 0, graph_ge = 0, graph_gn = 0, graph_nt = 0, graph_room = 0;
     std::string err;
 };
 
@@ -181,8 +179,7 @@ int rebuild_tables(ensc_batch* b) {
     std::vector<ensc::NodeView> views(static_cast<size_t>(b->slots));
     std::vector<int32_t> ei, eb, ni, nb;
     std::vector<ensc::ETileSrc> es;
-    const int64_t real = is_mixed(b) ? 4 : 8;
-    int used_slots = 0;
+    int used_slots = 0, room = is_mixed(b) ? 0 : static_cast<int>(ensc::Fp64Tile9::kBytes);
     for (int s = 0; s < b->slots; ++s) {
         const Slot& sl = b->inst[s];
         ensc::InstanceDesc& d = desc[s];
@@ -201,6 +198,7 @@ int rebuild_tables(ensc_batch* b) {
             ensc::set_mixed_consts(d.M);
         }
         d.active = 1;
+        if (!is_mixed(b)) room = std::max(room, static_cast<int>(sl.E.tile_bytes));
         d.patch = sl.PA.pf ? 1 : 0;
         d.pa = sl.PA;
         views[s] = ensc::node_view(d.E, d.N, d.M, d.ctl, &sl.PA);
@@ -209,18 +207,9 @@ int rebuild_tables(ensc_batch* b) {
             ei.push_back(s);
             eb.push_back(static_cast<int32_t>(e));
             const ensc::ElemArrays& E = sl.E;
-            auto at = [e](const void* p, int64_t size) { return static_cast<const void*>(static_cast<const char*>(p) + e * size); };
             ensc::ETileSrc t{};
-            t.conn = at(E.conn, 4);
-            t.bt = at(E.bt, real);
-            t.vol0 = at(E.vol0, 8);
-            t.cbrt_v0 = at(E.cbrt_v0, real);  // mixed: a float copy in the first words
-            t.cbrt_v0sq = at(E.cbrt_v0sq, 8);
-            t.sigma = at(E.sigma, real);
-            t.qia = at(E.qia, real);
-            t.eps_p = at(E.eps_p, real);
-            t.ne_pad = static_cast<int32_t>(E.ne_pad);
-            t.cnt = static_cast<int32_t>(std::min<int64_t>(E.ne_pad - e, b->etile));
+            t.tile = reinterpret_cast<const unsigned char*>(E.conn) + e / 32 * E.tile_bytes;
+            t.bytes = static_cast<int32_t>(std::min<int64_t>(E.ne_pad - e, b->etile) / 32 * E.tile_bytes);
             t.slot = s;
             t.base = static_cast<int32_t>(e);
             es.push_back(t);
@@ -256,16 +245,20 @@ int rebuild_tables(ensc_batch* b) {
     BCK(b, cudaStreamSynchronize(b->stream));
     b->n_etiles = static_cast<int64_t>(ei.size());
     b->n_ntiles = static_cast<int64_t>(ni.size());
+    if (room != b->T.tile_room) {
+        b->T.tile_room = room;
+        if (!is_mixed(b)) b->occ_e = std::max(1, ensc::occupancy_element_batch_fp64(room));
+    }
     b->dirty = false;
     return ENSC_OK;
 }
 
-void launch_cycle(ensc_batch* b, int ge, int gn, int nt, int ept, cudaStream_t st) {
+void launch_cycle(ensc_batch* b, int ge, int gn, int nt, cudaStream_t st) {
     ensc::launch_between_batch(b->T, b->slots, 0, st);
     ensc::launch_edge_prepass_batch(b->T, b->sms * b->occ_pre, st);
     if (is_mixed(b)) {
         const bool patch = b->assembly == ENSC_ASSEMBLY_PATCH;
-        ensc::launch_element_batch_mixed(b->T, ge, ept, patch, st);
+        ensc::launch_element_batch_mixed(b->T, ge, patch, st);
         ensc::launch_node_batch_mixed(b->T, gn, nt, patch, st);
     } else {
         ensc::launch_element_batch_fp64(b->T, ge, st);
@@ -280,10 +273,10 @@ int occupancy_node(ensc_batch* b, int threads) {
 
 int build_graph(ensc_batch* b, const Tune& t) {
     const int nt = t.node_threads;
-    const int ge = b->sms * (t.ept == 2 ? b->occ_e2 : b->occ_e) * t.mult_e;
+    const int ge = b->sms * b->occ_e * t.mult_e;
     const int gn = b->sms * occupancy_node(b, nt) * t.mult_n;
     if (b->graph && b->graph_chunk == t.chunk && b->graph_ge == ge && b->graph_gn == gn && b->graph_nt == nt &&
-        b->graph_ept == t.ept)
+        b->graph_room == b->T.tile_room)
         return ENSC_OK;
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -291,7 +284,7 @@ int build_graph(ensc_batch* b, const Tune& t) {
     }
     cudaGraph_t g = nullptr;
     BCK(b, cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
-    for (int c = 0; c < t.chunk; ++c) launch_cycle(b, ge, gn, nt, t.ept, b->cap_stream);
+    for (int c = 0; c < t.chunk; ++c) launch_cycle(b, ge, gn, nt, b->cap_stream);
     cudaError_t e = cudaStreamEndCapture(b->cap_stream, &g);
     if (e != cudaSuccess) return bcuda(b, "cudaStreamEndCapture", e);
     e = cudaGraphInstantiate(&b->graph, g, 0);
@@ -301,32 +294,23 @@ int build_graph(ensc_batch* b, const Tune& t) {
     b->graph_ge = ge;
     b->graph_gn = gn;
     b->graph_nt = nt;
-    b->graph_ept = t.ept;
+    b->graph_room = b->T.tile_room;
     return ENSC_OK;
 }
 
-// Picks the launch geometry (grid sizes, node-pass block size, elements per
-// thread of the mixed element pass) and graph length with the shortest time
-// per cycle on the batch as loaded.  The candidates differ only in how work
-// is spread over the GPU, not in arithmetic, so the cycles they run are
-// ordinary cycles of the solve (the state is identical whichever wins; the
-// energy sums are grouped per warp, so with 2 elements per thread they may
-// differ in the last bits).  Each candidate runs one warm-up
-// graph launch and one timed launch; a run too short for the next candidate
-// continues with the best so far, and the next run goes on from there.
-constexpr int kTuneCands = 9;
+// Picks the launch geometry (grid sizes, node-pass block size) and graph length
+// with the shortest time per cycle on the batch as loaded.  The candidates
+// differ only in how work is spread over the GPU, not in arithmetic, so the
+// cycles they run are ordinary cycles of the solve (the state is identical
+// whichever wins).  Each candidate runs one warm-up graph launch and one timed
+// launch; a run too short for the next candidate continues with the best so
+// far, and the next run goes on from there.
+constexpr int kTuneCands = 7;
 Tune tune_candidate(int i) {
     constexpr int kN = ensc::kNodeThreads;
-    const Tune cand[kTuneCands] = {{1, 1, 32, kN, 1},     {2, 1, 32, kN, 1},     {1, 2, 32, kN, 1},
-                                   {2, 2, 32, kN, 1},     {1, 1, 32, kN / 2, 1}, {1, 2, 32, kN / 2, 1},
-                                   {1, 1, 8, kN, 1},      {1, 1, 32, kN, 2},     {2, 1, 32, kN, 2}};
+    const Tune cand[kTuneCands] = {{1, 1, 32, kN},     {2, 1, 32, kN},     {1, 2, 32, kN}, {2, 2, 32, kN},
+                                   {1, 1, 32, kN / 2}, {1, 2, 32, kN / 2}, {1, 1, 8, kN}};
     return cand[i];
-}
-
-// 2 elements per thread: mixed precision, slot assembly (the patch sums take
-// one element per thread)
-bool candidate_applies(const ensc_batch* b, const Tune& t) {
-    return t.ept == 1 || (is_mixed(b) && b->assembly != ENSC_ASSEMBLY_PATCH);
 }
 
 int autotune(ensc_batch* b, int64_t* cycles_left) {
@@ -336,7 +320,6 @@ int autotune(ensc_batch* b, int64_t* cycles_left) {
     int rc = ENSC_OK;
     for (; b->tune_next < kTuneCands; ++b->tune_next) {
         Tune t = tune_candidate(b->tune_next);
-        if (!candidate_applies(b, t)) continue;
         if (b->fixed_chunk > 0) t.chunk = b->fixed_chunk;
         if (*cycles_left < 2 * t.chunk) break;
         rc = build_graph(b, t);
@@ -407,7 +390,7 @@ int ensc_batch_create(const ensc_params* params, int32_t max_instances, int64_t 
     b->budget = budget_bytes;
     b->slots = max_instances;
     // tiles: every instance rounds its element and node counts up to tiles
-    b->etile = ensc::batch_element_tile(params->precision == ENSC_MIXED);
+    b->etile = ensc::batch_element_tile(params->assembly == ENSC_ASSEMBLY_PATCH);
     b->ntile = ensc::batch_node_tile(params->precision == ENSC_MIXED);
     b->max_etiles = max_elements / b->etile + max_instances + 1;
     b->max_ntiles = max_nodes / b->ntile + max_instances + 1;
@@ -424,8 +407,7 @@ int ensc_batch_create(const ensc_params* params, int32_t max_instances, int64_t 
     cudaDeviceProp prop{};
     if (cudaGetDeviceProperties(&prop, b->device) != cudaSuccess) return fail(berr(b, ENSC_ERR_CUDA, "device query"));
     b->sms = prop.multiProcessorCount;
-    b->occ_e = std::max(1, is_mixed(b) ? ensc::occupancy_element_batch_mixed(1) : ensc::occupancy_element_batch_fp64());
-    b->occ_e2 = std::max(1, is_mixed(b) ? ensc::occupancy_element_batch_mixed(2) : 1);
+    if (is_mixed(b)) b->occ_e = std::max(1, ensc::occupancy_element_batch_mixed(b->assembly == ENSC_ASSEMBLY_PATCH));
     // arena: a memory pool that keeps released blocks for reuse
     cudaMemPoolProps pp{};
     pp.allocType = cudaMemAllocationTypePinned;
@@ -627,7 +609,6 @@ int ensc_batch_add_prepared(ensc_batch* b, const ensc_prepared* prep, const ensc
     sl.nn = ih.nn;
     sl.ne = ih.ne;
     sl.nn_pad = ih.nn_pad;
-    sl.ne_pad = ih.ne_pad;
     sl.plastic = ih.plastic;
     sl.kinetic0_done = false;
     ensc::material_from(mat, controls, sl.M);
@@ -807,18 +788,11 @@ int ensc_batch_download(ensc_batch* b, int32_t slot, double* x, double* u, doubl
     struct Item {
         double* dst;
         const void* src;
-        int64_t n, pad;
+        int64_t n;
         int comps;
-        bool f32;
-        const int32_t* at;
     };
-    const int32_t* ep = sl.PA.iperm;  // element fields: stored positions
-    const Item items[] = {{x, sl.N.x, sl.nn, sl.nn_pad, 3, false, nullptr},
-                          {u, sl.N.u, sl.nn, sl.nn_pad, 3, false, nullptr},
-                          {v, sl.N.v, sl.nn, sl.nn_pad, 3, mx, nullptr},
-                          {sigma, sl.E.sigma, sl.ne, sl.ne_pad, 6, mx, ep},
-                          {qia, sl.E.qia, sl.ne, sl.ne_pad, 12, mx, ep},
-                          {eps_p, sl.E.eps_p, sl.ne, sl.ne_pad, 1, mx, ep}};
+    const Item items[] = {{x, sl.N.x, sl.nn, 3},          {u, sl.N.u, sl.nn, 3},      {v, sl.N.v, sl.nn, 3},
+                          {sigma, sl.E.sigma, sl.ne, 6}, {qia, sl.E.qia, sl.ne, 12}, {eps_p, sl.E.eps_p, sl.ne, 1}};
     const size_t need = static_cast<size_t>(std::max<int64_t>(12 * sl.ne, 3 * sl.nn)) * sizeof(double);
     double* stage = nullptr;
     BCK(b, cudaMallocFromPoolAsync(reinterpret_cast<void**>(&stage), need, b->pool, b->stream));
@@ -828,7 +802,10 @@ int ensc_batch_download(ensc_batch* b, int32_t slot, double* x, double* u, doubl
         if (it.src == sl.N.v) ensc::launch_v_to_aos(sl.N, mx, stage, b->stream);
         else if (it.src == sl.N.u && mx && ENSC_MIXED_UREF)
             ensc::launch_disp_to_aos(sl.N.x, sl.N.u, sl.nn, sl.nn_pad, stage, b->stream);
-        else ensc::launch_soa_to_aos(it.src, it.n, it.pad, it.comps, it.f32, stage, b->stream, it.at);
+        else if (it.src == sl.N.x || it.src == sl.N.u)
+            ensc::launch_soa_to_aos(static_cast<const double*>(it.src), sl.nn, sl.nn_pad, 3, stage, b->stream);
+        else  // element fields, at their stored positions
+            ensc::launch_elem_to_aos(sl.E, it.src, it.comps, mx, stage, b->stream, sl.PA.iperm);
         cudaError_t e = cudaMemcpyAsync(it.dst, stage, it.n * it.comps * sizeof(double), cudaMemcpyDeviceToHost,
                                         b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
@@ -881,7 +858,7 @@ int ensc_batch_tuning(const ensc_batch* b, int32_t* mult_element, int32_t* mult_
     if (mult_node) *mult_node = t ? b->tune.mult_n : 0;
     if (graph_cycles) *graph_cycles = t ? b->tune.chunk : 0;
     if (node_threads) *node_threads = t ? b->tune.node_threads : 0;
-    if (elements_per_thread) *elements_per_thread = t ? b->tune.ept : 0;
+    if (elements_per_thread) *elements_per_thread = t ? 1 : 0;
     if (assembly) *assembly = b->assembly == ENSC_ASSEMBLY_PATCH ? ENSC_ASSEMBLY_PATCH : ENSC_ASSEMBLY_SLOT;
     return ENSC_OK;
 }

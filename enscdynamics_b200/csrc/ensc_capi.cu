@@ -33,7 +33,7 @@ struct ensc_handle {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaStream_t cap_stream = nullptr;
-    int64_t nn = 0, ne = 0, nn_pad = 0, ne_pad = 0;
+    int64_t nn = 0, ne = 0, nn_pad = 0;
     void* arena = nullptr;
     size_t arena_bytes = 0;
     double* staging = nullptr;     // device AoS staging for up/download
@@ -256,7 +256,6 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
     h->nn = ih.nn;
     h->ne = ih.ne;
     h->nn_pad = ih.nn_pad;
-    h->ne_pad = ih.ne_pad;
     h->chunk = params->graph_chunk > 0 ? params->graph_chunk : 32;
     DevGuard dg(h->device);
     auto fail = [&](int code) {
@@ -271,7 +270,7 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
         set_err(h, ENSC_ERR_CUDA, "cudaGetDeviceProperties failed");
         return fail(ENSC_ERR_CUDA);
     }
-    const int occ_e = std::max(1, mx ? ensc::occupancy_element_mixed(h->plastic) : ensc::occupancy_element_fp64(h->plastic));
+    const int occ_e = std::max(1, mx ? ensc::occupancy_element_mixed(h->plastic, ih.patch) : ensc::occupancy_element_fp64(h->plastic, ih.bt9));
     const int occ_n = std::max(1, mx ? ensc::occupancy_node_mixed() : ensc::occupancy_node_fp64());
     const int64_t ge = (h->ne + ensc::kElemThreads - 1) / ensc::kElemThreads;
     const int64_t node_threads = static_cast<int64_t>(ensc::kNodeThreads) * ensc::node_group_width(mx);
@@ -282,7 +281,7 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
     // resident runs where the mesh fits on chip (slot assembly)
     if (!ih.patch && prop.cooperativeLaunch)
         h->run = mx ? ensc::plan_run_mixed(h->ne, h->nn, h->plastic, prop.multiProcessorCount)
-                    : ensc::plan_run_fp64(h->ne, h->nn, h->plastic, prop.multiProcessorCount);
+                    : ensc::plan_run_fp64(h->ne, h->nn, h->plastic, ih.bt9, prop.multiProcessorCount);
 
     // ---- device memory: the instance block plus partial sums and control ----
     // (one partial slot per block of the larger of the two launch forms)
@@ -509,26 +508,22 @@ int ensc_download(ensc_handle* h, double* x, double* u, double* v, double* sigma
     struct Item {
         double* dst;
         const void* src;
-        int64_t n, pad;
+        int64_t n;
         int comps;
-        bool f32;
-        const int32_t* at;
     };
     const bool mx = mixed(h);
-    const int32_t* ep = h->PA.iperm;  // element fields: stored positions
-    const Item items[] = {{x, h->N.x, h->nn, h->nn_pad, 3, false, nullptr},
-                          {u, h->N.u, h->nn, h->nn_pad, 3, false, nullptr},
-                          {v, h->N.v, h->nn, h->nn_pad, 3, mx, nullptr},
-                          {sigma, h->E.sigma, h->ne, h->ne_pad, 6, mx, ep},
-                          {qia, h->E.qia, h->ne, h->ne_pad, 12, mx, ep},
-                          {eps_p, h->E.eps_p, h->ne, h->ne_pad, 1, mx, ep}};
+    const Item items[] = {{x, h->N.x, h->nn, 3},          {u, h->N.u, h->nn, 3},      {v, h->N.v, h->nn, 3},
+                          {sigma, h->E.sigma, h->ne, 6}, {qia, h->E.qia, h->ne, 12}, {eps_p, h->E.eps_p, h->ne, 1}};
     size_t used = 0;
     for (const Item& it : items) {
         if (!it.dst) continue;
         if (it.src == h->N.v) ensc::launch_v_to_aos(h->N, mx, h->staging, h->stream);
         else if (it.src == h->N.u && mx && ENSC_MIXED_UREF)
             ensc::launch_disp_to_aos(h->N.x, h->N.u, h->nn, h->nn_pad, h->staging, h->stream);
-        else ensc::launch_soa_to_aos(it.src, it.n, it.pad, it.comps, it.f32, h->staging, h->stream, it.at);
+        else if (it.src == h->N.x || it.src == h->N.u)
+            ensc::launch_soa_to_aos(static_cast<const double*>(it.src), h->nn, h->nn_pad, 3, h->staging, h->stream);
+        else  // element fields, at their stored positions
+            ensc::launch_elem_to_aos(h->E, it.src, it.comps, mx, h->staging, h->stream, h->PA.iperm);
         CK(h, cudaGetLastError());
         CK(h, cudaMemcpyAsync(it.dst, h->staging, it.n * it.comps * sizeof(double), cudaMemcpyDeviceToHost,
                               h->stream));
@@ -541,7 +536,7 @@ int ensc_download(ensc_handle* h, double* x, double* u, double* v, double* sigma
 int ensc_download_reactions(ensc_handle* h, double* rf) {
     if (!h || !rf) return ENSC_ERR_ARG;
     DevGuard dg(h->device);
-    ensc::launch_soa_to_aos(h->N.rf, h->nn, h->nn_pad, 3, false, h->staging, h->stream);
+    ensc::launch_soa_to_aos(h->N.rf, h->nn, h->nn_pad, 3, h->staging, h->stream);
     CK(h, cudaGetLastError());
     CK(h, cudaMemcpyAsync(rf, h->staging, h->nn * 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -556,19 +551,12 @@ int ensc_upload_state(ensc_handle* h, const double* x, const double* u, const do
     struct Item {
         const double* src;
         void* dst;
-        int64_t n, pad;
+        int64_t n;
         int comps;
-        bool f32;
-        const int32_t* at;
     };
     const bool mx = mixed(h);
-    const int32_t* ep = h->PA.iperm;  // element fields: stored positions
-    const Item items[] = {{x, h->N.x, h->nn, h->nn_pad, 3, false, nullptr},
-                          {u, h->N.u, h->nn, h->nn_pad, 3, false, nullptr},
-                          {v, h->N.v, h->nn, h->nn_pad, 3, mx, nullptr},
-                          {sigma, h->E.sigma, h->ne, h->ne_pad, 6, mx, ep},
-                          {qia, h->E.qia, h->ne, h->ne_pad, 12, mx, ep},
-                          {eps_p, h->E.eps_p, h->ne, h->ne_pad, 1, mx, ep}};
+    const Item items[] = {{x, h->N.x, h->nn, 3},          {u, h->N.u, h->nn, 3},      {v, h->N.v, h->nn, 3},
+                          {sigma, h->E.sigma, h->ne, 6}, {qia, h->E.qia, h->ne, 12}, {eps_p, h->E.eps_p, h->ne, 1}};
     size_t used = 0;
     // mixed: the u rows hold x - u; they hold u while x and u are replaced
     const bool uref = mx && ENSC_MIXED_UREF && (x || u);
@@ -584,7 +572,10 @@ int ensc_upload_state(ensc_handle* h, const double* x, const double* u, const do
             break;
         }
         if (it.dst == h->N.v) ensc::launch_aos_to_v(h->staging, h->N, mx, h->stream);
-        else ensc::launch_aos_to_soa(h->staging, it.n, it.pad, it.comps, it.dst, it.f32, h->stream, it.at);
+        else if (it.dst == h->N.x || it.dst == h->N.u)
+            ensc::launch_aos_to_soa(h->staging, h->nn, h->nn_pad, 3, static_cast<double*>(it.dst), h->stream);
+        else
+            ensc::launch_aos_to_elem(h->staging, h->E, it.comps, it.dst, mx, h->stream, h->PA.iperm);
         ue = cudaGetLastError();
         used = std::max(used, static_cast<size_t>(it.n * it.comps) * sizeof(double));
     }
@@ -645,12 +636,12 @@ int ensc_snapshot_begin(ensc_handle* h) {
     const bool mx = mixed(h);
     if (mx) ensc::launch_acceleration_mixed(h->E, h->N, h->M, h->ctl, d + 3 * nodes3, h->stream, h->PA);
     else ensc::launch_acceleration_fp64(h->E, h->N, h->M, h->ctl, d + 3 * nodes3, h->stream);
-    ensc::launch_soa_to_aos(h->N.x, h->nn, h->nn_pad, 3, false, d, h->stream);
+    ensc::launch_soa_to_aos(h->N.x, h->nn, h->nn_pad, 3, d, h->stream);
     if (mx && ENSC_MIXED_UREF) ensc::launch_disp_to_aos(h->N.x, h->N.u, h->nn, h->nn_pad, d + nodes3, h->stream);
-    else ensc::launch_soa_to_aos(h->N.u, h->nn, h->nn_pad, 3, false, d + nodes3, h->stream);
+    else ensc::launch_soa_to_aos(h->N.u, h->nn, h->nn_pad, 3, d + nodes3, h->stream);
     ensc::launch_v_to_aos(h->N, mx, d + 2 * nodes3, h->stream);
-    ensc::launch_soa_to_aos(h->N.rf, h->nn, h->nn_pad, 3, false, d + 4 * nodes3, h->stream);
-    ensc::launch_soa_to_aos(h->E.sigma, h->ne, h->ne_pad, 6, mx, d + 5 * nodes3, h->stream, h->PA.iperm);
+    ensc::launch_soa_to_aos(h->N.rf, h->nn, h->nn_pad, 3, d + 4 * nodes3, h->stream);
+    ensc::launch_elem_to_aos(h->E, h->E.sigma, 6, mx, d + 5 * nodes3, h->stream, h->PA.iperm);
     CK(h, cudaGetLastError());
     char* ctl_copy = reinterpret_cast<char*>(d) + (h->snap_bytes - sizeof(Ctl));
     CK(h, cudaMemcpyAsync(ctl_copy, h->ctl, sizeof(Ctl), cudaMemcpyDeviceToDevice, h->stream));

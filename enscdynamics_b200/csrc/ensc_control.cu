@@ -84,6 +84,21 @@ __global__ void __launch_bounds__(kCtlThreads) k_between(Ctl* ctl, Partials P, i
     cycle_begin(ctl);
 }
 
+// Minimum squared edge of element e from the current coordinates.
+__device__ __forceinline__ double element_edge_sq(const ElemArrays& E, const NodeArrays& N, int64_t np, int64_t e) {
+    const uint32_t* cn = tile_row(E, E.conn, e) + (e & 31);
+    const int64_t cs = tile_stride(E);
+    double xyz[8][3];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t n = cn[k * cs];
+        xyz[k][0] = N.x[n];
+        xyz[k][1] = N.x[np + n];
+        xyz[k][2] = N.x[2 * np + n];
+    }
+    return min_edge_sq(xyz);
+}
+
 // Minimum element edge over the current coordinates (min_ele_edge,
 // exDyna3D.cpp:1173-1220), needed before the element pass only in a cycle
 // where the total-time clamp may fire; the last block then applies the clamp
@@ -91,29 +106,11 @@ __global__ void __launch_bounds__(kCtlThreads) k_between(Ctl* ctl, Partials P, i
 __global__ void __launch_bounds__(128) k_edge_prepass(ElemArrays E, NodeArrays N, Ctl* ctl) {
     if (ctl->done || !ctl->need_exact) return;
     __shared__ unsigned long long red[4];
-    const int64_t ep = E.ne_pad, np = N.nn_pad;
+    const int64_t np = N.nn_pad;
     double m = DBL_MAX;
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < E.ne;
          e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        double xyz[8][3];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t n = E.conn[k * ep + e];
-            xyz[k][0] = N.x[n];
-            xyz[k][1] = N.x[np + n];
-            xyz[k][2] = N.x[2 * np + n];
-        }
-        constexpr int A0[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3};
-        constexpr int A1[12] = {1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7};
-        double mm = DBL_MAX;
-#pragma unroll
-        for (int k = 0; k < 12; ++k) {
-            const double dx = xyz[A1[k]][0] - xyz[A0[k]][0];
-            const double dy = xyz[A1[k]][1] - xyz[A0[k]][1];
-            const double dz = xyz[A1[k]][2] - xyz[A0[k]][2];
-            const double t = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));  // as the element pass
-            mm = t < mm ? t : mm;
-        }
+        const double mm = element_edge_sq(E, N, np, e);
         const double len = sqrt(mm);
         m = len < m ? len : m;
     }
@@ -213,15 +210,22 @@ __global__ void __launch_bounds__(kNodeThreads) k_kinetic(NodeArrays N, Partials
     }
 }
 
-// Entry e of the interleaved array is row position at[e] of the SoA rows
-// (at null: e).
+// Component c of entry s: rows of `pad` entries, or rows of 32 in tiles `tile`
+// entries apart (the element arrays).
+__device__ __forceinline__ int64_t row_entry(int64_t s, int c, int64_t pad, int64_t tile) {
+    return tile ? (s >> 5) * tile + c * 32 + (s & 31) : c * pad + s;
+}
+
+// Entry e of the interleaved array is row position at[e] of the rows (at
+// null: e).
 template <typename ST>
-__global__ void k_soa_to_aos(const ST* soa, int64_t n, int64_t pad, int comps, const int32_t* at, double* aos) {
+__global__ void k_soa_to_aos(const ST* soa, int64_t n, int64_t pad, int64_t tile, int comps, const int32_t* at,
+                             double* aos) {
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n * comps;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int64_t e = i / comps;
         const int c = static_cast<int>(i - e * comps);
-        aos[i] = static_cast<double>(soa[c * pad + (at ? at[e] : e)]);
+        aos[i] = static_cast<double>(soa[row_entry(at ? at[e] : e, c, pad, tile)]);
     }
 }
 
@@ -262,12 +266,13 @@ __global__ void k_aos_to_v(const double* aos, NodeArrays N) {
 }
 
 template <typename DT>
-__global__ void k_aos_to_soa(const double* aos, int64_t n, int64_t pad, int comps, const int32_t* at, DT* soa) {
+__global__ void k_aos_to_soa(const double* aos, int64_t n, int64_t pad, int64_t tile, int comps, const int32_t* at,
+                             DT* soa) {
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n * comps;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int64_t e = i / comps;
         const int c = static_cast<int>(i - e * comps);
-        soa[c * pad + (at ? at[e] : e)] = static_cast<DT>(aos[i]);
+        soa[row_entry(at ? at[e] : e, c, pad, tile)] = static_cast<DT>(aos[i]);
     }
 }
 
@@ -346,26 +351,7 @@ __global__ void __launch_bounds__(128) k_edge_prepass_batch(BatchTables T) {
         const int64_t end = base + T.etile < d.E.ne ? base + T.etile : d.E.ne;
         double m = DBL_MAX;
         for (int64_t e = base + lane; e < end; e += 32) {
-            const int64_t ep = d.E.ne_pad, np = d.N.nn_pad;
-            double xyz[8][3];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint32_t n = d.E.conn[k * ep + e];
-                xyz[k][0] = d.N.x[n];
-                xyz[k][1] = d.N.x[np + n];
-                xyz[k][2] = d.N.x[2 * np + n];
-            }
-            constexpr int A0[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3};
-            constexpr int A1[12] = {1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7};
-            double mm = DBL_MAX;
-#pragma unroll
-            for (int k = 0; k < 12; ++k) {
-                const double dx = xyz[A1[k]][0] - xyz[A0[k]][0];
-                const double dy = xyz[A1[k]][1] - xyz[A0[k]][1];
-                const double dz = xyz[A1[k]][2] - xyz[A0[k]][2];
-                const double tt = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));  // as the element pass
-                mm = tt < mm ? tt : mm;
-            }
+            const double mm = element_edge_sq(d.E, d.N, d.N.nn_pad, e);
             const double len = sqrt(mm);
             m = len < m ? len : m;
         }
@@ -435,11 +421,18 @@ void launch_kinetic0(const NodeArrays& N, const Partials& P, Ctl* ctl, bool fp32
     else k_kinetic<double><<<grid, kNodeThreads, 0, st>>>(N, P);
     k_between<<<1, kCtlThreads, 0, st>>>(ctl, P, 2);
 }
-void launch_soa_to_aos(const void* soa, int64_t n, int64_t pad, int comps, bool src_fp32, double* aos,
-                       cudaStream_t st, const int32_t* at) {
-    const int g = grid_for(n * comps, 256);
-    if (src_fp32) k_soa_to_aos<float><<<g, 256, 0, st>>>(static_cast<const float*>(soa), n, pad, comps, at, aos);
-    else k_soa_to_aos<double><<<g, 256, 0, st>>>(static_cast<const double*>(soa), n, pad, comps, at, aos);
+void launch_soa_to_aos(const double* soa, int64_t n, int64_t pad, int comps, double* aos, cudaStream_t st) {
+    k_soa_to_aos<double><<<grid_for(n * comps, 256), 256, 0, st>>>(soa, n, pad, 0, comps, nullptr, aos);
+}
+void launch_elem_to_aos(const ElemArrays& E, const void* rows, int comps, bool src_fp32, double* aos, cudaStream_t st,
+                        const int32_t* at) {
+    const int g = grid_for(E.ne * comps, 256);
+    if (src_fp32)
+        k_soa_to_aos<float><<<g, 256, 0, st>>>(static_cast<const float*>(rows), E.ne, 0, E.tile_bytes / 4, comps, at,
+                                               aos);
+    else
+        k_soa_to_aos<double><<<g, 256, 0, st>>>(static_cast<const double*>(rows), E.ne, 0, E.tile_bytes / 8, comps, at,
+                                                aos);
 }
 void launch_disp_to_aos(const double* x, const double* xr, int64_t n, int64_t pad, double* aos, cudaStream_t st) {
     k_disp_to_aos<<<grid_for(3 * n, 256), 256, 0, st>>>(x, xr, n, pad, aos);
@@ -457,11 +450,16 @@ void launch_aos_to_v(const double* aos, const NodeArrays& N, bool fp32_v, cudaSt
     if (fp32_v) k_aos_to_v<float><<<g, 256, 0, st>>>(aos, N);
     else k_aos_to_v<double><<<g, 256, 0, st>>>(aos, N);
 }
-void launch_aos_to_soa(const double* aos, int64_t n, int64_t pad, int comps, void* soa, bool dst_fp32,
-                       cudaStream_t st, const int32_t* at) {
-    const int g = grid_for(n * comps, 256);
-    if (dst_fp32) k_aos_to_soa<float><<<g, 256, 0, st>>>(aos, n, pad, comps, at, static_cast<float*>(soa));
-    else k_aos_to_soa<double><<<g, 256, 0, st>>>(aos, n, pad, comps, at, static_cast<double*>(soa));
+void launch_aos_to_soa(const double* aos, int64_t n, int64_t pad, int comps, double* soa, cudaStream_t st) {
+    k_aos_to_soa<double><<<grid_for(n * comps, 256), 256, 0, st>>>(aos, n, pad, 0, comps, nullptr, soa);
+}
+void launch_aos_to_elem(const double* aos, const ElemArrays& E, int comps, void* rows, bool dst_fp32, cudaStream_t st,
+                        const int32_t* at) {
+    const int g = grid_for(E.ne * comps, 256);
+    if (dst_fp32)
+        k_aos_to_soa<float><<<g, 256, 0, st>>>(aos, E.ne, 0, E.tile_bytes / 4, comps, at, static_cast<float*>(rows));
+    else
+        k_aos_to_soa<double><<<g, 256, 0, st>>>(aos, E.ne, 0, E.tile_bytes / 8, comps, at, static_cast<double*>(rows));
 }
 
 }  // namespace ensc

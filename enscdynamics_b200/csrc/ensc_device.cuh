@@ -1,12 +1,18 @@
 // Device-side data structures shared by the stepper kernels.
 //
-// Memory layout in HBM (structure of arrays, one array per component so a
-// warp of consecutive elements / nodes reads consecutive words):
-//   element arrays, length ne (padded stride ne_pad):
-//     conn[8][ne_pad] uint32         local node k of element e at conn[k*ne_pad + e]
-//     bt[24][ne_pad]                 B0^T row-major per element: (3*k + c)
-//     vol0, cbrt_v0, cbrt_v0sq [ne]  per-element constants
-//     sigma[6][ne_pad], qia[12][ne_pad], eps_p[ne]
+// Memory layout in HBM:
+//   element arrays: one tile of 32 consecutive elements after another
+//   (ElemTile below); within a tile every component is a row of 32 entries, so
+//   a warp of consecutive elements reads consecutive words, and a whole tile
+//   is one contiguous copy.  Instances on caller-owned memory (ensc_step_noalloc) keep
+//   plain rows of ne entries per component instead (tile_bytes 0).
+//     conn[8] uint32                 local node k of the element
+//     bt                             FP64: the 9 numbers the one-point B0^T
+//                                    rows are formed from, or its 24 numbers
+//                                    row-major (3*k + c); mixed: A as 9 hi and
+//                                    9 lo floats
+//     vol0, cbrt_v0, cbrt_v0sq       per-element constants
+//     sigma[6], qia[12], eps_p
 //     fe                             element nodal forces of the current cycle
 //                                    (the element -> node hand-off, scratch):
 //                                    [24][nn_pad] by node and local slot when
@@ -109,29 +115,62 @@ inline void set_mixed_consts(Material& M) {
     c.cq2_wos = M.cvisq * M.cvisq / M.wos;
 }
 
+// Byte offsets of the rows in a tile of 32 elements: what does not change
+// first, then the evolving rows, eps_p last (elastic instances do not copy
+// it).  The tile is copied to shared memory as it is.
+template <typename Real, int kGeom, int kConsts>
+struct ElemTile {
+    static constexpr uint32_t kRow = 32u * sizeof(Real);
+    static constexpr uint32_t kConn = 0;
+    static constexpr uint32_t kBt = 8u * 32u * 4u;
+    static constexpr uint32_t kVol0 = kBt + kGeom * kRow;          // doubles
+    static constexpr uint32_t kCb = kVol0 + 32u * 8u;              // cbrt(V0) (FP64: and cbrt(V0^2))
+    static constexpr uint32_t kState = kCb + kConsts * kRow;
+    static constexpr uint32_t kSig = kState;
+    static constexpr uint32_t kQia = kSig + 6u * kRow;
+    static constexpr uint32_t kEps = kQia + 12u * kRow;
+    static constexpr uint32_t kBytes = kEps + kRow;
+};
+using MixedTile = ElemTile<float, 18, 1>;    // 6,144 bytes
+using Fp64Tile9 = ElemTile<double, 9, 2>;    // 8,960 bytes
+using Fp64Tile24 = ElemTile<double, 24, 2>;  // 12,800 bytes
+
 struct ElemArrays {
     int64_t ne, ne_pad;
     const uint32_t* conn;
     const void* bt;            // double (FP64) or float (mixed)
     const double* vol0;
-    const double* cbrt_v0;
-    const double* cbrt_v0sq;
+    const void* cbrt_v0;       // double (FP64) or float (mixed)
+    const double* cbrt_v0sq;   // FP64
     void* sigma;
     void* qia;
     void* eps_p;
     void* fe;
-    // 1 when every element and node array starts 256-byte aligned and
-    // ne_pad / nn_pad are multiples of 32: rows of whole 32-entry tiles can be
-    // bulk-copied and read as 16-byte vectors (the staged element passes and
-    // the vectorised node passes)
-    int32_t tiles_aligned;
+    // bytes of a tile of 32 elements; the pointers above point into tile 0,
+    // which starts 256-byte aligned (node rows too, padded to 32 entries: the
+    // vectorised node passes).  0: plain rows of ne_pad entries.
+    int32_t tile_bytes;
     // 1: fe is node-major, fe[(3k + c) * nn_pad + conn[k][e]] -- the
     // reference's per-local-slot nodal vectors (exDyna3D.cpp:523-634), each
     // entry written by the one element that holds the node in slot k;
     // 0: fe is element-major, fe[(3k + c) * ne_pad + e], gathered through
     // ell / csr by the node pass
     int32_t slot_major;
+    int32_t bt9;               // FP64: bt holds 9 numbers per element (else 24)
+    int32_t pad;
 };
+
+// Entry e of a component array: its rows start at tile_row(E, p, e), `stride`
+// entries apart (tile_stride), with the element at e & 31.
+template <typename T>
+__host__ __device__ inline T* tile_row(const ElemArrays& E, T* p, int64_t e) {
+    if (E.tile_bytes) {
+        using B = const char;
+        return const_cast<T*>(reinterpret_cast<const T*>(reinterpret_cast<B*>(p) + (e >> 5) * E.tile_bytes));
+    }
+    return p + (e & ~int64_t(31));
+}
+__host__ __device__ inline int64_t tile_stride(const ElemArrays& E) { return E.tile_bytes ? 32 : E.ne_pad; }
 
 // Elements per patch of the mixed patch assembly: one staged tile.
 constexpr int kPatchElems = 64;
@@ -228,7 +267,7 @@ __host__ __device__ inline NodeView node_view(const ElemArrays& E, const NodeArr
     for (int c = 0; c < 3; ++c) v.gravity_dir[c] = M.gravity_dir[c];
     v.gravity_on = M.gravity_on;
     const bool patch = pa && pa->pf;
-    v.grouped = (E.slot_major && E.tiles_aligned) ? (patch ? 2 : 1) : 0;
+    v.grouped = (E.slot_major && E.tile_bytes) ? (patch ? 2 : 1) : 0;
     if (patch) {
         v.pf = pa->pf;
         v.nptr = pa->nptr;
@@ -259,24 +298,16 @@ struct StageHdr {
     int32_t live, pad;
 };
 
-// Where the staged batch element passes copy an element tile from: the
-// instance's element rows, each pointer already at the tile's first element.
-// A tile's record travels with the stage of the tile two visits earlier, so
-// the block that copies a tile reads its record from shared memory.
+// Where the batch element passes copy an element tile from.  A tile's record
+// travels with the stage of the tile two visits earlier, so the warp that copies
+// a tile reads its record from shared memory.
 struct alignas(16) ETileSrc {
-    const void* conn;
-    const void* bt;
-    const void* vol0;
-    const void* cbrt_v0;
-    const void* cbrt_v0sq;
-    const void* sigma;
-    const void* qia;
-    const void* eps_p;
-    int32_t ne_pad;   // row stride in elements
-    int32_t cnt;      // entries copied per row (tile size, or the rest of the padded rows)
+    const void* tile;
+    int32_t bytes;    // of the tiles the pass takes at once
     int32_t slot, base;
+    int32_t pad[3];
 };
-static_assert(sizeof(ETileSrc) == 80, "tile records are bulk-copied");
+static_assert(sizeof(ETileSrc) == 32, "tile records are bulk-copied");
 
 // Written into each stage by the thread that fills it: the tile's instance
 // slot and first element.
@@ -315,8 +346,16 @@ struct BatchTables {
     const NodeView* nview;       // [slots]
     const ETileSrc* etile_src;   // [etiles] copy sources of each element tile
     int32_t etile, ntile;        // elements / nodes per tile
+    int32_t tile_room;           // bytes the stages of the element pass have for a tile
+    int32_t pad;
 };
 static_assert(sizeof(InstanceDesc) % 16 == 0, "instance descriptors are bulk-copied");
+// behind the tile in a stage of the batched element passes: the descriptor, then
+constexpr uint32_t kBatchHdrOff = sizeof(InstanceDesc);
+constexpr uint32_t kBatchInfoOff = kBatchHdrOff + sizeof(StageHdr);
+constexpr uint32_t kBatchNextOff = kBatchInfoOff + sizeof(TileInfo);
+constexpr uint32_t kBatchTailBytes = (kBatchNextOff + sizeof(ETileSrc) + 127) / 128 * 128;
+static_assert(sizeof(StageHdr) == 16 && sizeof(TileInfo) == 16, "16-byte copies");
 
 // Amplitude factor of gravity in a cycle at `time` with step dt, as
 // exDyna3D::deal_amp computes it (exDyna3D.cpp:1222-1278), behaviour kept as

@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 namespace ensc {
 namespace {
@@ -42,21 +43,6 @@ __device__ __forceinline__ void inv3(const double m[3][3], double r[3][3]) {
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) r[i][j] = cof3(m, j, i) * invdet;
-}
-
-// Hourglass base vectors Gamma (exDyna3D.cpp:1003-1008) as signs.
-__device__ __forceinline__ constexpr int tau_sign(int k, int j) {
-    constexpr int T[4][8] = {{1, -1, 1, -1, 1, -1, 1, -1},
-                             {-1, -1, 1, 1, 1, 1, -1, -1},
-                             {-1, 1, 1, -1, 1, -1, -1, 1},
-                             {-1, 1, -1, 1, 1, -1, 1, -1}};
-    return T[k][j];
-}
-
-// Gamma row k as a bit mask: bit j set where the entry is +1.
-__device__ __forceinline__ double tau_of(int k, int j) {
-    constexpr unsigned kMask = 0x55u | (0x3Cu << 8) | (0x96u << 16) | (0x5Au << 24);
-    return ((kMask >> (8 * k + j)) & 1u) ? 1.0 : -1.0;
 }
 
 template <typename T>
@@ -129,31 +115,48 @@ __device__ __forceinline__ void block_min2(double a, double b, unsigned long lon
 }
 
 // Where one element's inputs are read from: rows of `stride` entries with the
-// element at `i` (the instance's global arrays, or a shared-memory stage
-// holding a tile of them); B0^T has its own rows so that it can stay in
-// global memory while the rest is staged.
+// element at `i`, in the instance's tiles or rows in global memory or in a tile
+// in shared memory.
 struct Fp64Src {
     const uint32_t* conn;   // [8] rows
-    const double* sig;      // [6] rows
-    const double* qia;      // [12] rows
+    const double* bt;       // [9] or [24] rows
     const double* vol0;
     const double* cb;       // cbrt(V0)
     const double* cb2;      // cbrt(V0^2)
+    const double* sig;      // [6] rows
+    const double* qia;      // [12] rows
     const double* eps;
     int64_t stride, i;
-    const double* bt;       // [24] rows
-    int64_t bt_stride, bt_i;
 };
 
+// TILED: the instance's arrays are in tiles, else plain rows (ElemArrays).
+template <bool TILED>
 __device__ __forceinline__ Fp64Src fp64_src_global(const ElemArrays& E, int64_t e) {
-    return Fp64Src{E.conn, static_cast<const double*>(E.sigma), static_cast<const double*>(E.qia), E.vol0,
-                   E.cbrt_v0, E.cbrt_v0sq, static_cast<const double*>(E.eps_p), E.ne_pad, e,
-                   static_cast<const double*>(E.bt), E.ne_pad, e};
+    if constexpr (!TILED)
+        return Fp64Src{E.conn,
+                       static_cast<const double*>(E.bt),
+                       E.vol0,
+                       static_cast<const double*>(E.cbrt_v0),
+                       E.cbrt_v0sq,
+                       static_cast<const double*>(E.sigma),
+                       static_cast<const double*>(E.qia),
+                       static_cast<const double*>(E.eps_p),
+                       E.ne_pad,
+                       e};
+    return Fp64Src{tile_row(E, E.conn, e),
+                   tile_row(E, static_cast<const double*>(E.bt), e),
+                   tile_row(E, E.vol0, e),
+                   tile_row(E, static_cast<const double*>(E.cbrt_v0), e),
+                   tile_row(E, E.cbrt_v0sq, e),
+                   tile_row(E, static_cast<const double*>(E.sigma), e),
+                   tile_row(E, static_cast<const double*>(E.qia), e),
+                   tile_row(E, static_cast<const double*>(E.eps_p), e),
+                   32,
+                   e & 31};
 }
 
-// Where one element's evolving rows are written: rows of `stride` entries
-// with the element at `i` (the instance's global arrays, or the shared-memory
-// tile that a resident run keeps them in).
+// Where one element's evolving rows are written: the instance's own arrays, or
+// the shared-memory tile that a resident run keeps them in.
 struct Fp64Out {
     double* sig;            // [6] rows
     double* qia;            // [12] rows
@@ -161,25 +164,100 @@ struct Fp64Out {
     int64_t stride, i;
 };
 
+template <bool TILED>
 __device__ __forceinline__ Fp64Out fp64_out_global(const ElemArrays& E, int64_t e) {
-    return Fp64Out{static_cast<double*>(E.sigma), static_cast<double*>(E.qia), static_cast<double*>(E.eps_p), E.ne_pad,
-                   e};
+    if constexpr (!TILED)
+        return Fp64Out{static_cast<double*>(E.sigma), static_cast<double*>(E.qia), static_cast<double*>(E.eps_p),
+                       E.ne_pad, e};
+    return Fp64Out{tile_row(E, static_cast<double*>(E.sigma), e), tile_row(E, static_cast<double*>(E.qia), e),
+                   tile_row(E, static_cast<double*>(E.eps_p), e), 32, e & 31};
+}
+
+// A tile of layout L (Fp64Tile9 / Fp64Tile24) in memory: row pointers of the
+// element at `lane`.
+template <typename L>
+__device__ __forceinline__ Fp64Src fp64_src_tile(const unsigned char* t, int lane) {
+    return Fp64Src{reinterpret_cast<const uint32_t*>(t),
+                   reinterpret_cast<const double*>(t + L::kBt),
+                   reinterpret_cast<const double*>(t + L::kVol0),
+                   reinterpret_cast<const double*>(t + L::kCb),
+                   reinterpret_cast<const double*>(t + L::kCb + L::kRow),
+                   reinterpret_cast<const double*>(t + L::kSig),
+                   reinterpret_cast<const double*>(t + L::kQia),
+                   reinterpret_cast<const double*>(t + L::kEps),
+                   32,
+                   lane};
+}
+template <typename L>
+__device__ __forceinline__ Fp64Out fp64_out_tile(unsigned char* t, int lane) {
+    return Fp64Out{reinterpret_cast<double*>(t + L::kSig), reinterpret_cast<double*>(t + L::kQia),
+                   reinterpret_cast<double*>(t + L::kEps), 32, lane};
+}
+
+// The four Gamma-signed sums of 8 values, each left to right from node 0 as
+// the oracle adds them; rows that agree up to sign so far share their partial
+// sum (rounding is symmetric in sign), 24 additions instead of 28.
+__device__ __forceinline__ void gamma_sums(const double (&v)[8], double (&t)[4]) {
+    const double d = v[0] - v[1], s = v[0] + v[1], q = (d + v[2]) - v[3];
+    t[0] = (((q + v[4]) - v[5]) + v[6]) - v[7];
+    t[1] = (((((v[2] - s) + v[3]) + v[4]) + v[5]) - v[6]) - v[7];
+    t[2] = (((((v[2] - d) - v[3]) + v[4]) - v[5]) - v[6]) + v[7];
+    t[3] = (((v[4] - q) - v[5]) + v[6]) - v[7];
+}
+
+// B0^T rows of an element.  9 numbers p = J^-1 / 8: row a is
+// (+-p0 +- p1) +- p2 with the corner signs of node a, and opposite corners have
+// opposite rows, so 4 rows of 3 carry all 8.  24 numbers: as stored.
+template <bool BT9, bool SMEM>
+struct B0Rows {
+    double r[4][3];  // BT9: nodes 6, 1, 2, 5
+    __device__ __forceinline__ void load(const Fp64Src& S) {
+        const double* b = S.bt + S.i;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double p0 = ldin<SMEM>(b + (3 * c) * S.stride), p1 = ldin<SMEM>(b + (3 * c + 1) * S.stride),
+                         p2 = ldin<SMEM>(b + (3 * c + 2) * S.stride);
+            const double u = p0 + p1, w = p0 - p1;
+            r[0][c] = u + p2;
+            r[1][c] = w - p2;
+            r[2][c] = u - p2;
+            r[3][c] = w + p2;
+        }
+    }
+    // row of node j: minus(j) ? -r[index(j)] : r[index(j)]
+    __device__ static constexpr int index(int j) {
+        constexpr int k[8] = {0, 1, 2, 3, 2, 3, 0, 1};
+        return k[j];
+    }
+    __device__ static constexpr bool minus(int j) { return j == 0 || j == 3 || j == 4 || j == 7; }
+    __device__ __forceinline__ double at(int j, int c) const { return minus(j) ? -r[index(j)][c] : r[index(j)][c]; }
+    // 24 numbers: row j as stored
+    __device__ __forceinline__ void row(const Fp64Src& S, int j, double (&bb)[3]) const {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) bb[c] = ldin<SMEM>(S.bt + (3 * j + c) * S.stride + S.i);
+    }
+};
+
+// Gamma row k, node j is +1 (exDyna3D.cpp:1003-1008).
+__device__ __forceinline__ constexpr bool gamma_plus(int k, int j) {
+    constexpr unsigned kMask = 0x55u | (0x3Cu << 8) | (0x96u << 16) | (0x5Au << 24);
+    return (kMask >> (8 * k + j)) & 1u;
 }
 
 // One element of the FP64 element pass (the kernel comment below has the
-// reference mapping), shared by the single-instance, staged, batched and
-// resident-run kernels; inputs come from S, the evolving rows go to O and the
-// forces to the instance's force array at element e.  Node rows are read with
-// plain loads: a resident run rewrites them between its cycles.  SMEM / BT_SMEM: S's rows / B0^T rows
-// are in shared memory.  PF: node rows the body reads later are prefetched
-// into L1 once the connectivity is known (bit 0 the velocities, bit 1 the
-// displacements).
-template <bool PLASTIC, bool INIT, bool SMEM = false, bool BT_SMEM = false, int PF = 0>
+// reference mapping), shared by the single-instance, batched and resident-run
+// kernels; inputs come from S, the evolving rows go to O and the forces to the
+// instance's force array at element e.  Node rows are read with plain loads: a
+// resident run rewrites them between its cycles.  SMEM: S's rows are in shared
+// memory.  BT9: its bt rows are the 9-number form.  PF: node rows the body reads
+// later are prefetched into L1 once the connectivity is known (bit 0 the
+// velocities, bit 1 the displacements).
+template <bool PLASTIC, bool INIT, bool BT9, bool SMEM = false, int PF = 0>
 __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArrays& N, const Material& M,
                                              const Fp64Src& S, const Fp64Out& O, const double dt1, const int64_t e,
                                              double& dts, double& len, double& e_int, double& e_hg, double& e_vis,
                                              int32_t& bad) {
-    const int64_t ss = S.stride, si = S.i, bs = S.bt_stride, os = O.stride, oi = O.i;
+    const int64_t ss = S.stride, si = S.i, os = O.stride, oi = O.i;
     const int64_t ep = E.ne_pad, np = N.nn_pad;
     double* fe = static_cast<double*>(E.fe);
     const double* X = N.x;
@@ -187,7 +265,6 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
     const double* V = static_cast<const double*>(N.v);
     const double G = M.G, lam = M.lambda;
 
-    const double* bte = S.bt + S.bt_i;
     uint32_t n[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) n[k] = ldin<SMEM>(S.conn + k * ss + si);
@@ -203,77 +280,109 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
 #pragma unroll
             for (int k = 0; k < 8; ++k) prefetch_l1(U + r * np + n[k]);
     }
-    // current coordinates: hourglass projections TAU x (exact, the
-    // Gamma entries are +-1) and the minimum edge (min_ele_edge :1173-1220)
+    // current coordinates: hourglass projections TAU x and the minimum edge
+    // (min_ele_edge :1173-1220)
     double TX[4][3];
     {
         double xyz[8][3];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            xyz[k][0] = X[n[k]];
-            xyz[k][1] = X[np + n[k]];
-            xyz[k][2] = X[2 * np + n[k]];
-        }
+        for (int c = 0; c < 3; ++c) {
+            double x[8], t[4];
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
+            for (int k = 0; k < 8; ++k) xyz[k][c] = x[k] = X[c * np + n[k]];
+            gamma_sums(x, t);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) TX[kk][c] = t[kk];
+        }
+        len = sqrt(min_edge_sq(xyz));
+    }
+    // F = I + u_e B0^T (:862-865); with B0 in its 9-number form one component
+    // at a time, else node by node (24 numbers would stay in registers)
+    B0Rows<BT9, SMEM> B;
+    double F[3][3];
+    if constexpr (BT9) {
+        B.load(S);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            double u[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) u[k] = U[r * np + n[k]];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                double t = tau_sign(kk, 0) > 0 ? xyz[0][c] : -xyz[0][c];
+                double t = 0.0;
 #pragma unroll
-                for (int j = 1; j < 8; ++j) t = tau_sign(kk, j) > 0 ? t + xyz[j][c] : t - xyz[j][c];
-                TX[kk][c] = t;
+                for (int k = 0; k < 8; ++k) t = __fma_rn(u[k], B.at(k, c), t);
+                F[r][c] = t;
             }
-        constexpr int A0[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3};
-        constexpr int A1[12] = {1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7};
-        double m = DBL_MAX;
-#pragma unroll
-        for (int k = 0; k < 12; ++k) {
-            const double dx = xyz[A1[k]][0] - xyz[A0[k]][0];
-            const double dy = xyz[A1[k]][1] - xyz[A0[k]][1];
-            const double dz = xyz[A1[k]][2] - xyz[A0[k]][2];
-            const double t = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
-            m = t < m ? t : m;
         }
-        len = sqrt(m);
-    }
-    // F = I + u_e B0^T (:862-865)
-    double F[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-#pragma unroll kNodeUnrollFp64
-    for (int k = 0; k < 8; ++k) {
-        const uint32_t nk = ldin<SMEM>(S.conn + k * ss + si);
-        const double uu[3] = {U[nk], U[np + nk], U[2 * np + nk]};
-        const double* bk = bte + 3 * k * bs;
-        const double bb[3] = {ldin<BT_SMEM>(bk), ldin<BT_SMEM>(bk + bs), ldin<BT_SMEM>(bk + 2 * bs)};
+    } else {
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+        for (int i = 0; i < 9; ++i) F[i / 3][i % 3] = 0.0;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) F[r][c] = __fma_rn(uu[r], bb[c], F[r][c]);
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t nk = ldin<SMEM>(S.conn + k * ss + si);
+            double bb[3];
+            B.row(S, k, bb);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const double u = U[r * np + nk];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) F[r][c] = __fma_rn(u, bb[c], F[r][c]);
+            }
+        }
     }
-    F[0][0] = 1.0 + F[0][0];
-    F[1][1] = 1.0 + F[1][1];
-    F[2][2] = 1.0 + F[2][2];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) F[r][r] = 1.0 + F[r][r];
     const double J = det3(F);
     double Fi[3][3];
     inv3(F, Fi);
     if (!(J > 0.0)) bad |= ST_INVERTED;
-    // per node: L0 = v_e B0^T, VT = v_e Gamma^T (signed sums), NX2 (:1024)
-    double L0[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-    double VT[3][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-    double nx2 = 0.0;
-#pragma unroll kNodeUnrollFp64
-    for (int j = 0; j < 8; ++j) {
-        const uint32_t nj = ldin<SMEM>(S.conn + j * ss + si);
-        const double* bk = bte + 3 * j * bs;
-        const double bb[3] = {ldin<BT_SMEM>(bk), ldin<BT_SMEM>(bk + bs), ldin<BT_SMEM>(bk + 2 * bs)};
-        const double vj[3] = {V[nj], V[np + nj], V[2 * np + nj]};
+    // L0 = v_e B0^T, VT = v_e Gamma^T (signed sums), NX2 (:1024)
+    double L0[3][3], VT[3][4], nx2 = 0.0;
+    if constexpr (BT9) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            double v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = V[r * np + n[j]];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double l = 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) l = __fma_rn(v[j], B.at(j, c), l);
+                L0[r][c] = l;
+            }
+            gamma_sums(v, VT[r]);
+        }
+        double sq[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            sq[j] = __fma_rn(B.r[j][2], B.r[j][2], __fma_rn(B.r[j][1], B.r[j][1], B.r[j][0] * B.r[j][0]));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) nx2 = nx2 + sq[B.index(j)];
+    } else {
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) L0[r][c] = __fma_rn(vj[r], bb[c], L0[r][c]);
+            for (int c = 0; c < 3; ++c) L0[r][c] = 0.0;
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) VT[r][kk] = tau_of(kk, j) > 0.0 ? VT[r][kk] + vj[r] : VT[r][kk] - vj[r];
+            for (int kk = 0; kk < 4; ++kk) VT[r][kk] = 0.0;
         }
-        nx2 = nx2 + __fma_rn(bb[2], bb[2], __fma_rn(bb[1], bb[1], bb[0] * bb[0]));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t nj = ldin<SMEM>(S.conn + j * ss + si);
+            double bb[3];
+            B.row(S, j, bb);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const double v = V[r * np + nj];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) L0[r][c] = __fma_rn(v, bb[c], L0[r][c]);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) VT[r][kk] = gamma_plus(kk, j) ? VT[r][kk] + v : VT[r][kk] - v;
+            }
+            nx2 = nx2 + __fma_rn(bb[2], bb[2], __fma_rn(bb[1], bb[1], bb[0] * bb[0]));
+        }
     }
     // L = L0 F^-1 (= v_e b^T, :928); HIA = VT - L0 TX^T (= v_e ATAU^T, :1020-1021)
     double L[3][3], HIA[3][4];
@@ -395,26 +504,45 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
         e_hg += hp * dt1;
     }
     // nodal forces f_j = -(B0_j Z) - Gamma_j Gq^T
-    // (= -b_j sigma V - h_j + p b_j V: :985-997, :1070, :1106)
-#pragma unroll kNodeUnrollFp64
-    for (int j = 0; j < 8; ++j) {
-        const double* bk = bte + 3 * j * bs;
-        const double b0 = ldin<BT_SMEM>(bk), b1 = ldin<BT_SMEM>(bk + bs), b2 = ldin<BT_SMEM>(bk + 2 * bs);
-        double* fej;
-        int64_t fst;
-        if (E.slot_major) {
-            fej = fe + 3 * j * np + ldin<SMEM>(S.conn + j * ss + si);
-            fst = np;
-        } else {
-            fej = fe + 3 * j * ep + e;
-            fst = ep;
-        }
+    // (= -b_j sigma V - h_j + p b_j V: :985-997, :1070, :1106).  Gamma_j Gq^T is
+    // summed over the four hourglass vectors in order, nodes with the same
+    // leading signs (or the opposite ones) sharing their partial sums; B0_j Z
+    // is evaluated once for two opposite corners.
+    {
+        B0Rows<BT9, SMEM> Bf;
+        if constexpr (BT9) Bf.load(S);
+        auto store = [&](int j, int i, double f) {
+            if (E.slot_major) fe[(3 * j + i) * np + ldin<SMEM>(S.conn + j * ss + si)] = f;
+            else fe[(3 * j + i) * ep + e] = f;
+        };
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            double tg = tau_of(0, j) > 0.0 ? Gq[i][0] : -Gq[i][0];
+            if constexpr (BT9) {
+                const double g0 = Gq[i][0], g1 = Gq[i][1], g2 = Gq[i][2], g3 = Gq[i][3];
+                const double d = g0 - g1, q = g0 + g1;
+                const double dm = d - g2, dp = d + g2, qm = g2 - q, qp = q + g2;
+                const double t[8] = {dm - g3, qm + g3, qp - g3, g3 - dp, qp + g3, -(dp + g3), dm + g3, qm - g3};
+                double bz[4];
 #pragma unroll
-            for (int kk = 1; kk < 4; ++kk) tg = tau_of(kk, j) > 0.0 ? tg + Gq[i][kk] : tg - Gq[i][kk];
-            fej[i * fst] = -__fma_rn(b2, Z[2][i], __fma_rn(b1, Z[1][i], b0 * Z[0][i])) - tg;
+                for (int j = 0; j < 4; ++j)
+                    bz[j] = __fma_rn(Bf.r[j][2], Z[2][i], __fma_rn(Bf.r[j][1], Z[1][i], Bf.r[j][0] * Z[0][i]));
+#pragma unroll
+                for (int j = 0; j < 8; ++j) store(j, i, (Bf.minus(j) ? bz[Bf.index(j)] : -bz[Bf.index(j)]) - t[j]);
+            }
+        }
+        if constexpr (!BT9) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                double bb[3];
+                Bf.row(S, j, bb);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    double tg = gamma_plus(0, j) ? Gq[i][0] : -Gq[i][0];
+#pragma unroll
+                    for (int kk = 1; kk < 4; ++kk) tg = gamma_plus(kk, j) ? tg + Gq[i][kk] : tg - Gq[i][kk];
+                    store(j, i, -__fma_rn(bb[2], Z[2][i], __fma_rn(bb[1], Z[1][i], bb[0] * Z[0][i])) - tg);
+                }
+            }
         }
     }
     // compute_dtStable (:828-834)
@@ -437,7 +565,7 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
 // per-node rows of b^T and ATAU are recomputed from B0^T (L1-resident) rather
 // than held, so no 8x3 / 4x8 array stays live.  Every value is the same
 // expression, in the same order, as the CPU restatement (explicit fma only).
-template <bool PLASTIC, bool INIT>
+template <bool PLASTIC, bool INIT, bool BT9, bool TILED>
 __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_FP64) k_element(ElemArrays E, NodeArrays N, Material M, Ctl* ctl,
                                                              Partials P) {
     if (ctl->done) return;
@@ -453,7 +581,9 @@ __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_FP64) k_element(E
         const bool live = e0 < ne;
         const int64_t e = live ? e0 : 0;
         double dts = DBL_MAX, len = DBL_MAX;
-        if (live) element_body<PLASTIC, INIT>(E, N, M, fp64_src_global(E, e), fp64_out_global(E, e), dt1, e, dts, len, e_int, e_hg, e_vis, bad);
+        if (live)
+            element_body<PLASTIC, INIT, BT9>(E, N, M, fp64_src_global<TILED>(E, e), fp64_out_global<TILED>(E, e), dt1, e,
+                                             dts, len, e_int, e_hg, e_vis, bad);
         dts_min = dts < dts_min ? dts : dts_min;
         len_min = len < len_min ? len : len_min;
     }
@@ -566,145 +696,6 @@ __device__ __forceinline__ void node_body(const ElemArrays& E, const NodeArrays&
     }
 }
 
-// ---- staged element pass ------------------------------------------------
-// As k_element, with each block walking tiles of kStageTileF64 consecutive
-// elements whose streamed inputs -- connectivity, sigma, QIA, V0, cbrt(V0),
-// cbrt(V0^2), eps_p and, when BT, B0^T -- thread 0 copies into one of two
-// shared-memory stages with bulk copies one tile ahead of the compute.  The
-// arithmetic is element_body's, so results are bit-identical to k_element.
-constexpr int kStageTileF64 = ENSC_STAGE_TILE_FP64;
-// resident blocks per SM of the staged FP64 passes (same threads per SM for
-// any tile size)
-constexpr int kStageMinbF64 = 256 / kStageTileF64;
-constexpr int kF64StageRows = 22;  // double rows before B0^T: 6 sigma, 12 QIA, V0, cbrt V0, cbrt V0^2, eps_p
-template <bool BT>
-constexpr uint32_t f64_stage_bytes() {
-    return 8u * kStageTileF64 * 4u + static_cast<uint32_t>(kF64StageRows + (BT ? 24 : 0)) * kStageTileF64 * 8u;
-}
-template <bool BT>
-constexpr size_t f64_stage_smem() {
-    return 2 * static_cast<size_t>(f64_stage_bytes<BT>()) + 16;
-}
-
-// double row r of the stage in global memory
-__device__ __forceinline__ const double* f64_stage_row(const ElemArrays& E, int r) {
-    const int64_t ep = E.ne_pad;
-    if (r < 6) return static_cast<const double*>(E.sigma) + r * ep;
-    if (r < 18) return static_cast<const double*>(E.qia) + (r - 6) * ep;
-    if (r == 18) return E.vol0;
-    if (r == 19) return E.cbrt_v0;
-    if (r == 20) return E.cbrt_v0sq;
-    if (r == 21) return static_cast<const double*>(E.eps_p);
-    return static_cast<const double*>(E.bt) + (r - kF64StageRows) * ep;
-}
-
-// Warp 0: the tile starting at element `base` into the stage at shared
-// address dst, completing on bar (rows padded to 32 entries and 256-byte
-// aligned: every copy is 16-byte aligned and a multiple of 128 bytes); lane
-// 0 arms the barrier, then the lanes start the row copies between them.
-__device__ __forceinline__ uint32_t f64_stage_count(const ElemArrays& E, int64_t base) {
-    const int64_t left = E.ne_pad - base;
-    return static_cast<uint32_t>(left < kStageTileF64 ? left : kStageTileF64);
-}
-template <bool PLASTIC, bool BT>
-__device__ __forceinline__ uint32_t f64_stage_tx_bytes(uint32_t cnt) {
-    constexpr int drows = kF64StageRows + (BT ? 24 : 0);
-    constexpr int dcopies = PLASTIC ? drows : drows - 1;
-    return 8u * cnt * 4u + static_cast<uint32_t>(dcopies) * cnt * 8u;
-}
-template <bool PLASTIC, bool BT>
-__device__ __forceinline__ void f64_stage_issue(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t base,
-                                                int lane) {
-    constexpr int drows = kF64StageRows + (BT ? 24 : 0);
-    const uint32_t cnt = f64_stage_count(E, base);
-    if (lane == 0) mbar_arrive_expect_tx(bar, f64_stage_tx_bytes<PLASTIC, BT>(cnt));
-    __syncwarp();
-    fence_proxy_async_smem();  // the block's reads of this stage come before the copies into it
-    const uint32_t dbase = dst + 8u * kStageTileF64 * 4u;
-    for (int q = lane; q < 8 + drows; q += 32) {
-        if (q < 8) {
-            bulk_g2s(dst + q * (kStageTileF64 * 4u), E.conn + q * E.ne_pad + base, cnt * 4u, bar);
-        } else {
-            const int r = q - 8;
-            if (PLASTIC || r != 21)  // eps_p is read only with J2
-                bulk_g2s(dbase + r * (kStageTileF64 * 8u), f64_stage_row(E, r) + base, cnt * 8u, bar);
-        }
-    }
-}
-
-template <bool PLASTIC, bool BT>
-__global__ void __launch_bounds__(kStageTileF64, BT ? kStageMinbF64 : kStageMinbF64 * 3 / 2)
-    k_element_staged(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
-    if (ctl->done) return;
-    extern __shared__ __align__(128) unsigned char smem[];
-    constexpr uint32_t SB = f64_stage_bytes<BT>();
-    constexpr int T = kStageTileF64;
-    const double dt1 = ctl->dt_i_1;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const uint32_t stage0 = smem_addr(smem);
-    const uint32_t bar0 = stage0 + 2 * SB;
-    const int64_t ntiles = (E.ne + T - 1) / T;
-    const int64_t gstride = gridDim.x;
-    if (tid == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar0 + 8, 1);
-        mbar_init_fence();
-    }
-    __syncthreads();
-    if (wid == 0) {
-        for (int s = 0; s < 2; ++s) {
-            const int64_t t = blockIdx.x + s * gstride;
-            if (t < ntiles) f64_stage_issue<PLASTIC, BT>(E, stage0 + s * SB, bar0 + 8 * s, t * T, lane);
-        }
-    }
-    double e_int = 0.0, e_hg = 0.0, e_vis = 0.0;
-    double dts_min = DBL_MAX, len_min = DBL_MAX;
-    int32_t bad = 0;
-    bool timed_out = false;
-    int it = 0;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gstride, ++it) {
-        const int s = it & 1;
-        const uint32_t bar = bar0 + 8 * s;
-        const bool ok = mbar_wait_bounded(bar, (it >> 1) & 1);
-        if (__syncthreads_or(!ok)) {
-            timed_out = true;
-            break;
-        }
-        const int64_t e = t * T + tid;
-        if (e < E.ne) {
-            const unsigned char* st = smem + s * SB;
-            const double* d = reinterpret_cast<const double*>(st + 8 * T * 4);
-            const Fp64Src S{reinterpret_cast<const uint32_t*>(st), d, d + 6 * T, d + 18 * T, d + 19 * T, d + 20 * T,
-                            d + 21 * T, T, tid,
-                            BT ? d + kF64StageRows * T : static_cast<const double*>(E.bt),
-                            BT ? static_cast<int64_t>(T) : E.ne_pad, BT ? static_cast<int64_t>(tid) : e};
-            double dts, len;
-            element_body<PLASTIC, false, true, BT>(E, N, M, S, fp64_out_global(E, e), dt1, e, dts, len, e_int, e_hg, e_vis, bad);
-            dts_min = dts < dts_min ? dts : dts_min;
-            len_min = len < len_min ? len : len_min;
-        }
-        __syncthreads();  // the block is done with stage s
-        const int64_t tn = t + 2 * gstride;
-        if (wid == 0 && tn < ntiles) f64_stage_issue<PLASTIC, BT>(E, stage0 + s * SB, bar, tn * T, lane);
-    }
-    if (timed_out) {
-        // record the failure and let the copies this block started land
-        // (bounded) before its shared memory is released
-        if (tid == 0) {
-            atomicOr(&ctl->status, ST_TIMEOUT);
-            for (int k = 0; k < 2; ++k) {
-                const int itk = it + k;
-                if (blockIdx.x + itk * gstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
-            }
-        }
-        __syncthreads();
-    }
-    if (bad) atomicOr(&ctl->status, bad);
-    block_min2<kStageTileF64>(dts_min, len_min, &ctl->dts_next, &ctl->len_min);
-    double v3[3] = {e_int, e_hg, e_vis};
-    block_sum<kStageTileF64, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
-}
-
 // ---- output: the last cycle's acceleration --------------------------------
 // solution_a as compute_a leaves it (exDyna3D.cpp:642-644) in the last cycle
 // -- assembled element forces, gravity, the acceleration boundary conditions,
@@ -717,7 +708,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration(ElemArrays E, Nod
                                                                double* a_out) {
     const int64_t np = N.nn_pad, ep = E.ne_pad;
     const double* __restrict__ fe = static_cast<const double*>(E.fe);
-    const bool grouped = E.slot_major && E.tiles_aligned;
+    const bool grouped = E.slot_major && E.tile_bytes;
     const double amp = (M.gravity_on && M.amp_n > 0) ? gravity_amplitude(M.amp, M.amp_n, ctl->time, ctl->dt_i) : 1.0;
     for (int64_t n = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; n < N.nn;
          n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -779,65 +770,51 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration(ElemArrays E, Nod
 }
 
 // ---- warp-pipelined element pass ---------------------------------------
-// As k_element_staged (B0^T staged too), but every warp runs its own
-// pipeline over tiles of 32 consecutive elements: its own two stages, its
-// own barriers, a stage reused as soon as its 32 lanes are done with it, and
-// no block-wide barrier per tile.  element_body's arithmetic, so results are
-// bit-identical to the other FP64 element passes.
-constexpr int kF64WarpTile = 32;
-// B0^T staged with the other rows (1) or read from global memory through L1
-// (0, a smaller stage: more warps fit in shared memory)
-constexpr bool kF64WarpBt = ENSC_F64_WARP_BT != 0;
-constexpr uint32_t kF64WarpStageBytes =
-    8u * kF64WarpTile * 4u + (kF64StageRows + (kF64WarpBt ? 24 : 0)) * kF64WarpTile * 8u;
+// Every warp runs its own pipeline over tiles of 32 consecutive elements: two
+// shared-memory stages, each filled by one bulk copy of a whole tile while
+// the other is computed, and no block-wide barrier per tile.  element_body's
+// arithmetic, so results are bit-identical to the other FP64 element passes.
 constexpr int kF64PipeWarps = ENSC_F64_PIPE_WARPS;
-constexpr size_t kF64WarpPipeSmem = static_cast<size_t>(kF64PipeWarps) * (2 * kF64WarpStageBytes + 16);
-
-template <bool PLASTIC>
-__device__ __forceinline__ void f64_warp_stage_issue(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t base,
-                                                     int lane) {
-    constexpr int drows = kF64StageRows + (kF64WarpBt ? 24 : 0);
-    // whole 32-entry tiles of rows padded to multiples of 32: 128- and
-    // 256-byte copies
-    if (lane == 0) mbar_arrive_expect_tx(bar, f64_stage_tx_bytes<PLASTIC, kF64WarpBt>(kF64WarpTile));
-    __syncwarp();
-    fence_proxy_async_smem();  // the warp's reads of this stage come before the copies into it
-    const uint32_t dbase = dst + 8u * kF64WarpTile * 4u;
-    for (int q = lane; q < 8 + drows; q += 32) {
-        if (q < 8) {
-            bulk_g2s(dst + q * (kF64WarpTile * 4u), E.conn + q * E.ne_pad + base, kF64WarpTile * 4u, bar);
-        } else {
-            const int r = q - 8;
-            if (PLASTIC || r != 21)  // eps_p is read only with J2
-                bulk_g2s(dbase + r * (kF64WarpTile * 8u), f64_stage_row(E, r) + base, kF64WarpTile * 8u, bar);
-        }
-    }
+template <typename L>
+constexpr size_t f64_pipe_smem() {
+    return static_cast<size_t>(kF64PipeWarps) * (2 * L::kBytes + 16);
 }
 
-template <bool PLASTIC>
+// Lane 0: the tile at src into shared memory at dst, completing on bar
+// (elastic instances leave out eps_p, the tile's last row).
+template <bool PLASTIC, typename L>
+__device__ __forceinline__ void f64_tile_issue(const void* src, uint32_t dst, uint32_t bar) {
+    constexpr uint32_t bytes = PLASTIC ? L::kBytes : L::kEps;
+    mbar_arrive_expect_tx(bar, bytes);
+    fence_proxy_async_smem();  // the warp's reads of this stage come before the copy into it
+    bulk_g2s(dst, src, bytes, bar);
+}
+
+template <bool PLASTIC, bool BT9>
 __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
     k_element_fp64_warp(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
+    using L = std::conditional_t<BT9, Fp64Tile9, Fp64Tile24>;
     if (ctl->done) return;
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int T = kF64WarpTile;
     const double dt1 = ctl->dt_i_1;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * kF64WarpStageBytes;
+    unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * L::kBytes;
     const uint32_t stage0 = smem_addr(wst);
-    const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kF64PipeWarps) * 2 * kF64WarpStageBytes) + 16u * wid;
-    const int64_t ntiles = (E.ne + T - 1) / T;
+    const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kF64PipeWarps) * 2 * L::kBytes) + 16u * wid;
+    const unsigned char* tiles = reinterpret_cast<const unsigned char*>(E.conn);
+    const int64_t ntiles = (E.ne + 31) / 32;
     const int64_t wstride = static_cast<int64_t>(gridDim.x) * kF64PipeWarps;
     const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kF64PipeWarps + wid;
     if (lane == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
+        for (int s = 0; s < 2; ++s) {
+            const int64_t t = w0 + s * wstride;
+            if (t < ntiles) f64_tile_issue<PLASTIC, L>(tiles + t * L::kBytes, stage0 + s * L::kBytes, bar0 + 8 * s);
+        }
     }
     __syncwarp();
-    for (int s = 0; s < 2; ++s) {
-        const int64_t t = w0 + s * wstride;
-        if (t < ntiles) f64_warp_stage_issue<PLASTIC>(E, stage0 + s * kF64WarpStageBytes, bar0 + 8 * s, t * T, lane);
-    }
     double e_int = 0.0, e_hg = 0.0, e_vis = 0.0;
     double dts_min = DBL_MAX, len_min = DBL_MAX;
     int32_t bad = 0;
@@ -851,23 +828,19 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
             timed_out = true;
             break;
         }
-        const int64_t e = t * T + lane;
+        const int64_t e = t * 32 + lane;
         if (e < E.ne) {
-            const unsigned char* st = wst + s * kF64WarpStageBytes;
-            const double* d = reinterpret_cast<const double*>(st + 8 * T * 4);
-            const Fp64Src S{reinterpret_cast<const uint32_t*>(st), d, d + 6 * T, d + 18 * T, d + 19 * T, d + 20 * T,
-                            d + 21 * T, T, lane,
-                            kF64WarpBt ? d + kF64StageRows * T : static_cast<const double*>(E.bt),
-                            kF64WarpBt ? static_cast<int64_t>(T) : E.ne_pad,
-                            kF64WarpBt ? static_cast<int64_t>(lane) : e};
+            unsigned char* g = const_cast<unsigned char*>(tiles) + t * L::kBytes;
             double dts, len;
-            element_body<PLASTIC, false, true, kF64WarpBt, ENSC_F64_PREFETCH>(E, N, M, S, fp64_out_global(E, e), dt1, e,
-                                                                              dts, len, e_int, e_hg, e_vis, bad);
+            element_body<PLASTIC, false, BT9, true, ENSC_F64_PREFETCH>(E, N, M, fp64_src_tile<L>(wst + s * L::kBytes, lane),
+                                                                       fp64_out_tile<L>(g, lane), dt1, e, dts, len,
+                                                                       e_int, e_hg, e_vis, bad);
             dts_min = dts < dts_min ? dts : dts_min;
             len_min = len < len_min ? len : len_min;
         }
+        __syncwarp();  // all lanes are done with stage s
         const int64_t tn = t + 2 * wstride;
-        if (tn < ntiles) f64_warp_stage_issue<PLASTIC>(E, stage0 + s * kF64WarpStageBytes, bar, tn * T, lane);
+        if (lane == 0 && tn < ntiles) f64_tile_issue<PLASTIC, L>(tiles + tn * L::kBytes, stage0 + s * L::kBytes, bar);
     }
     if (timed_out) {
         // record the failure and let the copies this warp started land
@@ -1060,7 +1033,7 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_FP64) k_node(Elem
     int32_t bad = 0;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (E.slot_major && E.tiles_aligned) {
+    if (E.slot_major && E.tile_bytes) {
         constexpr int W = kNodeGroupFp64;
         const NodeView nv = node_view(E, N, M, ctl);
         for (int64_t g = t0; g * W < nn; g += stride) node_group<W>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad);
@@ -1073,36 +1046,35 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_FP64) k_node(Elem
 }
 
 // ---- resident runs (ensc_run.cuh) -----------------------------------------
-// 8 warps per SM as in the warp-pipelined pass; a tile of 32 elements takes
-// 12.8 KB, so that 17 tiles fit an SM and 148 SMs hold 75,776 elements at two
-// tiles per warp.
+// 8 warps per SM as in the warp-pipelined pass; a tile takes 8,960 bytes, so
+// that 25 tiles fit an SM and 148 SMs hold 113,664 elements at three tiles per
+// warp.  (Only for B0 in its 9-number form, which every mesh whose constants
+// are computed here has.)
 constexpr int kRunWarpsF64 = 8;
 template <bool PLASTIC>
 struct RunFp64 {
-    static constexpr uint32_t kTileBytes = 8u * 32u * 4u + (kF64StageRows + 24) * 32u * 8u;
+    using L = Fp64Tile9;
+    static constexpr uint32_t kTileBytes = L::kBytes;
     __device__ static const uint32_t* conn(const unsigned char* tile) {
         return reinterpret_cast<const uint32_t*>(tile);
     }
-    __device__ static void load_tile(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t base, int lane) {
-        static_assert(kF64WarpBt && kF64WarpStageBytes == kTileBytes, "the warp-pipelined pass's stage");
-        f64_warp_stage_issue<PLASTIC>(E, dst, bar, base, lane);
+    __device__ static void load_tile(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t t, int lane) {
+        if (lane == 0)
+            f64_tile_issue<PLASTIC, L>(reinterpret_cast<const unsigned char*>(E.conn) + t * L::kBytes, dst, bar);
     }
-    __device__ static void store_tile(const ElemArrays& E, const unsigned char* tile, int64_t base, int lane) {
-        const double* d = reinterpret_cast<const double*>(tile + 8 * 32 * 4);
-        const int64_t e = base + lane;
-        if (e >= E.ne) return;
-        for (int r = 0; r < 18; ++r) const_cast<double*>(f64_stage_row(E, r))[e] = d[r * 32 + lane];
-        if (PLASTIC) const_cast<double*>(f64_stage_row(E, 21))[e] = d[21 * 32 + lane];
+    __device__ static void store_tile(const ElemArrays& E, const unsigned char* tile, int64_t t, int lane) {
+        // whole rows: the entries past ne are padding
+        unsigned char* g = const_cast<unsigned char*>(reinterpret_cast<const unsigned char*>(E.conn)) + t * L::kBytes;
+        constexpr uint32_t end = PLASTIC ? L::kBytes : L::kEps;
+        for (uint32_t o = L::kState + 8u * lane; o < end; o += 256)
+            *reinterpret_cast<double*>(g + o) = *reinterpret_cast<const double*>(tile + o);
     }
     __device__ static void element(const ElemArrays& E, const NodeArrays& N, const Material& M, unsigned char* tile,
                                    double dt1, int64_t e, int lane, double& dts, double& len, double& e_int,
                                    double& e_hg, double& e_vis, int32_t& bad) {
-        double* d = reinterpret_cast<double*>(tile + 8 * 32 * 4);
-        const Fp64Src S{conn(tile), d, d + 6 * 32, d + 18 * 32, d + 19 * 32, d + 20 * 32, d + 21 * 32, 32, lane,
-                        d + kF64StageRows * 32, 32, lane};
-        const Fp64Out O{d, d + 6 * 32, d + 21 * 32, 32, lane};
-        element_body<PLASTIC, false, true, true, ENSC_F64_PREFETCH>(E, N, M, S, O, dt1, e, dts, len, e_int, e_hg,
-                                                                     e_vis, bad);
+        element_body<PLASTIC, false, true, true, ENSC_F64_PREFETCH>(E, N, M, fp64_src_tile<L>(tile, lane),
+                                                                    fp64_out_tile<L>(tile, lane), dt1, e, dts, len,
+                                                                    e_int, e_hg, e_vis, bad);
     }
     // W nodes per thread, their rows loaded ahead of the forces; a thread's
     // further nodes (meshes with more than 2 per thread) load both together.
@@ -1153,10 +1125,10 @@ __global__ void __launch_bounds__(32 * kRunWarpsF64, 1)
 }
 
 // ---- batched instances --------------------------------------------------------
-// Element tiles of kStageTileF64 elements and node tiles of
-// 32 * kNodeGroupFp64 nodes, each inside one instance whose arrays, material
-// and control block come from the instance table.  The element pass runs the
-// staged pipeline over the tile list, one tile per block at a time; the node
+// Element tiles of 32 elements and node tiles of 32 * kNodeGroupFp64 nodes,
+// each inside one instance whose arrays, material and control block come from
+// the instance table.  The element pass runs one pipeline per warp over the
+// tile list; the node
 // pass gives each node tile to one warp.  Each tile accumulates its work terms across
 // cycles (one owner per tile and pass) and keeps its latest kinetic energy;
 // k_fold_batch folds them per instance in tile order, so the totals do not
@@ -1168,104 +1140,55 @@ __device__ __forceinline__ double warp_sum_b(double v) {
     return v;
 }
 
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w < v ? w : v;
-    }
-    return v;
-}
+// A batch stage: a tile, then its instance descriptor, its element-pass scalars
+// (StageHdr), the TileInfo the filling lane writes, and the ETileSrc record of
+// the tile that uses the stage next (as in the mixed batch pass).  The tile's
+// room is T.tile_room: 8,960 bytes, or 12,800 while the batch holds an
+// instance with its own 24-number B0^T.
 
-// A batch stage: the element rows of a tile of kF64BatchTile elements (as the
-// single-instance stage, B0^T included), then the tile's instance
-// descriptor, its element-pass scalars (StageHdr), the TileInfo the filling
-// warp writes, and the ETileSrc record of the tile that uses the stage next
-// (as in the mixed batch pass).
-constexpr int kF64BatchTile = ENSC_F64_BATCH_TILE;
-static_assert(kF64BatchTile % 32 == 0, "whole warps per tile");
-constexpr uint32_t kF64DescOff =
-    8u * kF64BatchTile * 4u + static_cast<uint32_t>(kF64StageRows + 24) * kF64BatchTile * 8u;
-constexpr uint32_t kF64HdrOff = kF64DescOff + sizeof(InstanceDesc);
-constexpr uint32_t kF64InfoOff = kF64HdrOff + sizeof(StageHdr);
-constexpr uint32_t kF64NextOff = kF64InfoOff + sizeof(TileInfo);
-constexpr uint32_t kF64BatchStageBytes = (kF64NextOff + sizeof(ETileSrc) + 127) / 128 * 128;
-constexpr size_t kF64BatchStageSmem = 2 * static_cast<size_t>(kF64BatchStageBytes) + 16;
-static_assert(sizeof(InstanceDesc) % 16 == 0, "16-byte copies");
-
-// double row r (as f64_stage_row) of a batch tile in global memory
-__device__ __forceinline__ const double* f64_tile_row(const ETileSrc& src, int r) {
-    const int64_t ep = src.ne_pad;
-    if (r < 6) return static_cast<const double*>(src.sigma) + r * ep;
-    if (r < 18) return static_cast<const double*>(src.qia) + (r - 6) * ep;
-    if (r == 18) return static_cast<const double*>(src.vol0);
-    if (r == 19) return static_cast<const double*>(src.cbrt_v0);
-    if (r == 20) return static_cast<const double*>(src.cbrt_v0sq);
-    if (r == 21) return static_cast<const double*>(src.eps_p);
-    return static_cast<const double*>(src.bt) + (r - kF64StageRows) * ep;
-}
-
-__device__ __forceinline__ void f64_batch_stage_issue(const BatchTables& T, const ETileSrc& src, int64_t t_next,
-                                                      int64_t ntiles, unsigned char* stage, uint32_t dst, uint32_t bar,
-                                                      int lane) {
-    constexpr int drows = kF64StageRows + 24;
-    const uint32_t cnt = static_cast<uint32_t>(src.cnt);
+// Lane 0 of a warp fills a stage.
+__device__ __forceinline__ void f64_batch_issue(const BatchTables& T, const ETileSrc& src, int64_t t_next,
+                                                int64_t ntiles, unsigned char* stage, uint32_t dst, uint32_t bar) {
     const bool next = t_next < ntiles;
-    if (lane == 0) {
-        TileInfo* ti = reinterpret_cast<TileInfo*>(stage + kF64InfoOff);
-        ti->slot = src.slot;
-        ti->base = src.base;
-        mbar_arrive_expect_tx(bar, f64_stage_tx_bytes<true, true>(cnt) + sizeof(InstanceDesc) + sizeof(StageHdr) +
-                                       (next ? sizeof(ETileSrc) : 0u));
-    }
-    __syncwarp();
-    fence_proxy_async_smem();  // the block's reads of this stage come before the copies into it
-    const uint32_t dbase = dst + 8u * kF64BatchTile * 4u;
-    for (int q = lane; q < 8 + drows + 3; q += 32) {
-        if (q < 8)
-            bulk_g2s(dst + q * (kF64BatchTile * 4u), static_cast<const uint32_t*>(src.conn) + q * src.ne_pad,
-                     cnt * 4u, bar);
-        else if (q < 8 + drows)
-            bulk_g2s(dbase + (q - 8) * (kF64BatchTile * 8u), f64_tile_row(src, q - 8), cnt * 8u, bar);
-        else if (q == 8 + drows)
-            bulk_g2s(dst + kF64DescOff, T.desc + src.slot, sizeof(InstanceDesc), bar);
-        else if (q == 8 + drows + 1)
-            bulk_g2s(dst + kF64HdrOff, T.sparam + src.slot, sizeof(StageHdr), bar);
-        else if (next)
-            bulk_g2s(dst + kF64NextOff, T.etile_src + t_next, sizeof(ETileSrc), bar);
-    }
+    const uint32_t o = static_cast<uint32_t>(T.tile_room);
+    TileInfo* ti = reinterpret_cast<TileInfo*>(stage + o + kBatchInfoOff);
+    ti->slot = src.slot;
+    ti->base = src.base;
+    mbar_arrive_expect_tx(bar, static_cast<uint32_t>(src.bytes) + sizeof(InstanceDesc) + sizeof(StageHdr) +
+                                   (next ? sizeof(ETileSrc) : 0u));
+    fence_proxy_async_smem();  // the warp's reads of this stage come before the copies into it
+    bulk_g2s(dst, src.tile, static_cast<uint32_t>(src.bytes), bar);
+    bulk_g2s(dst + o, T.desc + src.slot, sizeof(InstanceDesc), bar);
+    bulk_g2s(dst + o + kBatchHdrOff, T.sparam + src.slot, sizeof(StageHdr), bar);
+    if (next) bulk_g2s(dst + o + kBatchNextOff, T.etile_src + t_next, sizeof(ETileSrc), bar);
 }
 
-// The batched FP64 element pass: element_body's arithmetic per element, so
-// states are bit-identical to the single-instance pass.  A block's
-// consecutive tiles of one instance form a run whose sums and minima are
-// reduced once, into the partial slot of the run's first tile.
-__global__ void __launch_bounds__(kF64BatchTile, 256 / kF64BatchTile) k_element_batch_fp64(BatchTables T) {
+// The batched FP64 element pass: one pipeline per warp over tiles of 32
+// elements, element_body's arithmetic per element, so states are bit-identical
+// to the single-instance pass.  A warp's consecutive tiles of one instance form
+// a run whose sums and minima are reduced once, into the partial slot of the
+// run's first tile.
+__global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB) k_element_batch_fp64(BatchTables T) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int TT = kF64BatchTile;
-    constexpr int NW = TT / 32;
-    constexpr uint32_t SB = kF64BatchStageBytes;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const uint32_t stage0 = smem_addr(smem);
-    const uint32_t bar0 = stage0 + 2 * SB;
+    const uint32_t SB = static_cast<uint32_t>(T.tile_room) + kBatchTailBytes;
+    unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
+    const uint32_t stage0 = smem_addr(wst);
+    const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kF64PipeWarps) * 2 * SB) + 16u * wid;
     const int64_t ntiles = T.counts[0];
-    const int64_t gstride = gridDim.x;
-    if (tid == 0) {
+    const int64_t wstride = static_cast<int64_t>(gridDim.x) * kF64PipeWarps;
+    const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kF64PipeWarps + wid;
+    if (lane == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
-    }
-    __syncthreads();
-    if (wid == 0) {
         for (int s = 0; s < 2; ++s) {
-            const int64_t t = blockIdx.x + s * gstride;
-            if (t < ntiles) {
-                const ETileSrc src = T.etile_src[t];
-                f64_batch_stage_issue(T, src, t + 2 * gstride, ntiles, smem + s * SB, stage0 + s * SB, bar0 + 8 * s,
-                                      lane);
-            }
+            const int64_t t = w0 + s * wstride;
+            if (t < ntiles)
+                f64_batch_issue(T, T.etile_src[t], t + 2 * wstride, ntiles, wst + s * SB, stage0 + s * SB, bar0 + 8 * s);
         }
     }
+    __syncwarp();
     // the current run: instance slot, first tile, control block, liveness
     int run_slot = -1;
     int64_t run_tile = 0;
@@ -1277,11 +1200,11 @@ __global__ void __launch_bounds__(kF64BatchTile, 256 / kF64BatchTile) k_element_
         ei = warp_sum_b(ei);
         eh = warp_sum_b(eh);
         ev = warp_sum_b(ev);
-        const unsigned long long dmin = warp_min_u64(ord_bits(dts));
-        const unsigned long long lmin = warp_min_u64(ord_bits(len));
+        const unsigned long long dmin = run_warp_min(ord_bits(dts));
+        const unsigned long long lmin = run_warp_min(ord_bits(len));
         bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
         if (run_live && lane == 0) {
-            double* part = T.etile_part + 3 * (run_tile * NW + wid);
+            double* part = T.etile_part + 3 * run_tile;
             // one writer per slot and pass: the reductions (no return value)
             // add in cycle order without a round trip
             atomicAdd(part + 0, ei);
@@ -1297,19 +1220,20 @@ __global__ void __launch_bounds__(kF64BatchTile, 256 / kF64BatchTile) k_element_
     };
     bool timed_out = false;
     int it = 0;
-    int64_t t = blockIdx.x;
-    for (; t < ntiles; t += gstride, ++it) {
+    int64_t t = w0;
+    for (; t < ntiles; t += wstride, ++it) {
         const int s = it & 1;
         const uint32_t bar = bar0 + 8 * s;
         const bool ok = mbar_wait_bounded(bar, (it >> 1) & 1);
-        if (__syncthreads_or(!ok)) {
+        if (__any_sync(0xffffffffu, !ok)) {
             timed_out = true;
             break;
         }
-        unsigned char* st = smem + s * SB;
-        const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(st + kF64DescOff);
-        const StageHdr& h = *reinterpret_cast<const StageHdr*>(st + kF64HdrOff);
-        const TileInfo& ti = *reinterpret_cast<const TileInfo*>(st + kF64InfoOff);
+        unsigned char* st = wst + s * SB;
+        unsigned char* tail = st + T.tile_room;
+        const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(tail);
+        const StageHdr& h = *reinterpret_cast<const StageHdr*>(tail + kBatchHdrOff);
+        const TileInfo& ti = *reinterpret_cast<const TileInfo*>(tail + kBatchInfoOff);
         if (ti.slot != run_slot) {
             flush();
             run_slot = ti.slot;
@@ -1317,37 +1241,40 @@ __global__ void __launch_bounds__(kF64BatchTile, 256 / kF64BatchTile) k_element_
             run_ctl = d.ctl;
             run_live = h.live != 0;
         }
-        const int64_t e = static_cast<int64_t>(ti.base) + tid;
+        const int64_t e = static_cast<int64_t>(ti.base) + lane;
         if (run_live && e < d.E.ne) {
             // arrays copied to registers, material read at use
             const ElemArrays E = d.E;
             const NodeArrays N = d.N;
             const double dt1 = h.dt1;
-            const double* dr = reinterpret_cast<const double*>(st + 8 * TT * 4);
-            const Fp64Src S{reinterpret_cast<const uint32_t*>(st), dr, dr + 6 * TT, dr + 18 * TT, dr + 19 * TT,
-                            dr + 20 * TT, dr + 21 * TT, TT, tid, dr + kF64StageRows * TT, TT, tid};
             double d1, l1;
-            element_body<true, false, true, true, ENSC_F64_PREFETCH>(E, N, d.M, S, fp64_out_global(E, e), dt1, e, d1, l1,
-                                                                     ei, eh, ev, bad);
+            if (E.bt9)
+                element_body<true, false, true, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile9>(st, lane),
+                                                                         fp64_out_global<true>(E, e), dt1, e, d1, l1, ei, eh,
+                                                                         ev, bad);
+            else
+                element_body<true, false, false, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile24>(st, lane),
+                                                                          fp64_out_global<true>(E, e), dt1, e, d1, l1, ei, eh,
+                                                                          ev, bad);
             dts = d1 < dts ? d1 : dts;
             len = l1 < len ? l1 : len;
         }
-        __syncthreads();  // the block is done with stage s
-        const int64_t tn = t + 2 * gstride;
-        if (wid == 0 && tn < ntiles) {
-            const ETileSrc src = *reinterpret_cast<const ETileSrc*>(st + kF64NextOff);
-            f64_batch_stage_issue(T, src, tn + 2 * gstride, ntiles, st, stage0 + s * SB, bar, lane);
+        __syncwarp();  // all lanes are done with stage s
+        const int64_t tn = t + 2 * wstride;
+        if (lane == 0 && tn < ntiles) {
+            const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
+            f64_batch_issue(T, src, tn + 2 * wstride, ntiles, st, stage0 + s * SB, bar);
         }
     }
     if (!timed_out) {
         flush();
-    } else if (tid == 0) {
+    } else if (lane == 0) {
         // record the failure on the instance whose tile could not be read and
-        // let the copies this block started land (bounded) before exiting
+        // let the copies this warp started land (bounded) before exiting
         atomicOr(&T.desc[T.etile_inst[t]].ctl->status, ST_TIMEOUT);
         for (int k = 0; k < 2; ++k) {
             const int itk = it + k;
-            if (blockIdx.x + itk * gstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
+            if (w0 + itk * wstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
         }
     }
     element_pass_done(T);
@@ -1409,30 +1336,31 @@ __global__ void __launch_bounds__(NT, ENSC_NODE_MINB_FP64 * kNodeThreads / NT) k
 
 }  // namespace
 
-namespace {
-constexpr bool kStagedBt = ENSC_STAGED_FP64 == 2;
-}
-
 void launch_element_fp64(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl, const Partials& P,
                          int grid, bool init, cudaStream_t st) {
-    if (ENSC_WARP_PIPE_FP64 && !init && E.tiles_aligned) {
-        if (M.plastic) k_element_fp64_warp<true><<<grid, 32 * kF64PipeWarps, kF64WarpPipeSmem, st>>>(E, N, M, ctl, P);
-        else k_element_fp64_warp<false><<<grid, 32 * kF64PipeWarps, kF64WarpPipeSmem, st>>>(E, N, M, ctl, P);
+    if (!E.tile_bytes) {  // caller-owned rows (ensc_step_noalloc)
+        if (M.plastic) {
+            if (init) k_element<true, true, false, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+            else k_element<true, false, false, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+        } else {
+            if (init) k_element<false, true, false, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+            else k_element<false, false, false, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+        }
         return;
     }
-    if (ENSC_STAGED_FP64 && !init && E.tiles_aligned) {
-        constexpr size_t smem = f64_stage_smem<kStagedBt>();
-        if (M.plastic) k_element_staged<true, kStagedBt><<<grid, kStageTileF64, smem, st>>>(E, N, M, ctl, P);
-        else k_element_staged<false, kStagedBt><<<grid, kStageTileF64, smem, st>>>(E, N, M, ctl, P);
-        return;
-    }
-    if (M.plastic) {
-        if (init) k_element<true, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-        else k_element<true, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-    } else {
-        if (init) k_element<false, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-        else k_element<false, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-    }
+    auto pick = [&](auto bt9) {
+        constexpr bool B9 = decltype(bt9)::value;
+        constexpr size_t smem = f64_pipe_smem<std::conditional_t<B9, Fp64Tile9, Fp64Tile24>>();
+        if (M.plastic) {
+            if (init) k_element<true, true, B9, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+            else k_element_fp64_warp<true, B9><<<grid, 32 * kF64PipeWarps, smem, st>>>(E, N, M, ctl, P);
+        } else {
+            if (init) k_element<false, true, B9, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+            else k_element_fp64_warp<false, B9><<<grid, 32 * kF64PipeWarps, smem, st>>>(E, N, M, ctl, P);
+        }
+    };
+    if (E.bt9) pick(std::true_type{});
+    else pick(std::false_type{});
 }
 
 void launch_node_fp64(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl, const Partials& P,
@@ -1440,37 +1368,21 @@ void launch_node_fp64(const ElemArrays& E, const NodeArrays& N, const Material& 
     k_node<<<grid, kNodeThreads, 0, st>>>(E, N, M, ctl, P);
 }
 
-int occupancy_element_fp64(bool plastic) {
+int occupancy_element_fp64(bool plastic, bool bt9) {
+    // more than the default 48 KB of dynamic shared memory: set on the current
+    // device, before any launch or capture
     int nb = 0;
-    if (ENSC_WARP_PIPE_FP64) {
-        cudaFuncSetAttribute(k_element_fp64_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kF64WarpPipeSmem));
-        cudaFuncSetAttribute(k_element_fp64_warp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kF64WarpPipeSmem));
-        if (plastic)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_fp64_warp<true>, 32 * kF64PipeWarps,
-                                                          kF64WarpPipeSmem);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_fp64_warp<false>, 32 * kF64PipeWarps,
-                                                          kF64WarpPipeSmem);
-        return nb;
+    auto query = [&nb](auto kernel, size_t smem) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, 32 * kF64PipeWarps, smem);
+    };
+    if (bt9) {
+        if (plastic) query(k_element_fp64_warp<true, true>, f64_pipe_smem<Fp64Tile9>());
+        else query(k_element_fp64_warp<false, true>, f64_pipe_smem<Fp64Tile9>());
+    } else {
+        if (plastic) query(k_element_fp64_warp<true, false>, f64_pipe_smem<Fp64Tile24>());
+        else query(k_element_fp64_warp<false, false>, f64_pipe_smem<Fp64Tile24>());
     }
-    if (ENSC_STAGED_FP64) {
-        // more than the default 48 KB of dynamic shared memory: set on the
-        // current device, before any launch or capture
-        constexpr size_t smem = f64_stage_smem<kStagedBt>();
-        cudaFuncSetAttribute(k_element_staged<true, kStagedBt>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-        cudaFuncSetAttribute(k_element_staged<false, kStagedBt>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-        if (plastic)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_staged<true, kStagedBt>, kStageTileF64, smem);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_staged<false, kStagedBt>, kStageTileF64, smem);
-        return nb;
-    }
-    if (plastic) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element<true, false>, kElemThreads, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element<false, false>, kElemThreads, 0);
     return nb;
 }
 
@@ -1489,24 +1401,29 @@ int occupancy_node_fp64() {
 }
 
 
+static size_t f64_batch_smem(int tile_room) {
+    return static_cast<size_t>(kF64PipeWarps) * (2 * (static_cast<size_t>(tile_room) + kBatchTailBytes) + 16);
+}
 void launch_element_batch_fp64(const BatchTables& T, int grid, cudaStream_t st) {
-    k_element_batch_fp64<<<grid, kF64BatchTile, kF64BatchStageSmem, st>>>(T);
+    k_element_batch_fp64<<<grid, 32 * kF64PipeWarps, f64_batch_smem(T.tile_room), st>>>(T);
 }
 void launch_node_batch_fp64(const BatchTables& T, int grid, int threads, cudaStream_t st) {
     if (threads == kNodeThreads / 2) k_node_batch_fp64<kNodeThreads / 2><<<grid, threads, 0, st>>>(T);
     else k_node_batch_fp64<kNodeThreads><<<grid, kNodeThreads, 0, st>>>(T);
 }
-int occupancy_element_batch_fp64() {
+int occupancy_element_batch_fp64(int tile_room) {
     int nb = 0;
     // dynamic shared memory above the default 48 KB: set on the current
     // device before any launch or capture
     cudaFuncSetAttribute(k_element_batch_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kF64BatchStageSmem));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_batch_fp64, kF64BatchTile, kF64BatchStageSmem);
+                         static_cast<int>(f64_batch_smem(Fp64Tile24::kBytes)));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_batch_fp64, 32 * kF64PipeWarps,
+                                                  f64_batch_smem(tile_room));
     return nb;
 }
 
-RunPlan plan_run_fp64(int64_t ne, int64_t nn, bool plastic, int sms) {
+RunPlan plan_run_fp64(int64_t ne, int64_t nn, bool plastic, bool bt9, int sms) {
+    if (!bt9) return RunPlan{};
     return plastic ? plan_run(k_run_fp64<true, true, 1>, k_run_fp64<true, true, 2>, k_run_fp64<true, false, 1>,
                               k_run_fp64<true, false, 2>, ne, nn, sms, kRunWarpsF64, RunFp64<true>::kTileBytes)
                    : plan_run(k_run_fp64<false, true, 1>, k_run_fp64<false, true, 2>, k_run_fp64<false, false, 1>,
@@ -1522,7 +1439,6 @@ cudaError_t launch_run_fp64(const RunPlan& p, const ElemArrays& E, const NodeArr
                       sync, a);
 }
 
-int batch_element_tile_fp64() { return kF64BatchTile; }
 int occupancy_node_batch_fp64(int threads) {
     int nb = 0;
     if (threads == kNodeThreads / 2)

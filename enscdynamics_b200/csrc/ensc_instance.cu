@@ -35,13 +35,15 @@ void inv3h(const double m[3][3], double r[3][3]) {
 }
 
 void element_constants(int64_t nn, int64_t ne, const uint32_t* conn, const double* x0, double rho,
-                       std::vector<double>& bt, std::vector<double>& vol0, std::vector<double>& inv_mass) {
+                       std::vector<double>& bt, std::vector<double>& vol0, std::vector<double>& inv_mass,
+                       std::vector<double>& jinv) {
     static const double XI[8][3] = {{-1., -1., -1.}, {1., -1., -1.}, {1., 1., -1.}, {-1., 1., -1.},
                                     {-1., -1., 1.},  {1., -1., 1.},  {1., 1., 1.},  {-1., 1., 1.}};
     double dn[3][8];
     for (int a = 0; a < 8; ++a)
         for (int d = 0; d < 3; ++d) dn[d][a] = 1.0 / 8.0 * XI[a][d];
     bt.assign(static_cast<size_t>(24 * ne), 0.0);
+    jinv.resize(static_cast<size_t>(9 * ne));
     vol0.assign(static_cast<size_t>(ne), 0.0);
     std::vector<double> mass(static_cast<size_t>(3 * nn), 0.0);
     for (int64_t e = 0; e < ne; ++e) {
@@ -57,6 +59,8 @@ void element_constants(int64_t nn, int64_t ne, const uint32_t* conn, const doubl
             }
         double ij[3][3];
         inv3h(jac, ij);
+        for (int r = 0; r < 3; ++r)
+            for (int c = 0; c < 3; ++c) jinv[9 * e + 3 * r + c] = ij[r][c] * 0.125;
         const double detj = det3h(jac);
         for (int a = 0; a < 8; ++a)
             for (int r = 0; r < 3; ++r)
@@ -80,30 +84,69 @@ std::vector<T> to_soa(const double* aos, int64_t n, int64_t pad, int comps) {
     return out;
 }
 
-// The rows the upload copies as they are (InstanceHost::a_rows ...): the
-// element geometry in the precision's device form, x0 and v0 as SoA rows.
-// The caller's x0 and v0 are not read after this.
-void form_device_rows(InstanceHost& h) {
-    const int64_t ep = h.ne_pad, np = h.nn_pad;
-    if (h.mixed) {
-        // corner signs s_j of the reference hexahedron (Element_HexN8.cpp:49-91)
-        static const double kCorner[8][3] = {{-1, -1, -1}, {1, -1, -1}, {1, 1, -1}, {-1, 1, -1},
-                                             {-1, -1, 1},  {1, -1, 1},  {1, 1, 1},  {-1, 1, 1}};
-        h.a_rows.assign(static_cast<size_t>(18 * ep), 0.f);
-        for (int64_t el = 0; el < h.ne; ++el)
+// B0^T row a of an element from J^-1 / 8 (p, row-major): dN/dxi is +-1/8 of the
+// corner signs, so every product above is exact, and the sums are formed in the
+// same order.
+void bt_row(const double* p, int a, double out[3]) {
+    static const double XI[8][3] = {{-1., -1., -1.}, {1., -1., -1.}, {1., 1., -1.}, {-1., 1., -1.},
+                                    {-1., -1., 1.},  {1., -1., 1.},  {1., 1., 1.},  {-1., 1., 1.}};
+    for (int r = 0; r < 3; ++r) out[r] = (p[3 * r] * XI[a][0] + p[3 * r + 1] * XI[a][1]) + p[3 * r + 2] * XI[a][2];
+}
+
+// True when J^-1 / 8 gives every B0^T number (zeros of either sign alike).
+bool bt_from_jinv(const std::vector<double>& bt, const std::vector<double>& jinv, int64_t ne) {
+    for (int64_t e = 0; e < ne; ++e)
+        for (int a = 0; a < 8; ++a) {
+            double r[3];
+            bt_row(&jinv[9 * e], a, r);
+            for (int c = 0; c < 3; ++c)
+                if (!(r[c] == bt[24 * e + 3 * a + c])) return false;
+        }
+    return true;
+}
+
+template <typename T>
+T* tile_entry(InstanceHost& h, int64_t e, uint32_t off) {
+    return reinterpret_cast<T*>(h.tiles.data() + (e >> 5) * h.const_bytes + off) + (e & 31);
+}
+
+// What the upload copies as it is (InstanceHost::tiles ...): the element
+// geometry in the precision's device form, x0 and v0 as rows.  The caller's x0
+// and v0 are not read after this.  conn: in stored order, as bt and vol0.
+void form_device_rows(InstanceHost& h, const uint32_t* conn) {
+    const int64_t np = h.nn_pad;
+    h.tiles.assign(static_cast<size_t>(h.ne_pad / 32) * h.const_bytes, 0);
+    for (int64_t el = 0; el < h.ne; ++el) {
+        for (int k = 0; k < 8; ++k) tile_entry<uint32_t>(h, el, MixedTile::kConn)[32 * k] = conn[8 * el + k];
+        const double v0 = h.vol0[el], cb = std::cbrt(v0);
+        if (h.mixed) {
+            // corner signs s_j of the reference hexahedron (Element_HexN8.cpp:49-91)
+            static const double kCorner[8][3] = {{-1, -1, -1}, {1, -1, -1}, {1, 1, -1}, {-1, 1, -1},
+                                                 {-1, -1, 1},  {1, -1, 1},  {1, 1, 1},  {-1, 1, 1}};
+            float* a = tile_entry<float>(h, el, MixedTile::kBt);
             for (int c = 0; c < 3; ++c)
                 for (int m = 0; m < 3; ++m) {
                     double v = 0.0;
                     for (int j = 0; j < 8; ++j) v += h.bt[24 * el + 3 * j + c] * kCorner[j][m];
                     const float hi = static_cast<float>(v);
-                    h.a_rows[(3 * c + m) * ep + el] = hi;
-                    h.a_rows[(9 + 3 * c + m) * ep + el] = static_cast<float>(v - static_cast<double>(hi));
+                    a[32 * (3 * c + m)] = hi;
+                    a[32 * (9 + 3 * c + m)] = static_cast<float>(v - static_cast<double>(hi));
                 }
-        h.cb_f.assign(h.cb.begin(), h.cb.end());
-    } else {
-        h.bt_rows = to_soa<double>(h.bt.data(), h.ne, ep, 24);
+            *tile_entry<double>(h, el, MixedTile::kVol0) = v0;
+            *tile_entry<float>(h, el, MixedTile::kCb) = static_cast<float>(cb);
+        } else {
+            const double* src = h.bt9 ? &h.jinv[9 * el] : &h.bt[24 * el];
+            double* t = tile_entry<double>(h, el, Fp64Tile9::kBt);
+            for (int i = 0; i < (h.bt9 ? 9 : 24); ++i) t[32 * i] = src[i];
+            double* c = tile_entry<double>(h, el, h.bt9 ? Fp64Tile9::kVol0 : Fp64Tile24::kVol0);
+            c[0] = v0;
+            c[32] = cb;
+            c[64] = std::cbrt(v0 * v0);
+        }
     }
-    std::vector<double>().swap(h.bt);  // the device form replaces it
+    std::vector<double>().swap(h.bt);  // the device form replaces them
+    std::vector<double>().swap(h.jinv);
+    std::vector<double>().swap(h.vol0);
     h.x_rows = to_soa<double>(h.x0, h.nn, np, 3);
     if (h.v0) {
         if (h.mixed) {
@@ -268,7 +311,14 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
         h.vol0.assign(mesh->vol0, mesh->vol0 + ne);
         inv_mass_dof.assign(mesh->inv_mass, mesh->inv_mass + 3 * nn);
     } else {
-        element_constants(nn, ne, mesh->conn, mesh->x0, mat->rho, h.bt, h.vol0, inv_mass_dof);
+        element_constants(nn, ne, mesh->conn, mesh->x0, mat->rho, h.bt, h.vol0, inv_mass_dof, h.jinv);
+        h.bt9 = !mixed;
+    }
+    if (!mixed && !h.bt9) {
+        // a caller's own B0^T: the 9 numbers, where they give its very bits
+        std::vector<double> bt, vol0, inv_mass;
+        element_constants(nn, ne, mesh->conn, mesh->x0, mat->rho, bt, vol0, inv_mass, h.jinv);
+        h.bt9 = bt_from_jinv(h.bt, h.jinv, ne);
     }
 
     // no node repeating a local slot: slot-major forces, and patches allowed
@@ -316,18 +366,8 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
         build_patches(nn, ne, conn, h);
     }
 
-    h.cb.resize(ne);
-    h.cb2.resize(ne);
-    for (int64_t e = 0; e < ne; ++e) {
-        h.cb[e] = std::cbrt(h.vol0[e]);
-        h.cb2[e] = std::cbrt(h.vol0[e] * h.vol0[e]);
-    }
     h.im.assign(static_cast<size_t>(np), 1.0);
     for (int64_t n = 0; n < nn; ++n) h.im[n] = inv_mass_dof[3 * n];
-    h.conn_soa.assign(static_cast<size_t>(8 * ep), 0);
-    for (int64_t e = 0; e < ne; ++e)
-        for (int k = 0; k < 8; ++k) h.conn_soa[k * ep + e] = conn[8 * e + k];
-
     // node-to-element tables
     h.ell.assign(static_cast<size_t>(8 * np), ENSC_NONE);
     if (!h.clash) {
@@ -362,16 +402,9 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
     const size_t E8 = static_cast<size_t>(ep), N8 = static_cast<size_t>(np);
     const size_t fe_rows = h.clash ? E8 : N8;
     using P = InstanceHost::Piece;
-    h.size[P::CONN] = 8 * E8 * sizeof(uint32_t);
-    // FP64: B0^T rows as given; mixed: the 3x3 matrix A = sum_j B0_j s_j^T
-    // (B0_j = A s_j / 8) as 9 hi and 9 lo float rows
-    h.size[P::BT] = (mixed ? 18 : 24) * E8 * real;
-    h.size[P::VOL0] = E8 * 8;
-    h.size[P::CB] = E8 * 8;
-    h.size[P::CB2] = E8 * 8;
-    h.size[P::SIG] = 6 * E8 * real;
-    h.size[P::QIA] = 12 * E8 * real;
-    h.size[P::EPS] = E8 * real;
+    h.tile_bytes = mixed ? MixedTile::kBytes : (h.bt9 ? Fp64Tile9::kBytes : Fp64Tile24::kBytes);
+    h.const_bytes = mixed ? MixedTile::kState : (h.bt9 ? Fp64Tile9::kState : Fp64Tile24::kState);
+    h.size[P::TILES] = static_cast<size_t>(ep / 32) * h.tile_bytes;
     h.size[P::FE] = 24 * fe_rows * real;
     h.size[P::X] = 3 * N8 * 8;
     h.size[P::U] = 3 * N8 * 8;
@@ -401,7 +434,7 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
         total += (h.size[i] + 255) / 256 * 256;
     }
     h.bytes = total;
-    form_device_rows(h);
+    form_device_rows(h, conn);
     return ENSC_OK;
 }
 
@@ -411,17 +444,9 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     const int64_t ep = h.ne_pad, np = h.nn_pad;
     char* b = static_cast<char*>(block);
     cudaError_t e = cudaMemsetAsync(block, 0, h.bytes, st);
-    if (h.mixed) {
-        if (e == cudaSuccess) e = put(block, h.off[P::BT], h.a_rows, st);
-        if (e == cudaSuccess) e = put(block, h.off[P::VOL0], h.vol0, st);
-        if (e == cudaSuccess) e = put(block, h.off[P::CB], h.cb_f, st);
-    } else {
-        if (e == cudaSuccess) e = put(block, h.off[P::BT], h.bt_rows, st);
-        if (e == cudaSuccess) e = put(block, h.off[P::VOL0], h.vol0, st);
-        if (e == cudaSuccess) e = put(block, h.off[P::CB], h.cb, st);
-        if (e == cudaSuccess) e = put(block, h.off[P::CB2], h.cb2, st);
-    }
-    if (e == cudaSuccess) e = put(block, h.off[P::CONN], h.conn_soa, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpy2DAsync(b + h.off[P::TILES], h.tile_bytes, h.tiles.data(), h.const_bytes, h.const_bytes,
+                              static_cast<size_t>(ep / 32), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = put(block, h.off[P::IM], h.im, st);
     if (e == cudaSuccess) e = put(block, h.off[P::X], h.x_rows, st);
     // mixed: the u rows hold the reference position x - u, x0 at the start
@@ -461,16 +486,24 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     E = ElemArrays{};
     E.ne = h.ne;
     E.ne_pad = ep;
-    E.conn = reinterpret_cast<uint32_t*>(b + h.off[P::CONN]);
-    E.bt = b + h.off[P::BT];
-    E.vol0 = reinterpret_cast<double*>(b + h.off[P::VOL0]);
-    E.cbrt_v0 = reinterpret_cast<double*>(b + h.off[P::CB]);
-    E.cbrt_v0sq = reinterpret_cast<double*>(b + h.off[P::CB2]);
-    E.sigma = b + h.off[P::SIG];
-    E.qia = b + h.off[P::QIA];
-    E.eps_p = b + h.off[P::EPS];
+    auto point = [&](auto layout) {
+        using L = decltype(layout);
+        char* t = b + h.off[P::TILES];
+        E.conn = reinterpret_cast<uint32_t*>(t + L::kConn);
+        E.bt = t + L::kBt;
+        E.vol0 = reinterpret_cast<double*>(t + L::kVol0);
+        E.cbrt_v0 = t + L::kCb;
+        E.cbrt_v0sq = h.mixed ? nullptr : reinterpret_cast<double*>(t + L::kCb + L::kRow);
+        E.sigma = t + L::kSig;
+        E.qia = t + L::kQia;
+        E.eps_p = t + L::kEps;
+    };
+    if (h.mixed) point(MixedTile{});
+    else if (h.bt9) point(Fp64Tile9{});
+    else point(Fp64Tile24{});
     E.fe = b + h.off[P::FE];
-    E.tiles_aligned = 1;  // pieces are 256-byte aligned, ne_pad % 32 == 0
+    E.tile_bytes = h.tile_bytes;  // pieces are 256-byte aligned, rows padded to 32
+    E.bt9 = h.bt9 ? 1 : 0;
     E.slot_major = h.clash ? 0 : 1;
     PA = PatchArrays{};
     if (h.patch) {

@@ -19,9 +19,9 @@ namespace ensc {
 struct InstanceHost {
     int64_t nn = 0, ne = 0, nn_pad = 0, ne_pad = 0;
     bool mixed = false, plastic = false, clash = false;
-    std::vector<uint32_t> conn_soa;   // [8][ne_pad]
     std::vector<double> bt;           // [ne][24] row-major B0^T
-    std::vector<double> vol0, cb, cb2;  // [ne] V0, cbrt(V0), cbrt(V0^2)
+    std::vector<double> jinv;         // [ne][9] J^-1 / 8 where bt9
+    std::vector<double> vol0;         // [ne] V0
     std::vector<double> im;           // [nn_pad] inverse lumped mass per node
     std::vector<uint32_t> ell;        // [8][nn_pad] element in slot k, or ENSC_NONE
     std::vector<uint8_t> slot_mask;   // [nn_pad] occupied slots (clash-free meshes)
@@ -29,15 +29,18 @@ struct InstanceHost {
     std::vector<uint32_t> csr_ent;
     const double* x0 = nullptr;       // caller arrays, read by instance_prepare only
     const double* v0 = nullptr;
-    // the rows the upload copies as they are, formed by instance_prepare (so
-    // that a prepared instance's host work is done before its device part):
-    // mixed: A float pairs [18][ne_pad], cbrt(V0) as float [ne], v float
-    // rows [3][nn_pad] and their 16-bit residual rows [3][nn_pad]; FP64:
-    // B0^T [24][ne_pad], v [3][nn_pad]; both: x0 [3][nn_pad] (v rows empty
+    // what the upload copies as it is, formed by instance_prepare (so that a
+    // prepared instance's host work is done before its device part): the
+    // constant part of every element tile (connectivity, geometry, V0 and its
+    // roots), const_bytes each; x0 [3][nn_pad]; mixed: v float rows [3][nn_pad] and
+    // their 16-bit residual rows [3][nn_pad]; FP64: v [3][nn_pad] (v rows empty
     // when the mesh has no initial velocities)
-    std::vector<float> a_rows, cb_f, v_rows_f;
+    int32_t tile_bytes = 0, const_bytes = 0;
+    bool bt9 = false;                 // FP64: 9 numbers per element give B0^T bit for bit
+    std::vector<unsigned char> tiles;
+    std::vector<float> v_rows_f;
     std::vector<int16_t> v_lo_rows;
-    std::vector<double> bt_rows, x_rows, v_rows_d;
+    std::vector<double> x_rows, v_rows_d;
     // patch assembly (ElemArrays::patch): the stored order of the elements
     // and the patch tables; all element arrays above are in stored order
     bool patch = false;
@@ -50,7 +53,7 @@ struct InstanceHost {
     int64_t n_patches = 0, n_pnodes = 0;
     // device layout: byte offsets of the pieces in one 256-byte-aligned block
     enum Piece {
-        CONN, BT, VOL0, CB, CB2, SIG, QIA, EPS, FE, X, U, V, IM, BC, BCV, ELL, RF, CPTR, CENT, MASK,
+        TILES, FE, X, U, V, IM, BC, BCV, ELL, RF, CPTR, CENT, MASK,
         IPERM, PFOFF, PINCOFF, PINC, PF, NPTR, NENT, NPIECE
     };
     size_t off[NPIECE] = {};

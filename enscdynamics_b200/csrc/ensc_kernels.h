@@ -18,31 +18,13 @@ constexpr int kElemThreads = 128;
 #ifndef ENSC_ELEM_MINB_MIXED
 #define ENSC_ELEM_MINB_MIXED 6
 #endif
-// Unroll factor of the element passes' loops over the 8 nodes: more in-flight
-// gathers per thread against more live registers.
-#ifndef ENSC_NODE_UNROLL_FP64
-#define ENSC_NODE_UNROLL_FP64 8
+// the mixed element passes: warps per block, each with its own pipeline of
+// 32-element tiles, and resident blocks per SM
+#ifndef ENSC_MIXED_PIPE_WARPS
+#define ENSC_MIXED_PIPE_WARPS 4
 #endif
-#ifndef ENSC_NODE_UNROLL_MIXED
-#define ENSC_NODE_UNROLL_MIXED 4
-#endif
-constexpr int kNodeUnrollFp64 = ENSC_NODE_UNROLL_FP64;
-constexpr int kNodeUnrollMixed = ENSC_NODE_UNROLL_MIXED;
-// Mixed element pass with its streamed inputs staged in shared memory by
-// bulk copies (k_element_mixed_staged) instead of per-thread loads.
-#ifndef ENSC_STAGED_MIXED
-#define ENSC_STAGED_MIXED 1
-#endif
-// elements per stage (= threads per block) and resident blocks per SM of
-// the staged mixed pass; tuned on B200
-#ifndef ENSC_STAGE_TILE_MIXED
-#define ENSC_STAGE_TILE_MIXED 64
-#endif
-#ifndef ENSC_STAGE_MINB_MIXED
-#define ENSC_STAGE_MINB_MIXED 8
-#endif
-#ifndef ENSC_BATCH_MINB_MIXED
-#define ENSC_BATCH_MINB_MIXED 8
+#ifndef ENSC_MIXED_PIPE_MINB
+#define ENSC_MIXED_PIPE_MINB 4
 #endif
 // 1: the staged mixed element passes read A and the connectivity from the
 // stage again for the force step instead of keeping them in registers
@@ -63,12 +45,6 @@ constexpr int kNodeUnrollMixed = ENSC_NODE_UNROLL_MIXED;
 #ifndef ENSC_BATCH_MIXED_PREFETCH
 #define ENSC_BATCH_MIXED_PREFETCH 0
 #endif
-// how the batched mixed element pass reads the staged instance descriptor:
-// 1 all fields copied to registers per tile, 2 arrays copied and material
-// constants read at use, 0 everything read at use
-#ifndef ENSC_BATCH_DESC_MODE
-#define ENSC_BATCH_DESC_MODE 2
-#endif
 // 1: the grouped node passes sum all 8 force slots (empty ones hold zeros)
 // instead of reading the slot mask first (measured on B200, mixed: reading
 // the mask made the node pass 22% slower on the block and the batched
@@ -80,45 +56,19 @@ constexpr int kNodeUnrollMixed = ENSC_NODE_UNROLL_MIXED;
 #ifndef ENSC_NODE_BATCH_MINB_MIXED
 #define ENSC_NODE_BATCH_MINB_MIXED 2
 #endif
-// FP64 element pass staged the same way: 0 off, 1 staging all streamed
-// inputs except B0^T (read from global memory), 2 staging B0^T too.
-#ifndef ENSC_STAGED_FP64
-#define ENSC_STAGED_FP64 2
-#endif
-// 1: the single-instance FP64 element pass runs one bulk-copy pipeline per
-// warp (k_element_fp64_warp: 32-element tiles, two stages per warp, no
-// block-wide barrier per tile) instead of one per block (measured on B200
-// on the block workload: 0.6% faster; the same structure for the mixed
-// passes was 1-3% slower than their per-block pipelines)
-#ifndef ENSC_WARP_PIPE_FP64
-#define ENSC_WARP_PIPE_FP64 1
-#endif
+// the FP64 element passes: warps per block, each with its own pipeline of
+// 32-element tiles, and resident blocks per SM
 #ifndef ENSC_F64_PIPE_WARPS
 #define ENSC_F64_PIPE_WARPS 4
 #endif
-// 1: the warp-pipelined FP64 pass stages B0^T too; 0: reads it through L1
-#ifndef ENSC_F64_WARP_BT
-#define ENSC_F64_WARP_BT 1
+#ifndef ENSC_F64_PIPE_MINB
+#define ENSC_F64_PIPE_MINB 2
 #endif
 // The FP64 warp-pipelined element pass prefetches an element's node rows
 // into L1 once its connectivity is staged: bit 0 the velocities, bit 1 the
 // displacements
 #ifndef ENSC_F64_PREFETCH
 #define ENSC_F64_PREFETCH 3
-#endif
-// elements per tile of the batched FP64 element pass, one block of as many
-// threads per tile (32 would make every block one warp with its own
-// two-stage pipeline, as in the single-instance pass: 2% slower on the
-// 256-instance sweep, 0.6% faster on the block)
-#ifndef ENSC_F64_BATCH_TILE
-#define ENSC_F64_BATCH_TILE 128
-#endif
-#ifndef ENSC_F64_PIPE_MINB
-#define ENSC_F64_PIPE_MINB 2
-#endif
-// elements per stage (= threads per block) of the staged FP64 passes
-#ifndef ENSC_STAGE_TILE_FP64
-#define ENSC_STAGE_TILE_FP64 128
 #endif
 constexpr int kNodeThreads = 256;
 constexpr int kCtlThreads = 256;
@@ -152,7 +102,7 @@ struct RunPlan {
     int node_width = 1;        // nodes per thread of the node phase
     size_t smem = 0;
 };
-RunPlan plan_run_fp64(int64_t ne, int64_t nn, bool plastic, int sms);
+RunPlan plan_run_fp64(int64_t ne, int64_t nn, bool plastic, bool bt9, int sms);
 RunPlan plan_run_mixed(int64_t ne, int64_t nn, bool plastic, int sms);
 cudaError_t launch_run_fp64(const RunPlan& p, const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
                             const Partials& P, RunSync* sync, const RunArgs& a, cudaStream_t st);
@@ -164,7 +114,7 @@ void launch_element_fp64(const ElemArrays& E, const NodeArrays& N, const Materia
                          int grid, bool init, cudaStream_t st);
 void launch_node_fp64(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl, const Partials& P,
                       int grid, cudaStream_t st);
-int occupancy_element_fp64(bool plastic);
+int occupancy_element_fp64(bool plastic, bool bt9);
 // nodes per thread of the node pass on the padded slot-major layout
 #ifndef ENSC_NODE_GROUP_MIXED
 #define ENSC_NODE_GROUP_MIXED 4
@@ -194,7 +144,7 @@ void launch_element_mixed(const ElemArrays& E, const NodeArrays& N, const Materi
                           int grid, bool init, cudaStream_t st, const PatchArrays& PA = PatchArrays{});
 void launch_node_mixed(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl, const Partials& P,
                        int grid, cudaStream_t st, const PatchArrays& PA = PatchArrays{});
-int occupancy_element_mixed(bool plastic);
+int occupancy_element_mixed(bool plastic, bool patch);
 int occupancy_node_mixed();
 
 // the last cycle's acceleration (compute_a), interleaved xyz per node, from
@@ -208,16 +158,15 @@ void launch_acceleration_mixed(const ElemArrays& E, const NodeArrays& N, const M
 void launch_element_batch_fp64(const BatchTables& T, int grid, cudaStream_t st);
 // threads per block of the batched node passes: kNodeThreads or half of it
 void launch_node_batch_fp64(const BatchTables& T, int grid, int threads, cudaStream_t st);
-int occupancy_element_batch_fp64();
+int occupancy_element_batch_fp64(int tile_room);
 int occupancy_node_batch_fp64(int threads);
-void launch_element_batch_mixed(const BatchTables& T, int grid, int ept, bool patch, cudaStream_t st);
+void launch_element_batch_mixed(const BatchTables& T, int grid, bool patch, cudaStream_t st);
 void launch_node_batch_mixed(const BatchTables& T, int grid, int threads, bool patch, cudaStream_t st);
-int occupancy_element_batch_mixed(int ept);
+int occupancy_element_batch_mixed(bool patch);
 int occupancy_node_batch_mixed(int threads);
-// elements and nodes per batch tile (element tiles are the staged passes'
-// tiles; node tiles are one warp of node groups)
-int batch_element_tile(bool mixed_precision);
-int batch_element_tile_fp64();
+// elements and nodes per batch tile (element tiles are the tiles of 32, or
+// patches; node tiles are one warp of node groups)
+int batch_element_tile(bool patch);
 int batch_node_tile(bool mixed_precision);
 void launch_between_batch(const BatchTables& T, int slots, int mode, cudaStream_t st);
 void launch_edge_prepass_batch(const BatchTables& T, int grid, cudaStream_t st);
@@ -234,13 +183,15 @@ void launch_arm(Ctl* ctl, double step_end, long long max_cycles, cudaStream_t st
 void launch_apply_bc_v(const NodeArrays& N, bool fp32_v, cudaStream_t st);
 void launch_reset_init(Ctl* ctl, cudaStream_t st);
 void launch_kinetic0(const NodeArrays& N, const Partials& P, Ctl* ctl, bool fp32_v, int grid, cudaStream_t st);
-// layout conversion between caller AoS arrays and device SoA arrays
-// `at` (may be null): entry e of the interleaved array is SoA row position
-// at[e] -- an element's stored position under the patch order
-void launch_soa_to_aos(const void* soa, int64_t n, int64_t pad, int comps, bool src_fp32, double* aos,
-                       cudaStream_t st, const int32_t* at = nullptr);
-void launch_aos_to_soa(const double* aos, int64_t n, int64_t pad, int comps, void* soa, bool dst_fp32,
-                       cudaStream_t st, const int32_t* at = nullptr);
+// layout conversion between caller AoS arrays and node rows, or the element
+// rows at `rows` of E.  `at` (may be null): entry e of the interleaved array is
+// row position at[e] -- an element's stored position under the patch order
+void launch_soa_to_aos(const double* soa, int64_t n, int64_t pad, int comps, double* aos, cudaStream_t st);
+void launch_aos_to_soa(const double* aos, int64_t n, int64_t pad, int comps, double* soa, cudaStream_t st);
+void launch_elem_to_aos(const ElemArrays& E, const void* rows, int comps, bool src_fp32, double* aos, cudaStream_t st,
+                        const int32_t* at = nullptr);
+void launch_aos_to_elem(const double* aos, const ElemArrays& E, int comps, void* rows, bool dst_fp32, cudaStream_t st,
+                        const int32_t* at = nullptr);
 // displacements of a mixed instance (u rows holding xr = x - u) to
 // interleaved xyz doubles; and a <- x - a over three node rows
 void launch_disp_to_aos(const double* x, const double* xr, int64_t n, int64_t pad, double* aos, cudaStream_t st);

@@ -8,10 +8,10 @@
 // order is free here (FMA contraction on), accuracy is checked against the
 // FP64 path by relative displacement error and energy drift.
 //
-// Element arrays: the bt rows hold A = sum_j B0_j s_j^T (the one-point B0
-// rows are A s_j / 8, s_j the node's reference-corner signs) as a float pair,
-// 9 hi then 9 lo rows; sigma, qia, eps_p and fe are float; vol0 is double;
-// cbrt_v0 is a float copy (in the first ne words of its FP64 storage).
+// Element arrays (MixedTile): the bt rows hold A = sum_j B0_j s_j^T (the
+// one-point B0 rows are A s_j / 8, s_j the node's reference-corner signs) as a
+// float pair, 9 hi then 9 lo rows; cbrt_v0, sigma, qia, eps_p and fe are float;
+// vol0 is double.
 // Node arrays: x double; the u rows hold the reference position x - u
 // (double, ENSC_MIXED_UREF); v float with 16-bit residual rows.
 #include "ensc_device.cuh"
@@ -104,9 +104,8 @@ __device__ __forceinline__ void block_min2_d(double a, double b, unsigned long l
 // transforms below.  The hourglass force uses the reassociated sum
 // sum_k ATAU(k,j) (QIA(i,k) + CR HIA(i,k))  (exDyna3D.cpp:1053-1070).
 
-// Where one element's inputs are read from: rows of `stride` entries with the
-// element at `i` -- the instance's own arrays in global memory, or a
-// shared-memory stage that holds a tile of them.
+// Where one element's inputs are read from and its evolving rows written: a
+// tile of 32 elements, in global or shared memory, with the element at `i`.
 struct MixedSrc {
     const uint32_t* conn;   // [8] rows
     const float* a;         // [18] rows: A hi (3c+m), then A lo
@@ -115,19 +114,33 @@ struct MixedSrc {
     const float* sig;       // [6] rows
     const float* qia;       // [12] rows
     const float* eps;
-    int64_t stride, i;
+    int i;
 };
-
-__device__ __forceinline__ MixedSrc mixed_src_global(const ElemArrays& E, int64_t e) {
-    return MixedSrc{E.conn,
-                    static_cast<const float*>(E.bt),
-                    E.vol0,
-                    reinterpret_cast<const float*>(E.cbrt_v0),
-                    static_cast<const float*>(E.sigma),
-                    static_cast<const float*>(E.qia),
-                    static_cast<const float*>(E.eps_p),
-                    E.ne_pad,
-                    e};
+struct MixedOut {
+    float* sig;             // [6] rows
+    float* qia;             // [12] rows
+    float* eps;
+    int i;
+};
+__device__ __forceinline__ MixedSrc mixed_src_tile(const unsigned char* t, int lane) {
+    using L = MixedTile;
+    return MixedSrc{reinterpret_cast<const uint32_t*>(t),
+                    reinterpret_cast<const float*>(t + L::kBt),
+                    reinterpret_cast<const double*>(t + L::kVol0),
+                    reinterpret_cast<const float*>(t + L::kCb),
+                    reinterpret_cast<const float*>(t + L::kSig),
+                    reinterpret_cast<const float*>(t + L::kQia),
+                    reinterpret_cast<const float*>(t + L::kEps),
+                    lane};
+}
+__device__ __forceinline__ MixedOut mixed_out_tile(unsigned char* t, int lane) {
+    using L = MixedTile;
+    return MixedOut{reinterpret_cast<float*>(t + L::kSig), reinterpret_cast<float*>(t + L::kQia),
+                    reinterpret_cast<float*>(t + L::kEps), lane};
+}
+// tile t of an instance in global memory
+__device__ __forceinline__ unsigned char* mixed_tile(const ElemArrays& E, int64_t t) {
+    return const_cast<unsigned char*>(reinterpret_cast<const unsigned char*>(E.conn)) + t * MixedTile::kBytes;
 }
 
 // The one-point B0 row of local node j is A s_j / 8 with A = sum_j B0_j s_j^T
@@ -175,19 +188,6 @@ __device__ __forceinline__ void corner_values(T (&c)[8], T (&a)[8]) {
     for (int j = 0; j < 8; ++j) a[j] = c[kBits[j]];
 }
 
-// Where one element's evolving rows are written: the instance's own arrays,
-// or the shared-memory tile that a resident run keeps them in.
-struct MixedOut {
-    float* sig;             // [6] rows
-    float* qia;             // [12] rows
-    float* eps;
-    int64_t stride, i;
-};
-
-__device__ __forceinline__ MixedOut mixed_out_global(const ElemArrays& E, int64_t e) {
-    return MixedOut{static_cast<float*>(E.sigma), static_cast<float*>(E.qia), static_cast<float*>(E.eps_p), E.ne_pad, e};
-}
-
 // One element of the mixed element pass (see the kernel comment below);
 // shared by the single-instance, staged, batched and resident-run kernels.
 // Inputs come from S, the evolving rows go to O and the forces to the
@@ -203,7 +203,7 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
                                                    const double dt1d, const int64_t e, double& dts, double& len,
                                                    double& e_int, double& e_hg, double& e_vis, int32_t& bad,
                                                    float* fout = nullptr) {
-    const int64_t ep = E.ne_pad, np = N.nn_pad, ss = S.stride, si = S.i, os = O.stride, oi = O.i;
+    const int64_t ep = E.ne_pad, np = N.nn_pad, ss = 32, si = S.i, os = 32, oi = O.i;
     float* fe = static_cast<float*>(E.fe);
     const double* X = N.x;
     const float* V = static_cast<const float*>(N.v);
@@ -508,188 +508,141 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
     if (!isfinite(dts)) bad |= ST_NONFINITE;
 }
 
-template <bool PLASTIC, bool INIT>
+// The init force pass (dt = 0, no state written, no energy), from the tiles
+// in global memory.
+template <bool PLASTIC>
 __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_MIXED)
-    k_element_mixed(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
+    k_element_mixed_init(ElemArrays E, NodeArrays N, Material M, Ctl* ctl) {
     if (ctl->done) return;
-    const float dt1 = INIT ? 0.f : static_cast<float>(ctl->dt_i_1);
-    const double dt1d = INIT ? 0.0 : ctl->dt_i_1;
     const int64_t ne = E.ne;
     double e_int = 0.0, e_hg = 0.0, e_vis = 0.0;
     double dts_min = DBL_MAX, len_min = DBL_MAX;
     int32_t bad = 0;
-
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < ne; e += stride) {
+        unsigned char* g = mixed_tile(E, e >> 5);
+        const int lane = static_cast<int>(e & 31);
         double dts, len;
-        element_body_mixed<PLASTIC, INIT>(E, N, M, mixed_src_global(E, e), mixed_out_global(E, e), dt1, dt1d, e, dts, len,
+        element_body_mixed<PLASTIC, true>(E, N, M, mixed_src_tile(g, lane), mixed_out_tile(g, lane), 0.f, 0.0, e, dts, len,
                                           e_int, e_hg, e_vis, bad);
         dts_min = fmin(dts_min, dts);
         len_min = fmin(len_min, len);
     }
     if (bad) atomicOr(&ctl->status, bad);
     block_min2_d<kElemThreads>(dts_min, len_min, &ctl->dts_next, &ctl->len_min);
-    if (!INIT) {
-        double v3[3] = {e_int, e_hg, e_vis};
-        block_sum_d<kElemThreads, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
-    }
 }
 
-// ---- staged element pass ------------------------------------------------
-// Each block walks tiles of kStageTile consecutive elements.  Thread 0 copies
-// a tile's streamed inputs -- connectivity, the B0 matrix A (hi and lo),
-// sigma, QIA, cbrt(V0), eps_p and V0 -- into one of two
-// shared-memory stages with bulk copies, one tile ahead of the compute; the
-// block then evaluates the tile with element_body_mixed reading those inputs
-// from the stage while the next tile's copies are in flight.  Node data are
-// gathered from global memory as in the unstaged pass, and all outputs are
-// written there.
-constexpr int kStageTile = ENSC_STAGE_TILE_MIXED;
-// stage: 46 rows of 4-byte words (8 conn, 18 A, 6 sigma, 12 QIA, cbrt(V0),
-// eps_p), then V0 as a row of doubles
-constexpr int kStageWordRows = 46;
-constexpr uint32_t kStageV0Off = kStageWordRows * kStageTile * 4;
-constexpr uint32_t kStageBytes = kStageV0Off + kStageTile * 8;
-constexpr size_t kStageSmem = 2 * static_cast<size_t>(kStageBytes) + 16;  // two stages, two barriers
+// ---- warp-pipelined element pass -----------------------------------------
+// Every warp runs its own pipeline over tiles of 32 consecutive elements: two
+// shared-memory stages, each filled by one bulk copy of a whole tile while
+// the other is computed, and no block-wide barrier per tile.  Node data are
+// gathered from global memory, and all outputs are written there.
+constexpr int kMixedPipeWarps = ENSC_MIXED_PIPE_WARPS;
+constexpr size_t kMixedPipeSmem = static_cast<size_t>(kMixedPipeWarps) * (2 * MixedTile::kBytes + 16);
 
-// word row r of the stage in global memory
-__device__ __forceinline__ const float* stage_row(const ElemArrays& E, int r) {
-    const int64_t ep = E.ne_pad;
-    if (r < 8) return reinterpret_cast<const float*>(E.conn + r * ep);
-    if (r < 26) return static_cast<const float*>(E.bt) + (r - 8) * ep;
-    if (r < 32) return static_cast<const float*>(E.sigma) + (r - 26) * ep;
-    if (r < 44) return static_cast<const float*>(E.qia) + (r - 32) * ep;
-    if (r == 44) return reinterpret_cast<const float*>(E.cbrt_v0);
-    return static_cast<const float*>(E.eps_p);
-}
-
-// Warp 0 copies the tile starting at element `base` into the stage at
-// shared address dst, completing on bar: lane 0 arms the barrier with the
-// byte count, then the lanes start the row copies between them.  The rows
-// are padded to a multiple of 32 entries and start 256-byte aligned, so
-// every copy is 16-byte aligned and a multiple of 128 bytes long.
+// Lane 0: the tile at src into shared memory at dst, completing on bar
+// (elastic instances leave out eps_p, the tile's last row).
 template <bool PLASTIC>
-__device__ __forceinline__ uint32_t stage_count(const ElemArrays& E, int64_t base) {
-    const int64_t left = E.ne_pad - base;
-    return static_cast<uint32_t>(left < kStageTile ? left : kStageTile);
-}
-template <bool PLASTIC>
-__device__ __forceinline__ uint32_t stage_tx_bytes(uint32_t cnt) {
-    constexpr int rows = PLASTIC ? kStageWordRows : kStageWordRows - 1;  // eps_p last, J2 only
-    return rows * cnt * 4u + cnt * 8u;
-}
-template <bool PLASTIC>
-__device__ __forceinline__ void stage_issue(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t base, int lane) {
-    constexpr int rows = PLASTIC ? kStageWordRows : kStageWordRows - 1;
-    const uint32_t cnt = stage_count<PLASTIC>(E, base);
-    if (lane == 0) mbar_arrive_expect_tx(bar, stage_tx_bytes<PLASTIC>(cnt));
-    __syncwarp();
-    fence_proxy_async_smem();  // the block's reads of this stage come before the copies into it
-    for (int r = lane; r <= rows; r += 32) {
-        if (r < rows) bulk_g2s(dst + r * (kStageTile * 4u), stage_row(E, r) + base, cnt * 4u, bar);
-        else bulk_g2s(dst + kStageV0Off, E.vol0 + base, cnt * 8u, bar);
-    }
+__device__ __forceinline__ void mixed_tile_issue(const void* src, uint32_t dst, uint32_t bar) {
+    constexpr uint32_t bytes = PLASTIC ? MixedTile::kBytes : MixedTile::kEps;
+    mbar_arrive_expect_tx(bar, bytes);
+    fence_proxy_async_smem();  // the warp's reads of this stage come before the copy into it
+    bulk_g2s(dst, src, bytes, bar);
 }
 
 template <bool PLASTIC>
-__global__ void __launch_bounds__(kStageTile, ENSC_STAGE_MINB_MIXED)
-    k_element_mixed_staged(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
+__global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
+    k_element_mixed_warp(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
     if (ctl->done) return;
+    constexpr uint32_t SB = MixedTile::kBytes;
     extern __shared__ __align__(128) unsigned char smem[];
     const float dt1 = static_cast<float>(ctl->dt_i_1);
     const double dt1d = ctl->dt_i_1;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const uint32_t stage0 = smem_addr(smem);
-    const uint32_t bar0 = stage0 + 2 * kStageBytes;
-    const int64_t ntiles = (E.ne + kStageTile - 1) / kStageTile;
-    const int64_t gstride = gridDim.x;
-    if (tid == 0) {
+    unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
+    const uint32_t stage0 = smem_addr(wst);
+    const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kMixedPipeWarps) * 2 * SB) + 16u * wid;
+    const int64_t ntiles = (E.ne + 31) / 32;
+    const int64_t wstride = static_cast<int64_t>(gridDim.x) * kMixedPipeWarps;
+    const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kMixedPipeWarps + wid;
+    if (lane == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
-    }
-    __syncthreads();
-    if (wid == 0) {
         for (int s = 0; s < 2; ++s) {
-            const int64_t t = blockIdx.x + s * gstride;
-            if (t < ntiles) stage_issue<PLASTIC>(E, stage0 + s * kStageBytes, bar0 + 8 * s, t * kStageTile, lane);
+            const int64_t t = w0 + s * wstride;
+            if (t < ntiles) mixed_tile_issue<PLASTIC>(mixed_tile(E, t), stage0 + s * SB, bar0 + 8 * s);
         }
     }
+    __syncwarp();
     double e_int = 0.0, e_hg = 0.0, e_vis = 0.0;
     double dts_min = DBL_MAX, len_min = DBL_MAX;
     int32_t bad = 0;
     bool timed_out = false;
     int it = 0;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gstride, ++it) {
+    for (int64_t t = w0; t < ntiles; t += wstride, ++it) {
         const int s = it & 1;
         const uint32_t bar = bar0 + 8 * s;
         const bool ok = mbar_wait_bounded(bar, (it >> 1) & 1);
-        if (__syncthreads_or(!ok)) {
+        if (__any_sync(0xffffffffu, !ok)) {
             timed_out = true;
             break;
         }
-        const int64_t e = t * kStageTile + tid;
+        const int64_t e = t * 32 + lane;
         if (e < E.ne) {
-            const float* st = reinterpret_cast<const float*>(smem + s * kStageBytes);
-            const MixedSrc S{reinterpret_cast<const uint32_t*>(st),
-                             st + 8 * kStageTile,
-                             reinterpret_cast<const double*>(smem + s * kStageBytes + kStageV0Off),
-                             st + 44 * kStageTile,
-                             st + 26 * kStageTile,
-                             st + 32 * kStageTile,
-                             st + 45 * kStageTile,
-                             kStageTile,
-                             tid};
             double dts, len;
-            element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(E, N, M, S, mixed_out_global(E, e), dt1, dt1d, e,
-                                                                          dts, len, e_int, e_hg, e_vis, bad);
+            element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(
+                E, N, M, mixed_src_tile(wst + s * SB, lane), mixed_out_tile(mixed_tile(E, t), lane), dt1, dt1d, e, dts,
+                len, e_int, e_hg, e_vis, bad);
             dts_min = fmin(dts_min, dts);
             len_min = fmin(len_min, len);
         }
-        __syncthreads();  // the block is done with stage s
-        const int64_t tn = t + 2 * gstride;
-        if (wid == 0 && tn < ntiles) stage_issue<PLASTIC>(E, stage0 + s * kStageBytes, bar, tn * kStageTile, lane);
+        __syncwarp();  // all lanes are done with stage s
+        const int64_t tn = t + 2 * wstride;
+        if (lane == 0 && tn < ntiles) mixed_tile_issue<PLASTIC>(mixed_tile(E, tn), stage0 + s * SB, bar);
     }
     if (timed_out) {
-        // record the failure and let the copies this block started land
-        // (bounded) before its shared memory is released
-        if (tid == 0) {
+        // record the failure and let the copies this warp started land
+        // (bounded) before the block's shared memory is released
+        if (lane == 0) {
             atomicOr(&ctl->status, ST_TIMEOUT);
             for (int k = 0; k < 2; ++k) {
                 const int itk = it + k;
-                if (blockIdx.x + itk * gstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
+                if (w0 + itk * wstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
             }
         }
-        __syncthreads();
+        __syncwarp();
     }
     if (bad) atomicOr(&ctl->status, bad);
-    block_min2_d<kStageTile>(dts_min, len_min, &ctl->dts_next, &ctl->len_min);
+    block_min2_d<32 * kMixedPipeWarps>(dts_min, len_min, &ctl->dts_next, &ctl->len_min);
     double v3[3] = {e_int, e_hg, e_vis};
-    block_sum_d<kStageTile, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
+    block_sum_d<32 * kMixedPipeWarps, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
 }
 
-// ---- staged element pass with patch assembly ----------------------------
-// k_element_mixed_staged with one patch per tile.  After its element body a
-// thread holds its element's 24 nodal forces; once the whole block is done
-// with the stage's inputs, the forces go into the stage's memory as
-// [3][8 slots][kStageTile elements], and the block sums each of the patch's
-// nodes over its incidences in slot order (starting from zero) and writes the
-// node's partial to PA.pf.  INIT: the init force pass (dt = 0, no state
-// written, no energy).
-static_assert(kStageTile == kPatchElems, "one patch per staged tile");
-static_assert(3u * 8u * kStageTile * 4u <= kStageBytes, "the element forces fit in a stage");
+// ---- element pass with patch assembly -------------------------------------
+// One patch, two consecutive tiles, per 64-thread block at a time, through two
+// stages.  After its element body a thread holds its element's 24 nodal
+// forces; once the whole block is done with the stage's inputs, the forces go
+// into the stage's memory as [3][8 slots][kPatchElems elements], and the block
+// sums each of the patch's nodes over its incidences in slot order (starting
+// from zero) and writes the node's partial to PA.pf.  INIT: the init force pass
+// (dt = 0, no state written, no energy).
+constexpr uint32_t kPatchTiles = kPatchElems / 32;
+constexpr uint32_t kPatchStageBytes = kPatchTiles * MixedTile::kBytes;
+constexpr size_t kPatchSmem = 2 * static_cast<size_t>(kPatchStageBytes) + 16;
+static_assert(3u * 8u * kPatchElems * 4u <= kPatchStageBytes, "the element forces fit in a stage");
 
 __device__ __forceinline__ void patch_partials(const PatchArrays& E, const float* sf, int64_t t, int tid) {
     const uint32_t q0 = __ldg(E.pf_off + t), q1 = __ldg(E.pf_off + t + 1);
-    for (uint32_t q = q0 + tid; q < q1; q += kStageTile) {
+    for (uint32_t q = q0 + tid; q < q1; q += kPatchElems) {
         const uint32_t a = __ldg(E.pinc_off + q), b = __ldg(E.pinc_off + q + 1);
         float f0 = 0.f, f1 = 0.f, f2 = 0.f;
         for (uint32_t r = a; r < b; ++r) {
             const uint32_t u = __ldg(E.pinc + r);
-            const uint32_t col = (u & 7u) * kStageTile + (u >> 3);
+            const uint32_t col = (u & 7u) * kPatchElems + (u >> 3);
             f0 += sf[col];
-            f1 += sf[8 * kStageTile + col];
-            f2 += sf[16 * kStageTile + col];
+            f1 += sf[8 * kPatchElems + col];
+            f2 += sf[16 * kPatchElems + col];
         }
         E.pf[q] = f0;
         E.pf[E.pf_pad + q] = f1;
@@ -698,7 +651,7 @@ __device__ __forceinline__ void patch_partials(const PatchArrays& E, const float
 }
 
 template <bool PLASTIC, bool INIT>
-__global__ void __launch_bounds__(kStageTile, ENSC_STAGE_MINB_MIXED)
+__global__ void __launch_bounds__(kPatchElems, 8)
     k_element_mixed_patch(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P, PatchArrays PA) {
     if (ctl->done) return;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -706,81 +659,76 @@ __global__ void __launch_bounds__(kStageTile, ENSC_STAGE_MINB_MIXED)
     const double dt1d = INIT ? 0.0 : ctl->dt_i_1;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint32_t stage0 = smem_addr(smem);
-    const uint32_t bar0 = stage0 + 2 * kStageBytes;
-    const int64_t ntiles = (E.ne + kStageTile - 1) / kStageTile;
+    const uint32_t bar0 = stage0 + 2 * kPatchStageBytes;
+    const int64_t ntiles = (E.ne + 31) / 32, npatch = (E.ne + kPatchElems - 1) / kPatchElems;
     const int64_t gstride = gridDim.x;
+    auto issue = [&](int64_t p, int s) {
+        const int64_t left = ntiles - p * kPatchTiles;
+        const uint32_t bytes = static_cast<uint32_t>(left < kPatchTiles ? left : kPatchTiles) * MixedTile::kBytes;
+        mbar_arrive_expect_tx(bar0 + 8 * s, bytes);
+        fence_proxy_async_smem();  // the block's reads of this stage come before the copy into it
+        bulk_g2s(stage0 + s * kPatchStageBytes, mixed_tile(E, p * kPatchTiles), bytes, bar0 + 8 * s);
+    };
     if (tid == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
+        for (int s = 0; s < 2; ++s)
+            if (blockIdx.x + s * gstride < npatch) issue(blockIdx.x + s * gstride, s);
     }
     __syncthreads();
-    if (wid == 0) {
-        for (int s = 0; s < 2; ++s) {
-            const int64_t t = blockIdx.x + s * gstride;
-            if (t < ntiles) stage_issue<PLASTIC>(E, stage0 + s * kStageBytes, bar0 + 8 * s, t * kStageTile, lane);
-        }
-    }
     double e_int = 0.0, e_hg = 0.0, e_vis = 0.0;
     double dts_min = DBL_MAX, len_min = DBL_MAX;
     int32_t bad = 0;
     bool timed_out = false;
     int it = 0;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gstride, ++it) {
+    for (int64_t t = blockIdx.x; t < npatch; t += gstride, ++it) {
         const int s = it & 1;
-        const uint32_t bar = bar0 + 8 * s;
-        const bool ok = mbar_wait_bounded(bar, (it >> 1) & 1);
+        const bool ok = mbar_wait_bounded(bar0 + 8 * s, (it >> 1) & 1);
         if (__syncthreads_or(!ok)) {
             timed_out = true;
             break;
         }
-        const int64_t e = t * kStageTile + tid;
+        unsigned char* st = smem + s * kPatchStageBytes;
+        const int64_t e = t * kPatchElems + tid;
         const bool live = e < E.ne;
         float fo[24];
         if (live) {
-            const float* st = reinterpret_cast<const float*>(smem + s * kStageBytes);
-            const MixedSrc S{reinterpret_cast<const uint32_t*>(st),
-                             st + 8 * kStageTile,
-                             reinterpret_cast<const double*>(smem + s * kStageBytes + kStageV0Off),
-                             st + 44 * kStageTile,
-                             st + 26 * kStageTile,
-                             st + 32 * kStageTile,
-                             st + 45 * kStageTile,
-                             kStageTile,
-                             tid};
             double dts, len;
-            element_body_mixed<PLASTIC, INIT, true, ENSC_MIXED_PREFETCH, true>(E, N, M, S, mixed_out_global(E, e), dt1, dt1d,
-                                                                               e, dts, len, e_int, e_hg, e_vis, bad, fo);
+            element_body_mixed<PLASTIC, INIT, true, ENSC_MIXED_PREFETCH, true>(
+                E, N, M, mixed_src_tile(st + wid * MixedTile::kBytes, lane),
+                mixed_out_tile(mixed_tile(E, t * kPatchTiles + wid), lane), dt1, dt1d, e, dts, len, e_int, e_hg, e_vis, bad,
+                fo);
             dts_min = fmin(dts_min, dts);
             len_min = fmin(len_min, len);
         }
         __syncthreads();  // the stage's inputs are consumed
-        float* sf = reinterpret_cast<float*>(smem + s * kStageBytes);
+        float* sf = reinterpret_cast<float*>(st);
         if (live) {
 #pragma unroll
-            for (int i = 0; i < 24; ++i) sf[i * kStageTile + tid] = fo[i];
+            for (int i = 0; i < 24; ++i) sf[i * kPatchElems + tid] = fo[i];
         }
         __syncthreads();
         patch_partials(PA, sf, t, tid);
         __syncthreads();  // the block is done with stage s
         const int64_t tn = t + 2 * gstride;
-        if (wid == 0 && tn < ntiles) stage_issue<PLASTIC>(E, stage0 + s * kStageBytes, bar, tn * kStageTile, lane);
+        if (tid == 0 && tn < npatch) issue(tn, s);
     }
     if (timed_out) {
         if (tid == 0) {
             atomicOr(&ctl->status, ST_TIMEOUT);
             for (int k = 0; k < 2; ++k) {
                 const int itk = it + k;
-                if (blockIdx.x + itk * gstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
+                if (blockIdx.x + itk * gstride < npatch) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
             }
         }
         __syncthreads();
     }
     if (bad) atomicOr(&ctl->status, bad);
-    block_min2_d<kStageTile>(dts_min, len_min, &ctl->dts_next, &ctl->len_min);
+    block_min2_d<kPatchElems>(dts_min, len_min, &ctl->dts_next, &ctl->len_min);
     if (!INIT) {
         double v3[3] = {e_int, e_hg, e_vis};
-        block_sum_d<kStageTile, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
+        block_sum_d<kPatchElems, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
     }
 }
 
@@ -1107,7 +1055,7 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_MIXED) k_node_mix
     int32_t bad = 0;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (E.slot_major && E.tiles_aligned) {
+    if (E.slot_major && E.tile_bytes) {
         constexpr int W = kNodeGroupMixed;
         const NodeView nv = node_view(E, N, M, ctl, &PA);
         for (int64_t g = t0; g * W < nn; g += stride)
@@ -1121,41 +1069,33 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_MIXED) k_node_mix
 }
 
 // ---- resident runs (ensc_run.cuh) -----------------------------------------
-// 16 warps per SM as in the staged pass; a tile of 32 elements takes 6.1 KB,
-// so that 148 SMs hold 151,552 elements at two tiles per warp.
+// 16 warps per SM as in the warp-pipelined pass; a tile takes 6,144 bytes, so
+// that 37 tiles fit an SM and 148 SMs hold 151,552 elements at two tiles per
+// warp.
 constexpr int kRunWarpsMixed = 16;
 template <bool PLASTIC>
 struct RunMixed {
-    static constexpr uint32_t kV0Off = kStageWordRows * 32u * 4u;
-    static constexpr uint32_t kTileBytes = kV0Off + 32u * 8u;
+    static constexpr uint32_t kTileBytes = MixedTile::kBytes;
     __device__ static const uint32_t* conn(const unsigned char* tile) {
         return reinterpret_cast<const uint32_t*>(tile);
     }
-    __device__ static void load_tile(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t base, int lane) {
-        constexpr int rows = PLASTIC ? kStageWordRows : kStageWordRows - 1;
-        if (lane == 0) mbar_arrive_expect_tx(bar, rows * 32u * 4u + 32u * 8u);
-        __syncwarp();
-        for (int r = lane; r <= rows; r += 32) {
-            if (r < rows) bulk_g2s(dst + r * (32u * 4u), stage_row(E, r) + base, 32u * 4u, bar);
-            else bulk_g2s(dst + kV0Off, E.vol0 + base, 32u * 8u, bar);
-        }
+    __device__ static void load_tile(const ElemArrays& E, uint32_t dst, uint32_t bar, int64_t t, int lane) {
+        if (lane == 0) mixed_tile_issue<PLASTIC>(mixed_tile(E, t), dst, bar);
     }
-    __device__ static void store_tile(const ElemArrays& E, const unsigned char* tile, int64_t base, int lane) {
-        const float* d = reinterpret_cast<const float*>(tile);
-        const int64_t e = base + lane;
-        if (e >= E.ne) return;
-        for (int r = 26; r < 44; ++r) const_cast<float*>(stage_row(E, r))[e] = d[r * 32 + lane];
-        if (PLASTIC) const_cast<float*>(stage_row(E, 45))[e] = d[45 * 32 + lane];
+    __device__ static void store_tile(const ElemArrays& E, const unsigned char* tile, int64_t t, int lane) {
+        // whole rows: the entries past ne are padding
+        unsigned char* g = mixed_tile(E, t);
+        constexpr uint32_t end = PLASTIC ? MixedTile::kBytes : MixedTile::kEps;
+        for (uint32_t o = MixedTile::kState + 4u * lane; o < end; o += 128)
+            *reinterpret_cast<float*>(g + o) = *reinterpret_cast<const float*>(tile + o);
     }
     __device__ static void element(const ElemArrays& E, const NodeArrays& N, const Material& M, unsigned char* tile,
                                    double dt1, int64_t e, int lane, double& dts, double& len, double& e_int,
                                    double& e_hg, double& e_vis, int32_t& bad) {
-        float* st = reinterpret_cast<float*>(tile);
-        const MixedSrc S{conn(tile), st + 8 * 32, reinterpret_cast<const double*>(tile + kV0Off), st + 44 * 32,
-                         st + 26 * 32, st + 32 * 32, st + 45 * 32, 32, lane};
-        const MixedOut O{st + 26 * 32, st + 32 * 32, st + 45 * 32, 32, lane};
-        element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(E, N, M, S, O, static_cast<float>(dt1), dt1, e,
-                                                                      dts, len, e_int, e_hg, e_vis, bad);
+        element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(E, N, M, mixed_src_tile(tile, lane),
+                                                                      mixed_out_tile(tile, lane),
+                                                                      static_cast<float>(dt1), dt1, e, dts, len, e_int,
+                                                                      e_hg, e_vis, bad);
     }
     // as RunFp64::Nodes
     template <int W>
@@ -1212,7 +1152,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration_mixed(PatchArrays
                                                                      const Ctl* ctl, double* a_out) {
     const int64_t np = N.nn_pad, ep = E.ne_pad;
     const float* __restrict__ fe = static_cast<const float*>(E.fe);
-    const bool grouped = E.slot_major && E.tiles_aligned;
+    const bool grouped = E.slot_major && E.tile_bytes;
     const double amp = (M.gravity_on && M.amp_n > 0) ? gravity_amplitude(M.amp, M.amp_n, ctl->time, ctl->dt_i) : 1.0;
     for (int64_t n = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; n < N.nn;
          n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -1262,140 +1202,184 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration_mixed(PatchArrays
 }
 
 // ---- batched instances --------------------------------------------------------
-// Element tiles of kStageTile elements and node tiles of 32 * kNodeGroupBatchMixed
-// nodes, each inside one instance whose arrays, material and control block
-// come from the instance table.  The element pass runs the staged pipeline
-// over the tile list, one tile per block at a time; the node pass gives each
-// node tile to one warp.  Each tile accumulates its work terms across
-// cycles (one owner per tile and pass) and keeps its latest kinetic energy;
-// k_fold_batch folds them per instance in tile order, so the totals do not
-// depend on scheduling.
+// Element tiles of 32 elements (under the patch assembly: patches, two tiles)
+// and node tiles of 32 * kNodeGroupBatchMixed nodes, each inside one instance
+// whose arrays, material and control block come from the instance table.  The
+// element pass runs one pipeline per warp over the tile list (one per block
+// over patches); the node pass gives each node tile to one warp.  Each tile
+// accumulates its work terms across cycles (one owner per tile and pass) and
+// keeps its latest kinetic energy; k_fold_batch folds them per instance in tile
+// order, so the totals do not depend on scheduling.
 __device__ __forceinline__ double warp_sum_b(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w < v ? w : v;
-    }
-    return v;
-}
-
-// A batch stage: the single-instance stage, then the tile's instance
-// descriptor, its element-pass scalars (StageHdr), the TileInfo the filling
-// warp writes, and the ETileSrc record of the tile that uses the stage next.
-// Every tile is copied whole whether or not its instance runs this cycle;
-// the consumer skips the tiles of instances that do not.
-constexpr uint32_t kDescBytes = sizeof(InstanceDesc);
-constexpr uint32_t kBatchDescOff = kStageBytes;
-constexpr uint32_t kBatchHdrOff = kBatchDescOff + kDescBytes;
-constexpr uint32_t kBatchInfoOff = kBatchHdrOff + sizeof(StageHdr);
-constexpr uint32_t kBatchNextOff = kBatchInfoOff + sizeof(TileInfo);
-constexpr uint32_t kBatchStageBytes = (kBatchNextOff + sizeof(ETileSrc) + 127) / 128 * 128;
-constexpr size_t kBatchStageSmem = 2 * static_cast<size_t>(kBatchStageBytes) + 16;
-static_assert(kDescBytes % 16 == 0 && sizeof(StageHdr) == 16 && sizeof(TileInfo) == 16, "16-byte copies");
-
-// word row r of a batch tile in global memory
-__device__ __forceinline__ const void* tile_row(const ETileSrc& src, int r) {
-    const int64_t ep = src.ne_pad;
-    if (r < 8) return static_cast<const uint32_t*>(src.conn) + r * ep;
-    if (r < 26) return static_cast<const float*>(src.bt) + (r - 8) * ep;
-    if (r < 32) return static_cast<const float*>(src.sigma) + (r - 26) * ep;
-    if (r < 44) return static_cast<const float*>(src.qia) + (r - 32) * ep;
-    if (r == 44) return src.cbrt_v0;
-    return src.eps_p;
-}
-
-// Warp 0 fills a stage with the tile `src` describes (and the record of tile
-// t_next, if there is one): lane 0 writes the TileInfo and arms the barrier
-// with the byte count, then the lanes start the copies between them.
-__device__ __forceinline__ void batch_stage_issue(const BatchTables& T, const ETileSrc& src, int64_t t_next,
-                                                  int64_t ntiles, unsigned char* stage, uint32_t dst, uint32_t bar,
-                                                  int lane) {
-    const uint32_t cnt = static_cast<uint32_t>(src.cnt);
+// A batch stage: the tile (or patch), then its instance descriptor, its
+// element-pass scalars (StageHdr), the TileInfo the filling lane writes, and the
+// ETileSrc record of the tile that uses the stage next.  Every tile is copied
+// whole whether or not its instance runs this cycle; the consumer skips the
+// tiles of instances that do not.  One lane fills a stage.
+template <uint32_t ROOM>
+__device__ __forceinline__ void batch_issue(const BatchTables& T, const ETileSrc& src, int64_t t_next, int64_t ntiles,
+                                            unsigned char* stage, uint32_t dst, uint32_t bar) {
     const bool next = t_next < ntiles;
+    TileInfo* ti = reinterpret_cast<TileInfo*>(stage + ROOM + kBatchInfoOff);
+    ti->slot = src.slot;
+    ti->base = src.base;
+    mbar_arrive_expect_tx(bar, static_cast<uint32_t>(src.bytes) + sizeof(InstanceDesc) + sizeof(StageHdr) +
+                                   (next ? sizeof(ETileSrc) : 0u));
+    fence_proxy_async_smem();  // the reads of this stage come before the copies into it
+    bulk_g2s(dst, src.tile, static_cast<uint32_t>(src.bytes), bar);
+    bulk_g2s(dst + ROOM, T.desc + src.slot, sizeof(InstanceDesc), bar);
+    bulk_g2s(dst + ROOM + kBatchHdrOff, T.sparam + src.slot, sizeof(StageHdr), bar);
+    if (next) bulk_g2s(dst + ROOM + kBatchNextOff, T.etile_src + t_next, sizeof(ETileSrc), bar);
+}
+
+// A thread's sums over a run: consecutive tiles of one instance, reduced per
+// warp once, into the partial slot of the run's first tile.
+struct BatchRun {
+    int slot = -1;
+    double* part = nullptr;
+    Ctl* ctl = nullptr;
+    bool live = false;
+    double ei = 0.0, eh = 0.0, ev = 0.0, dts = DBL_MAX, len = DBL_MAX;
+    int32_t bad = 0;
+    __device__ __forceinline__ void flush(int lane) {
+        ei = warp_sum_b(ei);
+        eh = warp_sum_b(eh);
+        ev = warp_sum_b(ev);
+        const unsigned long long dmin = run_warp_min(ord_bits(dts));
+        const unsigned long long lmin = run_warp_min(ord_bits(len));
+        bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
+        if (live && lane == 0) {
+            // one writer per slot and pass: the reductions (no return value)
+            // add in cycle order without a round trip
+            atomicAdd(part + 0, ei);
+            atomicAdd(part + 1, eh);
+            atomicAdd(part + 2, ev);
+            atomicMin(&ctl->dts_next, dmin);
+            atomicMin(&ctl->len_min, lmin);
+            if (bad) atomicOr(&ctl->status, bad);
+        }
+        ei = eh = ev = 0.0;
+        dts = len = DBL_MAX;
+        bad = 0;
+    }
+};
+
+constexpr uint32_t kBatchStageMixed = MixedTile::kBytes + kBatchTailBytes;
+constexpr size_t kBatchMixedSmem = static_cast<size_t>(kMixedPipeWarps) * (2 * kBatchStageMixed + 16);
+
+__global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB) k_element_batch_mixed(BatchTables T) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr uint32_t SB = kBatchStageMixed;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
+    const uint32_t stage0 = smem_addr(wst);
+    const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kMixedPipeWarps) * 2 * SB) + 16u * wid;
+    const int64_t ntiles = T.counts[0];
+    const int64_t wstride = static_cast<int64_t>(gridDim.x) * kMixedPipeWarps;
+    const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kMixedPipeWarps + wid;
     if (lane == 0) {
-        TileInfo* ti = reinterpret_cast<TileInfo*>(stage + kBatchInfoOff);
-        ti->slot = src.slot;
-        ti->base = src.base;
-        mbar_arrive_expect_tx(bar, kStageWordRows * cnt * 4u + cnt * 8u + kDescBytes + sizeof(StageHdr) +
-                                       (next ? sizeof(ETileSrc) : 0u));
+        mbar_init(bar0, 1);
+        mbar_init(bar0 + 8, 1);
+        mbar_init_fence();
+        for (int s = 0; s < 2; ++s) {
+            const int64_t t = w0 + s * wstride;
+            if (t < ntiles)
+                batch_issue<MixedTile::kBytes>(T, T.etile_src[t], t + 2 * wstride, ntiles, wst + s * SB, stage0 + s * SB,
+                                               bar0 + 8 * s);
+        }
     }
     __syncwarp();
-    fence_proxy_async_smem();  // the block's reads of this stage come before the copies into it
-    for (int r = lane; r < kStageWordRows + 4; r += 32) {
-        if (r < kStageWordRows) bulk_g2s(dst + r * (kStageTile * 4u), tile_row(src, r), cnt * 4u, bar);
-        else if (r == kStageWordRows) bulk_g2s(dst + kStageV0Off, src.vol0, cnt * 8u, bar);
-        else if (r == kStageWordRows + 1) bulk_g2s(dst + kBatchDescOff, T.desc + src.slot, kDescBytes, bar);
-        else if (r == kStageWordRows + 2) bulk_g2s(dst + kBatchHdrOff, T.sparam + src.slot, sizeof(StageHdr), bar);
-        else if (next) bulk_g2s(dst + kBatchNextOff, T.etile_src + t_next, sizeof(ETileSrc), bar);
+    BatchRun run;
+    bool timed_out = false;
+    int it = 0;
+    int64_t t = w0;
+    for (; t < ntiles; t += wstride, ++it) {
+        const int s = it & 1;
+        const uint32_t bar = bar0 + 8 * s;
+        const bool ok = mbar_wait_bounded(bar, (it >> 1) & 1);
+        if (__any_sync(0xffffffffu, !ok)) {
+            timed_out = true;
+            break;
+        }
+        unsigned char* sb = wst + s * SB;
+        unsigned char* tail = sb + MixedTile::kBytes;
+        const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(tail);
+        const StageHdr& h = *reinterpret_cast<const StageHdr*>(tail + kBatchHdrOff);
+        const TileInfo& ti = *reinterpret_cast<const TileInfo*>(tail + kBatchInfoOff);
+        if (ti.slot != run.slot) {
+            run.flush(lane);
+            run.slot = ti.slot;
+            run.part = T.etile_part + 3 * t;
+            run.ctl = d.ctl;
+            run.live = h.live != 0;
+        }
+        const int64_t e = static_cast<int64_t>(ti.base) + lane;
+        if (run.live && e < d.E.ne) {
+            // arrays copied to registers (the body's stores could alias the
+            // stage as far as the compiler knows), material constants read at use
+            const ElemArrays E = d.E;
+            const NodeArrays N = d.N;
+            const double dt1d = h.dt1;
+            double d1, l1;
+            element_body_mixed<true, false, true, ENSC_BATCH_MIXED_PREFETCH>(
+                E, N, d.M, mixed_src_tile(sb, lane), mixed_out_tile(mixed_tile(E, ti.base >> 5), lane),
+                static_cast<float>(dt1d), dt1d, e, d1, l1, run.ei, run.eh, run.ev, run.bad);
+            run.dts = fmin(run.dts, d1);
+            run.len = fmin(run.len, l1);
+        }
+        __syncwarp();  // all lanes are done with stage s
+        const int64_t tn = t + 2 * wstride;
+        if (lane == 0 && tn < ntiles) {
+            const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
+            batch_issue<MixedTile::kBytes>(T, src, tn + 2 * wstride, ntiles, sb, stage0 + s * SB, bar);
+        }
     }
+    if (!timed_out) {
+        run.flush(lane);
+    } else if (lane == 0) {
+        // record the failure on the instance whose tile could not be read and
+        // let the copies this warp started land (bounded) before exiting
+        atomicOr(&T.desc[T.etile_inst[t]].ctl->status, ST_TIMEOUT);
+        for (int k = 0; k < 2; ++k) {
+            const int itk = it + k;
+            if (w0 + itk * wstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
+        }
+    }
+    element_pass_done(T);
 }
 
-// EPT elements per thread: the block has kStageTile / EPT threads, and each
-// thread evaluates elements tid, tid + kStageTile / EPT, ... of a tile in
-// turn (a tuning choice; EPT > 1 only under the slot assembly).  PATCH: the
-// batch's instances use the patch assembly (a batch has one assembly).
-template <int EPT, bool PATCH>
-__global__ void __launch_bounds__(kStageTile / EPT, ENSC_BATCH_MINB_MIXED) k_element_batch_mixed(BatchTables T) {
-    static_assert(EPT == 1 || !PATCH, "the patch sums take one element per thread");
+// The same under the patch assembly (a batch has one assembly): one patch per
+// block at a time, as k_element_mixed_patch.
+constexpr uint32_t kBatchStagePatch = kPatchStageBytes + kBatchTailBytes;
+constexpr size_t kBatchPatchSmem = 2 * static_cast<size_t>(kBatchStagePatch) + 16;
+
+__global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTables T) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int NW = kStageTile / 32;  // energy partial slots per tile
-    constexpr int NT = kStageTile / EPT;
+    constexpr uint32_t SB = kBatchStagePatch;
+    constexpr int NW = kPatchElems / 32;  // energy partial slots per patch
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint32_t stage0 = smem_addr(smem);
-    const uint32_t bar0 = stage0 + 2 * kBatchStageBytes;
+    const uint32_t bar0 = stage0 + 2 * SB;
     const int64_t ntiles = T.counts[0];
     const int64_t gstride = gridDim.x;
     if (tid == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
-    }
-    __syncthreads();
-    if (wid == 0) {
         for (int s = 0; s < 2; ++s) {
             const int64_t t = blockIdx.x + s * gstride;
-            if (t < ntiles) {
-                const ETileSrc src = T.etile_src[t];
-                batch_stage_issue(T, src, t + 2 * gstride, ntiles, smem + s * kBatchStageBytes,
-                                  stage0 + s * kBatchStageBytes, bar0 + 8 * s, lane);
-            }
+            if (t < ntiles)
+                batch_issue<kPatchStageBytes>(T, T.etile_src[t], t + 2 * gstride, ntiles, smem + s * SB, stage0 + s * SB,
+                                              bar0 + 8 * s);
         }
     }
-    // the current run: instance slot, first tile, control block, liveness
-    int run_slot = -1;
-    int64_t run_tile = 0;
-    Ctl* run_ctl = nullptr;
-    bool run_live = false;
-    double ei = 0.0, eh = 0.0, ev = 0.0, dts = DBL_MAX, len = DBL_MAX;
-    int32_t bad = 0;
-    auto flush = [&]() {
-        ei = warp_sum_b(ei);
-        eh = warp_sum_b(eh);
-        ev = warp_sum_b(ev);
-        const unsigned long long dmin = warp_min_u64(ord_bits(dts));
-        const unsigned long long lmin = warp_min_u64(ord_bits(len));
-        bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
-        if (run_live && lane == 0) {
-            double* part = T.etile_part + 3 * (run_tile * NW + wid);
-            // one writer per slot and pass: the reductions (no return value)
-            // add in cycle order without a round trip
-            atomicAdd(part + 0, ei);
-            atomicAdd(part + 1, eh);
-            atomicAdd(part + 2, ev);
-            atomicMin(&run_ctl->dts_next, dmin);
-            atomicMin(&run_ctl->len_min, lmin);
-            if (bad) atomicOr(&run_ctl->status, bad);
-        }
-        ei = eh = ev = 0.0;
-        dts = len = DBL_MAX;
-        bad = 0;
-    };
+    __syncthreads();
+    BatchRun run;
     bool timed_out = false;
     int it = 0;
     int64_t t = blockIdx.x;
@@ -1407,102 +1391,54 @@ __global__ void __launch_bounds__(kStageTile / EPT, ENSC_BATCH_MINB_MIXED) k_ele
             timed_out = true;
             break;
         }
-        unsigned char* sb = smem + s * kBatchStageBytes;
-        const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(sb + kBatchDescOff);
-        const StageHdr& h = *reinterpret_cast<const StageHdr*>(sb + kBatchHdrOff);
-        const TileInfo& ti = *reinterpret_cast<const TileInfo*>(sb + kBatchInfoOff);
-        if (ti.slot != run_slot) {
-            flush();
-            run_slot = ti.slot;
-            run_tile = t;
-            run_ctl = d.ctl;
-            run_live = h.live != 0;
+        unsigned char* sb = smem + s * SB;
+        unsigned char* tail = sb + kPatchStageBytes;
+        const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(tail);
+        const StageHdr& h = *reinterpret_cast<const StageHdr*>(tail + kBatchHdrOff);
+        const TileInfo& ti = *reinterpret_cast<const TileInfo*>(tail + kBatchInfoOff);
+        if (ti.slot != run.slot) {
+            run.flush(lane);
+            run.slot = ti.slot;
+            run.part = T.etile_part + 3 * (t * NW + wid);
+            run.ctl = d.ctl;
+            run.live = h.live != 0;
         }
-        constexpr bool patch = PATCH;
-        const PatchArrays* pe = &d.pa;
         float fo[24];
-        int64_t e = 0;
-#pragma unroll 1
-        for (int k = 0; k < EPT; ++k) {
-            const int li = tid + k * NT;
-            e = static_cast<int64_t>(ti.base) + li;
-            if (run_live && e < d.E.ne) {
-#if ENSC_BATCH_DESC_MODE == 1
-                // the instance's arrays and constants, read from the stage once:
-                // the body's stores could alias the stage as far as the compiler
-                // knows, so references into it would be re-read after each store
-                const ElemArrays E = d.E;
-                const NodeArrays N = d.N;
-                const Material M = d.M;
-#elif ENSC_BATCH_DESC_MODE == 2
-                // arrays copied to registers, material constants read at use
-                const ElemArrays E = d.E;
-                const NodeArrays N = d.N;
-                const Material& M = d.M;
-#else
-                const ElemArrays& E = d.E;
-                const NodeArrays& N = d.N;
-                const Material& M = d.M;
-#endif
-                const double dt1d = h.dt1;
-                const float dt1 = static_cast<float>(dt1d);
-                const float* st = reinterpret_cast<const float*>(sb);
-                const MixedSrc S{reinterpret_cast<const uint32_t*>(st),
-                                 st + 8 * kStageTile,
-                                 reinterpret_cast<const double*>(sb + kStageV0Off),
-                                 st + 44 * kStageTile,
-                                 st + 26 * kStageTile,
-                                 st + 32 * kStageTile,
-                                 st + 45 * kStageTile,
-                                 kStageTile,
-                                 li};
-                double d1, l1;
-                element_body_mixed<true, false, true, ENSC_BATCH_MIXED_PREFETCH, true>(E, N, M, S, mixed_out_global(E, e), dt1,
-                                                                                      dt1d, e, d1, l1, ei, eh, ev, bad, fo);
-                dts = fmin(dts, d1);
-                len = fmin(len, l1);
-                if (!patch) {
-                    // slot assembly: the forces to the instance's force array
-                    float* __restrict__ fe = static_cast<float*>(E.fe);
-                    const int64_t np = N.nn_pad, ep = E.ne_pad;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const uint32_t nj = S.conn[j * kStageTile + li];
-#pragma unroll
-                        for (int i = 0; i < 3; ++i) {
-                            if (E.slot_major) fe[(3 * j + i) * np + nj] = fo[8 * i + j];
-                            else fe[(3 * j + i) * ep + e] = fo[8 * i + j];
-                        }
-                    }
-                }
-            }
+        const int64_t e = static_cast<int64_t>(ti.base) + tid;
+        const int64_t ne = d.E.ne;
+        if (run.live && e < ne) {
+            const ElemArrays E = d.E;
+            const NodeArrays N = d.N;
+            const double dt1d = h.dt1;
+            double d1, l1;
+            element_body_mixed<true, false, true, ENSC_BATCH_MIXED_PREFETCH, true>(
+                E, N, d.M, mixed_src_tile(sb + wid * MixedTile::kBytes, lane),
+                mixed_out_tile(mixed_tile(E, (ti.base >> 5) + wid), lane), static_cast<float>(dt1d), dt1d, e, d1, l1, run.ei,
+                run.eh, run.ev, run.bad, fo);
+            run.dts = fmin(run.dts, d1);
+            run.len = fmin(run.len, l1);
         }
-        if (patch && run_live) {
-            // the tile's patch: its forces summed per patch node (see
-            // k_element_mixed_patch); the stage's element rows hold them
-            const PatchArrays PE = *pe;
-            const int64_t ne = d.E.ne;
+        if (run.live) {
+            const PatchArrays PE = d.pa;
             __syncthreads();  // the stage's inputs are consumed
             float* sf = reinterpret_cast<float*>(sb);
             if (e < ne) {
 #pragma unroll
-                for (int i = 0; i < 24; ++i) sf[i * kStageTile + tid] = fo[i];
+                for (int i = 0; i < 24; ++i) sf[i * kPatchElems + tid] = fo[i];
             }
             __syncthreads();
             patch_partials(PE, sf, static_cast<int64_t>(ti.base) / kPatchElems, tid);
         }
         __syncthreads();  // the block is done with stage s
         const int64_t tn = t + 2 * gstride;
-        if (wid == 0 && tn < ntiles) {
-            const ETileSrc src = *reinterpret_cast<const ETileSrc*>(sb + kBatchNextOff);
-            batch_stage_issue(T, src, tn + 2 * gstride, ntiles, sb, stage0 + s * kBatchStageBytes, bar, lane);
+        if (tid == 0 && tn < ntiles) {
+            const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
+            batch_issue<kPatchStageBytes>(T, src, tn + 2 * gstride, ntiles, sb, stage0 + s * SB, bar);
         }
     }
     if (!timed_out) {
-        flush();
+        run.flush(lane);
     } else if (tid == 0) {
-        // record the failure on the instance whose tile could not be read and
-        // let the copies this block started land (bounded) before exiting
         atomicOr(&T.desc[T.etile_inst[t]].ctl->status, ST_TIMEOUT);
         for (int k = 0; k < 2; ++k) {
             const int itk = it + k;
@@ -1577,25 +1513,18 @@ void launch_element_mixed(const ElemArrays& E, const NodeArrays& N, const Materi
                           int grid, bool init, cudaStream_t st, const PatchArrays& PA) {
     if (PA.pf) {
         if (M.plastic) {
-            if (init) k_element_mixed_patch<true, true><<<grid, kStageTile, kStageSmem, st>>>(E, N, M, ctl, P, PA);
-            else k_element_mixed_patch<true, false><<<grid, kStageTile, kStageSmem, st>>>(E, N, M, ctl, P, PA);
+            if (init) k_element_mixed_patch<true, true><<<grid, kPatchElems, kPatchSmem, st>>>(E, N, M, ctl, P, PA);
+            else k_element_mixed_patch<true, false><<<grid, kPatchElems, kPatchSmem, st>>>(E, N, M, ctl, P, PA);
         } else {
-            if (init) k_element_mixed_patch<false, true><<<grid, kStageTile, kStageSmem, st>>>(E, N, M, ctl, P, PA);
-            else k_element_mixed_patch<false, false><<<grid, kStageTile, kStageSmem, st>>>(E, N, M, ctl, P, PA);
+            if (init) k_element_mixed_patch<false, true><<<grid, kPatchElems, kPatchSmem, st>>>(E, N, M, ctl, P, PA);
+            else k_element_mixed_patch<false, false><<<grid, kPatchElems, kPatchSmem, st>>>(E, N, M, ctl, P, PA);
         }
-        return;
-    }
-    if (ENSC_STAGED_MIXED && !init && E.tiles_aligned) {
-        if (M.plastic) k_element_mixed_staged<true><<<grid, kStageTile, kStageSmem, st>>>(E, N, M, ctl, P);
-        else k_element_mixed_staged<false><<<grid, kStageTile, kStageSmem, st>>>(E, N, M, ctl, P);
-        return;
-    }
-    if (M.plastic) {
-        if (init) k_element_mixed<true, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-        else k_element_mixed<true, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+    } else if (M.plastic) {
+        if (init) k_element_mixed_init<true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl);
+        else k_element_mixed_warp<true><<<grid, 32 * kMixedPipeWarps, kMixedPipeSmem, st>>>(E, N, M, ctl, P);
     } else {
-        if (init) k_element_mixed<false, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-        else k_element_mixed<false, false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
+        if (init) k_element_mixed_init<false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl);
+        else k_element_mixed_warp<false><<<grid, 32 * kMixedPipeWarps, kMixedPipeSmem, st>>>(E, N, M, ctl, P);
     }
 }
 
@@ -1611,44 +1540,27 @@ void launch_node_mixed(const ElemArrays& E, const NodeArrays& N, const Material&
     else k_node_mixed<false><<<grid, kNodeThreads, 0, st>>>(E, N, M, ctl, P, PA);
 }
 
-// The staged passes need more than the default 48 KB of dynamic shared
+// The pipelined passes need more than the default 48 KB of dynamic shared
 // memory; the attribute is set on the current device before any launch or
 // capture.
-void set_element_mixed_attributes() {
-    cudaFuncSetAttribute(k_element_mixed_staged<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kStageSmem));
-    cudaFuncSetAttribute(k_element_mixed_staged<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kStageSmem));
-    cudaFuncSetAttribute(k_element_mixed_patch<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kStageSmem));
-    cudaFuncSetAttribute(k_element_mixed_patch<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kStageSmem));
-    cudaFuncSetAttribute(k_element_mixed_patch<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kStageSmem));
-    cudaFuncSetAttribute(k_element_mixed_patch<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kStageSmem));
+template <typename K>
+static int mixed_occupancy(K kernel, int threads, size_t smem) {
+    int nb = 0;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem);
+    return nb;
 }
 
-int occupancy_element_mixed(bool plastic) {
-    int nb = 0;
-    set_element_mixed_attributes();
-    if (ENSC_STAGED_MIXED) {
-        // the staged pass needs more than the default 48 KB of dynamic shared
-        // memory; the attribute is set here, on the current device, before
-        // any launch or capture
-        cudaFuncSetAttribute(k_element_mixed_staged<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kStageSmem));
-        cudaFuncSetAttribute(k_element_mixed_staged<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kStageSmem));
-        if (plastic)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_mixed_staged<true>, kStageTile, kStageSmem);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_mixed_staged<false>, kStageTile, kStageSmem);
-        return nb;
+int occupancy_element_mixed(bool plastic, bool patch) {
+    if (patch) {
+        // both the init and the cycle pass run
+        mixed_occupancy(k_element_mixed_patch<true, true>, kPatchElems, kPatchSmem);
+        mixed_occupancy(k_element_mixed_patch<false, true>, kPatchElems, kPatchSmem);
+        return plastic ? mixed_occupancy(k_element_mixed_patch<true, false>, kPatchElems, kPatchSmem)
+                       : mixed_occupancy(k_element_mixed_patch<false, false>, kPatchElems, kPatchSmem);
     }
-    if (plastic) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_mixed<true, false>, kElemThreads, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_mixed<false, false>, kElemThreads, 0);
-    return nb;
+    return plastic ? mixed_occupancy(k_element_mixed_warp<true>, 32 * kMixedPipeWarps, kMixedPipeSmem)
+                   : mixed_occupancy(k_element_mixed_warp<false>, 32 * kMixedPipeWarps, kMixedPipeSmem);
 }
 
 int occupancy_node_mixed() {
@@ -1658,10 +1570,9 @@ int occupancy_node_mixed() {
 }
 
 
-void launch_element_batch_mixed(const BatchTables& T, int grid, int ept, bool patch, cudaStream_t st) {
-    if (patch) k_element_batch_mixed<1, true><<<grid, kStageTile, kBatchStageSmem, st>>>(T);
-    else if (ept == 2) k_element_batch_mixed<2, false><<<grid, kStageTile / 2, kBatchStageSmem, st>>>(T);
-    else k_element_batch_mixed<1, false><<<grid, kStageTile, kBatchStageSmem, st>>>(T);
+void launch_element_batch_mixed(const BatchTables& T, int grid, bool patch, cudaStream_t st) {
+    if (patch) k_element_batch_patch<<<grid, kPatchElems, kBatchPatchSmem, st>>>(T);
+    else k_element_batch_mixed<<<grid, 32 * kMixedPipeWarps, kBatchMixedSmem, st>>>(T);
 }
 void launch_node_batch_mixed(const BatchTables& T, int grid, int threads, bool patch, cudaStream_t st) {
     if (patch) {
@@ -1672,23 +1583,11 @@ void launch_node_batch_mixed(const BatchTables& T, int grid, int threads, bool p
         else k_node_batch_mixed<kNodeThreads, false><<<grid, kNodeThreads, 0, st>>>(T);
     }
 }
-int occupancy_element_batch_mixed(int ept) {
-    int nb = 0;
-    set_element_mixed_attributes();  // the batch's init passes run the single-instance kernels
-    // dynamic shared memory above the default 48 KB: set on the current
-    // device before any launch or capture
-    cudaFuncSetAttribute(k_element_batch_mixed<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kBatchStageSmem));
-    cudaFuncSetAttribute(k_element_batch_mixed<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kBatchStageSmem));
-    cudaFuncSetAttribute(k_element_batch_mixed<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(kBatchStageSmem));
-    if (ept == 2)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_batch_mixed<2, false>, kStageTile / 2,
-                                                      kBatchStageSmem);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_element_batch_mixed<1, false>, kStageTile, kBatchStageSmem);
-    return nb;
+int occupancy_element_batch_mixed(bool patch) {
+    // the batch's init passes run the single-instance kernels
+    occupancy_element_mixed(true, patch);
+    return patch ? mixed_occupancy(k_element_batch_patch, kPatchElems, kBatchPatchSmem)
+                 : mixed_occupancy(k_element_batch_mixed, 32 * kMixedPipeWarps, kBatchMixedSmem);
 }
 
 RunPlan plan_run_mixed(int64_t ne, int64_t nn, bool plastic, int sms) {
@@ -1708,7 +1607,7 @@ cudaError_t launch_run_mixed(const RunPlan& p, const ElemArrays& E, const NodeAr
                       sync, a);
 }
 
-int batch_element_tile(bool mixed_precision) { return mixed_precision ? kStageTile : batch_element_tile_fp64(); }
+int batch_element_tile(bool patch) { return patch ? kPatchElems : 32; }
 int batch_node_tile(bool mixed_precision) { return 32 * (mixed_precision ? kNodeGroupBatchMixed : kNodeGroupFp64); }
 int occupancy_node_batch_mixed(int threads) {
     int nb = 0;

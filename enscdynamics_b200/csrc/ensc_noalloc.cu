@@ -130,7 +130,7 @@ int ensc_step_noalloc(const ensc_device_model* m, const ensc_material* mat, cons
 
     ensc::ElemArrays E{};
     E.ne = ne;
-    E.ne_pad = ne;
+    E.ne_pad = ne;  // plain rows (tile_bytes 0), B0^T as its 24 numbers (bt9 0)
     E.conn = m->conn;
     E.bt = m->bt;
     E.vol0 = m->vol0;

@@ -115,8 +115,8 @@ __device__ __forceinline__ void run_begin(RunShared& sh, int32_t status, int lau
 
 // The cycles of one launch.  Pol: the precision's element and node work.
 //   Pol::kTileBytes                       bytes of one staged tile of 32 elements
-//   Pol::load_tile(E, dst, bar, base, lane)   bulk copies of a tile
-//   Pol::store_tile(E, tile, base, lane)      its evolving rows back to global memory
+//   Pol::load_tile(E, dst, bar, t, lane)      bulk copy of tile t
+//   Pol::store_tile(E, tile, t, lane)         its evolving rows back to global memory
 //   Pol::element(E, N, M, tile, dt1, e, lane, ...)
 //   Pol::Nodes<W>                             a thread's W nodes: load (their rows), gather (their
 //                                             forces), update
@@ -165,7 +165,7 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
         }
         __syncwarp();
         for (int s = 0; s < mine; ++s)
-            Pol::load_tile(E, smem_addr(wtiles + s * Pol::kTileBytes), bar, (w0 + s * wstride) * 32, lane);
+            Pol::load_tile(E, smem_addr(wtiles + s * Pol::kTileBytes), bar, w0 + s * wstride, lane);
         loaded = mbar_wait_bounded(bar, 0);
         loaded = __all_sync(0xffffffffu, loaded);
     }
@@ -345,7 +345,7 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
     // ---- end of the launch: the evolving element rows, the energy partials
     // and the control block back to global memory
     for (int s = 0; s < mine && loaded; ++s)
-        Pol::store_tile(E, wtiles + s * Pol::kTileBytes, (w0 + s * wstride) * 32, lane);
+        Pol::store_tile(E, wtiles + s * Pol::kTileBytes, w0 + s * wstride, lane);
     if (tid == 0 && failed) atomicOr(&sync->status, ST_TIMEOUT);
     double kin = 0.0;
     for (int64_t n = t0; n < N.nn; n += stride) kin = kin + Pol::kinetic(N, n);

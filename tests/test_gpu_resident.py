@@ -87,8 +87,7 @@ def test_total_time_clamp_and_stop(dims):
 
 
 def test_a_mesh_beyond_the_chip_uses_the_phase_kernels():
-    m = M.box_mesh(296, 16, 16, 2.96, 0.16, 0.16)  # 75,776 elements fit in FP64
-    for n, launches in ((m.n_elements, 0), (m.n_elements + 1, 4)):
+    for n, launches in ((60_000, 0), (400_000, 4)):
         k = M.box_mesh(n, 1, 1, 0.01 * n, 0.01, 0.01)
         with capi.Stepper(k.x0, k.conn, None, material=M.Material(70e9, 0.33, 2700.0),
                           controls=M.Controls()) as s:
