@@ -787,25 +787,24 @@ int ensc_batch_download(ensc_batch* b, int32_t slot, double* x, double* u, doubl
     const bool mx = is_mixed(b);
     struct Item {
         double* dst;
-        const void* src;
+        const void* rows;   // element rows, or null: a node field
+        ensc::NodeField field;
         int64_t n;
         int comps;
     };
-    const Item items[] = {{x, sl.N.x, sl.nn, 3},          {u, sl.N.u, sl.nn, 3},      {v, sl.N.v, sl.nn, 3},
-                          {sigma, sl.E.sigma, sl.ne, 6}, {qia, sl.E.qia, sl.ne, 12}, {eps_p, sl.E.eps_p, sl.ne, 1}};
+    using F = ensc::NodeField;
+    const Item items[] = {{x, nullptr, F::X, sl.nn, 3},      {u, nullptr, F::U, sl.nn, 3},
+                          {v, nullptr, F::V, sl.nn, 3},      {sigma, sl.E.sigma, F::X, sl.ne, 6},
+                          {qia, sl.E.qia, F::X, sl.ne, 12},  {eps_p, sl.E.eps_p, F::X, sl.ne, 1}};
     const size_t need = static_cast<size_t>(std::max<int64_t>(12 * sl.ne, 3 * sl.nn)) * sizeof(double);
     double* stage = nullptr;
     BCK(b, cudaMallocFromPoolAsync(reinterpret_cast<void**>(&stage), need, b->pool, b->stream));
     int rc = ENSC_OK;
     for (const Item& it : items) {
         if (!it.dst) continue;
-        if (it.src == sl.N.v) ensc::launch_v_to_aos(sl.N, mx, stage, b->stream);
-        else if (it.src == sl.N.u && mx && ENSC_MIXED_UREF)
-            ensc::launch_disp_to_aos(sl.N.x, sl.N.u, sl.nn, sl.nn_pad, stage, b->stream);
-        else if (it.src == sl.N.x || it.src == sl.N.u)
-            ensc::launch_soa_to_aos(static_cast<const double*>(it.src), sl.nn, sl.nn_pad, 3, stage, b->stream);
+        if (!it.rows) ensc::launch_nodes_to_aos(sl.N, it.field, mx, stage, b->stream);
         else  // element fields, at their stored positions
-            ensc::launch_elem_to_aos(sl.E, it.src, it.comps, mx, stage, b->stream, sl.PA.iperm);
+            ensc::launch_elem_to_aos(sl.E, it.rows, it.comps, mx, stage, b->stream, sl.PA.iperm);
         cudaError_t e = cudaMemcpyAsync(it.dst, stage, it.n * it.comps * sizeof(double), cudaMemcpyDeviceToHost,
                                         b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

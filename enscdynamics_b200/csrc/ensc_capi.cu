@@ -507,23 +507,22 @@ int ensc_download(ensc_handle* h, double* x, double* u, double* v, double* sigma
     DevGuard dg(h->device);
     struct Item {
         double* dst;
-        const void* src;
+        const void* rows;   // element rows, or null: a node field
+        ensc::NodeField field;
         int64_t n;
         int comps;
     };
+    using F = ensc::NodeField;
     const bool mx = mixed(h);
-    const Item items[] = {{x, h->N.x, h->nn, 3},          {u, h->N.u, h->nn, 3},      {v, h->N.v, h->nn, 3},
-                          {sigma, h->E.sigma, h->ne, 6}, {qia, h->E.qia, h->ne, 12}, {eps_p, h->E.eps_p, h->ne, 1}};
+    const Item items[] = {{x, nullptr, F::X, h->nn, 3},          {u, nullptr, F::U, h->nn, 3},
+                          {v, nullptr, F::V, h->nn, 3},          {sigma, h->E.sigma, F::X, h->ne, 6},
+                          {qia, h->E.qia, F::X, h->ne, 12},      {eps_p, h->E.eps_p, F::X, h->ne, 1}};
     size_t used = 0;
     for (const Item& it : items) {
         if (!it.dst) continue;
-        if (it.src == h->N.v) ensc::launch_v_to_aos(h->N, mx, h->staging, h->stream);
-        else if (it.src == h->N.u && mx && ENSC_MIXED_UREF)
-            ensc::launch_disp_to_aos(h->N.x, h->N.u, h->nn, h->nn_pad, h->staging, h->stream);
-        else if (it.src == h->N.x || it.src == h->N.u)
-            ensc::launch_soa_to_aos(static_cast<const double*>(it.src), h->nn, h->nn_pad, 3, h->staging, h->stream);
+        if (!it.rows) ensc::launch_nodes_to_aos(h->N, it.field, mx, h->staging, h->stream);
         else  // element fields, at their stored positions
-            ensc::launch_elem_to_aos(h->E, it.src, it.comps, mx, h->staging, h->stream, h->PA.iperm);
+            ensc::launch_elem_to_aos(h->E, it.rows, it.comps, mx, h->staging, h->stream, h->PA.iperm);
         CK(h, cudaGetLastError());
         CK(h, cudaMemcpyAsync(it.dst, h->staging, it.n * it.comps * sizeof(double), cudaMemcpyDeviceToHost,
                               h->stream));
@@ -536,7 +535,7 @@ int ensc_download(ensc_handle* h, double* x, double* u, double* v, double* sigma
 int ensc_download_reactions(ensc_handle* h, double* rf) {
     if (!h || !rf) return ENSC_ERR_ARG;
     DevGuard dg(h->device);
-    ensc::launch_soa_to_aos(h->N.rf, h->nn, h->nn_pad, 3, h->staging, h->stream);
+    ensc::launch_reactions_to_aos(h->N, h->staging, h->stream);
     CK(h, cudaGetLastError());
     CK(h, cudaMemcpyAsync(rf, h->staging, h->nn * 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -550,17 +549,20 @@ int ensc_upload_state(ensc_handle* h, const double* x, const double* u, const do
     DevGuard dg(h->device);
     struct Item {
         const double* src;
-        void* dst;
+        void* rows;         // element rows, or null: a node field
+        ensc::NodeField field;
         int64_t n;
         int comps;
     };
+    using F = ensc::NodeField;
     const bool mx = mixed(h);
-    const Item items[] = {{x, h->N.x, h->nn, 3},          {u, h->N.u, h->nn, 3},      {v, h->N.v, h->nn, 3},
-                          {sigma, h->E.sigma, h->ne, 6}, {qia, h->E.qia, h->ne, 12}, {eps_p, h->E.eps_p, h->ne, 1}};
+    const Item items[] = {{x, nullptr, F::X, h->nn, 3},          {u, nullptr, F::U, h->nn, 3},
+                          {v, nullptr, F::V, h->nn, 3},          {sigma, h->E.sigma, F::X, h->ne, 6},
+                          {qia, h->E.qia, F::X, h->ne, 12},      {eps_p, h->E.eps_p, F::X, h->ne, 1}};
     size_t used = 0;
     // mixed: the u rows hold x - u; they hold u while x and u are replaced
-    const bool uref = mx && ENSC_MIXED_UREF && (x || u);
-    if (uref) ensc::launch_reflect_rows(h->N.x, h->N.u, h->nn, h->nn_pad, h->stream);
+    const bool uref = mx && (x || u);
+    if (uref) ensc::launch_reflect_rows(h->N, h->stream);
     cudaError_t ue = cudaGetLastError();
     const char* what = "ensc_upload_state";
     for (const Item& it : items) {
@@ -571,16 +573,13 @@ int ensc_upload_state(ensc_handle* h, const double* x, const double* u, const do
             what = "cudaMemcpyAsync(state upload)";
             break;
         }
-        if (it.dst == h->N.v) ensc::launch_aos_to_v(h->staging, h->N, mx, h->stream);
-        else if (it.dst == h->N.x || it.dst == h->N.u)
-            ensc::launch_aos_to_soa(h->staging, h->nn, h->nn_pad, 3, static_cast<double*>(it.dst), h->stream);
-        else
-            ensc::launch_aos_to_elem(h->staging, h->E, it.comps, it.dst, mx, h->stream, h->PA.iperm);
+        if (!it.rows) ensc::launch_aos_to_nodes(h->staging, h->N, it.field, mx, h->stream);
+        else ensc::launch_aos_to_elem(h->staging, h->E, it.comps, it.rows, mx, h->stream, h->PA.iperm);
         ue = cudaGetLastError();
         used = std::max(used, static_cast<size_t>(it.n * it.comps) * sizeof(double));
     }
     // back to x - u in the u rows, also when an upload above failed
-    if (uref) ensc::launch_reflect_rows(h->N.x, h->N.u, h->nn, h->nn_pad, h->stream);
+    if (uref) ensc::launch_reflect_rows(h->N, h->stream);
     if (ue == cudaSuccess) ue = cudaGetLastError();
     if (ue != cudaSuccess) {
         release_staging(h, used);
@@ -636,11 +635,10 @@ int ensc_snapshot_begin(ensc_handle* h) {
     const bool mx = mixed(h);
     if (mx) ensc::launch_acceleration_mixed(h->E, h->N, h->M, h->ctl, d + 3 * nodes3, h->stream, h->PA);
     else ensc::launch_acceleration_fp64(h->E, h->N, h->M, h->ctl, d + 3 * nodes3, h->stream);
-    ensc::launch_soa_to_aos(h->N.x, h->nn, h->nn_pad, 3, d, h->stream);
-    if (mx && ENSC_MIXED_UREF) ensc::launch_disp_to_aos(h->N.x, h->N.u, h->nn, h->nn_pad, d + nodes3, h->stream);
-    else ensc::launch_soa_to_aos(h->N.u, h->nn, h->nn_pad, 3, d + nodes3, h->stream);
-    ensc::launch_v_to_aos(h->N, mx, d + 2 * nodes3, h->stream);
-    ensc::launch_soa_to_aos(h->N.rf, h->nn, h->nn_pad, 3, d + 4 * nodes3, h->stream);
+    ensc::launch_nodes_to_aos(h->N, ensc::NodeField::X, mx, d, h->stream);
+    ensc::launch_nodes_to_aos(h->N, ensc::NodeField::U, mx, d + nodes3, h->stream);
+    ensc::launch_nodes_to_aos(h->N, ensc::NodeField::V, mx, d + 2 * nodes3, h->stream);
+    ensc::launch_reactions_to_aos(h->N, d + 4 * nodes3, h->stream);
     ensc::launch_elem_to_aos(h->E, h->E.sigma, 6, mx, d + 5 * nodes3, h->stream, h->PA.iperm);
     CK(h, cudaGetLastError());
     char* ctl_copy = reinterpret_cast<char*>(d) + (h->snap_bytes - sizeof(Ctl));

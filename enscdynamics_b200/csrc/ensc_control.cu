@@ -85,16 +85,15 @@ __global__ void __launch_bounds__(kCtlThreads) k_between(Ctl* ctl, Partials P, i
 }
 
 // Minimum squared edge of element e from the current coordinates.
-__device__ __forceinline__ double element_edge_sq(const ElemArrays& E, const NodeArrays& N, int64_t np, int64_t e) {
+__device__ __forceinline__ double element_edge_sq(const ElemArrays& E, const NodeArrays& N, int64_t e) {
     const uint32_t* cn = tile_row(E, E.conn, e) + (e & 31);
     const int64_t cs = tile_stride(E);
     double xyz[8][3];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const uint32_t n = cn[k * cs];
-        xyz[k][0] = N.x[n];
-        xyz[k][1] = N.x[np + n];
-        xyz[k][2] = N.x[2 * np + n];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) xyz[k][c] = *node_x(N, c, n);
     }
     return min_edge_sq(xyz);
 }
@@ -106,11 +105,10 @@ __device__ __forceinline__ double element_edge_sq(const ElemArrays& E, const Nod
 __global__ void __launch_bounds__(128) k_edge_prepass(ElemArrays E, NodeArrays N, Ctl* ctl) {
     if (ctl->done || !ctl->need_exact) return;
     __shared__ unsigned long long red[4];
-    const int64_t np = N.nn_pad;
     double m = DBL_MAX;
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < E.ne;
          e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const double mm = element_edge_sq(E, N, np, e);
+        const double mm = element_edge_sq(E, N, e);
         const double len = sqrt(mm);
         m = len < m ? len : m;
     }
@@ -153,23 +151,17 @@ __global__ void k_reset_init(Ctl* ctl) {
 
 // apply_boundary_condition_vec (exDyna3D.cpp:379-490): velocity conditions
 // first, fixed DOFs last.
-// One velocity component of a node: FP64, or the mixed stepper's float
-// (with its residual row, ENSC_MIXED_VLO).
+// One velocity component of a node: FP64, or the mixed stepper's float with
+// its residual row.
 template <typename VT>
 __device__ __forceinline__ double load_v(const NodeArrays& N, int c, int64_t n) {
-    const int64_t i = c * N.nn_pad + n;
-    if constexpr (sizeof(VT) == 4 && ENSC_MIXED_VLO)
-        return v_join(static_cast<const float*>(N.v)[i], v_lo_rows(N.v, N.nn_pad)[i]);
-    else
-        return static_cast<double>(static_cast<const VT*>(N.v)[i]);
+    if constexpr (sizeof(VT) == 4) return v_join(*node_vf(N, c, n), v_lo_rows(N.v, N.nn_pad)[c * N.nn_pad + n]);
+    else return *node_v64(N, c, n);
 }
 template <typename VT>
 __device__ __forceinline__ void store_v(const NodeArrays& N, int c, int64_t n, double v) {
-    const int64_t i = c * N.nn_pad + n;
-    if constexpr (sizeof(VT) == 4 && ENSC_MIXED_VLO)
-        v_split(v, static_cast<float*>(N.v)[i], v_lo_rows(N.v, N.nn_pad)[i]);
-    else
-        static_cast<VT*>(N.v)[i] = static_cast<VT>(v);
+    if constexpr (sizeof(VT) == 4) v_split(v, *node_vf(N, c, n), v_lo_rows(N.v, N.nn_pad)[c * N.nn_pad + n]);
+    else *node_v64(N, c, n) = v;
 }
 
 template <typename VT>
@@ -229,40 +221,41 @@ __global__ void k_soa_to_aos(const ST* soa, int64_t n, int64_t pad, int64_t tile
     }
 }
 
-// Displacements of a mixed instance, whose u rows hold the reference
-// position xr = x - u: interleaved u = x - xr.
-__global__ void k_disp_to_aos(const double* x, const double* xr, int64_t n, int64_t pad, double* aos) {
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < 3 * n;
+// a <- x - a over the u rows: turns the reference position rows of a mixed
+// instance into displacement rows and back
+__global__ void k_reflect_rows(NodeArrays N) {
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < 3 * N.nn;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t e = i / 3;
-        const int64_t k = (i - 3 * e) * pad + e;
-        aos[i] = x[k] - xr[k];
+        const int c = static_cast<int>(i / N.nn);
+        const int64_t n = i - c * N.nn, k = c * N.nn_pad + n;
+        N.u[k] = *node_x(N, c, n) - N.u[k];
     }
 }
 
-// a <- x - a over the three node rows: turns the reference position rows of
-// a mixed instance into displacement rows and back
-__global__ void k_reflect_rows(const double* x, double* a, int64_t n, int64_t pad) {
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < 3 * n;
+// Node fields between interleaved xyz doubles and the device layout.
+template <typename VT>
+__global__ void k_nodes_to_aos(NodeArrays N, NodeField field, double* aos) {
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < 3 * N.nn;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t c = i / n;
-        const int64_t k = c * pad + (i - c * n);
-        a[k] = x[k] - a[k];
+        const int64_t n = i / 3;
+        const int c = static_cast<int>(i - 3 * n);
+        if (field == NodeField::X) aos[i] = *node_x(N, c, n);
+        else if (field == NodeField::V) aos[i] = load_v<VT>(N, c, n);
+        else if (sizeof(VT) == 4) aos[i] = *node_x(N, c, n) - N.u[c * N.nn_pad + n];
+        else aos[i] = *node_u64(N, c, n);
     }
 }
-
-// Velocities between interleaved xyz doubles and the device rows.
 template <typename VT>
-__global__ void k_v_to_aos(NodeArrays N, double* aos) {
+__global__ void k_aos_to_nodes(const double* aos, NodeArrays N, NodeField field) {
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < 3 * N.nn;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        aos[i] = load_v<VT>(N, static_cast<int>(i % 3), i / 3);
-}
-template <typename VT>
-__global__ void k_aos_to_v(const double* aos, NodeArrays N) {
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < 3 * N.nn;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        store_v<VT>(N, static_cast<int>(i % 3), i / 3, aos[i]);
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t n = i / 3;
+        const int c = static_cast<int>(i - 3 * n);
+        if (field == NodeField::X) *node_x(N, c, n) = aos[i];
+        else if (field == NodeField::V) store_v<VT>(N, c, n, aos[i]);
+        else if (sizeof(VT) == 4) N.u[c * N.nn_pad + n] = aos[i];
+        else *node_u64(N, c, n) = aos[i];
+    }
 }
 
 template <typename DT>
@@ -351,7 +344,7 @@ __global__ void __launch_bounds__(128) k_edge_prepass_batch(BatchTables T) {
         const int64_t end = base + T.etile < d.E.ne ? base + T.etile : d.E.ne;
         double m = DBL_MAX;
         for (int64_t e = base + lane; e < end; e += 32) {
-            const double mm = element_edge_sq(d.E, d.N, d.N.nn_pad, e);
+            const double mm = element_edge_sq(d.E, d.N, e);
             const double len = sqrt(mm);
             m = len < m ? len : m;
         }
@@ -421,8 +414,8 @@ void launch_kinetic0(const NodeArrays& N, const Partials& P, Ctl* ctl, bool fp32
     else k_kinetic<double><<<grid, kNodeThreads, 0, st>>>(N, P);
     k_between<<<1, kCtlThreads, 0, st>>>(ctl, P, 2);
 }
-void launch_soa_to_aos(const double* soa, int64_t n, int64_t pad, int comps, double* aos, cudaStream_t st) {
-    k_soa_to_aos<double><<<grid_for(n * comps, 256), 256, 0, st>>>(soa, n, pad, 0, comps, nullptr, aos);
+void launch_reactions_to_aos(const NodeArrays& N, double* aos, cudaStream_t st) {
+    k_soa_to_aos<double><<<grid_for(3 * N.nn, 256), 256, 0, st>>>(N.rf, N.nn, N.nn_pad, 0, 3, nullptr, aos);
 }
 void launch_elem_to_aos(const ElemArrays& E, const void* rows, int comps, bool src_fp32, double* aos, cudaStream_t st,
                         const int32_t* at) {
@@ -434,24 +427,19 @@ void launch_elem_to_aos(const ElemArrays& E, const void* rows, int comps, bool s
         k_soa_to_aos<double><<<g, 256, 0, st>>>(static_cast<const double*>(rows), E.ne, 0, E.tile_bytes / 8, comps, at,
                                                 aos);
 }
-void launch_disp_to_aos(const double* x, const double* xr, int64_t n, int64_t pad, double* aos, cudaStream_t st) {
-    k_disp_to_aos<<<grid_for(3 * n, 256), 256, 0, st>>>(x, xr, n, pad, aos);
+void launch_reflect_rows(const NodeArrays& N, cudaStream_t st) {
+    k_reflect_rows<<<grid_for(3 * N.nn, 256), 256, 0, st>>>(N);
 }
-void launch_reflect_rows(const double* x, double* a, int64_t n, int64_t pad, cudaStream_t st) {
-    k_reflect_rows<<<grid_for(3 * n, 256), 256, 0, st>>>(x, a, n, pad);
+void launch_nodes_to_aos(const NodeArrays& N, NodeField field, bool mixed_precision, double* aos, cudaStream_t st) {
+    const int g = grid_for(3 * N.nn, 256);
+    if (mixed_precision) k_nodes_to_aos<float><<<g, 256, 0, st>>>(N, field, aos);
+    else k_nodes_to_aos<double><<<g, 256, 0, st>>>(N, field, aos);
 }
-void launch_v_to_aos(const NodeArrays& N, bool fp32_v, double* aos, cudaStream_t st) {
-    const int g = static_cast<int>(std::min<int64_t>((3 * N.nn + 255) / 256, 65535));
-    if (fp32_v) k_v_to_aos<float><<<g, 256, 0, st>>>(N, aos);
-    else k_v_to_aos<double><<<g, 256, 0, st>>>(N, aos);
-}
-void launch_aos_to_v(const double* aos, const NodeArrays& N, bool fp32_v, cudaStream_t st) {
-    const int g = static_cast<int>(std::min<int64_t>((3 * N.nn + 255) / 256, 65535));
-    if (fp32_v) k_aos_to_v<float><<<g, 256, 0, st>>>(aos, N);
-    else k_aos_to_v<double><<<g, 256, 0, st>>>(aos, N);
-}
-void launch_aos_to_soa(const double* aos, int64_t n, int64_t pad, int comps, double* soa, cudaStream_t st) {
-    k_aos_to_soa<double><<<grid_for(n * comps, 256), 256, 0, st>>>(aos, n, pad, 0, comps, nullptr, soa);
+void launch_aos_to_nodes(const double* aos, const NodeArrays& N, NodeField field, bool mixed_precision,
+                         cudaStream_t st) {
+    const int g = grid_for(3 * N.nn, 256);
+    if (mixed_precision) k_aos_to_nodes<float><<<g, 256, 0, st>>>(aos, N, field);
+    else k_aos_to_nodes<double><<<g, 256, 0, st>>>(aos, N, field);
 }
 void launch_aos_to_elem(const double* aos, const ElemArrays& E, int comps, void* rows, bool dst_fp32, cudaStream_t st,
                         const int32_t* at) {

@@ -15,20 +15,27 @@
 //     sigma[6], qia[12], eps_p
 //     fe                             element nodal forces of the current cycle
 //                                    (the element -> node hand-off, scratch):
-//                                    [24][nn_pad] by node and local slot when
-//                                    no node repeats a slot, else [24][ne_pad]
-//   node arrays, length nn (stride nn_pad):
-//     x[3][nn_pad], u[3][nn_pad] (FP64 always), v[3][nn_pad]
+//                                    by node and local slot when no node
+//                                    repeats a slot, else by element; per slot a
+//                                    row of (fx, fy) pairs, after the eight of
+//                                    them a row of fz per slot (force_xy, force_z)
+//   node arrays, length nn (stride nn_pad), in 32-byte records that one load
+//   brings in (rec 1):
+//     FP64:  x = [nn_pad] {x, y, z, ux}, u = [nn_pad] {uy, uz, vx, vy}, v = vz
+//     mixed: x = [nn_pad] {x, y, z, (vx, vy) as two floats}, v = vz as float, then
+//            the 16-bit residual rows [3][nn_pad] of v; u = [3][nn_pad] rows of
+//            the reference position x - u
+//     caller-owned memory (rec 0, FP64): plain rows [3][nn] of x, u and v
 //     inv_mass[nn]                   per node (equal for the 3 DOFs)
 //     bc[nn] uint8                   2 bits per DOF (bit0 fixed, bit1 velocity)
 //     bcv[3][nn_pad]                 prescribed velocities
-//     ell[8][nn_pad] uint32          element holding node n in local slot k, or
-//                                    ENSC_NONE; the gather sums slots k = 0..7
-//                                    in order, as the reference sums its 8
-//                                    slot vectors (exDyna3D.cpp:638-639)
-//     csr_ptr/csr_ent                general (slot, element)-sorted lists, used
-//                                    instead of ell when a node occupies the
-//                                    same slot in more than one element
+//     ell[8][nn] uint32              caller-owned memory: element holding node n
+//                                    in local slot k, or ENSC_NONE; the gather sums
+//                                    slots k = 0..7 in order, as the reference sums
+//                                    its 8 slot vectors (exDyna3D.cpp:638-639)
+//     csr_ptr/csr_ent                general (slot, element)-sorted lists, where
+//                                    a node occupies the same slot in more than
+//                                    one element
 #pragma once
 
 #include <cmath>
@@ -150,11 +157,10 @@ struct ElemArrays {
     // which starts 256-byte aligned (node rows too, padded to 32 entries: the
     // vectorised node passes).  0: plain rows of ne_pad entries.
     int32_t tile_bytes;
-    // 1: fe is node-major, fe[(3k + c) * nn_pad + conn[k][e]] -- the
-    // reference's per-local-slot nodal vectors (exDyna3D.cpp:523-634), each
-    // entry written by the one element that holds the node in slot k;
-    // 0: fe is element-major, fe[(3k + c) * ne_pad + e], gathered through
-    // ell / csr by the node pass
+    // 1: the entries of fe are nodes -- the reference's per-local-slot nodal
+    // vectors (exDyna3D.cpp:523-634), each entry written by the one element
+    // that holds the node in slot k; 0: elements, gathered through ell / csr by
+    // the node pass
     int32_t slot_major;
     int32_t bt9;               // FP64: bt holds 9 numbers per element (else 24)
     int32_t pad;
@@ -209,9 +215,21 @@ struct NodeArrays {
     const uint32_t* ell;
     const int64_t* csr_ptr;    // non-null: use the general lists
     const uint32_t* csr_ent;   // (e << 3) | slot
-    const uint8_t* slot_mask;  // slot-major forces: bit k set if slot k holds an element
     double* rf;                // reactions, [3][nn_pad]
+    int32_t rec;               // 1: x, u, v in records (head of this file), 0: rows
+    int32_t pad;
 };
+
+// Force hand-off of slot k, entry i (a node or an element; `np` entries per
+// row): (fx, fy) and fz.
+template <typename T>
+__host__ __device__ inline T* force_xy(T* fe, int64_t np, int k, int64_t i) {
+    return fe + 2 * (k * np + i);
+}
+template <typename T>
+__host__ __device__ inline T* force_z(T* fe, int64_t np, int k, int64_t i) {
+    return fe + (16 + k) * np + i;
+}
 
 // Partial sums written by each block of a pass, folded in fixed block order.
 struct Partials {
@@ -233,7 +251,6 @@ struct alignas(128) NodeView {
     double* x;
     const double* inv_mass;
     const uint8_t* bc;
-    const uint8_t* slot_mask;  // bit k: slot k holds an element
     double* rf;
     Ctl* ctl;
     int64_t nn, np;
@@ -258,7 +275,6 @@ __host__ __device__ inline NodeView node_view(const ElemArrays& E, const NodeArr
     v.x = N.x;
     v.inv_mass = N.inv_mass;
     v.bc = N.bc;
-    v.slot_mask = N.slot_mask;
     v.rf = N.rf;
     v.ctl = ctl;
     v.nn = N.nn;
@@ -408,11 +424,7 @@ __host__ __device__ inline double gravity_amplitude(const double* amp, int n, do
 // element pass reads) and a 16-bit residual `lo` in units of 2^-16 of hi's
 // spacing: v = hi + lo * ulp(hi) / 2^16, about 40 significant bits.  The node
 // pass updates v in FP64 and splits it again, so the velocity integration
-// does not drop FP32 rounding every cycle.  In memory the residual rows
-// follow the three float rows: [3][nn_pad] float, then [3][nn_pad] int16.
-#ifndef ENSC_MIXED_VLO
-#define ENSC_MIXED_VLO 1
-#endif
+// does not drop FP32 rounding every cycle.
 
 // The mixed stepper's element pass forms F from the current coordinates and
 // never reads the displacement, so it keeps the reference position
@@ -420,9 +432,6 @@ __host__ __device__ inline double gravity_amplitude(const double* amp, int n, do
 // u = x - xr is formed where the state is read (ensc_download, snapshots),
 // and an upload of x or u sets xr = x - u.  Both are FP64: u = x - xr is
 // within a rounding of x's magnitude of the separately accumulated u.
-#ifndef ENSC_MIXED_UREF
-#define ENSC_MIXED_UREF 1
-#endif
 
 // ulp(hi) / 2^16 and its inverse (normal or zero hi; hi's exponent field e
 // gives ulp(hi) = 2^(e - 150), with e = 1 for zero and subnormals)
@@ -457,7 +466,43 @@ __host__ __device__ inline void v_split(double v, float& hi, int16_t& lo) {
 }
 // the residual rows of a mixed velocity array
 __host__ __device__ inline int16_t* v_lo_rows(void* v, int64_t nn_pad) {
-    return reinterpret_cast<int16_t*>(static_cast<float*>(v) + 3 * nn_pad);
+    return reinterpret_cast<int16_t*>(static_cast<float*>(v) + nn_pad);
+}
+
+// One entry of the node state in either layout (FP64 displacement; the mixed
+// u rows are plain).
+__host__ __device__ inline double* node_x(const NodeArrays& N, int c, int64_t n) {
+    return N.rec ? N.x + 4 * n + c : N.x + c * N.nn_pad + n;
+}
+__host__ __device__ inline double* node_u64(const NodeArrays& N, int c, int64_t n) {
+    if (!N.rec) return N.u + c * N.nn_pad + n;
+    return c == 0 ? N.x + 4 * n + 3 : N.u + 4 * n + (c - 1);
+}
+__host__ __device__ inline double* node_v64(const NodeArrays& N, int c, int64_t n) {
+    double* v = static_cast<double*>(N.v);
+    if (!N.rec) return v + c * N.nn_pad + n;
+    return c < 2 ? N.u + 4 * n + 2 + c : v + n;
+}
+__host__ __device__ inline float* node_vf(const NodeArrays& N, int c, int64_t n) {
+    return c < 2 ? reinterpret_cast<float*>(N.x + 4 * n + 3) + c : static_cast<float*>(N.v) + n;
+}
+
+// A node record: 32 bytes in one load or store.  The load is volatile, as a
+// resident run's records change between its cycles.
+__device__ __forceinline__ void ld_rec(const double* p, double (&o)[4]) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+                 : "l"(p));
+}
+__device__ __forceinline__ void st_rec(double* p, const double (&v)[4]) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                 : "memory");
+}
+// the two floats of a mixed record's fourth word
+__device__ __forceinline__ float rec_vx(double w) { return __int_as_float(__double2loint(w)); }
+__device__ __forceinline__ float rec_vy(double w) { return __int_as_float(__double2hiint(w)); }
+__device__ __forceinline__ double rec_vxy(float vx, float vy) {
+    return __hiloint2double(__float_as_int(vy), __float_as_int(vx));
 }
 
 // Vector access to W consecutive entries of a padded SoA row (rows start

@@ -249,10 +249,11 @@ __device__ __forceinline__ constexpr bool gamma_plus(int k, int j) {
 // kernels; inputs come from S, the evolving rows go to O and the forces to the
 // instance's force array at element e.  Node rows are read with plain loads: a
 // resident run rewrites them between its cycles.  SMEM: S's rows are in shared
-// memory.  BT9: its bt rows are the 9-number form.  PF: node rows the body reads
-// later are prefetched into L1 once the connectivity is known (bit 0 the
-// velocities, bit 1 the displacements).
-template <bool PLASTIC, bool INIT, bool BT9, bool SMEM = false, int PF = 0>
+// memory.  BT9: its bt rows are the 9-number form.  REC: node records (three
+// loads per node; a record's last numbers are read when F and the velocity
+// gradient need them), else plain rows.  PF: the second record and vz of each
+// node are prefetched into L1 once the connectivity is known.
+template <bool PLASTIC, bool INIT, bool BT9, bool REC, bool SMEM = false, bool PF = false>
 __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArrays& N, const Material& M,
                                              const Fp64Src& S, const Fp64Out& O, const double dt1, const int64_t e,
                                              double& dts, double& len, double& e_int, double& e_hg, double& e_vis,
@@ -268,34 +269,57 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
     uint32_t n[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) n[k] = ldin<SMEM>(S.conn + k * ss + si);
-    if (PF & 1) {
+    if constexpr (REC && PF) {
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+        for (int k = 0; k < 8; ++k) prefetch_l1(U + 4 * static_cast<int64_t>(n[k]));
 #pragma unroll
-            for (int k = 0; k < 8; ++k) prefetch_l1(V + r * np + n[k]);
-    }
-    if (PF & 2) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) prefetch_l1(U + r * np + n[k]);
+        for (int k = 0; k < 8; ++k) prefetch_l1(V + n[k]);
     }
     // current coordinates: hourglass projections TAU x and the minimum edge
     // (min_ele_edge :1173-1220)
-    double TX[4][3];
+    double TX[4][3], ux[8];
     {
         double xyz[8][3];
+        if constexpr (REC) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                double q[4];
+                ld_rec(X + 4 * static_cast<int64_t>(n[k]), q);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) xyz[k][c] = q[c];
+                ux[k] = q[3];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) xyz[k][c] = X[c * np + n[k]];
+        }
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             double x[8], t[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) xyz[k][c] = x[k] = X[c * np + n[k]];
+            for (int k = 0; k < 8; ++k) x[k] = xyz[k][c];
             gamma_sums(x, t);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) TX[kk][c] = t[kk];
         }
         len = sqrt(min_edge_sq(xyz));
     }
+    // the second records: uy, uz, vx, vy
+    double q1[8][4];
+    if constexpr (REC) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ld_rec(U + 4 * static_cast<int64_t>(n[k]), q1[k]);
+    }
+    auto u_at = [&](int r, int k) -> double {
+        if constexpr (REC) return r == 0 ? ux[k] : q1[k][r - 1];
+        else return U[r * np + n[k]];
+    };
+    auto v_at = [&](int r, int k) -> double {
+        if constexpr (REC) return r < 2 ? q1[k][2 + r] : V[n[k]];
+        else return V[r * np + n[k]];
+    };
     // F = I + u_e B0^T (:862-865); with B0 in its 9-number form one component
     // at a time, else node by node (24 numbers would stay in registers)
     B0Rows<BT9, SMEM> B;
@@ -306,7 +330,7 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
         for (int r = 0; r < 3; ++r) {
             double u[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) u[k] = U[r * np + n[k]];
+            for (int k = 0; k < 8; ++k) u[k] = u_at(r, k);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 double t = 0.0;
@@ -320,12 +344,11 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
         for (int i = 0; i < 9; ++i) F[i / 3][i % 3] = 0.0;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const uint32_t nk = ldin<SMEM>(S.conn + k * ss + si);
             double bb[3];
             B.row(S, k, bb);
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-                const double u = U[r * np + nk];
+                const double u = u_at(r, k);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) F[r][c] = __fma_rn(u, bb[c], F[r][c]);
             }
@@ -344,7 +367,7 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
         for (int r = 0; r < 3; ++r) {
             double v[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = V[r * np + n[j]];
+            for (int j = 0; j < 8; ++j) v[j] = v_at(r, j);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 double l = 0.0;
@@ -370,12 +393,11 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const uint32_t nj = ldin<SMEM>(S.conn + j * ss + si);
             double bb[3];
             B.row(S, j, bb);
 #pragma unroll
             for (int r = 0; r < 3; ++r) {
-                const double v = V[r * np + nj];
+                const double v = v_at(r, j);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) L0[r][c] = __fma_rn(v, bb[c], L0[r][c]);
 #pragma unroll
@@ -510,14 +532,17 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
     // is evaluated once for two opposite corners.
     {
         B0Rows<BT9, SMEM> Bf;
-        if constexpr (BT9) Bf.load(S);
-        auto store = [&](int j, int i, double f) {
-            if (E.slot_major) fe[(3 * j + i) * np + ldin<SMEM>(S.conn + j * ss + si)] = f;
-            else fe[(3 * j + i) * ep + e] = f;
+        auto store = [&](int j, const double (&f)[3]) {
+            const int64_t row = E.slot_major ? np : ep;
+            const int64_t i = E.slot_major ? static_cast<int64_t>(ldin<SMEM>(S.conn + j * ss + si)) : e;
+            *reinterpret_cast<double2*>(force_xy(fe, row, j, i)) = make_double2(f[0], f[1]);
+            *force_z(fe, row, j, i) = f[2];
         };
+        if constexpr (BT9) {
+            Bf.load(S);
+            double f[8][3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            if constexpr (BT9) {
+            for (int i = 0; i < 3; ++i) {
                 const double g0 = Gq[i][0], g1 = Gq[i][1], g2 = Gq[i][2], g3 = Gq[i][3];
                 const double d = g0 - g1, q = g0 + g1;
                 const double dm = d - g2, dp = d + g2, qm = g2 - q, qp = q + g2;
@@ -527,21 +552,23 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
                 for (int j = 0; j < 4; ++j)
                     bz[j] = __fma_rn(Bf.r[j][2], Z[2][i], __fma_rn(Bf.r[j][1], Z[1][i], Bf.r[j][0] * Z[0][i]));
 #pragma unroll
-                for (int j = 0; j < 8; ++j) store(j, i, (Bf.minus(j) ? bz[Bf.index(j)] : -bz[Bf.index(j)]) - t[j]);
+                for (int j = 0; j < 8; ++j) f[j][i] = (Bf.minus(j) ? bz[Bf.index(j)] : -bz[Bf.index(j)]) - t[j];
             }
-        }
-        if constexpr (!BT9) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) store(j, f[j]);
+        } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                double bb[3];
+                double bb[3], f[3];
                 Bf.row(S, j, bb);
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
                     double tg = gamma_plus(0, j) ? Gq[i][0] : -Gq[i][0];
 #pragma unroll
                     for (int kk = 1; kk < 4; ++kk) tg = gamma_plus(kk, j) ? tg + Gq[i][kk] : tg - Gq[i][kk];
-                    store(j, i, -__fma_rn(bb[2], Z[2][i], __fma_rn(bb[1], Z[1][i], bb[0] * Z[0][i])) - tg);
+                    f[i] = -__fma_rn(bb[2], Z[2][i], __fma_rn(bb[1], Z[1][i], bb[0] * Z[0][i])) - tg;
                 }
+                store(j, f);
             }
         }
     }
@@ -582,7 +609,7 @@ __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_FP64) k_element(E
         const int64_t e = live ? e0 : 0;
         double dts = DBL_MAX, len = DBL_MAX;
         if (live)
-            element_body<PLASTIC, INIT, BT9>(E, N, M, fp64_src_global<TILED>(E, e), fp64_out_global<TILED>(E, e), dt1, e,
+            element_body<PLASTIC, INIT, BT9, TILED>(E, N, M, fp64_src_global<TILED>(E, e), fp64_out_global<TILED>(E, e), dt1, e,
                                              dts, len, e_int, e_hg, e_vis, bad);
         dts_min = dts < dts_min ? dts : dts_min;
         len_min = len < len_min ? len : len_min;
@@ -595,72 +622,74 @@ __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_FP64) k_element(E
     }
 }
 
-// One node of the node pass (see the kernel comment below); shared by the
+// The force of one node from per-element forces (E.slot_major 0): the
+// caller-owned table of one element per slot, or the general lists, sorted by
+// (slot, element): each slot's contributions are summed first (the reference's
+// per-slot += in element order), then added to the running total.
+__device__ __forceinline__ void listed_forces(const ElemArrays& E, const NodeArrays& N, const int64_t n,
+                                              double (&f)[3]) {
+    const int64_t np = N.nn_pad, ep = E.ne_pad;
+    const double* fe = static_cast<const double*>(E.fe);
+    auto at = [&](int k, uint32_t el, double (&r)[3]) {
+        const double2 xy = *reinterpret_cast<const double2*>(force_xy(fe, ep, k, el));
+        r[0] = xy.x;
+        r[1] = xy.y;
+        r[2] = *force_z(fe, ep, k, el);
+    };
+    f[0] = f[1] = f[2] = 0.0;
+    if (N.csr_ptr == nullptr) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t el = __ldg(N.ell + k * np + n);
+            if (el != ENSC_NONE) {
+                double r[3];
+                at(k, el, r);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) f[c] = f[c] + r[c];
+            }
+        }
+        return;
+    }
+    const int64_t b = N.csr_ptr[n], t = N.csr_ptr[n + 1];
+    int cur = -1;
+    double sl[3] = {0.0, 0.0, 0.0};
+    for (int64_t i = b; i < t; ++i) {
+        const uint32_t ent = N.csr_ent[i];
+        const int k = static_cast<int>(ent & 7u);
+        double r[3];
+        at(k, ent >> 3, r);
+        if (k != cur) {
+            if (cur >= 0) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) f[c] = f[c] + sl[c];
+            }
+            cur = k;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sl[c] = 0.0 + r[c];
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sl[c] = sl[c] + r[c];
+        }
+    }
+    if (cur >= 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = f[c] + sl[c];
+    }
+}
+
+// One node of the node pass where the forces are per element; shared by the
 // single-instance, batched and resident-run kernels (KIN: sum the kinetic
 // energy).
 template <bool KIN = true>
 __device__ __forceinline__ void node_body(const ElemArrays& E, const NodeArrays& N, const Material& M,
                                           const double dt_i, const double dt_i_1, const double amp, const int64_t n, double& kin,
                                           double& wext, int32_t& bad) {
-    const int64_t np = N.nn_pad, ep = E.ne_pad;
-    const double* fe = static_cast<const double*>(E.fe);
-    double* V = static_cast<double*>(N.v);
+    const int64_t np = N.nn_pad;
     const double half = (dt_i + dt_i_1);
     const double dt_avg = (dt_i + dt_i_1) / 2.0;
 
     double f[3];
-    if (E.slot_major) {
-        // the reference's ((((((a0+a1)+a2)+a3)+a4)+a5)+a6)+a7 over the
-        // slots that hold an element (an absent slot adds +0.0)
-        f[0] = f[1] = f[2] = 0.0;
-        const uint32_t msk = N.slot_mask[n];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if ((msk >> k) & 1u) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) f[c] = f[c] + fe[(3 * k + c) * np + n];
-            }
-        }
-    } else if (N.csr_ptr == nullptr) {
-        f[0] = f[1] = f[2] = 0.0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t el = __ldg(N.ell + k * np + n);
-            if (el != ENSC_NONE) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) f[c] = f[c] + fe[(3 * k + c) * ep + el];
-            }
-        }
-    } else {
-        // general lists: entries sorted by (slot, element); each slot's
-        // contributions are summed first (the reference's per-slot +=
-        // in element order), then added to the running total
-        f[0] = f[1] = f[2] = 0.0;
-        const int64_t b = N.csr_ptr[n], t = N.csr_ptr[n + 1];
-        int cur = -1;
-        double sl[3] = {0.0, 0.0, 0.0};
-        for (int64_t i = b; i < t; ++i) {
-            const uint32_t ent = N.csr_ent[i];
-            const int k = static_cast<int>(ent & 7u);
-            const uint32_t el = ent >> 3;
-            if (k != cur) {
-                if (cur >= 0) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) f[c] = f[c] + sl[c];
-                }
-                cur = k;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) sl[c] = 0.0 + fe[(3 * k + c) * ep + el];
-            } else {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) sl[c] = sl[c] + fe[(3 * k + c) * ep + el];
-            }
-        }
-        if (cur >= 0) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) f[c] = f[c] + sl[c];
-        }
-    }
+    listed_forces(E, N, n, f);
     const double im = N.inv_mass[n];
     const uint32_t code = N.bc[n];
 #pragma unroll
@@ -684,88 +713,16 @@ __device__ __forceinline__ void node_body(const ElemArrays& E, const NodeArrays&
         }
         if (cc) N.rf[c * np + n] = rf;
         a = a * im;
-        const double vo = V[c * np + n];
+        double *pv = node_v64(N, c, n), *pu = node_u64(N, c, n), *px = node_x(N, c, n);
+        const double vo = *pv;
         const double vn = vo + half * a / 2.0;
-        V[c * np + n] = vn;
-        N.u[c * np + n] = N.u[c * np + n] + dt_i * vn;
-        N.x[c * np + n] = N.x[c * np + n] + dt_i * vn;
+        *pv = vn;
+        *pu = *pu + dt_i * vn;
+        *px = *px + dt_i * vn;
         const double vb = 0.5 * (vo + vn);
         wext = wext + (g + r) * dt_avg * vb;
         if (KIN) kin = kin + 0.5 * (vn * vn) / im;
         if (!isfinite(vn)) bad |= ST_NONFINITE;
-    }
-}
-
-// ---- output: the last cycle's acceleration --------------------------------
-// solution_a as compute_a leaves it (exDyna3D.cpp:642-644) in the last cycle
-// -- assembled element forces, gravity, the acceleration boundary conditions,
-// times the inverse mass -- which output_results writes (:231).  The node
-// pass does not store it; this pass evaluates it again from the element
-// forces that the last force pass left in fe, with the node pass's
-// arithmetic in the node pass's order (the grouped layout adds all 8 slots,
-// empty ones as the zeros they hold).  Writes interleaved xyz per node.
-__global__ void __launch_bounds__(kNodeThreads) k_acceleration(ElemArrays E, NodeArrays N, Material M, const Ctl* ctl,
-                                                               double* a_out) {
-    const int64_t np = N.nn_pad, ep = E.ne_pad;
-    const double* __restrict__ fe = static_cast<const double*>(E.fe);
-    const bool grouped = E.slot_major && E.tile_bytes;
-    const double amp = (M.gravity_on && M.amp_n > 0) ? gravity_amplitude(M.amp, M.amp_n, ctl->time, ctl->dt_i) : 1.0;
-    for (int64_t n = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; n < N.nn;
-         n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        double f[3] = {0.0, 0.0, 0.0};
-        if (E.slot_major) {
-            const uint32_t msk = grouped ? 0xffu : N.slot_mask[n];
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if ((msk >> k) & 1u) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) f[c] = f[c] + fe[(3 * k + c) * np + n];
-                }
-        } else if (N.csr_ptr == nullptr) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint32_t el = N.ell[k * np + n];
-                if (el != ENSC_NONE) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) f[c] = f[c] + fe[(3 * k + c) * ep + el];
-                }
-            }
-        } else {
-            int cur = -1;
-            double sl[3] = {0.0, 0.0, 0.0};
-            for (int64_t i = N.csr_ptr[n]; i < N.csr_ptr[n + 1]; ++i) {
-                const uint32_t ent = N.csr_ent[i];
-                const int k = static_cast<int>(ent & 7u);
-                const uint32_t el = ent >> 3;
-                if (k != cur) {
-                    if (cur >= 0) {
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) f[c] = f[c] + sl[c];
-                    }
-                    cur = k;
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) sl[c] = 0.0 + fe[(3 * k + c) * ep + el];
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) sl[c] = sl[c] + fe[(3 * k + c) * ep + el];
-                }
-            }
-            if (cur >= 0) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) f[c] = f[c] + sl[c];
-            }
-        }
-        const double im = N.inv_mass[n];
-        const uint32_t code = N.bc[n];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            double a = f[c];
-            if (M.gravity_on) a = a + amp * M.gravity_value * M.gravity_dir[c] / im;
-            const uint32_t cc = (code >> (2 * c)) & 3u;
-            if (cc & 2u) a = 0.0;
-            if ((cc & 1u) && a != 0.0) a = 0.0;
-            a_out[3 * n + c] = a * im;
-        }
     }
 }
 
@@ -832,7 +789,7 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
         if (e < E.ne) {
             unsigned char* g = const_cast<unsigned char*>(tiles) + t * L::kBytes;
             double dts, len;
-            element_body<PLASTIC, false, BT9, true, ENSC_F64_PREFETCH>(E, N, M, fp64_src_tile<L>(wst + s * L::kBytes, lane),
+            element_body<PLASTIC, false, BT9, true, true, ENSC_F64_PREFETCH>(E, N, M, fp64_src_tile<L>(wst + s * L::kBytes, lane),
                                                                        fp64_out_tile<L>(g, lane), dt1, e, dts, len,
                                                                        e_int, e_hg, e_vis, bad);
             dts_min = dts < dts_min ? dts : dts_min;
@@ -860,34 +817,28 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
     block_sum<32 * kF64PipeWarps, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
 }
 
-// W consecutive nodes of the node pass with 16-byte row accesses: the same
-// arithmetic per node as node_body on the slot-major layout, in the same
-// order.  Slots the mask marks empty are skipped, or (ENSC_NODE_ALL_SLOTS)
-// added as the zeros they hold, as the reference adds all 8 slot vectors:
-// the slot-major rows start zeroed and only the slot's element writes them.
+// W consecutive nodes of the node pass on the slot-major layout.  Every slot is
+// added, empty ones as the zeros they hold, as the reference adds all 8 slot
+// vectors: the rows start zeroed and only the slot's element writes them.
 // Nodes at or past nn (row padding) are loaded and stored back unchanged.
 //
-// pre (resident runs): the nodes' own rows, loaded while the grid still works
+// pre (resident runs): the nodes' own records, loaded while the grid still works
 // on the forces; such a run sums its kinetic energy once, at its end.
 template <int W>
 struct NodeRowsF64 {
-    double im[W], rim[W], v[3][W], u[3][W], x[3][W];  // rim: 1 / im, under gravity
+    double im[W], rim[W], q0[W][4], q1[W][4], vz[W];  // rim: 1 / im, under gravity
     uint32_t code;
 };
 template <int W>
 __device__ __forceinline__ void node_rows_load(const NodeView& N, const int64_t n0, NodeRowsF64<W>& r) {
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        ld_rec(N.x + 4 * (n0 + j), r.q0[j]);
+        ld_rec(N.u + 4 * (n0 + j), r.q1[j]);
+    }
+    ld_row<W>(static_cast<const double*>(N.v) + n0, r.vz);
     ld_row<W>(N.inv_mass + n0, r.im);
     r.code = ld_bytes<W>(N.bc + n0);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        ld_row<W>(static_cast<const double*>(N.v) + c * N.np + n0, r.v[c]);
-        ld_row<W>(N.u + c * N.np + n0, r.u[c]);
-        ld_row<W>(N.x + c * N.np + n0, r.x[c]);
-    }
-    if (N.gravity_on) {
-#pragma unroll
-        for (int j = 0; j < W; ++j) r.rim[j] = 1.0 / r.im[j];
-    }
 }
 
 // The forces of W consecutive nodes, added up in slot order.
@@ -899,21 +850,16 @@ __device__ __forceinline__ void node_forces(const NodeView& N, const int64_t n0,
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int j = 0; j < W; ++j) f[c][j] = 0.0;
-    const uint32_t msk = ENSC_NODE_ALL_SLOTS ? 0xffffffffu : ld_bytes<W>(N.slot_mask + n0);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        uint32_t sel = 0;
+        double xy[2 * W], z[W];
+        ld_row<2 * W>(force_xy(fe, np, k, n0), xy);
+        ld_row<W>(force_z(fe, np, k, n0), z);
 #pragma unroll
-        for (int j = 0; j < W; ++j) sel |= ((msk >> (8 * j + k)) & 1u) << j;
-        if (sel) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                double r[W];
-                ld_row<W>(fe + (3 * k + c) * np + n0, r);
-#pragma unroll
-                for (int j = 0; j < W; ++j)
-                    if ((sel >> j) & 1u) f[c][j] = f[c][j] + r[j];
-            }
+        for (int j = 0; j < W; ++j) {
+            f[0][j] = f[0][j] + xy[2 * j];
+            f[1][j] = f[1][j] + xy[2 * j + 1];
+            f[2][j] = f[2][j] + z[j];
         }
     }
 }
@@ -925,9 +871,11 @@ __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i,
                                            const NodeRowsF64<W>* pre = nullptr,
                                            const double (*fpre)[W] = nullptr) {
     const int64_t np = N.np, nn = N.nn;
-    double* V = static_cast<double*>(N.v);
     const double half = (dt_i + dt_i_1);
     const double dt_avg = (dt_i + dt_i_1) / 2.0;
+    NodeRowsF64<W> own;
+    if constexpr (PRE) own = *pre;
+    else node_rows_load<W>(N, n0, own);
     double f[3][W];
     if constexpr (PRE) {
 #pragma unroll
@@ -937,46 +885,23 @@ __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i,
     } else {
         node_forces<W>(N, n0, f);
     }
-    double im[W];
-    uint32_t code;
-    if constexpr (PRE) {
 #pragma unroll
-        for (int j = 0; j < W; ++j) im[j] = pre->im[j];
-        code = pre->code;
-    } else {
-        ld_row<W>(N.inv_mass + n0, im);
-        code = ld_bytes<W>(N.bc + n0);
-    }
+    for (int j = 0; j < W; ++j) {
+        if (n0 + j >= nn) continue;
+        const double im = own.im[j];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        double vo[W], uo[W], xo[W], vn[W], un[W], xn[W];
-        if constexpr (PRE) {
-#pragma unroll
-            for (int j = 0; j < W; ++j) {
-                vo[j] = pre->v[c][j];
-                uo[j] = pre->u[c][j];
-                xo[j] = pre->x[c][j];
-            }
-        } else {
-            ld_row<W>(V + c * np + n0, vo);
-            ld_row<W>(N.u + c * np + n0, uo);
-            ld_row<W>(N.x + c * np + n0, xo);
-        }
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            vn[j] = vo[j];
-            un[j] = uo[j];
-            xn[j] = xo[j];
-            if (n0 + j >= nn) continue;
+        for (int c = 0; c < 3; ++c) {
+            double* pv = c == 2 ? &own.vz[j] : &own.q1[j][2 + c];
+            double* pu = c == 0 ? &own.q0[j][3] : &own.q1[j][c - 1];
             double a = f[c][j];
             double g = 0.0;
             if (N.gravity_on) {
                 const double w = amp * N.gravity_value * N.gravity_dir[c];
-                if constexpr (PRE) g = div_by(w, im[j], pre->rim[j]);
-                else g = w / im[j];
+                if constexpr (PRE) g = div_by(w, im, own.rim[j]);
+                else g = w / im;
                 a = a + g;
             }
-            const uint32_t cc = (code >> (8 * j + 2 * c)) & 3u;
+            const uint32_t cc = (own.code >> (8 * j + 2 * c)) & 3u;
             double r = 0.0, rf = 0.0;
             if (cc & 2u) {
                 r = -a;
@@ -988,18 +913,59 @@ __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i,
                 a = 0.0;
             }
             if (cc) N.rf[c * np + n0 + j] = rf;
-            a = a * im[j];
-            vn[j] = vo[j] + half * a / 2.0;
-            un[j] = uo[j] + dt_i * vn[j];
-            xn[j] = xo[j] + dt_i * vn[j];
-            const double vb = 0.5 * (vo[j] + vn[j]);
+            a = a * im;
+            const double vo = *pv, vn = vo + half * a / 2.0;
+            *pv = vn;
+            *pu = *pu + dt_i * vn;
+            own.q0[j][c] = own.q0[j][c] + dt_i * vn;
+            const double vb = 0.5 * (vo + vn);
             wext = wext + (g + r) * dt_avg * vb;
-            if (!PRE) kin = kin + 0.5 * (vn[j] * vn[j]) / im[j];
-            if (!isfinite(vn[j])) bad |= ST_NONFINITE;
+            if (!PRE) kin = kin + 0.5 * (vn * vn) / im;
+            if (!isfinite(vn)) bad |= ST_NONFINITE;
         }
-        st_row<W>(V + c * np + n0, vn);
-        st_row<W>(N.u + c * np + n0, un);
-        st_row<W>(N.x + c * np + n0, xn);
+    }
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        st_rec(N.x + 4 * (n0 + j), own.q0[j]);
+        st_rec(N.u + 4 * (n0 + j), own.q1[j]);
+    }
+    st_row<W>(static_cast<double*>(N.v) + n0, own.vz);
+}
+
+// ---- output: the last cycle's acceleration --------------------------------
+// solution_a as compute_a leaves it (exDyna3D.cpp:642-644) in the last cycle
+// -- assembled element forces, gravity, the acceleration boundary conditions,
+// times the inverse mass -- which output_results writes (:231).  The node
+// pass does not store it; this pass evaluates it again from the element
+// forces that the last force pass left in fe, with the node pass's
+// arithmetic in the node pass's order (the grouped layout adds all 8 slots,
+// empty ones as the zeros they hold).  Writes interleaved xyz per node.
+__global__ void __launch_bounds__(kNodeThreads) k_acceleration(ElemArrays E, NodeArrays N, Material M, const Ctl* ctl,
+                                                               double* a_out) {
+    const double amp = (M.gravity_on && M.amp_n > 0) ? gravity_amplitude(M.amp, M.amp_n, ctl->time, ctl->dt_i) : 1.0;
+    const NodeView nv = node_view(E, N, M, nullptr);
+    for (int64_t n = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; n < N.nn;
+         n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        double f[3];
+        if (E.slot_major) {
+            double g[3][1];
+            node_forces<1>(nv, n, g);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) f[c] = g[c][0];
+        } else {
+            listed_forces(E, N, n, f);
+        }
+        const double im = N.inv_mass[n];
+        const uint32_t code = N.bc[n];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double a = f[c];
+            if (M.gravity_on) a = a + amp * M.gravity_value * M.gravity_dir[c] / im;
+            const uint32_t cc = (code >> (2 * c)) & 3u;
+            if (cc & 2u) a = 0.0;
+            if ((cc & 1u) && a != 0.0) a = 0.0;
+            a_out[3 * n + c] = a * im;
+        }
     }
 }
 
@@ -1072,7 +1038,7 @@ struct RunFp64 {
     __device__ static void element(const ElemArrays& E, const NodeArrays& N, const Material& M, unsigned char* tile,
                                    double dt1, int64_t e, int lane, double& dts, double& len, double& e_int,
                                    double& e_hg, double& e_vis, int32_t& bad) {
-        element_body<PLASTIC, false, true, true, ENSC_F64_PREFETCH>(E, N, M, fp64_src_tile<L>(tile, lane),
+        element_body<PLASTIC, false, true, true, true, ENSC_F64_PREFETCH>(E, N, M, fp64_src_tile<L>(tile, lane),
                                                                     fp64_out_tile<L>(tile, lane), dt1, e, dts, len,
                                                                     e_int, e_hg, e_vis, bad);
     }
@@ -1084,7 +1050,14 @@ struct RunFp64 {
         NodeRowsF64<W> rows;
         double f[3][W];
         __device__ void load(const ElemArrays& E, const NodeArrays& N, const Material& M, int64_t t0) {
-            if (E.slot_major && t0 * W < N.nn) node_rows_load<W>(node_view(E, N, M, nullptr), t0 * W, rows);
+            if (E.slot_major && t0 * W < N.nn) {
+                node_rows_load<W>(node_view(E, N, M, nullptr), t0 * W, rows);
+                if (M.gravity_on) reciprocals();
+            }
+        }
+        __device__ void reciprocals() {
+#pragma unroll
+            for (int j = 0; j < W; ++j) rows.rim[j] = 1.0 / rows.im[j];
         }
         __device__ void gather(const ElemArrays& E, const NodeArrays& N, const Material& M, int64_t t0) {
             if (E.slot_major && t0 * W < N.nn) node_forces<W>(node_view(E, N, M, nullptr), t0 * W, f);
@@ -1098,6 +1071,7 @@ struct RunFp64 {
                 if (W > 1)
                     for (int64_t g = t0 + stride; g * W < N.nn; g += stride) {
                         node_rows_load<W>(nv, g * W, rows);
+                        if (M.gravity_on) reciprocals();
                         node_forces<W>(nv, g * W, f);
                         node_group<W, true>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad, &rows, f);
                     }
@@ -1108,10 +1082,9 @@ struct RunFp64 {
         }
     };
     __device__ static double kinetic(const NodeArrays& N, int64_t n) {
-        const double* V = static_cast<const double*>(N.v);
         double kin = 0.0;
         for (int c = 0; c < 3; ++c) {
-            const double v = V[c * N.nn_pad + n];
+            const double v = *node_v64(N, c, n);
             kin = kin + 0.5 * (v * v) / N.inv_mass[n];
         }
         return kin;
@@ -1249,11 +1222,11 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB) k_elem
             const double dt1 = h.dt1;
             double d1, l1;
             if (E.bt9)
-                element_body<true, false, true, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile9>(st, lane),
+                element_body<true, false, true, true, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile9>(st, lane),
                                                                          fp64_out_global<true>(E, e), dt1, e, d1, l1, ei, eh,
                                                                          ev, bad);
             else
-                element_body<true, false, false, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile24>(st, lane),
+                element_body<true, false, false, true, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile24>(st, lane),
                                                                           fp64_out_global<true>(E, e), dt1, e, d1, l1, ei, eh,
                                                                           ev, bad);
             dts = d1 < dts ? d1 : dts;

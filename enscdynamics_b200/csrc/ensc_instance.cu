@@ -75,15 +75,6 @@ void element_constants(int64_t nn, int64_t ne, const uint32_t* conn, const doubl
     for (int64_t i = 0; i < 3 * nn; ++i) inv_mass[i] = 1.0 / mass[i];
 }
 
-// Converts an AoS host array [n][comps] into SoA [comps][pad] of type T.
-template <typename T>
-std::vector<T> to_soa(const double* aos, int64_t n, int64_t pad, int comps) {
-    std::vector<T> out(static_cast<size_t>(comps * pad), T(0));
-    for (int64_t i = 0; i < n; ++i)
-        for (int c = 0; c < comps; ++c) out[c * pad + i] = static_cast<T>(aos[i * comps + c]);
-    return out;
-}
-
 // B0^T row a of an element from J^-1 / 8 (p, row-major): dN/dxi is +-1/8 of the
 // corner signs, so every product above is exact, and the sums are formed in the
 // same order.
@@ -147,17 +138,30 @@ void form_device_rows(InstanceHost& h, const uint32_t* conn) {
     std::vector<double>().swap(h.bt);  // the device form replaces them
     std::vector<double>().swap(h.jinv);
     std::vector<double>().swap(h.vol0);
-    h.x_rows = to_soa<double>(h.x0, h.nn, np, 3);
-    if (h.v0) {
-        if (h.mixed) {
-            h.v_rows_f = to_soa<float>(h.v0, h.nn, np, 3);
-#if ENSC_MIXED_VLO
-            h.v_lo_rows.assign(static_cast<size_t>(3 * np), 0);
-            for (int64_t n = 0; n < h.nn; ++n)
-                for (int c = 0; c < 3; ++c) v_split(h.v0[3 * n + c], h.v_rows_f[c * np + n], h.v_lo_rows[c * np + n]);
-#endif
-        } else {
-            h.v_rows_d = to_soa<double>(h.v0, h.nn, np, 3);
+    h.q0.assign(static_cast<size_t>(4 * np), 0.0);
+    for (int64_t n = 0; n < h.nn; ++n)
+        for (int c = 0; c < 3; ++c) h.q0[4 * n + c] = h.x0[3 * n + c];
+    if (h.mixed) {
+        h.x_rows.assign(static_cast<size_t>(3 * np), 0.0);
+        for (int64_t n = 0; n < h.nn; ++n)
+            for (int c = 0; c < 3; ++c) h.x_rows[c * np + n] = h.x0[3 * n + c];
+        if (h.v0) {
+            h.vz_f.assign(static_cast<size_t>(np), 0.f);
+            h.v_lo.assign(static_cast<size_t>(3 * np), 0);
+            for (int64_t n = 0; n < h.nn; ++n) {
+                float hi[3];
+                for (int c = 0; c < 3; ++c) v_split(h.v0[3 * n + c], hi[c], h.v_lo[c * np + n]);
+                std::memcpy(&h.q0[4 * n + 3], hi, 2 * sizeof(float));
+                h.vz_f[n] = hi[2];
+            }
+        }
+    } else if (h.v0) {
+        h.q1.assign(static_cast<size_t>(4 * np), 0.0);
+        h.vz_d.assign(static_cast<size_t>(np), 0.0);
+        for (int64_t n = 0; n < h.nn; ++n) {
+            h.q1[4 * n + 2] = h.v0[3 * n];
+            h.q1[4 * n + 3] = h.v0[3 * n + 1];
+            h.vz_d[n] = h.v0[3 * n + 2];
         }
     }
     h.x0 = nullptr;
@@ -368,23 +372,8 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
 
     h.im.assign(static_cast<size_t>(np), 1.0);
     for (int64_t n = 0; n < nn; ++n) h.im[n] = inv_mass_dof[3 * n];
-    // node-to-element tables
-    h.ell.assign(static_cast<size_t>(8 * np), ENSC_NONE);
-    if (!h.clash) {
-        for (int k = 0; k < 8; ++k)
-            for (int64_t e = 0; e < ne; ++e) h.ell[k * np + conn[8 * e + k]] = static_cast<uint32_t>(e);
-        h.slot_mask.assign(static_cast<size_t>(np), 0);
-        for (int k = 0; k < 8; ++k)
-            for (int64_t n = 0; n < nn; ++n)
-                if (h.ell[k * np + n] != ENSC_NONE) h.slot_mask[n] |= static_cast<uint8_t>(1u << k);
-    } else {
-        // ell keeps the first element per (slot, node) as before; the lists
-        // carry all of them
-        for (int k = 0; k < 8; ++k)
-            for (int64_t e = 0; e < ne; ++e) {
-                uint32_t& slot = h.ell[k * np + conn[8 * e + k]];
-                if (slot == ENSC_NONE) slot = static_cast<uint32_t>(e);
-            }
+    // meshes whose nodes repeat slots: the lists of the node pass
+    if (h.clash) {
         h.csr_ptr.assign(static_cast<size_t>(nn + 1), 0);
         for (int64_t i = 0; i < 8 * ne; ++i) h.csr_ptr[conn[i] + 1] += 1;
         for (int64_t n = 0; n < nn; ++n) h.csr_ptr[n + 1] += h.csr_ptr[n];
@@ -406,18 +395,16 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
     h.const_bytes = mixed ? MixedTile::kState : (h.bt9 ? Fp64Tile9::kState : Fp64Tile24::kState);
     h.size[P::TILES] = static_cast<size_t>(ep / 32) * h.tile_bytes;
     h.size[P::FE] = 24 * fe_rows * real;
-    h.size[P::X] = 3 * N8 * 8;
-    h.size[P::U] = 3 * N8 * 8;
-    // mixed: float rows, then the 16-bit velocity residual rows (v_lo_rows)
-    h.size[P::V] = 3 * N8 * real + ((mixed && ENSC_MIXED_VLO) ? 3 * N8 * sizeof(int16_t) : 0);
+    h.size[P::X] = 4 * N8 * 8;
+    h.size[P::U] = (mixed ? 3 : 4) * N8 * 8;
+    // vz; mixed: then the 16-bit velocity residual rows (v_lo_rows)
+    h.size[P::V] = N8 * real + (mixed ? 3 * N8 * sizeof(int16_t) : 0);
     h.size[P::IM] = N8 * 8;
     h.size[P::BC] = N8;
     h.size[P::BCV] = 3 * N8 * 8;
-    h.size[P::ELL] = 8 * N8 * sizeof(uint32_t);
     h.size[P::RF] = 3 * N8 * 8;
     h.size[P::CPTR] = h.clash ? static_cast<size_t>(nn + 1) * sizeof(int64_t) : 0;
     h.size[P::CENT] = h.clash ? static_cast<size_t>(8 * ne) * sizeof(uint32_t) : 0;
-    h.size[P::MASK] = h.clash ? 0 : N8;
     if (h.patch) {
         h.size[P::IPERM] = static_cast<size_t>(ne) * sizeof(int32_t);
         h.size[P::PFOFF] = static_cast<size_t>(h.n_patches + 1) * sizeof(uint32_t);
@@ -448,23 +435,15 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
         e = cudaMemcpy2DAsync(b + h.off[P::TILES], h.tile_bytes, h.tiles.data(), h.const_bytes, h.const_bytes,
                               static_cast<size_t>(ep / 32), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = put(block, h.off[P::IM], h.im, st);
-    if (e == cudaSuccess) e = put(block, h.off[P::X], h.x_rows, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::X], h.q0, st);
     // mixed: the u rows hold the reference position x - u, x0 at the start
-    if (h.mixed && ENSC_MIXED_UREF && e == cudaSuccess) e = put(block, h.off[P::U], h.x_rows, st);
-    if (h.mixed) {
-        if (e == cudaSuccess) e = put(block, h.off[P::V], h.v_rows_f, st);
-#if ENSC_MIXED_VLO
-        if (e == cudaSuccess) e = put(block, h.off[P::V] + 3 * np * sizeof(float), h.v_lo_rows, st);
-#endif
-    } else {
-        if (e == cudaSuccess) e = put(block, h.off[P::V], h.v_rows_d, st);
-    }
-    if (e == cudaSuccess) e = put(block, h.off[P::ELL], h.ell, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::U], h.mixed ? h.x_rows : h.q1, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::V], h.vz_d, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::V], h.vz_f, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::V] + np * sizeof(float), h.v_lo, st);
     if (h.clash) {
         if (e == cudaSuccess) e = put(block, h.off[P::CPTR], h.csr_ptr, st);
         if (e == cudaSuccess) e = put(block, h.off[P::CENT], h.csr_ent, st);
-    } else {
-        if (e == cudaSuccess) e = put(block, h.off[P::MASK], h.slot_mask, st);
     }
     std::vector<uint32_t> nptr_pad;
     if (h.patch) {
@@ -525,11 +504,10 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     N.inv_mass = reinterpret_cast<double*>(b + h.off[P::IM]);
     N.bc = reinterpret_cast<uint8_t*>(b + h.off[P::BC]);
     N.bcv = reinterpret_cast<double*>(b + h.off[P::BCV]);
-    N.ell = reinterpret_cast<uint32_t*>(b + h.off[P::ELL]);
+    N.rec = 1;
     N.csr_ptr = h.clash ? reinterpret_cast<int64_t*>(b + h.off[P::CPTR]) : nullptr;
     N.csr_ent = h.clash ? reinterpret_cast<uint32_t*>(b + h.off[P::CENT]) : nullptr;
     N.rf = reinterpret_cast<double*>(b + h.off[P::RF]);
-    N.slot_mask = h.clash ? nullptr : reinterpret_cast<uint8_t*>(b + h.off[P::MASK]);
     return ENSC_OK;
 }
 

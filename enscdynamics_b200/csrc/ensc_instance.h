@@ -23,8 +23,6 @@ struct InstanceHost {
     std::vector<double> jinv;         // [ne][9] J^-1 / 8 where bt9
     std::vector<double> vol0;         // [ne] V0
     std::vector<double> im;           // [nn_pad] inverse lumped mass per node
-    std::vector<uint32_t> ell;        // [8][nn_pad] element in slot k, or ENSC_NONE
-    std::vector<uint8_t> slot_mask;   // [nn_pad] occupied slots (clash-free meshes)
     std::vector<int64_t> csr_ptr;     // clash meshes: (slot, element)-sorted lists
     std::vector<uint32_t> csr_ent;
     const double* x0 = nullptr;       // caller arrays, read by instance_prepare only
@@ -32,15 +30,16 @@ struct InstanceHost {
     // what the upload copies as it is, formed by instance_prepare (so that a
     // prepared instance's host work is done before its device part): the
     // constant part of every element tile (connectivity, geometry, V0 and its
-    // roots), const_bytes each; x0 [3][nn_pad]; mixed: v float rows [3][nn_pad] and
-    // their 16-bit residual rows [3][nn_pad]; FP64: v [3][nn_pad] (v rows empty
-    // when the mesh has no initial velocities)
+    // roots), const_bytes each; the node records (NodeArrays) -- FP64: q0, q1 and
+    // vz; mixed: q0 with two velocities packed in, vz and the 16-bit residual rows
+    // [3][nn_pad], and the reference position rows x0 [3][nn_pad] (what only holds
+    // velocities stays empty when the mesh has none)
     int32_t tile_bytes = 0, const_bytes = 0;
     bool bt9 = false;                 // FP64: 9 numbers per element give B0^T bit for bit
     std::vector<unsigned char> tiles;
-    std::vector<float> v_rows_f;
-    std::vector<int16_t> v_lo_rows;
-    std::vector<double> x_rows, v_rows_d;
+    std::vector<double> q0, q1, vz_d, x_rows;
+    std::vector<float> vz_f;
+    std::vector<int16_t> v_lo;
     // patch assembly (ElemArrays::patch): the stored order of the elements
     // and the patch tables; all element arrays above are in stored order
     bool patch = false;
@@ -53,7 +52,7 @@ struct InstanceHost {
     int64_t n_patches = 0, n_pnodes = 0;
     // device layout: byte offsets of the pieces in one 256-byte-aligned block
     enum Piece {
-        TILES, FE, X, U, V, IM, BC, BCV, ELL, RF, CPTR, CENT, MASK,
+        TILES, FE, X, U, V, IM, BC, BCV, RF, CPTR, CENT,
         IPERM, PFOFF, PINCOFF, PINC, PF, NPTR, NENT, NPIECE
     };
     size_t off[NPIECE] = {};

@@ -31,28 +31,6 @@ constexpr int kElemThreads = 128;
 #ifndef ENSC_MIXED_REREAD
 #define ENSC_MIXED_REREAD 1
 #endif
-// The single-instance staged mixed element pass prefetches an element's node
-// rows into L1 before its coordinate phase: bit 0 the velocities, bit 1 the
-// coordinate components 1 and 2
-#ifndef ENSC_MIXED_PREFETCH
-#define ENSC_MIXED_PREFETCH 3
-#endif
-// The same for the batched mixed element pass, off: with the instance's
-// arrays in registers the prefetch addresses spill (measured on B200: the
-// velocity rows there spill 216 B per thread and cost 6%; with the
-// addresses formed inside the prefetch instruction the spill is 36 B and the
-// cost 4-6% on the block and on a 64-instance sweep)
-#ifndef ENSC_BATCH_MIXED_PREFETCH
-#define ENSC_BATCH_MIXED_PREFETCH 0
-#endif
-// 1: the grouped node passes sum all 8 force slots (empty ones hold zeros)
-// instead of reading the slot mask first (measured on B200, mixed: reading
-// the mask made the node pass 22% slower on the block and the batched
-// 64-instance sweep of plates and cantilevers, whose many boundary nodes have
-// empty slots, 5% slower)
-#ifndef ENSC_NODE_ALL_SLOTS
-#define ENSC_NODE_ALL_SLOTS 1
-#endif
 #ifndef ENSC_NODE_BATCH_MINB_MIXED
 #define ENSC_NODE_BATCH_MINB_MIXED 2
 #endif
@@ -64,11 +42,10 @@ constexpr int kElemThreads = 128;
 #ifndef ENSC_F64_PIPE_MINB
 #define ENSC_F64_PIPE_MINB 2
 #endif
-// The FP64 warp-pipelined element pass prefetches an element's node rows
-// into L1 once its connectivity is staged: bit 0 the velocities, bit 1 the
-// displacements
+// 1: the FP64 element passes prefetch an element's second node records and vz
+// into L1 once its connectivity is staged
 #ifndef ENSC_F64_PREFETCH
-#define ENSC_F64_PREFETCH 3
+#define ENSC_F64_PREFETCH 1
 #endif
 constexpr int kNodeThreads = 256;
 constexpr int kCtlThreads = 256;
@@ -127,7 +104,10 @@ int occupancy_element_fp64(bool plastic, bool bt9);
 #ifndef ENSC_NODE_MINB_FP64
 #define ENSC_NODE_MINB_FP64 4
 #endif
-constexpr int kNodeGroupFp64 = 2;
+#ifndef ENSC_NODE_GROUP_FP64
+#define ENSC_NODE_GROUP_FP64 1
+#endif
+constexpr int kNodeGroupFp64 = ENSC_NODE_GROUP_FP64;
 constexpr int kNodeGroupMixed = ENSC_NODE_GROUP_MIXED;
 // nodes per thread of the batched mixed node pass (with the nodes' rows
 // loaded first, 4 spill there; 2 were 1% faster on the block as a batch and
@@ -183,23 +163,22 @@ void launch_arm(Ctl* ctl, double step_end, long long max_cycles, cudaStream_t st
 void launch_apply_bc_v(const NodeArrays& N, bool fp32_v, cudaStream_t st);
 void launch_reset_init(Ctl* ctl, cudaStream_t st);
 void launch_kinetic0(const NodeArrays& N, const Partials& P, Ctl* ctl, bool fp32_v, int grid, cudaStream_t st);
-// layout conversion between caller AoS arrays and node rows, or the element
-// rows at `rows` of E.  `at` (may be null): entry e of the interleaved array is
-// row position at[e] -- an element's stored position under the patch order
-void launch_soa_to_aos(const double* soa, int64_t n, int64_t pad, int comps, double* aos, cudaStream_t st);
-void launch_aos_to_soa(const double* aos, int64_t n, int64_t pad, int comps, double* soa, cudaStream_t st);
+// Layout conversion between interleaved caller arrays and the device layout:
+// node fields, reactions, and the element rows at `rows` of E.  `at` (may be null):
+// entry e of the interleaved array is row position at[e] -- an element's stored
+// position under the patch order.  A mixed instance's u rows hold x - u: its
+// displacement is formed on the way out; on the way in the rows take u, between
+// two calls of launch_reflect_rows (a <- x - a over the u rows).
+enum class NodeField { X, U, V };
+void launch_nodes_to_aos(const NodeArrays& N, NodeField field, bool mixed_precision, double* aos, cudaStream_t st);
+void launch_aos_to_nodes(const double* aos, const NodeArrays& N, NodeField field, bool mixed_precision,
+                         cudaStream_t st);
+void launch_reactions_to_aos(const NodeArrays& N, double* aos, cudaStream_t st);
+void launch_reflect_rows(const NodeArrays& N, cudaStream_t st);
 void launch_elem_to_aos(const ElemArrays& E, const void* rows, int comps, bool src_fp32, double* aos, cudaStream_t st,
                         const int32_t* at = nullptr);
 void launch_aos_to_elem(const double* aos, const ElemArrays& E, int comps, void* rows, bool dst_fp32, cudaStream_t st,
                         const int32_t* at = nullptr);
-// displacements of a mixed instance (u rows holding xr = x - u) to
-// interleaved xyz doubles; and a <- x - a over three node rows
-void launch_disp_to_aos(const double* x, const double* xr, int64_t n, int64_t pad, double* aos, cudaStream_t st);
-void launch_reflect_rows(const double* x, double* a, int64_t n, int64_t pad, cudaStream_t st);
-// velocities (FP64 rows, or the mixed stepper's float rows and residual rows)
-// to and from interleaved xyz doubles
-void launch_v_to_aos(const NodeArrays& N, bool fp32_v, double* aos, cudaStream_t st);
-void launch_aos_to_v(const double* aos, const NodeArrays& N, bool fp32_v, cudaStream_t st);
 
 // thread-local message returned by ensc_last_error(NULL) (ensc_capi.cu)
 void set_thread_error(const std::string& msg);

@@ -12,8 +12,9 @@
 // one-point B0 rows are A s_j / 8, s_j the node's reference-corner signs) as a
 // float pair, 9 hi then 9 lo rows; cbrt_v0, sigma, qia, eps_p and fe are float;
 // vol0 is double.
-// Node arrays: x double; the u rows hold the reference position x - u
-// (double, ENSC_MIXED_UREF); v float with 16-bit residual rows.
+// Node arrays: records of x (double) and two velocity components (float), the
+// third as a row, with 16-bit residual rows; the u rows hold the reference
+// position x - u (double).
 #include "ensc_device.cuh"
 #include "ensc_kernels.h"
 #include "ensc_run.cuh"
@@ -193,11 +194,9 @@ __device__ __forceinline__ void corner_values(T (&c)[8], T (&a)[8]) {
 // Inputs come from S, the evolving rows go to O and the forces to the
 // instance's force array at element e.  Node rows are read with plain loads:
 // a resident run rewrites them between its cycles.
-// PF: node rows prefetched into L1 at the start (bit 0 velocities, bit 1
-// coordinate components 1 and 2).
 // FOUT: the 24 nodal forces go to fout[3 * 8] (component-major) instead of
 // the instance's force array, for the patch assembly.
-template <bool PLASTIC, bool INIT, bool SMEM = false, int PF = 0, bool FOUT = false>
+template <bool PLASTIC, bool INIT, bool SMEM = false, bool FOUT = false>
 __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const NodeArrays& N, const Material& M,
                                                    const MixedSrc& S, const MixedOut& O, const float dt1,
                                                    const double dt1d, const int64_t e, double& dts, double& len,
@@ -228,19 +227,13 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
     uint32_t nk[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) nk[k] = ldin<SMEM>(S.conn + k * ss + si);
-    // start the node rows the body reads later on their way into L1
-    if (PF & 1) {
+    // the node records, and vz
+    double q[8][4];
+    float vz[8];
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+    for (int k = 0; k < 8; ++k) ld_rec(X + 4 * static_cast<int64_t>(nk[k]), q[k]);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) prefetch_l1(V + r * np + nk[k]);
-    }
-    if (PF & 2) {
-#pragma unroll
-        for (int r = 1; r < 3; ++r)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) prefetch_l1(X + r * np + nk[k]);
-    }
+    for (int k = 0; k < 8; ++k) vz[k] = V[nk[k]];
     // coordinates relative to node 0, as FP64 differences, one component at a
     // time: hourglass projections TAU x = TAU (x - x0) (the Gamma rows sum to
     // zero) rounded to FP32; the minimum edge and F = sum_j (x_j - x_0) B0_j
@@ -257,16 +250,15 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
         double Gx[3][3];
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            const double* Xr = X + r * np;
-            const double xo = Xr[nk[0]];
+            const double xo = q[0][r];
             double xd[8];
             xd[0] = 0.0;
 #pragma unroll
-            for (int k = 1; k < 8; ++k) xd[k] = Xr[nk[k]] - xo;
+            for (int k = 1; k < 8; ++k) xd[k] = q[k][r] - xo;
 #pragma unroll
-            for (int q = 0; q < 12; ++q) {
-                const double d = xd[A1[q]] - xd[A0[q]];
-                e2[q] = r == 0 ? d * d : fma(d, d, e2[q]);
+            for (int i = 0; i < 12; ++i) {
+                const double d = xd[A1[i]] - xd[A0[i]];
+                e2[i] = r == 0 ? d * d : fma(d, d, e2[i]);
             }
             double c[8];
             corner_coeffs(xd, c);
@@ -290,7 +282,7 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
             }
         double m = DBL_MAX;
 #pragma unroll
-        for (int q = 0; q < 12; ++q) m = fmin(m, e2[q]);
+        for (int i = 0; i < 12; ++i) m = fmin(m, e2[i]);
         len = sqrt(m);
     }
     const float J = det3f(F);
@@ -311,7 +303,7 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
         for (int r = 0; r < 3; ++r) {
             float a[8], c[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) a[j] = V[r * np + nk[j]];
+            for (int j = 0; j < 8; ++j) a[j] = r == 0 ? rec_vx(q[j][3]) : r == 1 ? rec_vy(q[j][3]) : vz[j];
             corner_coeffs(a, c);
             Gv[r][0] = c[1];
             Gv[r][1] = c[2];
@@ -418,9 +410,9 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
-            const float q = fmaf(DR, HIA[i][kk], S.qia[(4 * i + kk) * ss + si]);
-            if (!INIT) O.qia[(4 * i + kk) * os + oi] = q;
-            Gq[i][kk] = fmaf(CR, HIA[i][kk], q);
+            const float h = fmaf(DR, HIA[i][kk], S.qia[(4 * i + kk) * ss + si]);
+            if (!INIT) O.qia[(4 * i + kk) * os + oi] = h;
+            Gq[i][kk] = fmaf(CR, HIA[i][kk], h);
         }
     const bool visc = !(fabsf(vr) < 1.0e-10f);
     float pv = 0.f;
@@ -485,17 +477,25 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
     // per force component: the node values of -(B0_j Z) - Gamma_j Gq^T from
     // their corner coefficients (-Y on xi, eta, zeta; -Gq on the hourglass
     // vectors, signed as Gamma)
+    float fx[8];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         float c[8] = {0.f,          -Y[0][i],     -Y[1][i],     -Gq[i][0],
                       -Y[2][i],     Gq[i][2],     Gq[i][1],     -Gq[i][3]};
         float f[8];
         corner_values(c, f);
+        if (FOUT) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) fout[8 * i + j] = f[j];
+            continue;
+        }
+        const int64_t row = E.slot_major ? np : ep;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            if (FOUT) fout[8 * i + j] = f[j];
-            else if (E.slot_major) fe[(3 * j + i) * np + nk[j]] = f[j];
-            else fe[(3 * j + i) * ep + e] = f[j];
+            const int64_t at = E.slot_major ? static_cast<int64_t>(nk[j]) : e;
+            if (i == 0) fx[j] = f[j];
+            else if (i == 1) *reinterpret_cast<float2*>(force_xy(fe, row, j, at)) = make_float2(fx[j], f[j]);
+            else *force_z(fe, row, j, at) = f[j];
         }
     }
     // element dt (compute_dtStable, exDyna3D.cpp:828-834), with the
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
         const int64_t e = t * 32 + lane;
         if (e < E.ne) {
             double dts, len;
-            element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(
+            element_body_mixed<PLASTIC, false, true>(
                 E, N, M, mixed_src_tile(wst + s * SB, lane), mixed_out_tile(mixed_tile(E, t), lane), dt1, dt1d, e, dts,
                 len, e_int, e_hg, e_vis, bad);
             dts_min = fmin(dts_min, dts);
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(kPatchElems, 8)
         float fo[24];
         if (live) {
             double dts, len;
-            element_body_mixed<PLASTIC, INIT, true, ENSC_MIXED_PREFETCH, true>(
+            element_body_mixed<PLASTIC, INIT, true, true>(
                 E, N, M, mixed_src_tile(st + wid * MixedTile::kBytes, lane),
                 mixed_out_tile(mixed_tile(E, t * kPatchTiles + wid), lane), dt1, dt1d, e, dts, len, e_int, e_hg, e_vis, bad,
                 fo);
@@ -744,18 +744,6 @@ __device__ __forceinline__ void patch_gather(const PatchArrays& PA, int64_t n, f
     }
 }
 
-#if !ENSC_MIXED_VLO
-// v + (dt_i + dt_i_1) / 2 * f * M^-1 in FP32 with the half step and the
-// inverse mass as float pairs: both are the same for many nodes and cycles,
-// so their FP32 rounding would scale all accelerations alike.
-__device__ __forceinline__ float velocity_update(float vo, float f, double im, float hdt, float hdt_lo) {
-    const float im_hi = static_cast<float>(im);
-    const float im_lo = static_cast<float>(im - static_cast<double>(im_hi));
-    const float acc = fmaf(f, im_hi, f * im_lo);
-    return fmaf(hdt, acc, fmaf(hdt_lo, acc, vo));
-}
-#endif
-
 // The velocity update in FP64 on the split velocity (hi float + 16-bit
 // residual, v_join / v_split): v + (dt_i + dt_i_1) / 2 * a with the FP32
 // acceleration a = f M^-1 (inverse mass as a float pair); returns the new
@@ -770,47 +758,34 @@ __device__ __forceinline__ double velocity_update_split(double vo, float f, doub
     return vn;
 }
 
-// One node of the mixed node pass; shared by the single-instance, batched and
-// resident-run kernels (KIN: sum the kinetic energy).
+// The force of one node from per-element forces, through the general lists
+// (meshes whose nodes repeat slots).
+__device__ __forceinline__ void listed_forces_mixed(const ElemArrays& E, const NodeArrays& N, const int64_t n,
+                                                    float (&f)[3]) {
+    const float* fe = static_cast<const float*>(E.fe);
+    f[0] = f[1] = f[2] = 0.f;
+    for (int64_t i = N.csr_ptr[n]; i < N.csr_ptr[n + 1]; ++i) {
+        const uint32_t ent = N.csr_ent[i];
+        const int k = static_cast<int>(ent & 7u);
+        const uint32_t el = ent >> 3;
+        const float2 xy = *reinterpret_cast<const float2*>(force_xy(fe, E.ne_pad, k, el));
+        f[0] += xy.x;
+        f[1] += xy.y;
+        f[2] += *force_z(fe, E.ne_pad, k, el);
+    }
+}
+
+// One node of the mixed node pass where the forces are per element; shared by
+// the single-instance, batched and resident-run kernels (KIN: sum the kinetic
+// energy).
 template <bool KIN = true>
 __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeArrays& N, const Material& M,
                                                 const double dt_i, const double dt_i_1, const double amp, const int64_t n,
                                                 double& kin, double& wext, int32_t& bad) {
-    const int64_t np = N.nn_pad, ep = E.ne_pad;
-    const float* fe = static_cast<const float*>(E.fe);
-    float* V = static_cast<float*>(N.v);
-    [[maybe_unused]] const float hdt = static_cast<float>(0.5 * (dt_i + dt_i_1));
-    [[maybe_unused]] const float hdt_lo = static_cast<float>(0.5 * (dt_i + dt_i_1) - static_cast<double>(hdt));
+    const int64_t np = N.nn_pad;
     const double dt_avg = 0.5 * (dt_i + dt_i_1);
-
-    float f[3] = {0.f, 0.f, 0.f};
-    if (E.slot_major) {
-        const uint32_t msk = N.slot_mask[n];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if ((msk >> k) & 1u) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) f[c] += fe[(3 * k + c) * np + n];
-            }
-        }
-    } else if (N.csr_ptr == nullptr) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t el = __ldg(N.ell + k * np + n);
-            if (el != ENSC_NONE) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) f[c] += fe[(3 * k + c) * ep + el];
-            }
-        }
-    } else {
-        for (int64_t i = N.csr_ptr[n]; i < N.csr_ptr[n + 1]; ++i) {
-            const uint32_t ent = N.csr_ent[i];
-            const int k = static_cast<int>(ent & 7u);
-            const uint32_t el = ent >> 3;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) f[c] += fe[(3 * k + c) * ep + el];
-        }
-    }
+    float f[3];
+    listed_forces_mixed(E, N, n, f);
     const double im = N.inv_mass[n];
     const uint32_t code = N.bc[n];
 #pragma unroll
@@ -833,56 +808,45 @@ __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeA
             a = 0.f;
         }
         if (cc) N.rf[c * np + n] = static_cast<double>(rf);
-#if ENSC_MIXED_VLO
-        int16_t* VL = v_lo_rows(N.v, np);
-        const double vod = v_join(V[c * np + n], VL[c * np + n]);
+        float* pv = node_vf(N, c, n);
+        int16_t* pl = v_lo_rows(N.v, np) + c * np + n;
+        double* px = node_x(N, c, n);
+        const double vod = v_join(*pv, *pl);
         float vn;
         int16_t vl;
         const double vnd = velocity_update_split(vod, a, im, dt_avg, vn, vl);
-        V[c * np + n] = vn;
-        VL[c * np + n] = vl;
-#else
-        const float vo = V[c * np + n];
-        const float vn = velocity_update(vo, a, im, hdt, hdt_lo);
-        V[c * np + n] = vn;
-        const double vnd = static_cast<double>(vn);
-        const double vod = static_cast<double>(vo);
-#endif
-        if (!ENSC_MIXED_UREF) N.u[c * np + n] += dt_i * vnd;
-        N.x[c * np + n] += dt_i * vnd;
+        *pv = vn;
+        *pl = vl;
+        *px += dt_i * vnd;
         wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
         if (KIN) kin += 0.5 * (vnd * vnd) / im;
         if (!isfinite(vnd)) bad |= ST_NONFINITE;
     }
 }
 
-// W consecutive nodes of the mixed node pass with 16-byte row accesses
-// (float4 force slots and velocities, pairs of doubles for x and the
-// inverse mass); per node the arithmetic of node_body_mixed.  Slots the mask
-// marks empty are skipped, or (ENSC_NODE_ALL_SLOTS) summed as the zeros they
-// hold: the slot-major rows start zeroed and only the slot's element writes
-// them.  Nodes at or past nn (row padding) are loaded and stored back
-// unchanged.
+// W consecutive nodes of the mixed node pass; per node the arithmetic of
+// node_body_mixed.  Every slot is added, empty ones as the zeros they hold: the
+// slot-major rows start zeroed and only the slot's element writes them.  Nodes
+// at or past nn (row padding) are loaded and stored back unchanged.
 //
-// pre (resident runs): the nodes' own rows, loaded while the grid still works
+// pre (resident runs): the nodes' own records, loaded while the grid still works
 // on the forces; such a run sums its kinetic energy once, at its end.
 template <int W>
 struct NodeRowsMixed {
-    double im[W], x[3][W];
-    float v[3][W];
+    double im[W], q[W][4];
+    float vz[W];
     int16_t lo[3][W];
     uint32_t code;
 };
 template <int W>
 __device__ __forceinline__ void node_rows_load(const NodeView& N, const int64_t n0, NodeRowsMixed<W>& r) {
+#pragma unroll
+    for (int j = 0; j < W; ++j) ld_rec(N.x + 4 * (n0 + j), r.q[j]);
+    ld_row<W>(static_cast<const float*>(N.v) + n0, r.vz);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) ld_row<W>(v_lo_rows(N.v, N.np) + c * N.np + n0, r.lo[c]);
     ld_row<W>(N.inv_mass + n0, r.im);
     r.code = ld_bytes<W>(N.bc + n0);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        ld_row<W>(static_cast<const float*>(N.v) + c * N.np + n0, r.v[c]);
-        ld_row<W>(N.x + c * N.np + n0, r.x[c]);
-        ld_row<W>(v_lo_rows(N.v, N.np) + c * N.np + n0, r.lo[c]);
-    }
 }
 
 // The forces of W consecutive nodes: their slots in order, or their patch
@@ -913,21 +877,16 @@ __device__ __forceinline__ void node_forces_mixed(const NodeView& N, const int64
             }
         }
     } else {
-        const uint32_t msk = ENSC_NODE_ALL_SLOTS ? 0xffffffffu : ld_bytes<W>(N.slot_mask + n0);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            uint32_t sel = 0;
+            float xy[2 * W], z[W];
+            ld_row<2 * W>(force_xy(fe, np, k, n0), xy);
+            ld_row<W>(force_z(fe, np, k, n0), z);
 #pragma unroll
-            for (int j = 0; j < W; ++j) sel |= ((msk >> (8 * j + k)) & 1u) << j;
-            if (sel) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    float r[W];
-                    ld_row<W>(fe + (3 * k + c) * np + n0, r);
-#pragma unroll
-                    for (int j = 0; j < W; ++j)
-                        if ((sel >> j) & 1u) f[c][j] += r[j];
-                }
+            for (int j = 0; j < W; ++j) {
+                f[0][j] += xy[2 * j];
+                f[1][j] += xy[2 * j + 1];
+                f[2][j] += z[j];
             }
         }
     }
@@ -940,17 +899,12 @@ __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double
                                                  int32_t& bad, const NodeRowsMixed<W>* pre = nullptr,
                                                  const float (*fpre)[W] = nullptr) {
     const int64_t np = N.np, nn = N.nn;
-    float* V = static_cast<float*>(N.v);
-    [[maybe_unused]] const float hdt = static_cast<float>(0.5 * (dt_i + dt_i_1));
-    [[maybe_unused]] const float hdt_lo = static_cast<float>(0.5 * (dt_i + dt_i_1) - static_cast<double>(hdt));
     const double dt_avg = 0.5 * (dt_i + dt_i_1);
     // the nodes' own rows first, so that their loads are in flight with the
-    // force slots' (measured on B200: node pass 4% faster, bit-identical)
+    // force slots'
     NodeRowsMixed<W> own;
     if constexpr (PRE) own = *pre;
     else node_rows_load<W>(N, n0, own);
-    const double (&im)[W] = own.im;
-    const uint32_t code = own.code;
     float f[3][W];
     if constexpr (PRE) {
 #pragma unroll
@@ -961,36 +915,19 @@ __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double
         node_forces_mixed<W, PATCH>(N, n0, f);
     }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        float vo[W], vn[W];
-        double uo[W], xo[W], un[W], xn[W];
-#if ENSC_MIXED_VLO
-        int16_t* VL = v_lo_rows(N.v, np);
-        int16_t lo[W], ln[W];
-#endif
+    for (int j = 0; j < W; ++j) {
+        if (n0 + j >= nn) continue;
+        const double im = own.im[j];
+        float v[3] = {rec_vx(own.q[j][3]), rec_vy(own.q[j][3]), own.vz[j]};
 #pragma unroll
-        for (int j = 0; j < W; ++j) {
-            vo[j] = own.v[c][j];
-            xo[j] = own.x[c][j];
-            lo[j] = own.lo[c][j];
-        }
-        if (!ENSC_MIXED_UREF) ld_row<W>(N.u + c * np + n0, uo);
-#pragma unroll
-        for (int j = 0; j < W; ++j) {
-            vn[j] = vo[j];
-#if ENSC_MIXED_VLO
-            ln[j] = lo[j];
-#endif
-            if (!ENSC_MIXED_UREF) un[j] = uo[j];
-            xn[j] = xo[j];
-            if (n0 + j >= nn) continue;
+        for (int c = 0; c < 3; ++c) {
             float a = f[c][j];
             float g = 0.f;
             if (N.gravity_on) {
-                g = static_cast<float>(amp * N.gravity_value * N.gravity_dir[c] / im[j]);
+                g = static_cast<float>(amp * N.gravity_value * N.gravity_dir[c] / im);
                 a += g;
             }
-            const uint32_t cc = (code >> (8 * j + 2 * c)) & 3u;
+            const uint32_t cc = (own.code >> (8 * j + 2 * c)) & 3u;
             float r = 0.f, rf = 0.f;
             if (cc & 2u) {
                 r = -a;
@@ -1002,32 +939,26 @@ __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double
                 a = 0.f;
             }
             if (cc) N.rf[c * np + n0 + j] = static_cast<double>(rf);
-#if ENSC_MIXED_VLO
-            const double vod = v_join(vo[j], lo[j]);
-            const double vnd = velocity_update_split(vod, a, im[j], dt_avg, vn[j], ln[j]);
-#else
-            vn[j] = velocity_update(vo[j], a, im[j], hdt, hdt_lo);
-            const double vnd = static_cast<double>(vn[j]);
-            const double vod = static_cast<double>(vo[j]);
-#endif
-            if (!ENSC_MIXED_UREF) un[j] = uo[j] + dt_i * vnd;
-            xn[j] = xo[j] + dt_i * vnd;
+            const double vod = v_join(v[c], own.lo[c][j]);
+            const double vnd = velocity_update_split(vod, a, im, dt_avg, v[c], own.lo[c][j]);
+            own.q[j][c] = own.q[j][c] + dt_i * vnd;
             wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
-            if (!PRE) kin += 0.5 * (vnd * vnd) / im[j];
+            if (!PRE) kin += 0.5 * (vnd * vnd) / im;
             if (!isfinite(vnd)) bad |= ST_NONFINITE;
         }
-        st_row<W>(V + c * np + n0, vn);
-#if ENSC_MIXED_VLO
-        st_row<W>(VL + c * np + n0, ln);
-#endif
-        if (!ENSC_MIXED_UREF) st_row<W>(N.u + c * np + n0, un);
-        st_row<W>(N.x + c * np + n0, xn);
+        own.q[j][3] = rec_vxy(v[0], v[1]);
+        own.vz[j] = v[2];
     }
+#pragma unroll
+    for (int j = 0; j < W; ++j) st_rec(N.x + 4 * (n0 + j), own.q[j]);
+    st_row<W>(static_cast<float*>(N.v) + n0, own.vz);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) st_row<W>(v_lo_rows(N.v, np) + c * np + n0, own.lo[c]);
 }
 
 // Node pass in mixed precision: FP32 slot-ordered gather and acceleration,
 // FP32 velocity, FP64 position accumulation and energy (the u rows hold the
-// reference position x - u and are not touched: ENSC_MIXED_UREF).
+// reference position x - u and are not touched).
 // PATCH: the instance uses the patch assembly (one instantiation each, so
 // the slot-assembly pass carries no code of the other).
 template <bool PATCH>
@@ -1092,7 +1023,7 @@ struct RunMixed {
     __device__ static void element(const ElemArrays& E, const NodeArrays& N, const Material& M, unsigned char* tile,
                                    double dt1, int64_t e, int lane, double& dts, double& len, double& e_int,
                                    double& e_hg, double& e_vis, int32_t& bad) {
-        element_body_mixed<PLASTIC, false, true, ENSC_MIXED_PREFETCH>(E, N, M, mixed_src_tile(tile, lane),
+        element_body_mixed<PLASTIC, false, true>(E, N, M, mixed_src_tile(tile, lane),
                                                                       mixed_out_tile(tile, lane),
                                                                       static_cast<float>(dt1), dt1, e, dts, len, e_int,
                                                                       e_hg, e_vis, bad);
@@ -1130,8 +1061,7 @@ struct RunMixed {
     __device__ static double kinetic(const NodeArrays& N, int64_t n) {
         double kin = 0.0;
         for (int c = 0; c < 3; ++c) {
-            const int64_t i = c * N.nn_pad + n;
-            const double v = v_join(static_cast<const float*>(N.v)[i], v_lo_rows(N.v, N.nn_pad)[i]);
+            const double v = v_join(*node_vf(N, c, n), v_lo_rows(N.v, N.nn_pad)[c * N.nn_pad + n]);
             kin += 0.5 * (v * v) / N.inv_mass[n];
         }
         return kin;
@@ -1150,40 +1080,20 @@ __global__ void __launch_bounds__(CLUSTER ? 128 : 32 * kRunWarpsMixed, 1)
 // as doubles, interleaved xyz per node.
 __global__ void __launch_bounds__(kNodeThreads) k_acceleration_mixed(PatchArrays PA, ElemArrays E, NodeArrays N, Material M,
                                                                      const Ctl* ctl, double* a_out) {
-    const int64_t np = N.nn_pad, ep = E.ne_pad;
-    const float* __restrict__ fe = static_cast<const float*>(E.fe);
-    const bool grouped = E.slot_major && E.tile_bytes;
     const double amp = (M.gravity_on && M.amp_n > 0) ? gravity_amplitude(M.amp, M.amp_n, ctl->time, ctl->dt_i) : 1.0;
+    const NodeView nv = node_view(E, N, M, nullptr, &PA);
     for (int64_t n = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; n < N.nn;
          n += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         float f[3] = {0.f, 0.f, 0.f};
         if (PA.pf) {
             patch_gather(PA, n, f);
         } else if (E.slot_major) {
-            const uint32_t msk = grouped ? 0xffu : N.slot_mask[n];
+            float g[3][1];
+            node_forces_mixed<1, false>(nv, n, g);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if ((msk >> k) & 1u) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) f[c] += fe[(3 * k + c) * np + n];
-                }
-        } else if (N.csr_ptr == nullptr) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const uint32_t el = N.ell[k * np + n];
-                if (el != ENSC_NONE) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) f[c] += fe[(3 * k + c) * ep + el];
-                }
-            }
+            for (int c = 0; c < 3; ++c) f[c] = g[c][0];
         } else {
-            for (int64_t i = N.csr_ptr[n]; i < N.csr_ptr[n + 1]; ++i) {
-                const uint32_t ent = N.csr_ent[i];
-                const int k = static_cast<int>(ent & 7u);
-                const uint32_t el = ent >> 3;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) f[c] += fe[(3 * k + c) * ep + el];
-            }
+            listed_forces_mixed(E, N, n, f);
         }
         const double im = N.inv_mass[n];
         const float im_hi = static_cast<float>(im);
@@ -1326,7 +1236,7 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB) k_
             const NodeArrays N = d.N;
             const double dt1d = h.dt1;
             double d1, l1;
-            element_body_mixed<true, false, true, ENSC_BATCH_MIXED_PREFETCH>(
+            element_body_mixed<true, false, true>(
                 E, N, d.M, mixed_src_tile(sb, lane), mixed_out_tile(mixed_tile(E, ti.base >> 5), lane),
                 static_cast<float>(dt1d), dt1d, e, d1, l1, run.ei, run.eh, run.ev, run.bad);
             run.dts = fmin(run.dts, d1);
@@ -1411,7 +1321,7 @@ __global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTab
             const NodeArrays N = d.N;
             const double dt1d = h.dt1;
             double d1, l1;
-            element_body_mixed<true, false, true, ENSC_BATCH_MIXED_PREFETCH, true>(
+            element_body_mixed<true, false, true, true>(
                 E, N, d.M, mixed_src_tile(sb + wid * MixedTile::kBytes, lane),
                 mixed_out_tile(mixed_tile(E, (ti.base >> 5) + wid), lane), static_cast<float>(dt1d), dt1d, e, d1, l1, run.ei,
                 run.eh, run.ev, run.bad, fo);

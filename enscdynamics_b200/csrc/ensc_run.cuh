@@ -187,7 +187,7 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
                 for (int k = 0; k < 8; ++k) {
                     const uint32_t n = cn[k * 32 + lane];
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) xyz[k][c] = N.x[c * N.nn_pad + n];
+                    for (int c = 0; c < 3; ++c) xyz[k][c] = *node_x(N, c, n);
                 }
                 const double t = sqrt(min_edge_sq(xyz));
                 m = t < m ? t : m;
