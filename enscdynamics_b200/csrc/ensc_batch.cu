@@ -478,6 +478,7 @@ int ensc_batch_create(const ensc_params* params, int32_t max_instances, int64_t 
     e = cudaMemcpy(b->d_ctl, b->h_ctl, sizeof(Ctl) * b->slots, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail(bcuda(b, "ctl init", e));
     b->T.desc = b->d_desc;
+    b->T.ctl = b->d_ctl;
     b->T.etile_inst = b->d_etile_inst;
     b->T.etile_base = b->d_etile_base;
     b->T.ntile_inst = b->d_ntile_inst;

@@ -35,7 +35,7 @@
 //                                    its 8 slot vectors (exDyna3D.cpp:638-639)
 //     csr_ptr/csr_ent                general (slot, element)-sorted lists, where
 //                                    a node occupies the same slot in more than
-//                                    one element
+//                                    one element and has more than 8 elements
 #pragma once
 
 #include <cmath>
@@ -153,14 +153,18 @@ struct ElemArrays {
     void* qia;
     void* eps_p;
     void* fe;
+    // meshes whose nodes repeat local slots, with at most 8 elements at a node:
+    // the row of fe that each local node's force goes to, 4 bits per local node
+    // (null: the slot itself)
+    const uint32_t* rows;
     // bytes of a tile of 32 elements; the pointers above point into tile 0,
     // which starts 256-byte aligned (node rows too, padded to 32 entries: the
     // vectorised node passes).  0: plain rows of ne_pad entries.
     int32_t tile_bytes;
     // 1: the entries of fe are nodes -- the reference's per-local-slot nodal
     // vectors (exDyna3D.cpp:523-634), each entry written by the one element
-    // that holds the node in slot k; 0: elements, gathered through ell / csr by
-    // the node pass
+    // that holds the node in slot k (or has row k at the node); 0: elements,
+    // gathered through ell / csr by the node pass
     int32_t slot_major;
     int32_t bt9;               // FP64: bt holds 9 numbers per element (else 24)
     int32_t pad;
@@ -215,6 +219,7 @@ struct NodeArrays {
     const uint32_t* ell;
     const int64_t* csr_ptr;    // non-null: use the general lists
     const uint32_t* csr_ent;   // (e << 3) | slot
+    const uint8_t* merge;      // with ElemArrays::rows: bit r set where row r holds the same slot as row r - 1
     double* rf;                // reactions, [3][nn_pad]
     int32_t rec;               // 1: x, u, v in records (head of this file), 0: rows
     int32_t pad;
@@ -251,6 +256,7 @@ struct alignas(128) NodeView {
     double* x;
     const double* inv_mass;
     const uint8_t* bc;
+    const uint8_t* merge;      // NodeArrays::merge
     double* rf;
     Ctl* ctl;
     int64_t nn, np;
@@ -275,6 +281,7 @@ __host__ __device__ inline NodeView node_view(const ElemArrays& E, const NodeArr
     v.x = N.x;
     v.inv_mass = N.inv_mass;
     v.bc = N.bc;
+    v.merge = N.merge;
     v.rf = N.rf;
     v.ctl = ctl;
     v.nn = N.nn;
@@ -345,6 +352,7 @@ struct alignas(16) InstanceDesc {
 
 struct BatchTables {
     const InstanceDesc* desc;    // [slots]
+    Ctl* ctl;                    // [slots] control blocks (desc[s].ctl is ctl + s)
     const int32_t* etile_inst;   // [etiles] instance slot of each element tile
     const int32_t* etile_base;   // first element of the tile within its instance
     const int32_t* ntile_inst;   // [ntiles]

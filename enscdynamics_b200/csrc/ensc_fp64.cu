@@ -259,8 +259,7 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
                                              double& dts, double& len, double& e_int, double& e_hg, double& e_vis,
                                              int32_t& bad) {
     const int64_t ss = S.stride, si = S.i, os = O.stride, oi = O.i;
-    const int64_t ep = E.ne_pad, np = N.nn_pad;
-    double* fe = static_cast<double*>(E.fe);
+    const int64_t np = N.nn_pad;
     const double* X = N.x;
     const double* U = N.u;
     const double* V = static_cast<const double*>(N.v);
@@ -269,6 +268,7 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
     uint32_t n[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) n[k] = ldin<SMEM>(S.conn + k * ss + si);
+    if (REC && E.rows) prefetch_l1(E.rows + e);  // read with the forces
     if constexpr (REC && PF) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) prefetch_l1(U + 4 * static_cast<int64_t>(n[k]));
@@ -532,11 +532,16 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
     // is evaluated once for two opposite corners.
     {
         B0Rows<BT9, SMEM> Bf;
+        // (the force array is looked up here: a batch reads it from the stage)
+        double* fe = static_cast<double*>(E.fe);
+        const int64_t row = E.slot_major ? N.nn_pad : E.ne_pad;
+        const bool mapped = REC && E.rows != nullptr;
+        const uint32_t rows = mapped ? __ldg(E.rows + e) : 0u;
         auto store = [&](int j, const double (&f)[3]) {
-            const int64_t row = E.slot_major ? np : ep;
             const int64_t i = E.slot_major ? static_cast<int64_t>(ldin<SMEM>(S.conn + j * ss + si)) : e;
-            *reinterpret_cast<double2*>(force_xy(fe, row, j, i)) = make_double2(f[0], f[1]);
-            *force_z(fe, row, j, i) = f[2];
+            const int k = mapped ? static_cast<int>((rows >> (4 * j)) & 7u) : j;
+            *reinterpret_cast<double2*>(force_xy(fe, row, k, i)) = make_double2(f[0], f[1]);
+            *force_z(fe, row, k, i) = f[2];
         };
         if constexpr (BT9) {
             Bf.load(S);
@@ -759,16 +764,16 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
     const uint32_t stage0 = smem_addr(wst);
     const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kF64PipeWarps) * 2 * L::kBytes) + 16u * wid;
     const unsigned char* tiles = reinterpret_cast<const unsigned char*>(E.conn);
-    const int64_t ntiles = (E.ne + 31) / 32;
-    const int64_t wstride = static_cast<int64_t>(gridDim.x) * kF64PipeWarps;
-    const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kF64PipeWarps + wid;
+    const int ntiles = static_cast<int>((E.ne + 31) / 32);
+    const int wstride = static_cast<int>(gridDim.x) * kF64PipeWarps;
+    const int w0 = static_cast<int>(blockIdx.x) * kF64PipeWarps + wid;
     if (lane == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
         for (int s = 0; s < 2; ++s) {
-            const int64_t t = w0 + s * wstride;
-            if (t < ntiles) f64_tile_issue<PLASTIC, L>(tiles + t * L::kBytes, stage0 + s * L::kBytes, bar0 + 8 * s);
+            const int t = w0 + s * wstride;
+            if (t < ntiles) f64_tile_issue<PLASTIC, L>(tiles + static_cast<int64_t>(t) * L::kBytes, stage0 + s * L::kBytes, bar0 + 8 * s);
         }
     }
     __syncwarp();
@@ -777,7 +782,7 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
     int32_t bad = 0;
     bool timed_out = false;
     int it = 0;
-    for (int64_t t = w0; t < ntiles; t += wstride, ++it) {
+    for (int t = w0; t < ntiles; t += wstride, ++it) {
         const int s = it & 1;
         const uint32_t bar = bar0 + 8 * s;
         const bool ok = mbar_wait_bounded(bar, (it >> 1) & 1);
@@ -785,9 +790,9 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
             timed_out = true;
             break;
         }
-        const int64_t e = t * 32 + lane;
+        const int e = t * 32 + lane;
         if (e < E.ne) {
-            unsigned char* g = const_cast<unsigned char*>(tiles) + t * L::kBytes;
+            unsigned char* g = const_cast<unsigned char*>(tiles) + static_cast<int64_t>(t) * L::kBytes;
             double dts, len;
             element_body<PLASTIC, false, BT9, true, true, ENSC_F64_PREFETCH>(E, N, M, fp64_src_tile<L>(wst + s * L::kBytes, lane),
                                                                        fp64_out_tile<L>(g, lane), dt1, e, dts, len,
@@ -796,8 +801,8 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
             len_min = len < len_min ? len : len_min;
         }
         __syncwarp();  // all lanes are done with stage s
-        const int64_t tn = t + 2 * wstride;
-        if (lane == 0 && tn < ntiles) f64_tile_issue<PLASTIC, L>(tiles + tn * L::kBytes, stage0 + s * L::kBytes, bar);
+        const int tn = t + 2 * wstride;
+        if (lane == 0 && tn < ntiles) f64_tile_issue<PLASTIC, L>(tiles + static_cast<int64_t>(tn) * L::kBytes, stage0 + s * L::kBytes, bar);
     }
     if (timed_out) {
         // record the failure and let the copies this warp started land
@@ -817,9 +822,9 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
     block_sum<32 * kF64PipeWarps, 3, 7u>(v3, P.elem, P.n_elem_blocks, blockIdx.x);
 }
 
-// W consecutive nodes of the node pass on the slot-major layout.  Every slot is
-// added, empty ones as the zeros they hold, as the reference adds all 8 slot
-// vectors: the rows start zeroed and only the slot's element writes them.
+// W consecutive nodes of the node pass where the force rows are by node.  Every
+// row is added, empty ones as the zeros they hold, as the reference adds all 8
+// slot vectors: the rows start zeroed and only the row's element writes them.
 // Nodes at or past nn (row padding) are loaded and stored back unchanged.
 //
 // pre (resident runs): the nodes' own records, loaded while the grid still works
@@ -841,15 +846,20 @@ __device__ __forceinline__ void node_rows_load(const NodeView& N, const int64_t 
     r.code = ld_bytes<W>(N.bc + n0);
 }
 
-// The forces of W consecutive nodes, added up in slot order.
-template <int W>
+// The forces of W consecutive nodes, added up in row order.  MERGE: where a node
+// repeats a slot (bit k of its merge byte: row k holds the slot of row k - 1),
+// that slot's rows are summed first, as the reference adds each element to its
+// slot's vector before it adds the vectors.
+template <int W, bool MERGE = false>
 __device__ __forceinline__ void node_forces(const NodeView& N, const int64_t n0, double (&f)[3][W]) {
     const int64_t np = N.np;
     const double* fe = static_cast<const double*>(N.fe);
+    const uint32_t merge = MERGE ? ld_bytes<W>(N.merge + n0) : 0u;
+    double sl[3][W];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int j = 0; j < W; ++j) f[c][j] = 0.0;
+        for (int j = 0; j < W; ++j) f[c][j] = sl[c][j] = 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         double xy[2 * W], z[W];
@@ -857,15 +867,28 @@ __device__ __forceinline__ void node_forces(const NodeView& N, const int64_t n0,
         ld_row<W>(force_z(fe, np, k, n0), z);
 #pragma unroll
         for (int j = 0; j < W; ++j) {
-            f[0][j] = f[0][j] + xy[2 * j];
-            f[1][j] = f[1][j] + xy[2 * j + 1];
-            f[2][j] = f[2][j] + z[j];
+            const double r[3] = {xy[2 * j], xy[2 * j + 1], z[j]};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if constexpr (MERGE) {
+                    const bool same = (merge >> (8 * j + k)) & 1u;
+                    f[c][j] = same ? f[c][j] : f[c][j] + sl[c][j];
+                    sl[c][j] = (same ? sl[c][j] : 0.0) + r[c];
+                } else {
+                    f[c][j] = f[c][j] + r[c];
+                }
+            }
         }
     }
+    if constexpr (MERGE)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int j = 0; j < W; ++j) f[c][j] = f[c][j] + sl[c][j];
 }
 
 // PRE: rows and forces come in pre and fpre.
-template <int W, bool PRE = false>
+template <int W, bool PRE = false, bool MERGE = false>
 __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i, const double dt_i_1, const double amp,
                                            const int64_t n0, double& kin, double& wext, int32_t& bad,
                                            const NodeRowsF64<W>* pre = nullptr,
@@ -883,7 +906,7 @@ __device__ __forceinline__ void node_group(const NodeView& N, const double dt_i,
 #pragma unroll
             for (int j = 0; j < W; ++j) f[c][j] = fpre[c][j];
     } else {
-        node_forces<W>(N, n0, f);
+        node_forces<W, MERGE>(N, n0, f);
     }
 #pragma unroll
     for (int j = 0; j < W; ++j) {
@@ -949,7 +972,8 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration(ElemArrays E, Nod
         double f[3];
         if (E.slot_major) {
             double g[3][1];
-            node_forces<1>(nv, n, g);
+            if (N.merge) node_forces<1, true>(nv, n, g);
+            else node_forces<1>(nv, n, g);
 #pragma unroll
             for (int c = 0; c < 3; ++c) f[c] = g[c][0];
         } else {
@@ -973,6 +997,8 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration(ElemArrays E, Nod
 // ((((((a0+a1)+a2)+a3)+a4)+a5)+a6)+a7, exDyna3D.cpp:638-639), gravity
 // (:819-824), boundary conditions on a (:2029-2145), a = f M^-1 (:642-644),
 // v += (dt_i + dt_i_1) a / 2, u += dt_i v, x += dt_i v (:646-654, :688-696).
+// MERGE: nodes repeat slots (ElemArrays::rows).
+template <bool MERGE>
 __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_FP64) k_node(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
     if (ctl->done) return;
     // stable dt of this cycle (update_minVertex_perMaterial_and_dt :673-679)
@@ -1002,7 +1028,12 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_FP64) k_node(Elem
     if (E.slot_major && E.tile_bytes) {
         constexpr int W = kNodeGroupFp64;
         const NodeView nv = node_view(E, N, M, ctl);
-        for (int64_t g = t0; g * W < nn; g += stride) node_group<W>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad);
+        // from the last nodes back: their forces are the latest in L2, and the
+        // first nodes' records stay there for the next element pass (B200,
+        // 2,097,152 elements: 3% of a mixed cycle, 2% of an FP64 one)
+        const int64_t ng = (nn + W - 1) / W;
+        for (int64_t g = t0; g < ng; g += stride)
+            node_group<W, false, MERGE>(nv, dt_i, dt_i_1, amp, (ng - 1 - g) * W, kin, wext, bad);
     } else {
         for (int64_t n = t0; n < nn; n += stride) node_body(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
     }
@@ -1059,8 +1090,12 @@ struct RunFp64 {
 #pragma unroll
             for (int j = 0; j < W; ++j) rows.rim[j] = 1.0 / rows.im[j];
         }
+        __device__ void forces(const NodeView& nv, int64_t n0) {
+            if (nv.merge) node_forces<W, true>(nv, n0, f);
+            else node_forces<W>(nv, n0, f);
+        }
         __device__ void gather(const ElemArrays& E, const NodeArrays& N, const Material& M, int64_t t0) {
-            if (E.slot_major && t0 * W < N.nn) node_forces<W>(node_view(E, N, M, nullptr), t0 * W, f);
+            if (E.slot_major && t0 * W < N.nn) forces(node_view(E, N, M, nullptr), t0 * W);
         }
         __device__ void update(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i, double dt_i_1,
                                double amp, int64_t t0, int64_t stride, double& wext, int32_t& bad) {
@@ -1072,7 +1107,7 @@ struct RunFp64 {
                     for (int64_t g = t0 + stride; g * W < N.nn; g += stride) {
                         node_rows_load<W>(nv, g * W, rows);
                         if (M.gravity_on) reciprocals();
-                        node_forces<W>(nv, g * W, f);
+                        forces(nv, g * W);
                         node_group<W, true>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad, &rows, f);
                     }
             } else {
@@ -1107,12 +1142,6 @@ __global__ void __launch_bounds__(32 * kRunWarpsF64, 1)
 // k_fold_batch folds them per instance in tile order, so the totals do not
 // depend on scheduling.  Arithmetic per element and node is that of
 // the single-instance kernels, so states are bit-identical to them.
-__device__ __forceinline__ double warp_sum_b(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // A batch stage: a tile, then its instance descriptor, its element-pass scalars
 // (StageHdr), the TileInfo the filling lane writes, and the ETileSrc record of
 // the tile that uses the stage next (as in the mixed batch pass).  The tile's
@@ -1138,9 +1167,9 @@ __device__ __forceinline__ void f64_batch_issue(const BatchTables& T, const ETil
 
 // The batched FP64 element pass: one pipeline per warp over tiles of 32
 // elements, element_body's arithmetic per element, so states are bit-identical
-// to the single-instance pass.  A warp's consecutive tiles of one instance form
-// a run whose sums and minima are reduced once, into the partial slot of the
-// run's first tile.
+// to the single-instance pass.  Sums are kept over a warp's consecutive tiles of
+// one instance and reduced into the partial slot of the first: reducing per tile
+// took 3% more of a 24-instance sweep's cycle.
 __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB) k_element_batch_fp64(BatchTables T) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1148,52 +1177,28 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB) k_elem
     unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
     const uint32_t stage0 = smem_addr(wst);
     const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kF64PipeWarps) * 2 * SB) + 16u * wid;
-    const int64_t ntiles = T.counts[0];
-    const int64_t wstride = static_cast<int64_t>(gridDim.x) * kF64PipeWarps;
-    const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kF64PipeWarps + wid;
+    const int ntiles = T.counts[0];
+    const int wstride = static_cast<int>(gridDim.x) * kF64PipeWarps;
+    const int w0 = static_cast<int>(blockIdx.x) * kF64PipeWarps + wid;
     if (lane == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
         for (int s = 0; s < 2; ++s) {
-            const int64_t t = w0 + s * wstride;
+            const int t = w0 + s * wstride;
             if (t < ntiles)
                 f64_batch_issue(T, T.etile_src[t], t + 2 * wstride, ntiles, wst + s * SB, stage0 + s * SB, bar0 + 8 * s);
         }
     }
     __syncwarp();
-    // the current run: instance slot, first tile, control block, liveness
-    int run_slot = -1;
-    int64_t run_tile = 0;
-    Ctl* run_ctl = nullptr;
-    bool run_live = false;
-    double ei = 0.0, eh = 0.0, ev = 0.0, dts = DBL_MAX, len = DBL_MAX;
-    int32_t bad = 0;
-    auto flush = [&]() {
-        ei = warp_sum_b(ei);
-        eh = warp_sum_b(eh);
-        ev = warp_sum_b(ev);
-        const unsigned long long dmin = run_warp_min(ord_bits(dts));
-        const unsigned long long lmin = run_warp_min(ord_bits(len));
-        bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
-        if (run_live && lane == 0) {
-            double* part = T.etile_part + 3 * run_tile;
-            // one writer per slot and pass: the reductions (no return value)
-            // add in cycle order without a round trip
-            atomicAdd(part + 0, ei);
-            atomicAdd(part + 1, eh);
-            atomicAdd(part + 2, ev);
-            atomicMin(&run_ctl->dts_next, dmin);
-            atomicMin(&run_ctl->len_min, lmin);
-            if (bad) atomicOr(&run_ctl->status, bad);
-        }
-        ei = eh = ev = 0.0;
-        dts = len = DBL_MAX;
-        bad = 0;
-    };
     bool timed_out = false;
     int it = 0;
-    int64_t t = w0;
+    int t = w0;
+    // the current run, consecutive tiles of one instance: its slot, first tile and sums
+    int run_slot = -1, run_tile = 0;
+    bool live = false;
+    double ei = 0.0, eh = 0.0, ev = 0.0, dts = DBL_MAX, len = DBL_MAX;
+    int32_t bad = 0;
     for (; t < ntiles; t += wstride, ++it) {
         const int s = it & 1;
         const uint32_t bar = bar0 + 8 * s;
@@ -1207,44 +1212,47 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB) k_elem
         const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(tail);
         const StageHdr& h = *reinterpret_cast<const StageHdr*>(tail + kBatchHdrOff);
         const TileInfo& ti = *reinterpret_cast<const TileInfo*>(tail + kBatchInfoOff);
-        if (ti.slot != run_slot) {
-            flush();
-            run_slot = ti.slot;
+        const int slot = ti.slot, e = ti.base + lane;
+        if (slot != run_slot) {
+            if (live) batch_tile_sums(T, run_tile, run_slot, lane, ei, eh, ev, dts, len, bad);
+            ei = eh = ev = 0.0;
+            dts = len = DBL_MAX;
+            bad = 0;
+            run_slot = slot;
             run_tile = t;
-            run_ctl = d.ctl;
-            run_live = h.live != 0;
+            live = h.live != 0;
         }
-        const int64_t e = static_cast<int64_t>(ti.base) + lane;
-        if (run_live && e < d.E.ne) {
+        if (live && e < d.E.ne) {
             // arrays copied to registers, material read at use
             const ElemArrays E = d.E;
             const NodeArrays N = d.N;
             const double dt1 = h.dt1;
+            unsigned char* g = tile_row(E, const_cast<unsigned char*>(reinterpret_cast<const unsigned char*>(E.conn)), ti.base);
             double d1, l1;
             if (E.bt9)
                 element_body<true, false, true, true, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile9>(st, lane),
-                                                                         fp64_out_global<true>(E, e), dt1, e, d1, l1, ei, eh,
+                                                                         fp64_out_tile<Fp64Tile9>(g, lane), dt1, e, d1, l1, ei, eh,
                                                                          ev, bad);
             else
                 element_body<true, false, false, true, true, ENSC_F64_PREFETCH>(E, N, d.M, fp64_src_tile<Fp64Tile24>(st, lane),
-                                                                          fp64_out_global<true>(E, e), dt1, e, d1, l1, ei, eh,
+                                                                          fp64_out_tile<Fp64Tile24>(g, lane), dt1, e, d1, l1, ei, eh,
                                                                           ev, bad);
             dts = d1 < dts ? d1 : dts;
             len = l1 < len ? l1 : len;
         }
         __syncwarp();  // all lanes are done with stage s
-        const int64_t tn = t + 2 * wstride;
+        const int tn = t + 2 * wstride;
         if (lane == 0 && tn < ntiles) {
             const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
             f64_batch_issue(T, src, tn + 2 * wstride, ntiles, st, stage0 + s * SB, bar);
         }
     }
     if (!timed_out) {
-        flush();
+        if (live) batch_tile_sums(T, run_tile, run_slot, lane, ei, eh, ev, dts, len, bad);
     } else if (lane == 0) {
         // record the failure on the instance whose tile could not be read and
         // let the copies this warp started land (bounded) before exiting
-        atomicOr(&T.desc[T.etile_inst[t]].ctl->status, ST_TIMEOUT);
+        atomicOr(&T.ctl[T.etile_inst[t]].status, ST_TIMEOUT);
         for (int k = 0; k < 2; ++k) {
             const int itk = it + k;
             if (w0 + itk * wstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
@@ -1282,16 +1290,18 @@ __global__ void __launch_bounds__(NT, ENSC_NODE_MINB_FP64 * kNodeThreads / NT) k
             int32_t bad = 0;
             const int64_t n0 = static_cast<int64_t>(base) + static_cast<int64_t>(lane) * W;
             if (n0 < v.nn) {
-                if (v.grouped) {
+                if (v.grouped && !v.merge) {
                     node_group<W>(v, dt_i, dt_i_1, amp, n0, kin, wext, bad);
+                } else if (v.grouped) {
+                    node_group<W, false, true>(v, dt_i, dt_i_1, amp, n0, kin, wext, bad);
                 } else {
                     const InstanceDesc& d = T.desc[slot];
                     for (int j = 0; j < W && n0 + j < v.nn; ++j)
                         node_body(d.E, d.N, d.M, dt_i, dt_i_1, amp, n0 + j, kin, wext, bad);
                 }
             }
-            kin = warp_sum_b(kin);
-            wext = warp_sum_b(wext);
+            kin = batch_warp_sum(kin);
+            wext = batch_warp_sum(wext);
             bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
             if (lane == 0) {
                 double* part = T.ntile_part + 2 * static_cast<int64_t>(t);
@@ -1338,7 +1348,8 @@ void launch_element_fp64(const ElemArrays& E, const NodeArrays& N, const Materia
 
 void launch_node_fp64(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl, const Partials& P,
                       int grid, cudaStream_t st) {
-    k_node<<<grid, kNodeThreads, 0, st>>>(E, N, M, ctl, P);
+    if (N.merge) k_node<true><<<grid, kNodeThreads, 0, st>>>(E, N, M, ctl, P);
+    else k_node<false><<<grid, kNodeThreads, 0, st>>>(E, N, M, ctl, P);
 }
 
 int occupancy_element_fp64(bool plastic, bool bt9) {
@@ -1369,7 +1380,7 @@ int node_group_width(bool mixed_precision) { return mixed_precision ? kNodeGroup
 
 int occupancy_node_fp64() {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_node, kNodeThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_node<false>, kNodeThreads, 0);
     return nb;
 }
 

@@ -384,12 +384,37 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
                 const uint32_t n = conn[8 * e + k];
                 h.csr_ent[fill[n]++] = (static_cast<uint32_t>(e) << 3) | static_cast<uint32_t>(k);
             }
+        // at most 8 elements at every node: each entry of a node's list gets its own
+        // row of the force array, so that the hand-off and its sums stay those of
+        // meshes without clashes.  Rows rise along the list and keep to the slots
+        // where they can: neighbouring elements then write neighbouring entries.
+        bool fits = true;
+        for (int64_t n = 0; n < nn && fits; ++n) fits = h.csr_ptr[n + 1] - h.csr_ptr[n] <= 8;
+        if (fits) {
+            h.rows.assign(static_cast<size_t>(ep), 0);
+            if (!mixed) h.merge.assign(static_cast<size_t>(np), 0);
+            for (int64_t n = 0; n < nn; ++n) {
+                const int m = static_cast<int>(h.csr_ptr[n + 1] - h.csr_ptr[n]);
+                const uint32_t* list = h.csr_ent.data() + h.csr_ptr[n];
+                int row = -1;
+                for (int i = 0; i < m; ++i) {
+                    const int k = static_cast<int>(list[i] & 7u);
+                    row = std::min(std::max(row + 1, k), 8 - (m - i));
+                    h.rows[list[i] >> 3] |= static_cast<uint32_t>(row) << (4 * k);
+                    if (!mixed && i > 0 && static_cast<int>(list[i - 1] & 7u) == k)
+                        h.merge[n] |= static_cast<uint8_t>(1u << row);
+                }
+            }
+            std::vector<int64_t>().swap(h.csr_ptr);
+            std::vector<uint32_t>().swap(h.csr_ent);
+        }
     }
+    const bool listed = !h.csr_ptr.empty();
 
     // device layout
     const size_t real = mixed ? 4 : 8;  // element state, forces and velocity
     const size_t E8 = static_cast<size_t>(ep), N8 = static_cast<size_t>(np);
-    const size_t fe_rows = h.clash ? E8 : N8;
+    const size_t fe_rows = listed ? E8 : N8;
     using P = InstanceHost::Piece;
     h.tile_bytes = mixed ? MixedTile::kBytes : (h.bt9 ? Fp64Tile9::kBytes : Fp64Tile24::kBytes);
     h.const_bytes = mixed ? MixedTile::kState : (h.bt9 ? Fp64Tile9::kState : Fp64Tile24::kState);
@@ -403,8 +428,10 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
     h.size[P::BC] = N8;
     h.size[P::BCV] = 3 * N8 * 8;
     h.size[P::RF] = 3 * N8 * 8;
-    h.size[P::CPTR] = h.clash ? static_cast<size_t>(nn + 1) * sizeof(int64_t) : 0;
-    h.size[P::CENT] = h.clash ? static_cast<size_t>(8 * ne) * sizeof(uint32_t) : 0;
+    h.size[P::ROWS] = h.rows.size() * sizeof(uint32_t);
+    h.size[P::MERGE] = h.merge.size();
+    h.size[P::CPTR] = listed ? static_cast<size_t>(nn + 1) * sizeof(int64_t) : 0;
+    h.size[P::CENT] = listed ? static_cast<size_t>(8 * ne) * sizeof(uint32_t) : 0;
     if (h.patch) {
         h.size[P::IPERM] = static_cast<size_t>(ne) * sizeof(int32_t);
         h.size[P::PFOFF] = static_cast<size_t>(h.n_patches + 1) * sizeof(uint32_t);
@@ -441,10 +468,10 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     if (e == cudaSuccess) e = put(block, h.off[P::V], h.vz_d, st);
     if (e == cudaSuccess) e = put(block, h.off[P::V], h.vz_f, st);
     if (e == cudaSuccess) e = put(block, h.off[P::V] + np * sizeof(float), h.v_lo, st);
-    if (h.clash) {
-        if (e == cudaSuccess) e = put(block, h.off[P::CPTR], h.csr_ptr, st);
-        if (e == cudaSuccess) e = put(block, h.off[P::CENT], h.csr_ent, st);
-    }
+    if (e == cudaSuccess) e = put(block, h.off[P::ROWS], h.rows, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::MERGE], h.merge, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::CPTR], h.csr_ptr, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::CENT], h.csr_ent, st);
     std::vector<uint32_t> nptr_pad;
     if (h.patch) {
         // padding nodes have no partials: nptr stays at the total past nn
@@ -483,7 +510,9 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     E.fe = b + h.off[P::FE];
     E.tile_bytes = h.tile_bytes;  // pieces are 256-byte aligned, rows padded to 32
     E.bt9 = h.bt9 ? 1 : 0;
-    E.slot_major = h.clash ? 0 : 1;
+    const bool listed = !h.csr_ptr.empty();
+    E.slot_major = listed ? 0 : 1;
+    E.rows = h.rows.empty() ? nullptr : reinterpret_cast<uint32_t*>(b + h.off[P::ROWS]);
     PA = PatchArrays{};
     if (h.patch) {
         PA.pf_off = reinterpret_cast<uint32_t*>(b + h.off[P::PFOFF]);
@@ -505,8 +534,9 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     N.bc = reinterpret_cast<uint8_t*>(b + h.off[P::BC]);
     N.bcv = reinterpret_cast<double*>(b + h.off[P::BCV]);
     N.rec = 1;
-    N.csr_ptr = h.clash ? reinterpret_cast<int64_t*>(b + h.off[P::CPTR]) : nullptr;
-    N.csr_ent = h.clash ? reinterpret_cast<uint32_t*>(b + h.off[P::CENT]) : nullptr;
+    N.csr_ptr = listed ? reinterpret_cast<int64_t*>(b + h.off[P::CPTR]) : nullptr;
+    N.csr_ent = listed ? reinterpret_cast<uint32_t*>(b + h.off[P::CENT]) : nullptr;
+    N.merge = h.merge.empty() ? nullptr : reinterpret_cast<uint8_t*>(b + h.off[P::MERGE]);
     N.rf = reinterpret_cast<double*>(b + h.off[P::RF]);
     return ENSC_OK;
 }

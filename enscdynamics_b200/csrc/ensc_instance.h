@@ -23,7 +23,12 @@ struct InstanceHost {
     std::vector<double> jinv;         // [ne][9] J^-1 / 8 where bt9
     std::vector<double> vol0;         // [ne] V0
     std::vector<double> im;           // [nn_pad] inverse lumped mass per node
-    std::vector<int64_t> csr_ptr;     // clash meshes: (slot, element)-sorted lists
+    // clash meshes (a node repeats a local slot): with at most 8 elements at
+    // every node, rows of the force array [ne_pad] (ElemArrays::rows) and
+    // merge flags [nn_pad] (NodeArrays::merge); else (slot, element)-sorted lists
+    std::vector<uint32_t> rows;
+    std::vector<uint8_t> merge;
+    std::vector<int64_t> csr_ptr;
     std::vector<uint32_t> csr_ent;
     const double* x0 = nullptr;       // caller arrays, read by instance_prepare only
     const double* v0 = nullptr;
@@ -52,7 +57,7 @@ struct InstanceHost {
     int64_t n_patches = 0, n_pnodes = 0;
     // device layout: byte offsets of the pieces in one 256-byte-aligned block
     enum Piece {
-        TILES, FE, X, U, V, IM, BC, BCV, RF, CPTR, CENT,
+        TILES, FE, X, U, V, IM, BC, BCV, RF, ROWS, MERGE, CPTR, CENT,
         IPERM, PFOFF, PINCOFF, PINC, PF, NPTR, NENT, NPIECE
     };
     size_t off[NPIECE] = {};

@@ -102,7 +102,7 @@ int occupancy_element_fp64(bool plastic, bool bt9);
 #define ENSC_NODE_MINB_MIXED 2
 #endif
 #ifndef ENSC_NODE_MINB_FP64
-#define ENSC_NODE_MINB_FP64 4
+#define ENSC_NODE_MINB_FP64 3
 #endif
 #ifndef ENSC_NODE_GROUP_FP64
 #define ENSC_NODE_GROUP_FP64 1

@@ -202,8 +202,8 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
                                                    const double dt1d, const int64_t e, double& dts, double& len,
                                                    double& e_int, double& e_hg, double& e_vis, int32_t& bad,
                                                    float* fout = nullptr) {
-    const int64_t ep = E.ne_pad, np = N.nn_pad, ss = 32, si = S.i, os = 32, oi = O.i;
-    float* fe = static_cast<float*>(E.fe);
+    constexpr int ss = 32, os = 32;
+    const int si = S.i, oi = O.i;
     const double* X = N.x;
     const float* V = static_cast<const float*>(N.v);
     const float G = M.mc.G;
@@ -213,17 +213,7 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
     const float cvisl = M.mc.cvisl, cvisq = M.mc.cvisq;
     const float y0 = M.mc.y0, H = M.mc.H;
     const float DRc = M.mc.DRc, CRc = M.mc.CRc;
-    // A = sum_j B0_j s_j^T as a float pair (hi + lo); B0 enters every
-    // product through A, so no FP32 rounding of the reference geometry is
-    // shared by all elements of a uniform mesh
-    float Ah[3][3], Al[3][3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            Ah[c][m] = ldin<SMEM>(S.a + (3 * c + m) * ss + si);
-            Al[c][m] = ldin<SMEM>(S.a + (9 + 3 * c + m) * ss + si);
-        }
+    if (!FOUT && E.rows) prefetch_l1(E.rows + e);  // read with the forces
     uint32_t nk[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) nk[k] = ldin<SMEM>(S.conn + k * ss + si);
@@ -243,6 +233,7 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
     // every element and shift the stiffness and the stable dt of all of them
     float TX[4][3];
     float F[3][3];
+    float Ah[3][3], Al[3][3];
     {
         constexpr int A0[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3};
         constexpr int A1[12] = {1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7};
@@ -270,6 +261,16 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
             TX[2][r] = static_cast<float>(-c[5]);
             TX[3][r] = static_cast<float>(c[7]);
         }
+        // A = sum_j B0_j s_j^T as a float pair (hi + lo); B0 enters every
+        // product through A, so no FP32 rounding of the reference geometry is
+        // shared by all elements of a uniform mesh
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                Ah[c][m] = ldin<SMEM>(S.a + (3 * c + m) * ss + si);
+                Al[c][m] = ldin<SMEM>(S.a + (9 + 3 * c + m) * ss + si);
+            }
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -477,25 +478,33 @@ __device__ __forceinline__ void element_body_mixed(const ElemArrays& E, const No
     // per force component: the node values of -(B0_j Z) - Gamma_j Gq^T from
     // their corner coefficients (-Y on xi, eta, zeta; -Gq on the hourglass
     // vectors, signed as Gamma)
-    float fx[8];
+    float f[3][8];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         float c[8] = {0.f,          -Y[0][i],     -Y[1][i],     -Gq[i][0],
                       -Y[2][i],     Gq[i][2],     Gq[i][1],     -Gq[i][3]};
-        float f[8];
-        corner_values(c, f);
-        if (FOUT) {
+        corner_values(c, f[i]);
+    }
+    if (FOUT) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) fout[8 * i + j] = f[j];
-            continue;
-        }
-        const int64_t row = E.slot_major ? np : ep;
+        for (int i = 0; i < 24; ++i) fout[i] = f[i / 8][i % 8];
+    } else {
+        // (the force array is looked up here: a batch reads it from the stage)
+        float* fe = static_cast<float*>(E.fe);
+        auto store = [&](int j, int k, int64_t row, int64_t at) {
+            *reinterpret_cast<float2*>(force_xy(fe, row, k, at)) = make_float2(f[0][j], f[1][j]);
+            *force_z(fe, row, k, at) = f[2][j];
+        };
+        if (!E.slot_major) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int64_t at = E.slot_major ? static_cast<int64_t>(nk[j]) : e;
-            if (i == 0) fx[j] = f[j];
-            else if (i == 1) *reinterpret_cast<float2*>(force_xy(fe, row, j, at)) = make_float2(fx[j], f[j]);
-            else *force_z(fe, row, j, at) = f[j];
+            for (int j = 0; j < 8; ++j) store(j, j, E.ne_pad, e);
+        } else if (E.rows) {
+            const uint32_t rows = __ldg(E.rows + e);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) store(j, static_cast<int>((rows >> (4 * j)) & 7u), N.nn_pad, nk[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) store(j, j, N.nn_pad, nk[j]);
         }
     }
     // element dt (compute_dtStable, exDyna3D.cpp:828-834), with the
@@ -562,15 +571,15 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
     unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
     const uint32_t stage0 = smem_addr(wst);
     const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kMixedPipeWarps) * 2 * SB) + 16u * wid;
-    const int64_t ntiles = (E.ne + 31) / 32;
-    const int64_t wstride = static_cast<int64_t>(gridDim.x) * kMixedPipeWarps;
-    const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kMixedPipeWarps + wid;
+    const int ntiles = static_cast<int>((E.ne + 31) / 32);
+    const int wstride = static_cast<int>(gridDim.x) * kMixedPipeWarps;
+    const int w0 = static_cast<int>(blockIdx.x) * kMixedPipeWarps + wid;
     if (lane == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
         for (int s = 0; s < 2; ++s) {
-            const int64_t t = w0 + s * wstride;
+            const int t = w0 + s * wstride;
             if (t < ntiles) mixed_tile_issue<PLASTIC>(mixed_tile(E, t), stage0 + s * SB, bar0 + 8 * s);
         }
     }
@@ -580,7 +589,7 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
     int32_t bad = 0;
     bool timed_out = false;
     int it = 0;
-    for (int64_t t = w0; t < ntiles; t += wstride, ++it) {
+    for (int t = w0; t < ntiles; t += wstride, ++it) {
         const int s = it & 1;
         const uint32_t bar = bar0 + 8 * s;
         const bool ok = mbar_wait_bounded(bar, (it >> 1) & 1);
@@ -588,7 +597,7 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
             timed_out = true;
             break;
         }
-        const int64_t e = t * 32 + lane;
+        const int e = t * 32 + lane;
         if (e < E.ne) {
             double dts, len;
             element_body_mixed<PLASTIC, false, true>(
@@ -598,7 +607,7 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
             len_min = fmin(len_min, len);
         }
         __syncwarp();  // all lanes are done with stage s
-        const int64_t tn = t + 2 * wstride;
+        const int tn = t + 2 * wstride;
         if (lane == 0 && tn < ntiles) mixed_tile_issue<PLASTIC>(mixed_tile(E, tn), stage0 + s * SB, bar);
     }
     if (timed_out) {
@@ -989,8 +998,12 @@ __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_MIXED) k_node_mix
     if (E.slot_major && E.tile_bytes) {
         constexpr int W = kNodeGroupMixed;
         const NodeView nv = node_view(E, N, M, ctl, &PA);
-        for (int64_t g = t0; g * W < nn; g += stride)
-            node_group_mixed<W, PATCH>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad);
+        // from the last nodes back: their forces are the latest in L2, and the
+        // first nodes' records stay there for the next element pass (B200,
+        // 2,097,152 elements: 3% of a mixed cycle, 2% of an FP64 one)
+        const int64_t ng = (nn + W - 1) / W;
+        for (int64_t g = t0; g < ng; g += stride)
+            node_group_mixed<W, PATCH>(nv, dt_i, dt_i_1, amp, (ng - 1 - g) * W, kin, wext, bad);
     } else {
         for (int64_t n = t0; n < nn; n += stride) node_body_mixed(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
     }
@@ -1120,12 +1133,6 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration_mixed(PatchArrays
 // accumulates its work terms across cycles (one owner per tile and pass) and
 // keeps its latest kinetic energy; k_fold_batch folds them per instance in tile
 // order, so the totals do not depend on scheduling.
-__device__ __forceinline__ double warp_sum_b(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // A batch stage: the tile (or patch), then its instance descriptor, its
 // element-pass scalars (StageHdr), the TileInfo the filling lane writes, and the
 // ETileSrc record of the tile that uses the stage next.  Every tile is copied
@@ -1147,38 +1154,6 @@ __device__ __forceinline__ void batch_issue(const BatchTables& T, const ETileSrc
     if (next) bulk_g2s(dst + ROOM + kBatchNextOff, T.etile_src + t_next, sizeof(ETileSrc), bar);
 }
 
-// A thread's sums over a run: consecutive tiles of one instance, reduced per
-// warp once, into the partial slot of the run's first tile.
-struct BatchRun {
-    int slot = -1;
-    double* part = nullptr;
-    Ctl* ctl = nullptr;
-    bool live = false;
-    double ei = 0.0, eh = 0.0, ev = 0.0, dts = DBL_MAX, len = DBL_MAX;
-    int32_t bad = 0;
-    __device__ __forceinline__ void flush(int lane) {
-        ei = warp_sum_b(ei);
-        eh = warp_sum_b(eh);
-        ev = warp_sum_b(ev);
-        const unsigned long long dmin = run_warp_min(ord_bits(dts));
-        const unsigned long long lmin = run_warp_min(ord_bits(len));
-        bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
-        if (live && lane == 0) {
-            // one writer per slot and pass: the reductions (no return value)
-            // add in cycle order without a round trip
-            atomicAdd(part + 0, ei);
-            atomicAdd(part + 1, eh);
-            atomicAdd(part + 2, ev);
-            atomicMin(&ctl->dts_next, dmin);
-            atomicMin(&ctl->len_min, lmin);
-            if (bad) atomicOr(&ctl->status, bad);
-        }
-        ei = eh = ev = 0.0;
-        dts = len = DBL_MAX;
-        bad = 0;
-    }
-};
-
 constexpr uint32_t kBatchStageMixed = MixedTile::kBytes + kBatchTailBytes;
 constexpr size_t kBatchMixedSmem = static_cast<size_t>(kMixedPipeWarps) * (2 * kBatchStageMixed + 16);
 
@@ -1189,25 +1164,24 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB) k_
     unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
     const uint32_t stage0 = smem_addr(wst);
     const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kMixedPipeWarps) * 2 * SB) + 16u * wid;
-    const int64_t ntiles = T.counts[0];
-    const int64_t wstride = static_cast<int64_t>(gridDim.x) * kMixedPipeWarps;
-    const int64_t w0 = static_cast<int64_t>(blockIdx.x) * kMixedPipeWarps + wid;
+    const int ntiles = T.counts[0];
+    const int wstride = static_cast<int>(gridDim.x) * kMixedPipeWarps;
+    const int w0 = static_cast<int>(blockIdx.x) * kMixedPipeWarps + wid;
     if (lane == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
         mbar_init_fence();
         for (int s = 0; s < 2; ++s) {
-            const int64_t t = w0 + s * wstride;
+            const int t = w0 + s * wstride;
             if (t < ntiles)
                 batch_issue<MixedTile::kBytes>(T, T.etile_src[t], t + 2 * wstride, ntiles, wst + s * SB, stage0 + s * SB,
                                                bar0 + 8 * s);
         }
     }
     __syncwarp();
-    BatchRun run;
     bool timed_out = false;
     int it = 0;
-    int64_t t = w0;
+    int t = w0;
     for (; t < ntiles; t += wstride, ++it) {
         const int s = it & 1;
         const uint32_t bar = bar0 + 8 * s;
@@ -1221,40 +1195,30 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB) k_
         const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(tail);
         const StageHdr& h = *reinterpret_cast<const StageHdr*>(tail + kBatchHdrOff);
         const TileInfo& ti = *reinterpret_cast<const TileInfo*>(tail + kBatchInfoOff);
-        if (ti.slot != run.slot) {
-            run.flush(lane);
-            run.slot = ti.slot;
-            run.part = T.etile_part + 3 * t;
-            run.ctl = d.ctl;
-            run.live = h.live != 0;
-        }
-        const int64_t e = static_cast<int64_t>(ti.base) + lane;
-        if (run.live && e < d.E.ne) {
-            // arrays copied to registers (the body's stores could alias the
-            // stage as far as the compiler knows), material constants read at use
-            const ElemArrays E = d.E;
-            const NodeArrays N = d.N;
+        double ei = 0.0, eh = 0.0, ev = 0.0, dts = DBL_MAX, len = DBL_MAX;
+        int32_t bad = 0;
+        const int slot = ti.slot, e = ti.base + lane;
+        const bool live = h.live != 0;
+        if (live && e < d.E.ne) {
+            const ElemArrays& E = d.E;
+            const NodeArrays& N = d.N;
             const double dt1d = h.dt1;
-            double d1, l1;
             element_body_mixed<true, false, true>(
                 E, N, d.M, mixed_src_tile(sb, lane), mixed_out_tile(mixed_tile(E, ti.base >> 5), lane),
-                static_cast<float>(dt1d), dt1d, e, d1, l1, run.ei, run.eh, run.ev, run.bad);
-            run.dts = fmin(run.dts, d1);
-            run.len = fmin(run.len, l1);
+                static_cast<float>(dt1d), dt1d, e, dts, len, ei, eh, ev, bad);
         }
         __syncwarp();  // all lanes are done with stage s
-        const int64_t tn = t + 2 * wstride;
+        const int tn = t + 2 * wstride;
         if (lane == 0 && tn < ntiles) {
             const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
             batch_issue<MixedTile::kBytes>(T, src, tn + 2 * wstride, ntiles, sb, stage0 + s * SB, bar);
         }
+        if (live) batch_tile_sums(T, t, slot, lane, ei, eh, ev, dts, len, bad);
     }
-    if (!timed_out) {
-        run.flush(lane);
-    } else if (lane == 0) {
+    if (timed_out && lane == 0) {
         // record the failure on the instance whose tile could not be read and
         // let the copies this warp started land (bounded) before exiting
-        atomicOr(&T.desc[T.etile_inst[t]].ctl->status, ST_TIMEOUT);
+        atomicOr(&T.ctl[T.etile_inst[t]].status, ST_TIMEOUT);
         for (int k = 0; k < 2; ++k) {
             const int itk = it + k;
             if (w0 + itk * wstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
@@ -1289,7 +1253,6 @@ __global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTab
         }
     }
     __syncthreads();
-    BatchRun run;
     bool timed_out = false;
     int it = 0;
     int64_t t = blockIdx.x;
@@ -1306,29 +1269,23 @@ __global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTab
         const InstanceDesc& d = *reinterpret_cast<const InstanceDesc*>(tail);
         const StageHdr& h = *reinterpret_cast<const StageHdr*>(tail + kBatchHdrOff);
         const TileInfo& ti = *reinterpret_cast<const TileInfo*>(tail + kBatchInfoOff);
-        if (ti.slot != run.slot) {
-            run.flush(lane);
-            run.slot = ti.slot;
-            run.part = T.etile_part + 3 * (t * NW + wid);
-            run.ctl = d.ctl;
-            run.live = h.live != 0;
-        }
+        double ei = 0.0, eh = 0.0, ev = 0.0, dts = DBL_MAX, len = DBL_MAX;
+        int32_t bad = 0;
+        const int slot = ti.slot;
+        const bool live = h.live != 0;
         float fo[24];
         const int64_t e = static_cast<int64_t>(ti.base) + tid;
         const int64_t ne = d.E.ne;
-        if (run.live && e < ne) {
-            const ElemArrays E = d.E;
-            const NodeArrays N = d.N;
+        if (live && e < ne) {
+            const ElemArrays& E = d.E;
+            const NodeArrays& N = d.N;
             const double dt1d = h.dt1;
-            double d1, l1;
             element_body_mixed<true, false, true, true>(
                 E, N, d.M, mixed_src_tile(sb + wid * MixedTile::kBytes, lane),
-                mixed_out_tile(mixed_tile(E, (ti.base >> 5) + wid), lane), static_cast<float>(dt1d), dt1d, e, d1, l1, run.ei,
-                run.eh, run.ev, run.bad, fo);
-            run.dts = fmin(run.dts, d1);
-            run.len = fmin(run.len, l1);
+                mixed_out_tile(mixed_tile(E, (ti.base >> 5) + wid), lane), static_cast<float>(dt1d), dt1d, e, dts, len, ei, eh,
+                ev, bad, fo);
         }
-        if (run.live) {
+        if (live) {
             const PatchArrays PE = d.pa;
             __syncthreads();  // the stage's inputs are consumed
             float* sf = reinterpret_cast<float*>(sb);
@@ -1345,11 +1302,10 @@ __global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTab
             const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
             batch_issue<kPatchStageBytes>(T, src, tn + 2 * gstride, ntiles, sb, stage0 + s * SB, bar);
         }
+        if (live) batch_tile_sums(T, static_cast<int>(t) * NW + wid, slot, lane, ei, eh, ev, dts, len, bad);
     }
-    if (!timed_out) {
-        run.flush(lane);
-    } else if (tid == 0) {
-        atomicOr(&T.desc[T.etile_inst[t]].ctl->status, ST_TIMEOUT);
+    if (timed_out && tid == 0) {
+        atomicOr(&T.ctl[T.etile_inst[t]].status, ST_TIMEOUT);
         for (int k = 0; k < 2; ++k) {
             const int itk = it + k;
             if (blockIdx.x + itk * gstride < ntiles) mbar_wait_bounded(bar0 + 8 * (itk & 1), (itk >> 1) & 1);
@@ -1400,8 +1356,8 @@ __global__ void __launch_bounds__(NT, ENSC_NODE_BATCH_MINB_MIXED * kNodeThreads 
                         node_body_mixed(d.E, d.N, d.M, dt_i, dt_i_1, amp, n0 + j, kin, wext, bad);
                 }
             }
-            kin = warp_sum_b(kin);
-            wext = warp_sum_b(wext);
+            kin = batch_warp_sum(kin);
+            wext = batch_warp_sum(wext);
             bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
             if (lane == 0) {
                 double* part = T.ntile_part + 2 * static_cast<int64_t>(t);

@@ -53,6 +53,37 @@ __device__ __forceinline__ unsigned long long run_warp_min(unsigned long long v)
     return (static_cast<unsigned long long>(h) << 32) | l;
 }
 
+// ---- batched element passes: a warp's sums over one tile ----
+__device__ __forceinline__ double batch_warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// Reduced per tile: between a warp's tiles, 100,000 elements and more apart, the
+// instance changes almost always, and sums kept across tiles took the
+// registers of the gathers.
+__device__ __forceinline__ void batch_tile_sums(const BatchTables& T, int part, int slot, int lane, double ei,
+                                                double eh, double ev, double dts, double len, int32_t bad) {
+    ei = batch_warp_sum(ei);
+    eh = batch_warp_sum(eh);
+    ev = batch_warp_sum(ev);
+    const unsigned long long dmin = run_warp_min(ord_bits(dts));
+    const unsigned long long lmin = run_warp_min(ord_bits(len));
+    bad = static_cast<int32_t>(__reduce_or_sync(0xffffffffu, static_cast<unsigned>(bad)));
+    if (lane == 0) {
+        // one writer per partial slot and pass: the reductions (no return
+        // value) add in cycle order without a round trip
+        double* p = T.etile_part + 3 * static_cast<int64_t>(part);
+        Ctl* ctl = T.ctl + slot;
+        atomicAdd(p + 0, ei);
+        atomicAdd(p + 1, eh);
+        atomicAdd(p + 2, ev);
+        atomicMin(&ctl->dts_next, dmin);
+        atomicMin(&ctl->len_min, lmin);
+        if (bad) atomicOr(&ctl->status, bad);
+    }
+}
+
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
