@@ -195,8 +195,8 @@ constexpr int kPatchElems = 64;
 // incidences are pinc[pinc_off[q] .. pinc_off[q + 1]) as (element in patch
 // << 3 | slot), in slot order, and its partial goes to pf[c * pf_pad + q].
 // Node n's force is the sum of its partials nent[nptr[n] .. nptr[n + 1]),
-// in patch order.  iperm maps an element of the caller's numbering to its
-// stored position.
+// in patch order.  iperm (also without patches; null: the same) maps an element
+// of the caller's numbering to its stored position.
 struct PatchArrays {
     const uint32_t* pf_off;
     const uint32_t* pinc_off;

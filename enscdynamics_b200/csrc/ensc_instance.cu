@@ -177,6 +177,38 @@ cudaError_t put(void* block, size_t off, const std::vector<T>& v, cudaStream_t s
 
 }  // namespace
 
+std::vector<int32_t> local_order(int64_t nn, int64_t ne, const uint32_t* conn) {
+    // node groups of 4 (a sector of FP32 force pairs) that a warp's lanes touch
+    // per slot, counted as changes between neighbouring elements
+    auto changes = [&](const int32_t* perm) {
+        int64_t c = 0;
+        for (int64_t s = 1; s < ne; ++s) {
+            const uint32_t* a = conn + 8 * (perm ? perm[s - 1] : s - 1);
+            const uint32_t* b = conn + 8 * (perm ? perm[s] : s);
+            for (int k = 0; k < 8; ++k) c += (a[k] >> 2) != (b[k] >> 2);
+        }
+        return c;
+    };
+    const int64_t own = changes(nullptr);
+    if (own <= 3 * ne) return {};
+    // counting sort by the largest of the four lowest nodes: on layered meshes
+    // the corner of the layer below, so that rows of elements follow rows of nodes
+    std::vector<uint32_t> key(static_cast<size_t>(ne));
+    std::vector<int32_t> at(static_cast<size_t>(nn + 1), 0);
+    for (int64_t e = 0; e < ne; ++e) {
+        uint32_t n[8];
+        std::memcpy(n, conn + 8 * e, sizeof(n));
+        std::nth_element(n, n + 3, n + 8);
+        key[e] = n[3];
+        at[n[3] + 1] += 1;
+    }
+    for (int64_t n = 0; n < nn; ++n) at[n + 1] += at[n];
+    std::vector<int32_t> perm(static_cast<size_t>(ne));
+    for (int64_t e = 0; e < ne; ++e) perm[at[key[e]]++] = static_cast<int32_t>(e);
+    if (5 * changes(perm.data()) > 4 * own) return {};
+    return perm;
+}
+
 std::vector<int32_t> patch_order(int64_t ne, const uint32_t* conn, const double* x0) {
     std::vector<double> cen(static_cast<size_t>(3 * ne));
     double lo[3], hi[3], ext[3];
@@ -349,30 +381,36 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
     }
     h.patch = assembly == ENSC_ASSEMBLY_PATCH;
 
-    // stored element order: the caller's, or patch order
+    // stored element order: the caller's, or one in which neighbours share nodes,
+    // or patch order
     const uint32_t* conn = mesh->conn;
     std::vector<uint32_t> pconn;
-    if (h.patch) {
-        const std::vector<int32_t> perm = patch_order(ne, mesh->conn, mesh->x0);
+    const std::vector<int32_t> perm =
+        h.patch ? patch_order(ne, mesh->conn, mesh->x0) : local_order(nn, ne, mesh->conn);
+    if (!perm.empty()) {
         pconn.resize(static_cast<size_t>(8 * ne));
         std::vector<double> bt(static_cast<size_t>(24 * ne)), vol0(static_cast<size_t>(ne));
+        std::vector<double> jinv(h.bt9 ? static_cast<size_t>(9 * ne) : 0);
         h.iperm.resize(static_cast<size_t>(ne));
         for (int64_t sidx = 0; sidx < ne; ++sidx) {
             const int64_t e = perm[sidx];
             h.iperm[e] = static_cast<int32_t>(sidx);
             std::memcpy(&pconn[8 * sidx], &mesh->conn[8 * e], 8 * sizeof(uint32_t));
             std::memcpy(&bt[24 * sidx], &h.bt[24 * e], 24 * sizeof(double));
+            if (h.bt9) std::memcpy(&jinv[9 * sidx], &h.jinv[9 * e], 9 * sizeof(double));
             vol0[sidx] = h.vol0[e];
         }
         h.bt.swap(bt);
         h.vol0.swap(vol0);
+        if (h.bt9) h.jinv.swap(jinv);
         conn = pconn.data();
-        build_patches(nn, ne, conn, h);
+        if (h.patch) build_patches(nn, ne, conn, h);
     }
 
     h.im.assign(static_cast<size_t>(np), 1.0);
     for (int64_t n = 0; n < nn; ++n) h.im[n] = inv_mass_dof[3 * n];
-    // meshes whose nodes repeat slots: the lists of the node pass
+    // meshes whose nodes repeat slots: the lists of the node pass, of stored
+    // elements in the caller's order
     if (h.clash) {
         h.csr_ptr.assign(static_cast<size_t>(nn + 1), 0);
         for (int64_t i = 0; i < 8 * ne; ++i) h.csr_ptr[conn[i] + 1] += 1;
@@ -381,8 +419,9 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
         std::vector<int64_t> fill(h.csr_ptr.begin(), h.csr_ptr.end() - 1);
         for (int k = 0; k < 8; ++k)
             for (int64_t e = 0; e < ne; ++e) {
-                const uint32_t n = conn[8 * e + k];
-                h.csr_ent[fill[n]++] = (static_cast<uint32_t>(e) << 3) | static_cast<uint32_t>(k);
+                const uint32_t n = mesh->conn[8 * e + k];
+                const uint32_t at = static_cast<uint32_t>(perm.empty() ? e : h.iperm[e]);
+                h.csr_ent[fill[n]++] = (at << 3) | static_cast<uint32_t>(k);
             }
         // at most 8 elements at every node: each entry of a node's list gets its own
         // row of the force array, so that the hand-off and its sums stay those of
@@ -432,8 +471,8 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
     h.size[P::MERGE] = h.merge.size();
     h.size[P::CPTR] = listed ? static_cast<size_t>(nn + 1) * sizeof(int64_t) : 0;
     h.size[P::CENT] = listed ? static_cast<size_t>(8 * ne) * sizeof(uint32_t) : 0;
+    h.size[P::IPERM] = h.iperm.size() * sizeof(int32_t);
     if (h.patch) {
-        h.size[P::IPERM] = static_cast<size_t>(ne) * sizeof(int32_t);
         h.size[P::PFOFF] = static_cast<size_t>(h.n_patches + 1) * sizeof(uint32_t);
         h.size[P::PINCOFF] = static_cast<size_t>(h.n_pnodes + 1) * sizeof(uint32_t);
         h.size[P::PINC] = static_cast<size_t>(8 * ne) * sizeof(uint16_t);
@@ -472,12 +511,12 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     if (e == cudaSuccess) e = put(block, h.off[P::MERGE], h.merge, st);
     if (e == cudaSuccess) e = put(block, h.off[P::CPTR], h.csr_ptr, st);
     if (e == cudaSuccess) e = put(block, h.off[P::CENT], h.csr_ent, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::IPERM], h.iperm, st);
     std::vector<uint32_t> nptr_pad;
     if (h.patch) {
         // padding nodes have no partials: nptr stays at the total past nn
         nptr_pad.assign(static_cast<size_t>(np + 1), h.nptr.empty() ? 0u : h.nptr.back());
         std::copy(h.nptr.begin(), h.nptr.end(), nptr_pad.begin());
-        if (e == cudaSuccess) e = put(block, h.off[P::IPERM], h.iperm, st);
         if (e == cudaSuccess) e = put(block, h.off[P::PFOFF], h.pf_off, st);
         if (e == cudaSuccess) e = put(block, h.off[P::PINCOFF], h.pinc_off, st);
         if (e == cudaSuccess) e = put(block, h.off[P::PINC], h.pinc, st);
@@ -522,8 +561,8 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
         PA.pf_pad = pad32(h.n_pnodes);
         PA.nptr = reinterpret_cast<uint32_t*>(b + h.off[P::NPTR]);
         PA.nent = reinterpret_cast<uint32_t*>(b + h.off[P::NENT]);
-        PA.iperm = reinterpret_cast<int32_t*>(b + h.off[P::IPERM]);
     }
+    PA.iperm = h.iperm.empty() ? nullptr : reinterpret_cast<int32_t*>(b + h.off[P::IPERM]);
     N = NodeArrays{};
     N.nn = h.nn;
     N.nn_pad = np;

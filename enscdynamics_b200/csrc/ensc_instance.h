@@ -45,10 +45,11 @@ struct InstanceHost {
     std::vector<double> q0, q1, vz_d, x_rows;
     std::vector<float> vz_f;
     std::vector<int16_t> v_lo;
-    // patch assembly (ElemArrays::patch): the stored order of the elements
-    // and the patch tables; all element arrays above are in stored order
+    // element of the caller's numbering -> stored position; empty: the same.  All
+    // element arrays above are in stored order
+    std::vector<int32_t> iperm;
+    // patch assembly: the patch tables
     bool patch = false;
-    std::vector<int32_t> iperm;       // [ne] element of the caller's numbering -> stored position
     std::vector<uint32_t> pf_off;     // [n_patches + 1]
     std::vector<uint32_t> pinc_off;   // [n_pnodes + 1]
     std::vector<uint16_t> pinc;       // [8 ne]
@@ -69,6 +70,14 @@ struct InstanceHost {
 // compute_invMassMatrix does unless the caller supplies them).
 int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool mixed, int assembly,
                      InstanceHost& h, std::string& err);
+
+// Stored order of the slot assembly, as patch_order; empty: the caller's order.
+// Warps gather node records and store forces best where the elements of a tile
+// follow the node numbering.  Where a slot's node leaves its group of 4 from one
+// element to the next in more than 3 of 8 slots (a block's rows: 2.2), the
+// elements are sorted by their nodes; the sorted order is taken where it leaves
+// at most 4/5 of the changes.
+std::vector<int32_t> local_order(int64_t nn, int64_t ne, const uint32_t* conn);
 
 // Stored order of the patch assembly: elements sorted by the Morton key of
 // their centroid's cell on a grid of the smallest element extent per axis,
