@@ -53,6 +53,7 @@ __device__ double fixed_sum_strided(const double* a, int n, int stride) {
 // partials, which accumulate over cycles between folds (the host folds
 // before it reads energies); 2: fold as the initial kinetic energy.
 __global__ void __launch_bounds__(kCtlThreads) k_between(Ctl* ctl, Partials P, int mode) {
+    cycle_kernel_enter();
     if (mode != 0 && (ctl->energy_pending || mode == 2)) {
         const double ei = fixed_sum(P.elem + 0 * P.n_elem_blocks, P.n_elem_blocks);
         const double eh = fixed_sum(P.elem + 1 * P.n_elem_blocks, P.n_elem_blocks);
@@ -103,6 +104,7 @@ __device__ __forceinline__ double element_edge_sq(const ElemArrays& E, const Nod
 // where the total-time clamp may fire; the last block then applies the clamp
 // (begin_exact).
 __global__ void __launch_bounds__(128) k_edge_prepass(ElemArrays E, NodeArrays N, Ctl* ctl) {
+    cycle_kernel_enter();
     if (ctl->done || !ctl->need_exact) return;
     __shared__ unsigned long long red[4];
     double m = DBL_MAX;
@@ -277,6 +279,7 @@ __global__ void k_aos_to_soa(const double* aos, int64_t n, int64_t pad, int64_t 
 // until k_fold_batch.  Each slot's element-pass scalars (dt_i_1, live) go to
 // T.sparam; the edge prepass rewrites them where it decides dt.
 __global__ void k_begin_batch(BatchTables T, int begin) {
+    cycle_kernel_enter();
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= T.counts[2]) return;
     const InstanceDesc& d = T.desc[slot];
@@ -332,6 +335,7 @@ __global__ void __launch_bounds__(kCtlThreads) k_fold_batch(BatchTables T) {
 // Minimum element edge for the instances whose cycle may hit the total-time
 // clamp (see k_edge_prepass), one warp per element tile of T.etile elements.
 __global__ void __launch_bounds__(128) k_edge_prepass_batch(BatchTables T) {
+    cycle_kernel_enter();
     if (*T.exact_count == 0) return;
     const int lane = threadIdx.x & 31;
     const int warp = static_cast<int>((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
@@ -389,16 +393,17 @@ int grid_for(int64_t work, int threads) {
 
 void launch_between_batch(const BatchTables& T, int slots, int mode, cudaStream_t st) {
     if (mode == 1) k_fold_batch<<<slots, kCtlThreads, 0, st>>>(T);
-    k_begin_batch<<<(slots + 127) / 128, 128, 0, st>>>(T, mode == 0 ? 1 : 0);
+    launch_cycle_kernel(k_begin_batch, (slots + 127) / 128, 128, 0, st, T, mode == 0 ? 1 : 0);
 }
 void launch_edge_prepass_batch(const BatchTables& T, int grid, cudaStream_t st) {
-    k_edge_prepass_batch<<<grid, 128, 0, st>>>(T);
+    launch_cycle_kernel(k_edge_prepass_batch, grid, 128, 0, st, T);
 }
 void launch_between(Ctl* ctl, const Partials& P, int mode, cudaStream_t st) {
-    k_between<<<1, kCtlThreads, 0, st>>>(ctl, P, mode);
+    if (mode == 0) launch_cycle_kernel(k_between, 1, 32, 0, st, ctl, P, mode);
+    else k_between<<<1, kCtlThreads, 0, st>>>(ctl, P, mode);
 }
 void launch_edge_prepass(const ElemArrays& E, const NodeArrays& N, Ctl* ctl, int grid, cudaStream_t st) {
-    k_edge_prepass<<<grid, 128, 0, st>>>(E, N, ctl);
+    launch_cycle_kernel(k_edge_prepass, grid, 128, 0, st, E, N, ctl);
 }
 void launch_arm(Ctl* ctl, double step_end, long long max_cycles, cudaStream_t st, double pause) {
     k_arm<<<1, 1, 0, st>>>(ctl, step_end, max_cycles, pause);

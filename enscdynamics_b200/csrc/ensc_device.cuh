@@ -588,6 +588,16 @@ __device__ __forceinline__ NodeParam ld_param(const NodeParam* p) {
     memcpy(&v, w, sizeof(v));
     return v;
 }
+// ---- programmatic launches (launch_cycle_kernel) ----
+// A kernel launched while the one before it still runs waits here until that
+// one has completed and its writes are visible.  Only then may the next be
+// launched, so that what the kernel before the last one wrote can be read
+// ahead of the wait.
+__device__ __forceinline__ void cycle_kernel_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }

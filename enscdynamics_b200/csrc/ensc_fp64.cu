@@ -756,6 +756,7 @@ template <bool PLASTIC, bool BT9>
 __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB)
     k_element_fp64_warp(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
     using L = std::conditional_t<BT9, Fp64Tile9, Fp64Tile24>;
+    cycle_kernel_enter();
     if (ctl->done) return;
     extern __shared__ __align__(128) unsigned char smem[];
     const double dt1 = ctl->dt_i_1;
@@ -1000,6 +1001,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_acceleration(ElemArrays E, Nod
 // MERGE: nodes repeat slots (ElemArrays::rows).
 template <bool MERGE>
 __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_FP64) k_node(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
+    cycle_kernel_enter();
     if (ctl->done) return;
     // stable dt of this cycle (update_minVertex_perMaterial_and_dt :673-679)
     double dt_i;
@@ -1177,6 +1179,7 @@ __global__ void __launch_bounds__(32 * kF64PipeWarps, ENSC_F64_PIPE_MINB) k_elem
     unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
     const uint32_t stage0 = smem_addr(wst);
     const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kF64PipeWarps) * 2 * SB) + 16u * wid;
+    cycle_kernel_enter();
     const int ntiles = T.counts[0];
     const int wstride = static_cast<int>(gridDim.x) * kF64PipeWarps;
     const int w0 = static_cast<int>(blockIdx.x) * kF64PipeWarps + wid;
@@ -1269,6 +1272,7 @@ __global__ void __launch_bounds__(NT, ENSC_NODE_MINB_FP64 * kNodeThreads / NT) k
     const int lane = threadIdx.x & 31;
     const int warp = static_cast<int>((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
     const int nwarps = static_cast<int>((static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5);
+    cycle_kernel_enter();
     const int ntiles = T.counts[1];
     int slot = warp < ntiles ? __ldg(T.ntile_inst + warp) : 0;
     int slot_n = warp + nwarps < ntiles ? __ldg(T.ntile_inst + warp + nwarps) : 0;
@@ -1336,10 +1340,10 @@ void launch_element_fp64(const ElemArrays& E, const NodeArrays& N, const Materia
         constexpr size_t smem = f64_pipe_smem<std::conditional_t<B9, Fp64Tile9, Fp64Tile24>>();
         if (M.plastic) {
             if (init) k_element<true, true, B9, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-            else k_element_fp64_warp<true, B9><<<grid, 32 * kF64PipeWarps, smem, st>>>(E, N, M, ctl, P);
+            else launch_cycle_kernel(k_element_fp64_warp<true, B9>, grid, 32 * kF64PipeWarps, smem, st, E, N, M, ctl, P);
         } else {
             if (init) k_element<false, true, B9, true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl, P);
-            else k_element_fp64_warp<false, B9><<<grid, 32 * kF64PipeWarps, smem, st>>>(E, N, M, ctl, P);
+            else launch_cycle_kernel(k_element_fp64_warp<false, B9>, grid, 32 * kF64PipeWarps, smem, st, E, N, M, ctl, P);
         }
     };
     if (E.bt9) pick(std::true_type{});
@@ -1389,7 +1393,7 @@ static size_t f64_batch_smem(int tile_room) {
     return static_cast<size_t>(kF64PipeWarps) * (2 * (static_cast<size_t>(tile_room) + kBatchTailBytes) + 16);
 }
 void launch_element_batch_fp64(const BatchTables& T, int grid, cudaStream_t st) {
-    k_element_batch_fp64<<<grid, 32 * kF64PipeWarps, f64_batch_smem(T.tile_room), st>>>(T);
+    launch_cycle_kernel(k_element_batch_fp64, grid, 32 * kF64PipeWarps, f64_batch_smem(T.tile_room), st, T);
 }
 void launch_node_batch_fp64(const BatchTables& T, int grid, int threads, cudaStream_t st) {
     if (threads == kNodeThreads / 2) k_node_batch_fp64<kNodeThreads / 2><<<grid, threads, 0, st>>>(T);

@@ -562,11 +562,8 @@ __device__ __forceinline__ void mixed_tile_issue(const void* src, uint32_t dst, 
 template <bool PLASTIC>
 __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
     k_element_mixed_warp(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P) {
-    if (ctl->done) return;
     constexpr uint32_t SB = MixedTile::kBytes;
     extern __shared__ __align__(128) unsigned char smem[];
-    const float dt1 = static_cast<float>(ctl->dt_i_1);
-    const double dt1d = ctl->dt_i_1;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
     const uint32_t stage0 = smem_addr(wst);
@@ -584,6 +581,14 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB)
         }
     }
     __syncwarp();
+    cycle_kernel_enter();  // (the last element pass completed before the kernel before this one began)
+    if (ctl->done) {
+        for (int s = 0; s < 2; ++s)
+            if (w0 + s * wstride < ntiles) mbar_wait_bounded(bar0 + 8 * s, 0);
+        return;
+    }
+    const double dt1d = ctl->dt_i_1;
+    const float dt1 = static_cast<float>(dt1d);
     double e_int = 0.0, e_hg = 0.0, e_vis = 0.0;
     double dts_min = DBL_MAX, len_min = DBL_MAX;
     int32_t bad = 0;
@@ -662,6 +667,7 @@ __device__ __forceinline__ void patch_partials(const PatchArrays& E, const float
 template <bool PLASTIC, bool INIT>
 __global__ void __launch_bounds__(kPatchElems, 8)
     k_element_mixed_patch(ElemArrays E, NodeArrays N, Material M, Ctl* ctl, Partials P, PatchArrays PA) {
+    cycle_kernel_enter();
     if (ctl->done) return;
     extern __shared__ __align__(128) unsigned char smem[];
     const float dt1 = INIT ? 0.f : static_cast<float>(ctl->dt_i_1);
@@ -973,6 +979,7 @@ __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double
 template <bool PATCH>
 __global__ void __launch_bounds__(kNodeThreads, ENSC_NODE_MINB_MIXED) k_node_mixed(ElemArrays E, NodeArrays N, Material M, Ctl* ctl,
                                                              Partials P, PatchArrays PA) {
+    cycle_kernel_enter();
     if (ctl->done) return;
     double dt_i;
     const double dt_i_1 = ctl->dt_i_1;
@@ -1164,6 +1171,7 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB) k_
     unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
     const uint32_t stage0 = smem_addr(wst);
     const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kMixedPipeWarps) * 2 * SB) + 16u * wid;
+    cycle_kernel_enter();
     const int ntiles = T.counts[0];
     const int wstride = static_cast<int>(gridDim.x) * kMixedPipeWarps;
     const int w0 = static_cast<int>(blockIdx.x) * kMixedPipeWarps + wid;
@@ -1239,6 +1247,7 @@ __global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTab
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint32_t stage0 = smem_addr(smem);
     const uint32_t bar0 = stage0 + 2 * SB;
+    cycle_kernel_enter();
     const int64_t ntiles = T.counts[0];
     const int64_t gstride = gridDim.x;
     if (tid == 0) {
@@ -1325,6 +1334,7 @@ __global__ void __launch_bounds__(NT, ENSC_NODE_BATCH_MINB_MIXED * kNodeThreads 
     const int lane = threadIdx.x & 31;
     const int warp = static_cast<int>((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
     const int nwarps = static_cast<int>((static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5);
+    cycle_kernel_enter();
     const int ntiles = T.counts[1];
     int slot = warp < ntiles ? __ldg(T.ntile_inst + warp) : 0;
     int slot_n = warp + nwarps < ntiles ? __ldg(T.ntile_inst + warp + nwarps) : 0;
@@ -1387,10 +1397,10 @@ void launch_element_mixed(const ElemArrays& E, const NodeArrays& N, const Materi
         }
     } else if (M.plastic) {
         if (init) k_element_mixed_init<true><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl);
-        else k_element_mixed_warp<true><<<grid, 32 * kMixedPipeWarps, kMixedPipeSmem, st>>>(E, N, M, ctl, P);
+        else launch_cycle_kernel(k_element_mixed_warp<true>, grid, 32 * kMixedPipeWarps, kMixedPipeSmem, st, E, N, M, ctl, P);
     } else {
         if (init) k_element_mixed_init<false><<<grid, kElemThreads, 0, st>>>(E, N, M, ctl);
-        else k_element_mixed_warp<false><<<grid, 32 * kMixedPipeWarps, kMixedPipeSmem, st>>>(E, N, M, ctl, P);
+        else launch_cycle_kernel(k_element_mixed_warp<false>, grid, 32 * kMixedPipeWarps, kMixedPipeSmem, st, E, N, M, ctl, P);
     }
 }
 
@@ -1437,8 +1447,8 @@ int occupancy_node_mixed() {
 
 
 void launch_element_batch_mixed(const BatchTables& T, int grid, bool patch, cudaStream_t st) {
-    if (patch) k_element_batch_patch<<<grid, kPatchElems, kBatchPatchSmem, st>>>(T);
-    else k_element_batch_mixed<<<grid, 32 * kMixedPipeWarps, kBatchMixedSmem, st>>>(T);
+    if (patch) launch_cycle_kernel(k_element_batch_patch, grid, kPatchElems, kBatchPatchSmem, st, T);
+    else launch_cycle_kernel(k_element_batch_mixed, grid, 32 * kMixedPipeWarps, kBatchMixedSmem, st, T);
 }
 void launch_node_batch_mixed(const BatchTables& T, int grid, int threads, bool patch, cudaStream_t st) {
     if (patch) {
