@@ -45,16 +45,50 @@ __device__ double fixed_sum_strided(const double* a, int n, int stride) {
     return r;
 }
 
-// mode 0: the first half of update_minVertex_perMaterial_and_dt for the
-// next cycle: rotate dt_i_1 <- dt_i, advance time (computeSate :775-780) and
-// fix dt_i_1 unless the total-time clamp (:682-685) could fire, which needs
-// this cycle's minimum element edge first (the edge prepass).
+// A warp's view of a control block: all of it in one trip to L2, scalar work on
+// the copy by lane 0, and one trip back.  Read field by field, between the
+// branches that need them, the same work took 7.7 us of a batch's cycle on
+// B200 (2.9 us this way).
+constexpr int kCtlWords = sizeof(Ctl) / 8;
+static_assert(sizeof(Ctl) % 8 == 0 && kCtlWords <= 32, "a control block is one word per lane");
+struct CtlCopy {
+    union {
+        Ctl c;
+        unsigned long long w[kCtlWords];
+    };
+    __device__ CtlCopy() {}
+    __device__ void load(const Ctl* g, int lane) {
+        if (lane < kCtlWords) w[lane] = reinterpret_cast<const unsigned long long*>(g)[lane];
+        __syncwarp();
+    }
+    __device__ void store(Ctl* g, int lane) {
+        __syncwarp();
+        if (lane < kCtlWords) reinterpret_cast<unsigned long long*>(g)[lane] = w[lane];
+    }
+};
+
+// The first half of update_minVertex_perMaterial_and_dt for the next cycle:
+// rotate dt_i_1 <- dt_i, advance time (computeSate :775-780) and fix dt_i_1
+// unless the total-time clamp (:682-685) could fire, which needs this cycle's
+// minimum element edge first (the edge prepass).  One warp.
+__global__ void k_begin(Ctl* ctl) {
+    cycle_kernel_enter();
+    __shared__ CtlCopy s;
+    s.load(ctl, threadIdx.x);
+    if (s.c.done) return;
+    __syncwarp();
+    if (threadIdx.x == 0) {
+        if (cycle_stops(&s.c, s.c.status)) s.c.done = 1;
+        else cycle_begin(&s.c);
+    }
+    s.store(ctl, threadIdx.x);
+}
+
 // mode 1: fold the energy partials into the control block and clear the work
 // partials, which accumulate over cycles between folds (the host folds
 // before it reads energies); 2: fold as the initial kinetic energy.
 __global__ void __launch_bounds__(kCtlThreads) k_between(Ctl* ctl, Partials P, int mode) {
-    cycle_kernel_enter();
-    if (mode != 0 && (ctl->energy_pending || mode == 2)) {
+    if (ctl->energy_pending || mode == 2) {
         const double ei = fixed_sum(P.elem + 0 * P.n_elem_blocks, P.n_elem_blocks);
         const double eh = fixed_sum(P.elem + 1 * P.n_elem_blocks, P.n_elem_blocks);
         const double ev = fixed_sum(P.elem + 2 * P.n_elem_blocks, P.n_elem_blocks);
@@ -76,13 +110,6 @@ __global__ void __launch_bounds__(kCtlThreads) k_between(Ctl* ctl, Partials P, i
         for (int i = threadIdx.x; i < 3 * P.n_elem_blocks; i += kCtlThreads) P.elem[i] = 0.0;
         for (int i = threadIdx.x; i < P.n_node_blocks; i += kCtlThreads) P.node[P.n_node_blocks + i] = 0.0;
     }
-    if (mode != 0 || threadIdx.x != 0 || ctl->done) return;
-    if (ctl->status || !(ctl->time < ctl->step_end) || ctl->cycles_done >= ctl->cycles_target ||
-        !(ctl->time < ctl->pause_time)) {
-        ctl->done = 1;
-        return;
-    }
-    cycle_begin(ctl);
 }
 
 // Minimum squared edge of element e from the current coordinates.
@@ -278,27 +305,34 @@ __global__ void k_aos_to_soa(const double* aos, int64_t n, int64_t pad, int64_t 
 // the edge prepass.  The energy terms stay in the per-tile accumulators
 // until k_fold_batch.  Each slot's element-pass scalars (dt_i_1, live) go to
 // T.sparam; the edge prepass rewrites them where it decides dt.
-__global__ void k_begin_batch(BatchTables T, int begin) {
+__global__ void __launch_bounds__(128) k_begin_batch(BatchTables T, int begin) {
+    // one warp per slot; the tables stay as they are while a batch steps
+    __shared__ CtlCopy copies[4];
+    const int lane = threadIdx.x & 31, slot = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const bool used = slot < T.counts[2];
+    const int active = used ? T.desc[slot].active : 0;
     cycle_kernel_enter();
-    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= T.counts[2]) return;
-    const InstanceDesc& d = T.desc[slot];
+    if (!used) return;
     StageHdr h{0.0, 0, 0};
-    if (d.active) {
-        Ctl* ctl = d.ctl;
-        if (!ctl->done) {
-            if (ctl->status || !(ctl->time < ctl->step_end) || ctl->cycles_done >= ctl->cycles_target ||
-                !(ctl->time < ctl->pause_time)) {
-                ctl->done = 1;
-            } else if (begin) {
-                cycle_begin(ctl);
-                if (ctl->need_exact) atomicAdd(T.exact_count, 1);
-                h.dt1 = ctl->dt_i_1;
-                h.live = 1;
+    if (active) {
+        CtlCopy& s = copies[threadIdx.x >> 5];
+        s.load(T.ctl + slot, lane);
+        if (!s.c.done) {
+            __syncwarp();
+            if (lane == 0) {
+                if (cycle_stops(&s.c, s.c.status)) {
+                    s.c.done = 1;
+                } else if (begin) {
+                    cycle_begin(&s.c);
+                    if (s.c.need_exact) atomicAdd(T.exact_count, 1);
+                    h.dt1 = s.c.dt_i_1;
+                    h.live = 1;
+                }
             }
+            s.store(T.ctl + slot, lane);
         }
     }
-    T.sparam[slot] = h;
+    if (lane == 0) T.sparam[slot] = h;
 }
 
 // Folds an instance's tile accumulators into its control block (one block
@@ -393,13 +427,13 @@ int grid_for(int64_t work, int threads) {
 
 void launch_between_batch(const BatchTables& T, int slots, int mode, cudaStream_t st) {
     if (mode == 1) k_fold_batch<<<slots, kCtlThreads, 0, st>>>(T);
-    launch_cycle_kernel(k_begin_batch, (slots + 127) / 128, 128, 0, st, T, mode == 0 ? 1 : 0);
+    launch_cycle_kernel(k_begin_batch, (slots + 3) / 4, 128, 0, st, T, mode == 0 ? 1 : 0);
 }
 void launch_edge_prepass_batch(const BatchTables& T, int grid, cudaStream_t st) {
     launch_cycle_kernel(k_edge_prepass_batch, grid, 128, 0, st, T);
 }
 void launch_between(Ctl* ctl, const Partials& P, int mode, cudaStream_t st) {
-    if (mode == 0) launch_cycle_kernel(k_between, 1, 32, 0, st, ctl, P, mode);
+    if (mode == 0) launch_cycle_kernel(k_begin, 1, 32, 0, st, ctl);
     else k_between<<<1, kCtlThreads, 0, st>>>(ctl, P, mode);
 }
 void launch_edge_prepass(const ElemArrays& E, const NodeArrays& N, Ctl* ctl, int grid, cudaStream_t st) {

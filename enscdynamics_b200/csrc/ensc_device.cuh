@@ -618,26 +618,29 @@ __device__ __forceinline__ T ldin(const T* p) {
 // edge minimum is read through L2.
 __device__ inline void node_params_slot(const BatchTables& T, int slot) {
     const InstanceDesc& d = T.desc[slot];
+    Ctl* ctl = T.ctl + slot;
     NodeParam p{0.0, 0.0, 1.0, 0, 0};
-    Ctl* ctl = d.ctl;
-    if (d.active && !ctl->done) {
-        double dt_i;
-        const int dt_final = ctl->dt_final;
-        if (dt_final) {
-            dt_i = ctl->dt_i;
-        } else {
-            double dd = __longlong_as_double(static_cast<long long>(__ldcg(&ctl->len_min))) / ctl->wos;
-            const double tmp = ctl->dts_cur;
-            dd = dd < tmp ? dd : tmp;
-            dt_i = dd * ctl->factor;
+    // all that it may need at once, not load after branch
+    const int active = d.active, gravity = d.M.gravity_on && d.M.amp_n > 0;
+    const int done = ctl->done, dt_final = ctl->dt_final;
+    const double len = __longlong_as_double(static_cast<long long>(__ldcg(&ctl->len_min)));
+    const double wos = ctl->wos, dts = ctl->dts_cur, factor = ctl->factor, time = ctl->time, fixed = ctl->dt_i;
+    const double dt_i_1 = ctl->dt_i_1;
+    const long long cycles = ctl->cycles_done;
+    if (active && !done) {
+        double dt_i = fixed;
+        if (!dt_final) {
+            double dd = len / wos;
+            dd = dd < dts ? dd : dts;
+            dt_i = dd * factor;
         }
         if (!(dt_i > 0.0) || !isfinite(dt_i)) atomicOr(&ctl->status, ST_BAD_DT);
         if (!dt_final) ctl->dt_i = dt_i;
-        ctl->cycles_done += 1;
+        ctl->cycles_done = cycles + 1;
         ctl->energy_pending = 1;
         p.dt_i = dt_i;
-        p.dt_i_1 = ctl->dt_i_1;
-        p.amp = (d.M.gravity_on && d.M.amp_n > 0) ? gravity_amplitude(d.M.amp, d.M.amp_n, ctl->time, dt_i) : 1.0;
+        p.dt_i_1 = dt_i_1;
+        p.amp = gravity ? gravity_amplitude(d.M.amp, d.M.amp_n, time, dt_i) : 1.0;
         p.live = 1;
     }
     T.nparam[slot] = p;
