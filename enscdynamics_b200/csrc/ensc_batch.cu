@@ -646,21 +646,12 @@ int ensc_batch_set_bcs(ensc_batch* b, int32_t slot, const int8_t* dof_code, cons
     DevGuard dg(b->device);
     Slot& sl = b->inst[slot];
     cudaStream_t st = slot_stream(b, sl);
-    std::vector<uint8_t> bc(static_cast<size_t>(sl.nn_pad), 0);
-    std::vector<double> bcv(static_cast<size_t>(3 * sl.nn_pad), 0.0);
-    if (dof_code) {
-        for (int64_t n = 0; n < sl.nn; ++n) {
-            uint32_t packed = 0;
-            for (int c = 0; c < 3; ++c) {
-                const uint32_t cc = static_cast<uint32_t>(dof_code[3 * n + c]) & 3u;
-                packed |= cc << (2 * c);
-                if ((cc & ENSC_BC_VELOCITY) && dof_value) bcv[c * sl.nn_pad + n] = dof_value[3 * n + c];
-            }
-            bc[n] = static_cast<uint8_t>(packed);
-        }
-    }
+    std::vector<uint8_t> bc;
+    std::vector<double> bcv;
+    ensc::pack_bcs(sl.nn, sl.nn_pad, dof_code, dof_value, bc, bcv);
     BCK(b, cudaMemcpyAsync(const_cast<uint8_t*>(sl.N.bc), bc.data(), bc.size(), cudaMemcpyHostToDevice, st));
-    BCK(b, cudaMemcpyAsync(const_cast<double*>(sl.N.bcv), bcv.data(), bcv.size() * 8, cudaMemcpyHostToDevice, st));
+    if (!bcv.empty())
+        BCK(b, cudaMemcpyAsync(const_cast<double*>(sl.N.bcv), bcv.data(), bcv.size() * 8, cudaMemcpyHostToDevice, st));
     ensc::launch_apply_bc_v(sl.N, is_mixed(b), st);
     if (!sl.kinetic0_done) {
         ensc::Partials P{};

@@ -378,21 +378,11 @@ int ensc_create(const ensc_mesh_desc* mesh, const ensc_material* mat, const ensc
 int ensc_set_bcs(ensc_handle* h, const int8_t* dof_code, const double* dof_value) {
     if (!h) return ENSC_ERR_ARG;
     DevGuard dg(h->device);
-    std::vector<uint8_t> bc(static_cast<size_t>(h->nn_pad), 0);
-    std::vector<double> bcv(static_cast<size_t>(3 * h->nn_pad), 0.0);
-    if (dof_code) {
-        for (int64_t n = 0; n < h->nn; ++n) {
-            uint32_t packed = 0;
-            for (int c = 0; c < 3; ++c) {
-                const uint32_t cc = static_cast<uint32_t>(dof_code[3 * n + c]) & 3u;
-                packed |= cc << (2 * c);
-                if ((cc & ENSC_BC_VELOCITY) && dof_value) bcv[c * h->nn_pad + n] = dof_value[3 * n + c];
-            }
-            bc[n] = static_cast<uint8_t>(packed);
-        }
-    }
+    std::vector<uint8_t> bc;
+    std::vector<double> bcv;
+    ensc::pack_bcs(h->nn, h->nn_pad, dof_code, dof_value, bc, bcv);
     int rc = upload(h, const_cast<uint8_t*>(h->N.bc), bc);
-    if (!rc) rc = upload(h, const_cast<double*>(h->N.bcv), bcv);
+    if (!rc && !bcv.empty()) rc = upload(h, const_cast<double*>(h->N.bcv), bcv);
     if (rc) return rc;
     ensc::launch_apply_bc_v(h->N, mixed(h), h->stream);
     if (!h->kinetic0_done) {

@@ -1,6 +1,8 @@
 // Host-side preparation and device layout of one solver instance.
 #include "ensc_instance.h"
 
+#include "ensc_kernels.h"
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -142,9 +144,6 @@ void form_device_rows(InstanceHost& h, const uint32_t* conn) {
     for (int64_t n = 0; n < h.nn; ++n)
         for (int c = 0; c < 3; ++c) h.q0[4 * n + c] = h.x0[3 * n + c];
     if (h.mixed) {
-        h.x_rows.assign(static_cast<size_t>(3 * np), 0.0);
-        for (int64_t n = 0; n < h.nn; ++n)
-            for (int c = 0; c < 3; ++c) h.x_rows[c * np + n] = h.x0[3 * n + c];
         if (h.v0) {
             h.vz_f.assign(static_cast<size_t>(np), 0.f);
             h.v_lo.assign(static_cast<size_t>(3 * np), 0);
@@ -491,6 +490,22 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
     return ENSC_OK;
 }
 
+void pack_bcs(int64_t nn, int64_t nn_pad, const int8_t* dof_code, const double* dof_value, std::vector<uint8_t>& bc,
+              std::vector<double>& bcv) {
+    bc.assign(static_cast<size_t>(nn_pad), 0);
+    bcv.clear();
+    if (!dof_code) return;
+    for (int64_t n = 0; n < nn; ++n) {
+        uint32_t packed = 0;
+        for (int c = 0; c < 3; ++c) packed |= (static_cast<uint32_t>(dof_code[3 * n + c]) & 3u) << (2 * c);
+        bc[n] = static_cast<uint8_t>(packed);
+        if (!(packed & 0x2au)) continue;  // ENSC_BC_VELOCITY of any component
+        if (bcv.empty()) bcv.assign(static_cast<size_t>(3 * nn_pad), 0.0);
+        for (int c = 0; c < 3; ++c)
+            if (((packed >> (2 * c)) & ENSC_BC_VELOCITY) && dof_value) bcv[c * nn_pad + n] = dof_value[3 * n + c];
+    }
+}
+
 int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArrays& E, NodeArrays& N,
                     PatchArrays& PA, std::string& err) {
     using P = InstanceHost::Piece;
@@ -502,8 +517,7 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
                               static_cast<size_t>(ep / 32), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = put(block, h.off[P::IM], h.im, st);
     if (e == cudaSuccess) e = put(block, h.off[P::X], h.q0, st);
-    // mixed: the u rows hold the reference position x - u, x0 at the start
-    if (e == cudaSuccess) e = put(block, h.off[P::U], h.mixed ? h.x_rows : h.q1, st);
+    if (e == cudaSuccess) e = put(block, h.off[P::U], h.q1, st);
     if (e == cudaSuccess) e = put(block, h.off[P::V], h.vz_d, st);
     if (e == cudaSuccess) e = put(block, h.off[P::V], h.vz_f, st);
     if (e == cudaSuccess) e = put(block, h.off[P::V] + np * sizeof(float), h.v_lo, st);
@@ -522,11 +536,6 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
         if (e == cudaSuccess) e = put(block, h.off[P::PINC], h.pinc, st);
         if (e == cudaSuccess) e = put(block, h.off[P::NPTR], nptr_pad, st);
         if (e == cudaSuccess) e = put(block, h.off[P::NENT], h.nent, st);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-        err = std::string("instance upload: ") + cudaGetErrorString(e);
-        return ENSC_ERR_CUDA;
     }
     E = ElemArrays{};
     E.ne = h.ne;
@@ -577,6 +586,16 @@ int instance_upload(const InstanceHost& h, void* block, cudaStream_t st, ElemArr
     N.csr_ent = listed ? reinterpret_cast<uint32_t*>(b + h.off[P::CENT]) : nullptr;
     N.merge = h.merge.empty() ? nullptr : reinterpret_cast<uint8_t*>(b + h.off[P::MERGE]);
     N.rf = reinterpret_cast<double*>(b + h.off[P::RF]);
+    if (e == cudaSuccess && h.mixed) {
+        // the u rows hold the reference position x - u: x - 0, from the records
+        launch_reflect_rows(N, st);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        err = std::string("instance upload: ") + cudaGetErrorString(e);
+        return ENSC_ERR_CUDA;
+    }
     return ENSC_OK;
 }
 

@@ -37,12 +37,11 @@ struct InstanceHost {
     // constant part of every element tile (connectivity, geometry, V0 and its
     // roots), const_bytes each; the node records (NodeArrays) -- FP64: q0, q1 and
     // vz; mixed: q0 with two velocities packed in, vz and the 16-bit residual rows
-    // [3][nn_pad], and the reference position rows x0 [3][nn_pad] (what only holds
-    // velocities stays empty when the mesh has none)
+    // [3][nn_pad] (what only holds velocities stays empty when the mesh has none)
     int32_t tile_bytes = 0, const_bytes = 0;
     bool bt9 = false;                 // FP64: 9 numbers per element give B0^T bit for bit
     std::vector<unsigned char> tiles;
-    std::vector<double> q0, q1, vz_d, x_rows;
+    std::vector<double> q0, q1, vz_d;
     std::vector<float> vz_f;
     std::vector<int16_t> v_lo;
     // element of the caller's numbering -> stored position; empty: the same.  All
@@ -88,6 +87,12 @@ std::vector<int32_t> patch_order(int64_t ne, const uint32_t* conn, const double*
 // Builds the patch tables of h (pf_off, pinc_off, pinc, nptr, nent) for the
 // stored connectivity conn [ne][8].
 void build_patches(int64_t nn, int64_t ne, const uint32_t* conn, InstanceHost& h);
+
+// The device form of a call's boundary conditions: bc[n] packs the codes of node
+// n's components, 2 bits each; bcv[3][nn_pad] holds the prescribed velocities and
+// stays empty when no component has one (they are read only where one has).
+void pack_bcs(int64_t nn, int64_t nn_pad, const int8_t* dof_code, const double* dof_value, std::vector<uint8_t>& bc,
+              std::vector<double>& bcv);
 
 // Copies the instance into `block` (h.bytes bytes, 256-byte aligned) on
 // stream `st`, waits for the copies, and fills the array descriptors (PA
