@@ -105,13 +105,15 @@ T* tile_entry(InstanceHost& h, int64_t e, uint32_t off) {
 
 // What the upload copies as it is (InstanceHost::tiles ...): the element
 // geometry in the precision's device form, x0 and v0 as rows.  The caller's x0
-// and v0 are not read after this.  conn: in stored order, as bt and vol0.
-void form_device_rows(InstanceHost& h, const uint32_t* conn) {
+// and v0 are not read after this.  conn, bt, jinv and vol0 are in the caller's
+// order; perm: the element at each stored position (empty: the same).
+void form_device_rows(InstanceHost& h, const uint32_t* conn, const std::vector<int32_t>& perm) {
     const int64_t np = h.nn_pad;
     h.tiles.assign(static_cast<size_t>(h.ne_pad / 32) * h.const_bytes, 0);
     for (int64_t el = 0; el < h.ne; ++el) {
-        for (int k = 0; k < 8; ++k) tile_entry<uint32_t>(h, el, MixedTile::kConn)[32 * k] = conn[8 * el + k];
-        const double v0 = h.vol0[el], cb = std::cbrt(v0);
+        const int64_t e = perm.empty() ? el : perm[el];
+        for (int k = 0; k < 8; ++k) tile_entry<uint32_t>(h, el, MixedTile::kConn)[32 * k] = conn[8 * e + k];
+        const double v0 = h.vol0[e], cb = std::cbrt(v0);
         if (h.mixed) {
             // corner signs s_j of the reference hexahedron (Element_HexN8.cpp:49-91)
             static const double kCorner[8][3] = {{-1, -1, -1}, {1, -1, -1}, {1, 1, -1}, {-1, 1, -1},
@@ -120,7 +122,7 @@ void form_device_rows(InstanceHost& h, const uint32_t* conn) {
             for (int c = 0; c < 3; ++c)
                 for (int m = 0; m < 3; ++m) {
                     double v = 0.0;
-                    for (int j = 0; j < 8; ++j) v += h.bt[24 * el + 3 * j + c] * kCorner[j][m];
+                    for (int j = 0; j < 8; ++j) v += h.bt[24 * e + 3 * j + c] * kCorner[j][m];
                     const float hi = static_cast<float>(v);
                     a[32 * (3 * c + m)] = hi;
                     a[32 * (9 + 3 * c + m)] = static_cast<float>(v - static_cast<double>(hi));
@@ -128,7 +130,7 @@ void form_device_rows(InstanceHost& h, const uint32_t* conn) {
             *tile_entry<double>(h, el, MixedTile::kVol0) = v0;
             *tile_entry<float>(h, el, MixedTile::kCb) = static_cast<float>(cb);
         } else {
-            const double* src = h.bt9 ? &h.jinv[9 * el] : &h.bt[24 * el];
+            const double* src = h.bt9 ? &h.jinv[9 * e] : &h.bt[24 * e];
             double* t = tile_entry<double>(h, el, Fp64Tile9::kBt);
             for (int i = 0; i < (h.bt9 ? 9 : 24); ++i) t[32 * i] = src[i];
             double* c = tile_entry<double>(h, el, h.bt9 ? Fp64Tile9::kVol0 : Fp64Tile24::kVol0);
@@ -382,28 +384,17 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
 
     // stored element order: the caller's, or one in which neighbours share nodes,
     // or patch order
-    const uint32_t* conn = mesh->conn;
-    std::vector<uint32_t> pconn;
     const std::vector<int32_t> perm =
         h.patch ? patch_order(ne, mesh->conn, mesh->x0) : local_order(nn, ne, mesh->conn);
     if (!perm.empty()) {
-        pconn.resize(static_cast<size_t>(8 * ne));
-        std::vector<double> bt(static_cast<size_t>(24 * ne)), vol0(static_cast<size_t>(ne));
-        std::vector<double> jinv(h.bt9 ? static_cast<size_t>(9 * ne) : 0);
         h.iperm.resize(static_cast<size_t>(ne));
-        for (int64_t sidx = 0; sidx < ne; ++sidx) {
-            const int64_t e = perm[sidx];
-            h.iperm[e] = static_cast<int32_t>(sidx);
-            std::memcpy(&pconn[8 * sidx], &mesh->conn[8 * e], 8 * sizeof(uint32_t));
-            std::memcpy(&bt[24 * sidx], &h.bt[24 * e], 24 * sizeof(double));
-            if (h.bt9) std::memcpy(&jinv[9 * sidx], &h.jinv[9 * e], 9 * sizeof(double));
-            vol0[sidx] = h.vol0[e];
-        }
-        h.bt.swap(bt);
-        h.vol0.swap(vol0);
-        if (h.bt9) h.jinv.swap(jinv);
-        conn = pconn.data();
-        if (h.patch) build_patches(nn, ne, conn, h);
+        for (int64_t sidx = 0; sidx < ne; ++sidx) h.iperm[perm[sidx]] = static_cast<int32_t>(sidx);
+    }
+    if (h.patch) {
+        std::vector<uint32_t> conn(static_cast<size_t>(8 * ne));
+        for (int64_t sidx = 0; sidx < ne; ++sidx)
+            std::memcpy(&conn[8 * sidx], &mesh->conn[8 * static_cast<int64_t>(perm[sidx])], 8 * sizeof(uint32_t));
+        build_patches(nn, ne, conn.data(), h);
     }
 
     h.im.assign(static_cast<size_t>(np), 1.0);
@@ -412,7 +403,7 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
     // elements in the caller's order
     if (h.clash) {
         h.csr_ptr.assign(static_cast<size_t>(nn + 1), 0);
-        for (int64_t i = 0; i < 8 * ne; ++i) h.csr_ptr[conn[i] + 1] += 1;
+        for (int64_t i = 0; i < 8 * ne; ++i) h.csr_ptr[mesh->conn[i] + 1] += 1;
         for (int64_t n = 0; n < nn; ++n) h.csr_ptr[n + 1] += h.csr_ptr[n];
         h.csr_ent.resize(static_cast<size_t>(8 * ne));
         std::vector<int64_t> fill(h.csr_ptr.begin(), h.csr_ptr.end() - 1);
@@ -486,7 +477,7 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
         total += (h.size[i] + 255) / 256 * 256;
     }
     h.bytes = total;
-    form_device_rows(h, conn);
+    form_device_rows(h, mesh->conn, perm);
     return ENSC_OK;
 }
 

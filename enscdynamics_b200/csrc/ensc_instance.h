@@ -19,6 +19,7 @@ namespace ensc {
 struct InstanceHost {
     int64_t nn = 0, ne = 0, nn_pad = 0, ne_pad = 0;
     bool mixed = false, plastic = false, clash = false;
+    // (bt, jinv and vol0 in the caller's order, and only until the tiles hold them)
     std::vector<double> bt;           // [ne][24] row-major B0^T
     std::vector<double> jinv;         // [ne][9] J^-1 / 8 where bt9
     std::vector<double> vol0;         // [ne] V0
@@ -44,8 +45,8 @@ struct InstanceHost {
     std::vector<double> q0, q1, vz_d;
     std::vector<float> vz_f;
     std::vector<int16_t> v_lo;
-    // element of the caller's numbering -> stored position; empty: the same.  All
-    // element arrays above are in stored order
+    // element of the caller's numbering -> stored position; empty: the same.
+    // Tiles, rows and lists are of stored elements
     std::vector<int32_t> iperm;
     // patch assembly: the patch tables
     bool patch = false;
