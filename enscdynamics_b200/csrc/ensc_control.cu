@@ -299,8 +299,8 @@ __global__ void k_aos_to_soa(const double* aos, int64_t n, int64_t pad, int64_t 
 }
 
 // ---- batched instances ---------------------------------------------------------
-// Begins every instance's next cycle exactly as k_between does for one
-// instance (one thread per instance slot), after marking instances that have
+// Begins every instance's next cycle exactly as k_begin does for one
+// instance (one warp per instance slot), after marking instances that have
 // reached their limits as done, and counts the instances whose cycle needs
 // the edge prepass.  The energy terms stay in the per-tile accumulators
 // until k_fold_batch.  Each slot's element-pass scalars (dt_i_1, live) go to

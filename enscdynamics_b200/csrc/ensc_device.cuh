@@ -16,8 +16,9 @@
 //     fe                             element nodal forces of the current cycle
 //                                    (the element -> node hand-off, scratch):
 //                                    by node and local slot when no node
-//                                    repeats a slot, else by element; per slot a
-//                                    row of (fx, fy) pairs, after the eight of
+//                                    repeats a slot, by node and row (rows) when
+//                                    none has more than 8 elements, else by
+//                                    element; per slot a row of (fx, fy) pairs, after the eight of
 //                                    them a row of fz per slot (force_xy, force_z)
 //   node arrays, length nn (stride nn_pad), in 32-byte records that one load
 //   brings in (rec 1):

@@ -5,8 +5,9 @@
 //
 // One cycle (exDyna3D::run loop body, Explicit3D/source/exDyna3D.cpp:86-100)
 // is the kernel sequence
-//   between  -> [edge_prepass -> begin_exact] -> element -> node
-// launched inside a CUDA graph; see ensc_capi.cu for the orchestration.
+//   begin  -> [edge_prepass -> begin_exact] -> element -> node
+// launched inside a CUDA graph, or the phases of a resident run
+// (ensc_run.cuh); see ensc_capi.cu for the orchestration.
 #include "ensc_device.cuh"
 #include "ensc_kernels.h"
 #include "ensc_run.cuh"
@@ -1077,7 +1078,7 @@ struct RunFp64 {
     }
     // W nodes per thread, their rows loaded ahead of the forces; a thread's
     // further nodes (meshes with more than 2 per thread) load both together.
-    // Meshes whose nodes repeat slots read their lists node by node.
+    // Meshes with node lists read them node by node.
     template <int W>
     struct Nodes {
         NodeRowsF64<W> rows;

@@ -175,11 +175,9 @@ int batch_element_tile(bool patch);
 int batch_node_tile(bool mixed_precision);
 void launch_between_batch(const BatchTables& T, int slots, int mode, cudaStream_t st);
 void launch_edge_prepass_batch(const BatchTables& T, int grid, cudaStream_t st);
-// per-instance node-pass scalars (and the control-block updates of the node
-// pass); runs between the element and node passes
 
 // control (ensc_control.cu, built with -fmad=false)
-// mode 0: fold energy partials + begin next cycle; 1: fold only; 2: fold as initial KE
+// mode 0: begin the next cycle; 1: fold the energy partials; 2: fold them as the initial kinetic energy
 void launch_between(Ctl* ctl, const Partials& P, int mode, cudaStream_t st);
 void launch_edge_prepass(const ElemArrays& E, const NodeArrays& N, Ctl* ctl, int grid, cudaStream_t st);
 // pause: the instance stops after the cycle in which its time reaches pause

@@ -1171,6 +1171,8 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB) k_
     unsigned char* wst = smem + static_cast<size_t>(wid) * 2 * SB;
     const uint32_t stage0 = smem_addr(wst);
     const uint32_t bar0 = smem_addr(smem + static_cast<size_t>(kMixedPipeWarps) * 2 * SB) + 16u * wid;
+    __shared__ SentMinima sent[kMixedPipeWarps];
+    if (lane == 0) sent[wid].slot = -1;
     cycle_kernel_enter();
     const int ntiles = T.counts[0];
     const int wstride = static_cast<int>(gridDim.x) * kMixedPipeWarps;
@@ -1221,7 +1223,7 @@ __global__ void __launch_bounds__(32 * kMixedPipeWarps, ENSC_MIXED_PIPE_MINB) k_
             const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
             batch_issue<MixedTile::kBytes>(T, src, tn + 2 * wstride, ntiles, sb, stage0 + s * SB, bar);
         }
-        if (live) batch_tile_sums(T, t, slot, lane, ei, eh, ev, dts, len, bad);
+        if (live) batch_tile_sums(T, t, slot, lane, ei, eh, ev, dts, len, bad, &sent[wid]);
     }
     if (timed_out && lane == 0) {
         // record the failure on the instance whose tile could not be read and
@@ -1247,6 +1249,8 @@ __global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTab
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint32_t stage0 = smem_addr(smem);
     const uint32_t bar0 = stage0 + 2 * SB;
+    __shared__ SentMinima sent[kPatchElems / 32];
+    if (lane == 0) sent[wid].slot = -1;
     cycle_kernel_enter();
     const int64_t ntiles = T.counts[0];
     const int64_t gstride = gridDim.x;
@@ -1311,7 +1315,7 @@ __global__ void __launch_bounds__(kPatchElems, 8) k_element_batch_patch(BatchTab
             const ETileSrc src = *reinterpret_cast<const ETileSrc*>(tail + kBatchNextOff);
             batch_issue<kPatchStageBytes>(T, src, tn + 2 * gstride, ntiles, sb, stage0 + s * SB, bar);
         }
-        if (live) batch_tile_sums(T, static_cast<int>(t) * NW + wid, slot, lane, ei, eh, ev, dts, len, bad);
+        if (live) batch_tile_sums(T, static_cast<int>(t) * NW + wid, slot, lane, ei, eh, ev, dts, len, bad, &sent[wid]);
     }
     if (timed_out && tid == 0) {
         atomicOr(&T.ctl[T.etile_inst[t]].status, ST_TIMEOUT);

@@ -59,11 +59,20 @@ __device__ __forceinline__ double batch_warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
+// The minima that a warp has sent to an instance's control block in this pass, in
+// shared memory (lane 0's).  All tiles of a large instance would meet at two
+// addresses there: a block of 2,097,152 elements alone in a batch took 326 us a
+// cycle with two atomics per tile.
+struct SentMinima {
+    int32_t slot, pad;
+    unsigned long long dts, len;
+};
 // Reduced per tile: between a warp's tiles, 100,000 elements and more apart, the
 // instance changes almost always, and sums kept across tiles took the
 // registers of the gathers.
 __device__ __forceinline__ void batch_tile_sums(const BatchTables& T, int part, int slot, int lane, double ei,
-                                                double eh, double ev, double dts, double len, int32_t bad) {
+                                                double eh, double ev, double dts, double len, int32_t bad,
+                                                SentMinima* sent = nullptr) {
     ei = batch_warp_sum(ei);
     eh = batch_warp_sum(eh);
     ev = batch_warp_sum(ev);
@@ -78,8 +87,18 @@ __device__ __forceinline__ void batch_tile_sums(const BatchTables& T, int part, 
         atomicAdd(p + 0, ei);
         atomicAdd(p + 1, eh);
         atomicAdd(p + 2, ev);
-        atomicMin(&ctl->dts_next, dmin);
-        atomicMin(&ctl->len_min, lmin);
+        if (sent && sent->slot != slot) {
+            sent->slot = slot;
+            sent->dts = sent->len = kInfBits;
+        }
+        if (!sent || dmin < sent->dts) {
+            atomicMin(&ctl->dts_next, dmin);
+            if (sent) sent->dts = dmin;
+        }
+        if (!sent || lmin < sent->len) {
+            atomicMin(&ctl->len_min, lmin);
+            if (sent) sent->len = lmin;
+        }
         if (bad) atomicOr(&ctl->status, bad);
     }
 }

@@ -377,7 +377,7 @@ int32_t ensc_batch_instances(const ensc_batch* b);
  * the reference has no batched stepper): grid multipliers over one wave of
  * resident blocks of the element and node passes, cycles per graph launch,
  * threads per block of the node pass and elements per thread of the element
- * pass -- zero until the first tuning completes; the autotuner spreads its
+ * pass (1 once tuned) -- zero until the first tuning completes; the autotuner spreads its
  * candidates over the first runs and tunes again when the batch's element
  * count changes four-fold -- and the force assembly of the batch's
  * instances (ENSC_ASSEMBLY_SLOT or _PATCH, fixed at ensc_batch_create:
