@@ -16,8 +16,11 @@
 // arithmetic per element and node is that of the per-phase kernels, and the
 // minima are exact, so the state is bit-identical to theirs.
 //
-// Every wait on the counter is bounded (kStageWaitCycles); when one expires
-// the block raises ST_TIMEOUT and leaves, and so do the others.
+// Every wait on the counter and on a tile's copy is bounded (kStageWaitCycles);
+// when one expires the block raises ST_TIMEOUT and leaves, and so do the others.
+// The hardware barrier of a cluster has no limit of its own: all blocks of a
+// cluster run at the same time, take the same decisions, and hold no wait
+// without a limit between two of its barriers.
 #pragma once
 
 #include "ensc_cycle.cuh"
@@ -201,11 +204,15 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
     }
     __syncthreads();
     if (!sh.go) {
-        // nothing to run: only the limits and `done` change, to the same
-        // values whichever of the old and new ones another block reads
+        // nothing to run, in any block of the launch: only the limits and `done`
+        // change, to the same values whichever of the old and new ones another
+        // block reads
         if (tid == 0 && block == 0) *ctl = sh.c;
         return;
     }
+    // another block's shared memory may be written once that block runs: every
+    // block of a cluster arrives here, and waits before its first such store
+    if (CLUSTER) cluster_arrive();
     bool loaded = true;
     if (mine > 0) {
         const uint32_t bar = smem_addr(&sh.mbar[wid]);
@@ -219,6 +226,7 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
         loaded = mbar_wait_bounded(bar, 0);
         loaded = __all_sync(0xffffffffu, loaded);
     }
+    if (CLUSTER) cluster_wait();
     double e_int = 0.0, e_hg = 0.0, e_vis = 0.0, wext = 0.0;
     const int64_t t0 = static_cast<int64_t>(block) * blockDim.x + tid;
     const int64_t stride = static_cast<int64_t>(nblocks) * blockDim.x;
