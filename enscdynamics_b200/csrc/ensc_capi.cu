@@ -161,6 +161,12 @@ int loads_changed(ensc_handle* h) { return h->graph ? build_graph(h) : ENSC_OK; 
 // Enqueues up to `cycles` cycles of a step call: its first (arm, which sets
 // the call's limits: max_cycles in all) or a later part.
 int enqueue_cycles(ensc_handle* h, int64_t cycles, bool arm, int64_t max_cycles, double step_end, double pause) {
+    // in a stream under capture every launch form refuses, not the graph's alone:
+    // the cycles would be recorded with this call's limits, and none would run
+    cudaStreamCaptureStatus capture;
+    CK(h, cudaStreamIsCapturing(h->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone)
+        return cuda_err(h, "step call", cudaErrorStreamCaptureUnsupported);
     if (h->run.grid) {
         int64_t left = cycles;
         while (left > 0) {

@@ -180,7 +180,8 @@ int ensc_step_until(ensc_handle* h, int64_t max_cycles, double step_end_time, do
                     ensc_step_report* report);
 
 /* Enqueues the same work without waiting (for callers that time the stream
- * themselves); finish with ensc_sync. */
+ * themselves); finish with ensc_sync.  Step calls are refused (ENSC_ERR_CUDA)
+ * while their stream is under capture. */
 int ensc_step_async(ensc_handle* h, int64_t max_cycles, double step_end_time);
 int ensc_sync(ensc_handle* h, ensc_step_report* report);
 
