@@ -153,6 +153,17 @@ int build_graph(ensc_handle* h) {
 // resident): the host looks at the control block between launches.
 constexpr int64_t kRunCycles = 4096;
 
+// Before kernels that fill the partial slots in another way than the cycles
+// before them: folds what those left, and leaves no kinetic energy in slots that
+// the kernels to come may not fill (a resident run fills one per block of its
+// grid, the node pass and the initial sum grid_n of them).
+int settle_energy(ensc_handle* h) {
+    ensc::launch_between(h->ctl, h->P, 1, h->stream);
+    CK(h, cudaGetLastError());
+    CK(h, cudaMemsetAsync(h->P.node, 0, h->P.n_node_blocks * sizeof(double), h->stream));
+    return ENSC_OK;
+}
+
 // The launches that rebuild what a handle steps with after its material or
 // loads changed: the graph carries them by value, a resident run takes them
 // with every launch.
@@ -404,6 +415,7 @@ int ensc_set_bcs(ensc_handle* h, const int8_t* dof_code, const double* dof_value
     if (rc) return rc;
     ensc::launch_apply_bc_v(h->N, mixed(h), h->stream);
     if (!h->kinetic0_done) {
+        if (int rs = settle_energy(h)) return rs;  // cycles may have run before the first conditions
         ensc::launch_kinetic0(h->N, h->P, h->ctl, mixed(h), h->grid_n, h->stream);
         h->kinetic0_done = true;
     }
@@ -712,12 +724,8 @@ int ensc_profile(ensc_handle* h, int64_t max_cycles, double step_end_time, doubl
     }
     cudaEvent_t ev[6];
     for (int i = 0; i < 6; ++i) CK(h, cudaEventCreate(&ev[i]));
-    if (h->run.grid) {
-        // the node pass fills fewer partial slots than a resident run: what
-        // the runs left is folded, and no kinetic energy stays in the others
-        ensc::launch_between(h->ctl, h->P, 1, h->stream);
-        CK(h, cudaMemsetAsync(h->P.node, 0, h->P.n_node_blocks * sizeof(double), h->stream));
-    }
+    if (h->run.grid)
+        if (int rs = settle_energy(h)) return rs;
     ensc::launch_arm(h->ctl, step_end_time, max_cycles, h->stream);
     int rc = ENSC_OK;
     for (int64_t c = 0; c < max_cycles && rc == ENSC_OK; ++c) {
