@@ -191,6 +191,7 @@ int enqueue_cycles(ensc_handle* h, int64_t cycles, bool arm, int64_t max_cycles,
                 // the per-phase kernels need no resident grid
                 cudaGetLastError();
                 h->run = ensc::RunPlan{};
+                if (int rs = settle_energy(h)) return rs;
                 break;
             }
             if (e != cudaSuccess) return cuda_err(h, "resident run", e);
