@@ -1055,6 +1055,7 @@ template <bool PLASTIC>
 struct RunFp64 {
     using L = Fp64Tile9;
     static constexpr uint32_t kTileBytes = L::kBytes;
+    static constexpr bool kKinInUpdate = false;  // velocities are stored as they are computed
     __device__ static const uint32_t* conn(const unsigned char* tile) {
         return reinterpret_cast<const uint32_t*>(tile);
     }

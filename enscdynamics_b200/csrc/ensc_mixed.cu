@@ -790,10 +790,14 @@ __device__ __forceinline__ void listed_forces_mixed(const ElemArrays& E, const N
     }
 }
 
+// The work of a node update: all of it; all but the kinetic energy (a resident run
+// in every cycle); or the kinetic energy of the velocities that the update will
+// form and nothing else (a resident run ahead of its last update).
+enum NodeWork { kNodeAll, kNodeUpdate, kNodeKinetic };
+
 // One node of the mixed node pass where the forces are per element; shared by
-// the single-instance, batched and resident-run kernels (KIN: sum the kinetic
-// energy).
-template <bool KIN = true>
+// the single-instance, batched and resident-run kernels.
+template <NodeWork WORK = kNodeAll>
 __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeArrays& N, const Material& M,
                                                 const double dt_i, const double dt_i_1, const double amp, const int64_t n,
                                                 double& kin, double& wext, int32_t& bad) {
@@ -822,7 +826,7 @@ __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeA
             r = -a;
             a = 0.f;
         }
-        if (cc) N.rf[c * np + n] = static_cast<double>(rf);
+        if (WORK != kNodeKinetic && cc) N.rf[c * np + n] = static_cast<double>(rf);
         float* pv = node_vf(N, c, n);
         int16_t* pl = v_lo_rows(N.v, np) + c * np + n;
         double* px = node_x(N, c, n);
@@ -830,11 +834,12 @@ __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeA
         float vn;
         int16_t vl;
         const double vnd = velocity_update_split(vod, a, im, dt_avg, vn, vl);
+        if (WORK != kNodeUpdate) kin += 0.5 * (vnd * vnd) / im;
+        if (WORK == kNodeKinetic) continue;
         *pv = vn;
         *pl = vl;
         *px += dt_i * vnd;
         wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
-        if (KIN) kin += 0.5 * (vnd * vnd) / im;
         if (!isfinite(vnd)) bad |= ST_NONFINITE;
     }
 }
@@ -845,7 +850,7 @@ __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeA
 // at or past nn (row padding) are loaded and stored back unchanged.
 //
 // pre (resident runs): the nodes' own records, loaded while the grid still works
-// on the forces; such a run sums its kinetic energy once, at its end.
+// on the forces.
 template <int W>
 struct NodeRowsMixed {
     double im[W], q[W][4];
@@ -908,7 +913,7 @@ __device__ __forceinline__ void node_forces_mixed(const NodeView& N, const int64
 }
 
 // PRE: rows and forces come in pre and fpre.
-template <int W, bool PATCH, bool PRE = false>
+template <int W, bool PATCH, bool PRE = false, NodeWork WORK = kNodeAll>
 __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double dt_i, const double dt_i_1,
                                                  const double amp, const int64_t n0, double& kin, double& wext,
                                                  int32_t& bad, const NodeRowsMixed<W>* pre = nullptr,
@@ -953,17 +958,19 @@ __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double
                 r = -a;
                 a = 0.f;
             }
-            if (cc) N.rf[c * np + n0 + j] = static_cast<double>(rf);
+            if (WORK != kNodeKinetic && cc) N.rf[c * np + n0 + j] = static_cast<double>(rf);
             const double vod = v_join(v[c], own.lo[c][j]);
             const double vnd = velocity_update_split(vod, a, im, dt_avg, v[c], own.lo[c][j]);
+            if (WORK != kNodeUpdate) kin += 0.5 * (vnd * vnd) / im;
+            if (WORK == kNodeKinetic) continue;
             own.q[j][c] = own.q[j][c] + dt_i * vnd;
             wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
-            if (!PRE) kin += 0.5 * (vnd * vnd) / im;
             if (!isfinite(vnd)) bad |= ST_NONFINITE;
         }
         own.q[j][3] = rec_vxy(v[0], v[1]);
         own.vz[j] = v[2];
     }
+    if (WORK == kNodeKinetic) return;
 #pragma unroll
     for (int j = 0; j < W; ++j) st_rec(N.x + 4 * (n0 + j), own.q[j]);
     st_row<W>(static_cast<float*>(N.v) + n0, own.vz);
@@ -1027,6 +1034,7 @@ constexpr int kRunWarpsMixed = 16;
 template <bool PLASTIC>
 struct RunMixed {
     static constexpr uint32_t kTileBytes = MixedTile::kBytes;
+    static constexpr bool kKinInUpdate = true;
     __device__ static const uint32_t* conn(const unsigned char* tile) {
         return reinterpret_cast<const uint32_t*>(tile);
     }
@@ -1059,23 +1067,38 @@ struct RunMixed {
         __device__ void gather(const ElemArrays& E, const NodeArrays& N, const Material& M, int64_t t0) {
             if (E.slot_major && t0 * W < N.nn) node_forces_mixed<W, false>(node_view(E, N, M, nullptr), t0 * W, f);
         }
-        __device__ void update(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i, double dt_i_1,
-                               double amp, int64_t t0, int64_t stride, double& wext, int32_t& bad) {
-            double kin = 0.0;
+        template <NodeWork WORK>
+        __device__ void pass(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i, double dt_i_1,
+                             double amp, int64_t t0, int64_t stride, double& kin, double& wext, int32_t& bad) {
             if (E.slot_major) {
                 const NodeView nv = node_view(E, N, M, nullptr);
                 if (t0 * W < N.nn)
-                    node_group_mixed<W, false, true>(nv, dt_i, dt_i_1, amp, t0 * W, kin, wext, bad, &rows, f);
+                    node_group_mixed<W, false, true, WORK>(nv, dt_i, dt_i_1, amp, t0 * W, kin, wext, bad, &rows, f);
                 if (W > 1)
                     for (int64_t g = t0 + stride; g * W < N.nn; g += stride) {
-                        node_rows_load<W>(nv, g * W, rows);
-                        node_forces_mixed<W, false>(nv, g * W, f);
-                        node_group_mixed<W, false, true>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad, &rows, f);
+                        NodeRowsMixed<W> r;
+                        float fg[3][W];
+                        node_rows_load<W>(nv, g * W, r);
+                        node_forces_mixed<W, false>(nv, g * W, fg);
+                        node_group_mixed<W, false, true, WORK>(nv, dt_i, dt_i_1, amp, g * W, kin, wext, bad, &r, fg);
                     }
             } else {
                 for (int64_t n = t0; n < N.nn; n += stride)
-                    node_body_mixed<false>(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
+                    node_body_mixed<WORK>(E, N, M, dt_i, dt_i_1, amp, n, kin, wext, bad);
             }
+        }
+        __device__ void update(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i, double dt_i_1,
+                               double amp, int64_t t0, int64_t stride, double& wext, int32_t& bad) {
+            double kin = 0.0;
+            pass<kNodeUpdate>(E, N, M, dt_i, dt_i_1, amp, t0, stride, kin, wext, bad);
+        }
+        // the kinetic energy of the velocities that the update will form
+        __device__ double kinetic_after(const ElemArrays& E, const NodeArrays& N, const Material& M, double dt_i,
+                                        double dt_i_1, double amp, int64_t t0, int64_t stride) {
+            double kin = 0.0, wext = 0.0;
+            int32_t bad = 0;
+            pass<kNodeKinetic>(E, N, M, dt_i, dt_i_1, amp, t0, stride, kin, wext, bad);
+            return kin;
         }
     };
     __device__ static double kinetic(const NodeArrays& N, int64_t n) {

@@ -40,6 +40,7 @@ struct RunShared {
     int32_t go, exact;
     double dt1, dt_i, dt_i_1, amp;
     int32_t cycles;                // cycles begun in this launch
+    int32_t limit;                 // and the most that it may begin
     int32_t last;
     unsigned int bar;              // arrivals that complete the next barrier
     unsigned long long w_dts[kRunMaxWarps], w_len[kRunMaxWarps];
@@ -173,13 +174,17 @@ __device__ __forceinline__ void run_begin(RunShared& sh, int32_t status, int lau
 //   Pol::element(E, N, M, tile, dt1, e, lane, ...)
 //   Pol::Nodes<W>                             a thread's W nodes: load (their rows), gather (their
 //                                             forces), update
-//   Pol::kinetic(N, n)                        kinetic energy of node n
+//   Pol::kinetic(N, n)                        kinetic energy of node n from its stored velocity
+//   Pol::kKinInUpdate                         its velocities have more bits in the update than stored: the
+//                                             kinetic energy is summed ahead of the last cycle's update
+//                                             (Nodes::kinetic_after)
 // Blocks of 32 * nw threads; warp w of the grid owns the tiles w, w + W, ...
 template <class Pol, bool CLUSTER, int W>
 __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays& N, const Material& M, Ctl* ctl,
                                            const Partials& P, RunSync* sync, const RunArgs& a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ RunShared sh;
+    __shared__ double red[5][kRunMaxWarps];  // the warps' sums at the end of the launch
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
     const int nblocks = gridDim.x, block = blockIdx.x;
     const int64_t ntiles = (E.ne + 31) / 32;
@@ -197,6 +202,8 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
             sh.c.done = 0;
         }
         sh.cycles = 0;
+        const long long left = sh.c.cycles_target - sh.c.cycles_done;
+        sh.limit = left < a.launch_cycles ? static_cast<int32_t>(left) : a.launch_cycles;
         sh.bar = 0;
         sh.go = 0;
         sh.exact = 0;
@@ -231,6 +238,7 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
     const int64_t t0 = static_cast<int64_t>(block) * blockDim.x + tid;
     const int64_t stride = static_cast<int64_t>(nblocks) * blockDim.x;
     bool failed = false;
+    bool ends = false;  // the cycle is the launch's last, unless an error makes an earlier one so
     int32_t err = 0;  // warp 0: an error was published
     while (sh.go) {
         const int set = sh.cycles % 3;
@@ -323,6 +331,10 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
         // the thread's own node rows are on their way while the grid finishes
         typename Pol::template Nodes<W> nodes;
         if (CLUSTER) cluster_arrive();
+        // (by every thread while it waits: decided by thread 0 along with dt, it took
+        // 0.25 us of a 4.6 us cycle)
+        if (Pol::kKinInUpdate)
+            ends = !(sh.c.time < sh.c.step_end) | !(sh.c.time < sh.c.pause_time) | (sh.cycles >= sh.limit);
         nodes.load(E, N, M, t0);
         if (CLUSTER) {
             cluster_wait();
@@ -335,6 +347,7 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
             }
             if (__syncthreads_or(failed)) {
                 failed = true;
+                ends = false;
                 break;
             }
         }
@@ -376,6 +389,11 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
         __syncthreads();
         // ---- node phase
         int32_t nbad = 0;
+        if constexpr (Pol::kKinInUpdate)
+            if (ends) {
+                const double k = batch_warp_sum(nodes.kinetic_after(E, N, M, sh.dt_i, sh.dt_i_1, sh.amp, t0, stride));
+                if (lane == 0) red[4][wid] = k;
+            }
         nodes.update(E, N, M, sh.dt_i, sh.dt_i_1, sh.amp, t0, stride, wext, nbad);
         if (nbad) atomicOr(&sync->status, nbad);
         any_bad = __syncthreads_or(nbad);
@@ -405,16 +423,16 @@ __device__ __forceinline__ void run_cycles(const ElemArrays& E, const NodeArrays
     for (int s = 0; s < mine && loaded; ++s)
         Pol::store_tile(E, wtiles + s * Pol::kTileBytes, w0 + s * wstride, lane);
     if (tid == 0 && failed) atomicOr(&sync->status, ST_TIMEOUT);
+    // kinetic energy, unless the last cycle has summed it (a mixed run that an error
+    // ended did not know its last cycle)
     double kin = 0.0;
-    for (int64_t n = t0; n < N.nn; n += stride) kin = kin + Pol::kinetic(N, n);
+    if (!ends)
+        for (int64_t n = t0; n < N.nn; n += stride) kin = kin + Pol::kinetic(N, n);
     double v5[5] = {e_int, e_hg, e_vis, wext, kin};
-    __shared__ double red[5][kRunMaxWarps];
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
-        double s = v5[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) red[i][wid] = s;
+        const double s = batch_warp_sum(v5[i]);
+        if (lane == 0 && !(i == 4 && ends)) red[i][wid] = s;
     }
     __syncthreads();
     if (tid < 5) {
