@@ -38,14 +38,14 @@ void inv3h(const double m[3][3], double r[3][3]) {
 
 void element_constants(int64_t nn, int64_t ne, const uint32_t* conn, const double* x0, double rho,
                        std::vector<double>& bt, std::vector<double>& vol0, std::vector<double>& inv_mass,
-                       std::vector<double>& jinv) {
+                       std::vector<double>* jinv) {
     static const double XI[8][3] = {{-1., -1., -1.}, {1., -1., -1.}, {1., 1., -1.}, {-1., 1., -1.},
                                     {-1., -1., 1.},  {1., -1., 1.},  {1., 1., 1.},  {-1., 1., 1.}};
     double dn[3][8];
     for (int a = 0; a < 8; ++a)
         for (int d = 0; d < 3; ++d) dn[d][a] = 1.0 / 8.0 * XI[a][d];
     bt.assign(static_cast<size_t>(24 * ne), 0.0);
-    jinv.resize(static_cast<size_t>(9 * ne));
+    if (jinv) jinv->resize(static_cast<size_t>(9 * ne));
     vol0.assign(static_cast<size_t>(ne), 0.0);
     std::vector<double> mass(static_cast<size_t>(3 * nn), 0.0);
     for (int64_t e = 0; e < ne; ++e) {
@@ -61,8 +61,9 @@ void element_constants(int64_t nn, int64_t ne, const uint32_t* conn, const doubl
             }
         double ij[3][3];
         inv3h(jac, ij);
-        for (int r = 0; r < 3; ++r)
-            for (int c = 0; c < 3; ++c) jinv[9 * e + 3 * r + c] = ij[r][c] * 0.125;
+        if (jinv)
+            for (int r = 0; r < 3; ++r)
+                for (int c = 0; c < 3; ++c) (*jinv)[9 * e + 3 * r + c] = ij[r][c] * 0.125;
         const double detj = det3h(jac);
         for (int a = 0; a < 8; ++a)
             for (int r = 0; r < 3; ++r)
@@ -112,6 +113,15 @@ void form_device_rows(InstanceHost& h, const uint32_t* conn, const std::vector<i
     h.tiles.assign(static_cast<size_t>(h.ne_pad / 32) * h.const_bytes, 0);
     for (int64_t el = 0; el < h.ne; ++el) {
         const int64_t e = perm.empty() ? el : perm[el];
+        if (!perm.empty() && el + 16 < h.ne) {
+            // in another order every element is elsewhere in memory: ask for it ahead
+            const int64_t a = perm[el + 16];
+            const int n = h.bt9 ? 9 : 24;
+            const double* g = h.bt9 ? &h.jinv[9 * a] : &h.bt[24 * a];
+            for (int i = 0; i < n; i += 8) __builtin_prefetch(g + i);
+            __builtin_prefetch(conn + 8 * a);
+            __builtin_prefetch(&h.vol0[a]);
+        }
         for (int k = 0; k < 8; ++k) tile_entry<uint32_t>(h, el, MixedTile::kConn)[32 * k] = conn[8 * e + k];
         const double v0 = h.vol0[e], cb = std::cbrt(v0);
         if (h.mixed) {
@@ -348,13 +358,14 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
         h.vol0.assign(mesh->vol0, mesh->vol0 + ne);
         inv_mass_dof.assign(mesh->inv_mass, mesh->inv_mass + 3 * nn);
     } else {
-        element_constants(nn, ne, mesh->conn, mesh->x0, mat->rho, h.bt, h.vol0, inv_mass_dof, h.jinv);
+        element_constants(nn, ne, mesh->conn, mesh->x0, mat->rho, h.bt, h.vol0, inv_mass_dof,
+                          mixed ? nullptr : &h.jinv);
         h.bt9 = !mixed;
     }
     if (!mixed && !h.bt9) {
         // a caller's own B0^T: the 9 numbers, where they give its very bits
         std::vector<double> bt, vol0, inv_mass;
-        element_constants(nn, ne, mesh->conn, mesh->x0, mat->rho, bt, vol0, inv_mass, h.jinv);
+        element_constants(nn, ne, mesh->conn, mesh->x0, mat->rho, bt, vol0, inv_mass, &h.jinv);
         h.bt9 = bt_from_jinv(h.bt, h.jinv, ne);
     }
 
