@@ -12,10 +12,11 @@ namespace ensc {
 // division does (P. Markstein, "Computation of elementary functions on the IBM
 // RISC System/6000 processor", 1990: an estimate within one unit in the last
 // place and one correction with a correctly rounded reciprocal suffice; the
-// first correction brings the estimate there).  For normal x, c and quotient;
-// zero stays zero and a non-finite x gives a non-finite quotient.  Five
-// dependent operations without the branch and the call of a general
-// division.
+// first correction brings the estimate there).  For |x| >= 2^-969, below which
+// the remainder x - q c may underflow, with c, rc and the quotient normal; a
+// smaller x is off by a few units in the last place at most, a zero of either
+// sign gives +0, and a non-finite x a non-finite quotient.  Five dependent
+// operations without the branch and the call of a general division.
 __device__ __forceinline__ double div_by(double x, double c, double rc) {
     double q = x * rc;
     q = __fma_rn(__fma_rn(-q, c, x), rc, q);
