@@ -302,7 +302,8 @@ int build_graph(ensc_batch* b, const Tune& t) {
 // with the shortest time per cycle on the batch as loaded.  The candidates
 // differ only in how work is spread over the GPU, not in arithmetic, so the
 // cycles they run are ordinary cycles of the solve (the state is identical
-// whichever wins).  Each candidate runs one warm-up graph launch and one timed
+// whichever wins; FP64 element energies are grouped by the grid and may differ in
+// the last bits).  Each candidate runs one warm-up graph launch and one timed
 // launch; a run too short for the next candidate continues with the best so
 // far, and the next run goes on from there.
 constexpr int kTuneCands = 7;

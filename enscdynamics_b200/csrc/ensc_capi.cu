@@ -8,7 +8,9 @@
 //                 allocation, and the init force pass with dt = 0 that seeds
 //                 the stable time step.
 //   ensc_set_bcs  setCurrentStep's boundary update (:1760-1940, :1911).
-//   ensc_step     run()'s loop body (:86-100), as a CUDA graph of cycles.
+//   ensc_step     run()'s loop body (:86-100): resident runs where the mesh fits on
+//                 chip, else CUDA graphs of cycles and up to half a graph's
+//                 cycles one by one.
 //   ensc_download copies state back in the reference's array layouts.
 #include "ensc_gpu.h"
 #include "ensc_device.cuh"

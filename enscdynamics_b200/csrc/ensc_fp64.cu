@@ -591,13 +591,12 @@ __device__ __forceinline__ void element_body(const ElemArrays& E, const NodeArra
 // Element pass: add_inForce_to_rhs's element loop body
 // (exDyna3D.cpp:556-573): kinematics, Jaumann stress (+ J2 return),
 // hourglass, bulk viscosity, element dt and min edge.  Writes the element's
-// 8x3 nodal forces to fe for the node-centric gather.
-//
-// Register-lean structure: the element's nodes are streamed once for the
-// kinematics (b^T, L, hourglass vectors, HIA) and once more for the forces;
-// per-node rows of b^T and ATAU are recomputed from B0^T (L1-resident) rather
-// than held, so no 8x3 / 4x8 array stays live.  Every value is the same
+// 8x3 nodal forces to fe for the node-centric gather.  Every value is the same
 // expression, in the same order, as the CPU restatement (explicit fma only).
+//
+// One element per thread from global memory: the init force pass, and every pass
+// over caller-owned rows (ensc_step_noalloc).  Cycles over tiles run
+// k_element_fp64_warp.
 template <bool PLASTIC, bool INIT, bool BT9, bool TILED>
 __global__ void __launch_bounds__(kElemThreads, ENSC_ELEM_MINB_FP64) k_element(ElemArrays E, NodeArrays N, Material M, Ctl* ctl,
                                                              Partials P) {
@@ -1141,11 +1140,12 @@ __global__ void __launch_bounds__(32 * kRunWarpsF64, 1)
 // each inside one instance whose arrays, material and control block come from
 // the instance table.  The element pass runs one pipeline per warp over the
 // tile list; the node
-// pass gives each node tile to one warp.  Each tile accumulates its work terms across
-// cycles (one owner per tile and pass) and keeps its latest kinetic energy;
-// k_fold_batch folds them per instance in tile order, so the totals do not
-// depend on scheduling.  Arithmetic per element and node is that of
-// the single-instance kernels, so states are bit-identical to them.
+// pass gives each node tile to one warp.  Work terms add up across cycles in a
+// partial slot per node tile and per run of element tiles (below), one owner per
+// slot and pass; a node tile keeps its latest kinetic energy.  k_fold_batch folds
+// them per instance in tile order.  Arithmetic per element and node is that of
+// the single-instance kernels, so states are bit-identical to them; the element
+// sums are grouped by the grid, so their last bits may change with it.
 // A batch stage: a tile, then its instance descriptor, its element-pass scalars
 // (StageHdr), the TileInfo the filling lane writes, and the ETileSrc record of
 // the tile that uses the stage next (as in the mixed batch pass).  The tile's

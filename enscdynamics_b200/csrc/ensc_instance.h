@@ -74,9 +74,20 @@ int instance_prepare(const ensc_mesh_desc* mesh, const ensc_material* mat, bool 
 // Stored order of the slot assembly, as patch_order; empty: the caller's order.
 // Warps gather node records and store forces best where the elements of a tile
 // follow the node numbering.  Where a slot's node leaves its group of 4 from one
-// element to the next in more than 3 of 8 slots (a block's rows: 2.2), the
+// element to the next in more than 3 of 8 slots (a block's rows: 2.0 to 2.2), the
 // elements are sorted by their nodes; the sorted order is taken where it leaves
-// at most 4/5 of the changes.
+// at most 4/5 of the changes.  B200, us a cycle of 196,608 elements (FP64, mixed)
+// as given and sorted, a block's element order cut into shuffled runs:
+//   changes 8.0   69.8, 56.3   44.4, 30.4        3.0   48.1, 33.2   44.4, 29.8
+//           5.0   53.5, 40.7   44.4, 30.2        2.5   46.5, 31.5   44.5, 30.5
+//           3.5   48.5, 34.1   44.4, 30.3        2.0   44.3, 30.4   44.5, 30.2
+// and with the node numbers shuffled too, within 8, 64 and all of the nodes:
+//   8.0, sorted 5.3   71.0, 56.9   45.9, 31.4
+//   8.0, sorted 7.4   72.2, 59.2   49.6, 34.1
+//   8.0, sorted 8.0   66.4, 53.3   68.9, 57.1
+// So the first line lies where sorting still gives 8 to 12%, and the second, left
+// on the safe side, keeps an order that sorting may lose to (3 to 7% at the
+// last); numberings between 4/5 and 1 stay as given although many would gain.
 std::vector<int32_t> local_order(int64_t nn, int64_t ne, const uint32_t* conn);
 
 // Stored order of the patch assembly: elements sorted by the Morton key of

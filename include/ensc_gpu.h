@@ -167,7 +167,12 @@ int ensc_set_gravity_amplitude(ensc_handle* h, int32_t n_points, const double* t
 
 /* Runs the body of run()'s step loop (exDyna3D.cpp:86-100) -- stable dt,
  * last-step clamp, computeSate -- while time < step_end_time, at most
- * max_cycles cycles.  Blocks until done; report may be NULL. */
+ * max_cycles cycles.  Blocks until done; report may be NULL.
+ * An instance that stays on chip (ensc_kernels_per_cycle 0) is stepped by
+ * launches of up to 4096 cycles whose blocks run all at once, on every SM but
+ * for the smallest meshes (one cluster of at most 16): a launch starts when
+ * other streams' blocks leave it room, and work of other streams that finds no
+ * room beside it waits for its end. */
 int ensc_step(ensc_handle* h, int64_t max_cycles, double step_end_time, ensc_step_report* report);
 
 /* ensc_step that also stops after the cycle in which time first reaches
@@ -249,7 +254,9 @@ int ensc_download_reactions(ensc_handle* h, double* rf);
  * kernel instead of as a graph) with CUDA events around every kernel on the
  * handle's stream, and returns each kernel's summed duration in milliseconds
  * and launch count.  Kernel order: [0] cycle begin, [1] edge prepass,
- * [2] exact-dt begin, [3] element pass, [4] node pass.  For measurement. */
+ * [2] exact-dt begin, [3] element pass, [4] node pass.  For measurement.  An
+ * instance that stays on chip is profiled with these kernels too, although its
+ * step calls do not use them (ensc_kernels_per_cycle 0). */
 int ensc_profile(ensc_handle* h, int64_t max_cycles, double step_end_time, double ms[5], int64_t launches[5]);
 
 /* Device bytes held by the handle. */
@@ -279,7 +286,8 @@ void ensc_destroy(ensc_handle* h);
  * share its precision and stream.  Results of an instance do not depend on
  * the other instances in the batch: its state and energies are those of the
  * same solve with ensc_create (state bit-identical; energy sums may differ in
- * the last bits, being summed per 32-element tile). */
+ * the last bits, being grouped by tiles, in FP64 by the tiles of one instance
+ * that a warp visits). */
 typedef struct ensc_batch ensc_batch;
 
 /* params: precision, device, stream (NULL: own stream) and graph_chunk
