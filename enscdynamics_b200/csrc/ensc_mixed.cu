@@ -834,13 +834,14 @@ __device__ __forceinline__ void node_body_mixed(const ElemArrays& E, const NodeA
         float vn;
         int16_t vl;
         const double vnd = velocity_update_split(vod, a, im, dt_avg, vn, vl);
+        if (WORK != kNodeKinetic) {
+            *pv = vn;
+            *pl = vl;
+            *px += dt_i * vnd;
+            wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
+        }
         if (WORK != kNodeUpdate) kin += 0.5 * (vnd * vnd) / im;
-        if (WORK == kNodeKinetic) continue;
-        *pv = vn;
-        *pl = vl;
-        *px += dt_i * vnd;
-        wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
-        if (!isfinite(vnd)) bad |= ST_NONFINITE;
+        if (WORK != kNodeKinetic && !isfinite(vnd)) bad |= ST_NONFINITE;
     }
 }
 
@@ -961,11 +962,12 @@ __device__ __forceinline__ void node_group_mixed(const NodeView& N, const double
             if (WORK != kNodeKinetic && cc) N.rf[c * np + n0 + j] = static_cast<double>(rf);
             const double vod = v_join(v[c], own.lo[c][j]);
             const double vnd = velocity_update_split(vod, a, im, dt_avg, v[c], own.lo[c][j]);
+            if (WORK != kNodeKinetic) {
+                own.q[j][c] = own.q[j][c] + dt_i * vnd;
+                wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
+            }
             if (WORK != kNodeUpdate) kin += 0.5 * (vnd * vnd) / im;
-            if (WORK == kNodeKinetic) continue;
-            own.q[j][c] = own.q[j][c] + dt_i * vnd;
-            wext += static_cast<double>(g + r) * dt_avg * 0.5 * (vod + vnd);
-            if (!isfinite(vnd)) bad |= ST_NONFINITE;
+            if (WORK != kNodeKinetic && !isfinite(vnd)) bad |= ST_NONFINITE;
         }
         own.q[j][3] = rec_vxy(v[0], v[1]);
         own.vz[j] = v[2];
