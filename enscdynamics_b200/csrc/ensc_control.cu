@@ -171,13 +171,6 @@ __global__ void k_arm(Ctl* ctl, double step_end, long long max_cycles, double pa
     ctl->done = 0;
 }
 
-__global__ void k_reset_init(Ctl* ctl) {
-    ctl->done = 0;
-    ctl->dts_next = kInfBits;
-    ctl->len_min = kInfBits;
-    ctl->status = 0;
-}
-
 // apply_boundary_condition_vec (exDyna3D.cpp:379-490): velocity conditions
 // first, fixed DOFs last.
 // One velocity component of a node: FP64, or the mixed stepper's float with
@@ -442,7 +435,6 @@ void launch_edge_prepass(const ElemArrays& E, const NodeArrays& N, Ctl* ctl, int
 void launch_arm(Ctl* ctl, double step_end, long long max_cycles, cudaStream_t st, double pause) {
     k_arm<<<1, 1, 0, st>>>(ctl, step_end, max_cycles, pause);
 }
-void launch_reset_init(Ctl* ctl, cudaStream_t st) { k_reset_init<<<1, 1, 0, st>>>(ctl); }
 void launch_apply_bc_v(const NodeArrays& N, bool fp32_v, cudaStream_t st) {
     const int g = grid_for(N.nn, 256);
     if (fp32_v) k_apply_bc_v<float><<<g, 256, 0, st>>>(N);

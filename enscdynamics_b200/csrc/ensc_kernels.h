@@ -184,7 +184,6 @@ void launch_edge_prepass(const ElemArrays& E, const NodeArrays& N, Ctl* ctl, int
 // (dt is not clamped to it)
 void launch_arm(Ctl* ctl, double step_end, long long max_cycles, cudaStream_t st, double pause = HUGE_VAL);
 void launch_apply_bc_v(const NodeArrays& N, bool fp32_v, cudaStream_t st);
-void launch_reset_init(Ctl* ctl, cudaStream_t st);
 void launch_kinetic0(const NodeArrays& N, const Partials& P, Ctl* ctl, bool fp32_v, int grid, cudaStream_t st);
 // Layout conversion between interleaved caller arrays and the device layout:
 // node fields, reactions, and the element rows at `rows` of E.  `at` (may be null):
